@@ -485,12 +485,14 @@ __global__ void __launch_bounds__(256) ep_layout_hist_kernel(LayoutParams p) {
     int* hist = smem_i32;  // [E]
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int t = blockIdx.x * nthr + tid;
-    int e[kMaxTopk];
-    load_token_choices(p.topk_idx, t, p.T, p.K, p.E, e);
+    // The first kernel of a call may be chained to the kernel that WRITES the index
+    // matrix (the elastic calls' route kernel): nothing is read before the wait.
     for (int i = tid; i < p.E; i += nthr) hist[i] = 0;
-    __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    int e[kMaxTopk];
+    load_token_choices(p.topk_idx, t, p.T, p.K, p.E, e);
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kMaxTopk; ++k)
         if (e[k] >= 0) atomicAdd(&hist[e[k]], 1);

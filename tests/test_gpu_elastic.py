@@ -267,3 +267,47 @@ def test_buffer_of_an_odd_size_keeps_the_records_aligned():
     outs = _dispatch(bufs, xs, idxs, ws, E, M, 1, False, keep)
     _check_dispatch(outs, eo.elastic_dispatch(xs, idxs, ws, E, M), False, True, K)
     assert all(b.runtime.status() == 0 for b in bufs)
+
+
+@pytest.mark.parametrize("T,H,E,K,expand", [(1, 128, 4, 1, False), (300, 256, 8, 4, False), (1000, 128, 16, 2, False),
+                                            (1024, 256, 8, 4, True), (2001, 128, 32, 8, False)])
+def test_routing_changes_from_call_to_call(T, H, E, K, expand):
+    """One buffer, back-to-back calls without a wait between them, each with a
+    routing of its own (a different set of padding tokens every time): no call may
+    see anything of the routing of an earlier one."""
+    bufs = _group(1, T, H, K, False)
+    calls = []
+    keep = []
+    ins = []
+    for c in range(5):
+        x, idx, w = make_rank_inputs(70 + c, 0, T, H, E, K, "uniform")
+        idx[torch.randperm(T, generator=torch.Generator().manual_seed(c))[:T * c // 6]] = -1
+        ins.append((x, idx, w))
+    dev = [tuple(t.cuda() for t in i) for i in ins]
+    for x, idx, w in dev:  # queued one behind the other
+        calls.append(_enqueue_single(bufs[0], x, idx, w, E, T, expand))
+    torch.cuda.synchronize()
+    for (x, idx, w), d in zip(ins, calls):
+        want = eo.elastic_dispatch([x], [idx], [w], E, T, 1, expand)
+        _check_dispatch([d], want, expand, True, K)
+    assert bufs[0].runtime.status() == 0
+
+
+def _enqueue_single(buf, x, idx, w, E, M, expand):
+    """One single-rank elastic dispatch on the current stream, not waited for."""
+    T, H = x.shape
+    K = idx.shape[1]
+    cap = M * K if expand else M
+    i32 = lambda *s: torch.full(s, -7, dtype=torch.int32, device="cuda")  # noqa: E731
+    d = dict(x=x, idx=idx, w=w, active=torch.ones(1, dtype=torch.int32, device="cuda"), psum_rank=i32(1),
+             psum_expert=i32(E + 1), slot=i32(T, K), md=i32(M, K + 2),
+             recv_x=torch.zeros((cap, H), dtype=torch.bfloat16, device="cuda"),
+             recv_idx=torch.full((M, K), -7, dtype=torch.int64, device="cuda"),
+             recv_w=torch.full((cap,) if expand else (M, K), -7.0, device="cuda"),
+             copied=torch.full((T, K), -7, dtype=torch.int64, device="cuda"))
+    buf.runtime.elastic_dispatch(
+        x.data_ptr(), 2, 0, T, H, 0, 0, 0, idx.data_ptr(), K, w.data_ptr(), d["active"].data_ptr(), E, M, 1, expand,
+        False, torch.cuda.current_stream().cuda_stream, False, d["psum_rank"].data_ptr(), d["psum_expert"].data_ptr(),
+        d["slot"].data_ptr(), d["recv_x"].data_ptr(), 0, d["recv_idx"].data_ptr(), d["recv_w"].data_ptr(),
+        d["md"].data_ptr(), 200_000, d["copied"].data_ptr())
+    return d
