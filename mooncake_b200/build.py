@@ -1,4 +1,5 @@
-"""Builds libmcep.so (the CUDA kernels and the C ABI) in-tree with nvcc, for sm_100a only."""
+"""Builds, in-tree, libmcep.so (the CUDA kernels and the C ABI, nvcc, for sm_100a only) and
+_mcep_torch.so (the native part of the Python binding, g++ against torch's headers)."""
 from __future__ import annotations
 
 import fcntl
@@ -78,5 +79,67 @@ def _build_locked(force: bool, verbose: bool) -> str:
     return LIB
 
 
+# ---- the torch binding ------------------------------------------------------------
+BINDING = os.path.join(HERE, "_mcep_torch.so")
+BINDING_STAMP = BINDING + ".sources"
+BINDING_SOURCES = ["ep_py_torch.cpp", os.path.join("..", "..", "include", "mcep.h")]
+
+
+def _binding_digest() -> str:
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {sys.version_info[:2]}".encode())
+    for f in BINDING_SOURCES:
+        path = os.path.join(CSRC, f)
+        if os.path.exists(path):
+            with open(path, "rb") as fh:
+                h.update(fh.read())
+    return h.hexdigest()
+
+
+def _binding_stale() -> bool:
+    if not os.path.exists(BINDING):
+        return True
+    try:
+        with open(BINDING_STAMP) as fh:
+            return fh.read().strip() != _binding_digest()
+    except OSError:
+        return True
+
+
+def build_binding(force: bool = False) -> str:
+    if not force and not _binding_stale():
+        return BINDING
+    with open(BINDING + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if not force and not _binding_stale():
+                return BINDING
+            cxx = shutil.which("g++")
+            if cxx is None:
+                if os.path.exists(BINDING) and not force:
+                    return BINDING  # a prebuilt binding and no compiler: use what is there
+                raise RuntimeError("mooncake_b200: g++ not found; cannot build _mcep_torch.so")
+            import sysconfig
+            import torch
+            root = os.path.dirname(torch.__file__)
+            cuda = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
+            include = [os.path.join(HERE, "..", "include"), sysconfig.get_paths()["include"],
+                       os.path.join(root, "include"),
+                       os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                       os.path.join(cuda, "include")]
+            cmd = [cxx, "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden",
+                   f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            cmd += [a for d in include for a in ("-isystem", d)]
+            cmd += [os.path.join(CSRC, BINDING_SOURCES[0]), "-o", BINDING, "-L", os.path.join(root, "lib"),
+                    "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+            subprocess.run(cmd, check=True)
+            with open(BINDING_STAMP, "w") as fh:
+                fh.write(_binding_digest())
+            return BINDING
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_binding(force="--force" in sys.argv))

@@ -1,0 +1,572 @@
+// The Python side of a call, in native code: a CPython extension over the C ABI
+// (include/mcep.h) that checks the tensors, allocates the outputs and makes the
+// call in one step. The package's `Buffer` / `ElasticBuffer` wrappers and
+// `ep.Buffer` are thin classes over it.
+//
+// Why it exists: a decode-sized layer keeps the GPU busy for 10 - 15 us, while
+// the same steps written in Python (about twenty assertions, five torch.empty,
+// eighteen ctypes conversions per call) took 50 us per layer of host time, so
+// the host bounded every small call (DeepSeek-V3-shaped decode layer, 128
+// tokens: 50.2 us per layer, of which the device was busy for 14.5).
+//
+// The module holds no state of its own; it calls the library through the
+// addresses `bind` was given, so it always drives the same libmcep.so as the
+// ctypes declarations of ep.py.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstring>
+#include <initializer_list>
+#include <string>
+
+#include "mcep.h"
+
+namespace {
+
+// ---- the library ---------------------------------------------------------------------
+struct Library {
+    decltype(&mcep_last_error) last_error;
+    decltype(&mcep_dispatch) dispatch;
+    decltype(&mcep_combine) combine;
+    decltype(&mcep_elastic_dispatch) elastic_dispatch;
+    decltype(&mcep_elastic_combine) elastic_combine;
+    decltype(&mcep_buffer_next_recv_x) next_recv_x;
+    decltype(&mcep_event_create) event_create;
+    decltype(&mcep_event_current_stream_wait) event_wait;
+    decltype(&mcep_event_synchronize) event_synchronize;
+    decltype(&mcep_event_free) event_free;
+    decltype(&mcep_hook_run) hook_run;
+    decltype(&mcep_hook_free) hook_free;
+} lib;
+
+const char* const kSymbols[] = {"mcep_last_error", "mcep_dispatch", "mcep_combine", "mcep_elastic_dispatch",
+                                "mcep_elastic_combine", "mcep_buffer_next_recv_x", "mcep_event_create",
+                                "mcep_event_current_stream_wait", "mcep_event_synchronize", "mcep_event_free",
+                                "mcep_hook_run", "mcep_hook_free"};
+constexpr size_t kNumSymbols = sizeof(kSymbols) / sizeof(kSymbols[0]);
+static_assert(sizeof(Library) == kNumSymbols * sizeof(void*), "one address per name");
+
+PyObject* fail() {
+    PyErr_SetString(PyExc_RuntimeError, lib.last_error());
+    return nullptr;
+}
+
+// bind({name: address}): where the entry points of the loaded libmcep.so are.
+PyObject* py_bind(PyObject*, PyObject* table) {
+    void** slots = reinterpret_cast<void**>(&lib);
+    for (size_t i = 0; i < kNumSymbols; ++i) {
+        PyObject* v = PyDict_GetItemString(table, kSymbols[i]);
+        if (v == nullptr) return PyErr_Format(PyExc_KeyError, "%s", kSymbols[i]);
+        slots[i] = PyLong_AsVoidPtr(v);
+        if (PyErr_Occurred()) return nullptr;
+    }
+    Py_RETURN_NONE;
+}
+
+// ---- arguments -----------------------------------------------------------------------
+// Positional and keyword arguments of a call into `out[0..n)` (borrowed; null = not given).
+bool collect(const char* const* names, int n, int required, PyObject* const* args, Py_ssize_t nargs,
+             PyObject* kwnames, PyObject** out, const char* fname) {
+    if (nargs > n) {
+        PyErr_Format(PyExc_TypeError, "%s() takes %d arguments (%zd given)", fname, n, nargs);
+        return false;
+    }
+    for (Py_ssize_t i = 0; i < n; ++i) out[i] = i < nargs ? args[i] : nullptr;
+    const Py_ssize_t nk = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+    for (Py_ssize_t j = 0; j < nk; ++j) {
+        PyObject* key = PyTuple_GET_ITEM(kwnames, j);
+        int at = -1;
+        for (int i = 0; i < n && at < 0; ++i)
+            if (PyUnicode_CompareWithASCIIString(key, names[i]) == 0) at = i;
+        if (at < 0 || out[at] != nullptr) {
+            PyErr_Format(PyExc_TypeError, "%s() got an unexpected or repeated keyword argument '%U'", fname, key);
+            return false;
+        }
+        out[at] = args[nargs + j];
+    }
+    for (int i = 0; i < required; ++i)
+        if (out[i] == nullptr) {
+            PyErr_Format(PyExc_TypeError, "%s() missing required argument: '%s'", fname, names[i]);
+            return false;
+        }
+    return true;
+}
+
+// Reads integers, addresses and truth values; the first failure sticks.
+struct Reader {
+    PyObject** v;
+    bool ok = true;
+    long long num(int i, long long dflt = 0) {
+        if (v[i] == nullptr || v[i] == Py_None) return dflt;
+        const long long r = PyLong_AsLongLong(v[i]);
+        if (r == -1 && PyErr_Occurred()) ok = false;
+        return r;
+    }
+    int i32(int i, int dflt = 0) { return (int)num(i, dflt); }
+    int flag(int i) {
+        if (v[i] == nullptr) return 0;
+        const int r = PyObject_IsTrue(v[i]);
+        if (r < 0) ok = false;
+        return r > 0;
+    }
+    void* ptr(int i) {
+        if (v[i] == nullptr || v[i] == Py_None) return nullptr;
+        void* r = PyLong_AsVoidPtr(v[i]);
+        if (r == nullptr && PyErr_Occurred()) ok = false;
+        return r;
+    }
+};
+
+// ---- events and hooks ------------------------------------------------------------------
+struct EventObject {
+    PyObject_HEAD
+    mcep_event* ev;
+};
+PyTypeObject* event_type = nullptr;
+
+PyObject* wrap_event(mcep_event* ev) {
+    if (ev == nullptr) Py_RETURN_NONE;
+    EventObject* o = PyObject_New(EventObject, event_type);
+    if (o == nullptr) {
+        lib.event_free(ev);
+        return nullptr;
+    }
+    o->ev = ev;
+    return reinterpret_cast<PyObject*>(o);
+}
+
+PyObject* event_new(PyTypeObject* type, PyObject* args, PyObject* kw) {
+    static const char* names[] = {"stream_ptr", nullptr};
+    unsigned long long stream = 0;
+    if (!PyArg_ParseTupleAndKeywords(args, kw, "|K", const_cast<char**>(names), &stream)) return nullptr;
+    mcep_event* ev = nullptr;
+    if (lib.event_create(stream, &ev)) return fail();
+    EventObject* o = reinterpret_cast<EventObject*>(type->tp_alloc(type, 0));
+    if (o == nullptr) {
+        lib.event_free(ev);
+        return nullptr;
+    }
+    o->ev = ev;
+    return reinterpret_cast<PyObject*>(o);
+}
+
+void event_dealloc(PyObject* self) {
+    PyTypeObject* type = Py_TYPE(self);
+    lib.event_free(reinterpret_cast<EventObject*>(self)->ev);
+    type->tp_free(self);
+    Py_DECREF(type);
+}
+
+PyObject* event_stream_wait(PyObject* self, PyObject* stream) {
+    const unsigned long long s = PyLong_AsUnsignedLongLong(stream);
+    if (PyErr_Occurred()) return nullptr;
+    if (lib.event_wait(reinterpret_cast<EventObject*>(self)->ev, s)) return fail();
+    Py_RETURN_NONE;
+}
+
+PyObject* event_sync(PyObject* self, PyObject*) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = lib.event_synchronize(reinterpret_cast<EventObject*>(self)->ev);
+    Py_END_ALLOW_THREADS if (rc) return fail();
+    Py_RETURN_NONE;
+}
+
+PyMethodDef event_methods[] = {
+    {"current_stream_wait", event_stream_wait, METH_O, "Make the stream (a cudaStream_t as an integer) wait."},
+    {"synchronize", event_sync, METH_NOARGS, "Wait for the event on the host."},
+    {nullptr, nullptr, 0, nullptr}};
+PyType_Slot event_slots[] = {
+    {Py_tp_doc, const_cast<char*>("mooncake-ep/include/mooncake_ep_event.h:9-44: a CUDA event recorded on\n"
+                                  "`stream_ptr` at construction.")},
+    {Py_tp_new, reinterpret_cast<void*>(event_new)},
+    {Py_tp_dealloc, reinterpret_cast<void*>(event_dealloc)},
+    {Py_tp_methods, event_methods},
+    {0, nullptr}};
+PyType_Spec event_spec = {"mooncake_b200._mcep_torch.EventHandle", sizeof(EventObject), 0,
+                          Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE, event_slots};
+
+struct HookObject {
+    PyObject_HEAD
+    mcep_hook* hook;
+};
+PyTypeObject* hook_type = nullptr;
+
+PyObject* wrap_hook(mcep_hook* hook) {
+    if (hook == nullptr) Py_RETURN_NONE;
+    HookObject* o = PyObject_New(HookObject, hook_type);
+    if (o == nullptr) {
+        lib.hook_free(hook);
+        return nullptr;
+    }
+    o->hook = hook;
+    return reinterpret_cast<PyObject*>(o);
+}
+
+void hook_dealloc(PyObject* self) {
+    PyTypeObject* type = Py_TYPE(self);
+    lib.hook_free(reinterpret_cast<HookObject*>(self)->hook);
+    type->tp_free(self);
+    Py_DECREF(type);
+}
+
+PyObject* hook_call(PyObject* self, PyObject*, PyObject*) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = lib.hook_run(reinterpret_cast<HookObject*>(self)->hook);
+    Py_END_ALLOW_THREADS if (rc) return fail();
+    Py_RETURN_NONE;
+}
+
+PyType_Slot hook_slots[] = {
+    {Py_tp_doc, const_cast<char*>("The receive-phase callback (the `std::function<void()>` of the reference).")},
+    {Py_tp_dealloc, reinterpret_cast<void*>(hook_dealloc)},
+    {Py_tp_call, reinterpret_cast<void*>(hook_call)},
+    {0, nullptr}};
+PyType_Spec hook_spec = {"mooncake_b200._mcep_torch.Hook", sizeof(HookObject), 0,
+                         Py_TPFLAGS_DEFAULT | Py_TPFLAGS_DISALLOW_INSTANTIATION, hook_slots};
+
+// ---- tensors -------------------------------------------------------------------------
+const at::Tensor* tensor_of(PyObject* o) { return o && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+bool matrix(const at::Tensor* t, at::ScalarType type) {
+    return t && t->is_cuda() && t->dim() == 2 && t->scalar_type() == type && t->is_contiguous();
+}
+bool usable_mask(const at::Tensor* t, int64_t ranks) {
+    return t && t->is_cuda() && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
+}
+
+at::Tensor empty(at::IntArrayRef size, at::ScalarType type, at::Device dev) {
+    return at::detail::empty_cuda(size, type, dev, std::nullopt);
+}
+
+// Several small output tensors cut out of one allocation: the caching allocator
+// is asked once (an allocation costs about as much as everything else that has
+// to be done for a small tensor).
+class Arena {
+public:
+    explicit Arena(at::Device dev) : dev_(dev) {}
+    int64_t reserve(int64_t bytes) {
+        const int64_t at = size_;
+        size_ += (bytes + 255) / 256 * 256;
+        return at;
+    }
+    void allocate() {
+        base_ = empty({size_ ? size_ : 1}, at::kByte, dev_);
+        data_ = static_cast<char*>(base_.data_ptr());
+    }
+    char* at(int64_t offset) const { return data_ + offset; }
+    at::Tensor view(int64_t offset, at::ScalarType type, at::IntArrayRef size) const {
+        const auto meta = c10::scalarTypeToTypeMeta(type);
+        at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base_.storage()), base_.key_set(), meta);
+        t.unsafeGetTensorImpl()->set_storage_offset(offset / (int64_t)meta.itemsize());
+        t.unsafeGetTensorImpl()->set_sizes_contiguous(size);
+        return t;
+    }
+
+private:
+    at::Device dev_;
+    int64_t size_ = 0;
+    at::Tensor base_;
+    char* data_ = nullptr;
+};
+
+PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
+
+// A new tuple that takes over the references of `items`; null if any is null.
+PyObject* pack(std::initializer_list<PyObject*> items) {
+    bool ok = true;
+    for (PyObject* o : items) ok = ok && o != nullptr;
+    PyObject* t = ok ? PyTuple_New((Py_ssize_t)items.size()) : nullptr;
+    if (t == nullptr) {
+        for (PyObject* o : items) Py_XDECREF(o);
+        return nullptr;
+    }
+    Py_ssize_t i = 0;
+    for (PyObject* o : items) PyTuple_SET_ITEM(t, i++, o);
+    return t;
+}
+
+PyObject* new_ref(PyObject* o) {
+    Py_INCREF(o);
+    return o;
+}
+
+uint64_t current_stream() { return reinterpret_cast<uint64_t>(c10::cuda::getCurrentCUDAStream().stream()); }
+
+PyObject* py_current_stream(PyObject*, PyObject*) { return PyLong_FromUnsignedLongLong(current_stream()); }
+
+// ---- the runtime object -----------------------------------------------------------------
+struct RuntimeObject {
+    PyObject_HEAD
+    mcep_buffer* buf;
+    int num_ranks;
+};
+
+RuntimeObject* self_of(PyObject* o) { return reinterpret_cast<RuntimeObject*>(o); }
+
+bool alive(RuntimeObject* s) {
+    if (s->buf != nullptr) return true;
+    PyErr_SetString(PyExc_RuntimeError, "the buffer has been destroyed");
+    return false;
+}
+
+PyObject* runtime_adopt(PyObject* self, PyObject* args) {
+    PyObject* h;
+    int ranks;
+    if (!PyArg_ParseTuple(args, "Oi", &h, &ranks)) return nullptr;
+    self_of(self)->buf = h == Py_None ? nullptr : static_cast<mcep_buffer*>(PyLong_AsVoidPtr(h));
+    self_of(self)->num_ranks = ranks;
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+}
+
+int call_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** ev, mcep_hook** hk) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = lib.dispatch(b, a, ev, hk);
+    Py_END_ALLOW_THREADS return rc;
+}
+int call_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** ev, mcep_hook** hk) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = lib.combine(b, a, ev, hk);
+    Py_END_ALLOW_THREADS return rc;
+}
+
+const char* const kDispatchNames[] = {
+    "x_ptr", "topk_idx_ptr", "active_ranks_ptr", "num_tokens", "hidden", "num_topk",
+    "num_max_dispatch_tokens_per_rank", "num_experts", "timeout_us", "use_fp8", "packed_recv_x_ptr",
+    "packed_recv_x_scales_ptr", "packed_recv_count_ptr", "packed_recv_src_info_ptr",
+    "packed_recv_layout_range_ptr", "async_finish", "return_recv_hook", "compute_stream_ptr"};
+
+PyObject* runtime_dispatch(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+    PyObject* v[18];
+    if (!collect(kDispatchNames, 18, 18, args, nargs, kwnames, v, "dispatch") || !alive(self_of(self))) return nullptr;
+    Reader r{v};
+    mcep_dispatch_args a = {};
+    a.x = r.ptr(0), a.topk_idx = static_cast<int64_t*>(r.ptr(1)), a.active_ranks = static_cast<int32_t*>(r.ptr(2));
+    a.num_tokens = r.i32(3), a.hidden = r.i32(4), a.num_topk = r.i32(5);
+    a.num_max_dispatch_tokens_per_rank = r.i32(6), a.num_experts = r.i32(7), a.timeout_us = r.num(8);
+    a.use_fp8 = r.flag(9), a.packed_recv_x = r.ptr(10), a.packed_recv_x_scales = static_cast<float*>(r.ptr(11));
+    a.packed_recv_count = static_cast<int32_t*>(r.ptr(12)), a.packed_recv_src_info = static_cast<int32_t*>(r.ptr(13));
+    a.packed_recv_layout_range = static_cast<int64_t*>(r.ptr(14));
+    a.async_finish = r.flag(15), a.return_recv_hook = r.flag(16);
+    a.compute_stream = reinterpret_cast<uint64_t>(r.ptr(17));
+    if (!r.ok) return nullptr;
+    mcep_event* ev = nullptr;
+    mcep_hook* hk = nullptr;
+    if (call_dispatch(self_of(self)->buf, &a, &ev, &hk)) return fail();
+    return pack({wrap_event(ev), wrap_hook(hk)});
+}
+
+const char* const kCombineNames[] = {
+    "x_ptr", "topk_idx_ptr", "topk_weights_ptr", "src_info_ptr", "layout_range_ptr", "active_ranks_ptr",
+    "num_local_experts", "num_combined_tokens", "hidden", "num_topk", "num_max_dispatch_tokens_per_rank",
+    "num_experts", "timeout_us", "zero_copy", "combined_x_ptr", "async_finish", "return_recv_hook",
+    "compute_stream_ptr"};
+
+PyObject* runtime_combine(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+    PyObject* v[18];
+    if (!collect(kCombineNames, 18, 18, args, nargs, kwnames, v, "combine") || !alive(self_of(self))) return nullptr;
+    Reader r{v};
+    mcep_combine_args a = {};
+    a.x = r.ptr(0), a.topk_idx = static_cast<int64_t*>(r.ptr(1)), a.topk_weights = static_cast<float*>(r.ptr(2));
+    a.src_info = static_cast<int32_t*>(r.ptr(3)), a.layout_range = static_cast<int64_t*>(r.ptr(4));
+    a.active_ranks = static_cast<int32_t*>(r.ptr(5)), a.num_local_experts = r.i32(6);
+    a.num_combined_tokens = r.i32(7), a.hidden = r.i32(8), a.num_topk = r.i32(9);
+    a.num_max_dispatch_tokens_per_rank = r.i32(10), a.num_experts = r.i32(11), a.timeout_us = r.num(12);
+    a.zero_copy = r.flag(13), a.combined_x = r.ptr(14), a.async_finish = r.flag(15), a.return_recv_hook = r.flag(16);
+    a.compute_stream = reinterpret_cast<uint64_t>(r.ptr(17));
+    if (!r.ok) return nullptr;
+    mcep_event* ev = nullptr;
+    mcep_hook* hk = nullptr;
+    if (call_combine(self_of(self)->buf, &a, &ev, &hk)) return fail();
+    return pack({wrap_event(ev), wrap_hook(hk)});
+}
+
+// next_recv_x(M, hidden, num_experts, use_fp8) -> (pointer, bytes)
+PyObject* runtime_next_recv_x(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+    static const char* const names[] = {"num_max_dispatch_tokens_per_rank", "hidden", "num_experts", "use_fp8"};
+    PyObject* v[4];
+    if (!collect(names, 4, 4, args, nargs, kwnames, v, "next_recv_x") || !alive(self_of(self))) return nullptr;
+    Reader r{v};
+    const int M = r.i32(0), H = r.i32(1), E = r.i32(2), fp8 = r.flag(3);
+    if (!r.ok) return nullptr;
+    void* p = nullptr;
+    size_t n = 0;
+    if (lib.next_recv_x(self_of(self)->buf, M, H, E, fp8, &p, &n)) return fail();
+    return pack({PyLong_FromVoidPtr(p), PyLong_FromSize_t(n)});
+}
+
+// dispatch_tensors(x, topk_idx, active_ranks, M, E, timeout_us, use_fp8, async_finish,
+//                  return_recv_hook, in_place or None)
+// `in_place`(pointer, bytes, L, R*M, H, use_fp8, x) makes the tensor over the symmetric memory in
+// which a group's rows land; without it, or for a single rank, the rows get a tensor of their own.
+//   -> (recv_x, scales or None, recv_count, src_info, layout_range, event, hook)
+// or None when an argument is not what the call takes (the wrapper then says which).
+PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    RuntimeObject* s = self_of(self);
+    if (nargs != 10) return PyErr_Format(PyExc_TypeError, "dispatch_tensors() takes 10 arguments");
+    if (!alive(s)) return nullptr;
+    Reader r{const_cast<PyObject**>(args)};
+    const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *active = tensor_of(args[2]);
+    const int64_t M = r.num(3), E = r.num(4), timeout = r.num(5), R = s->num_ranks;
+    const int fp8 = r.flag(6), async = r.flag(7), hooked = r.flag(8);
+    if (!r.ok) return nullptr;
+    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !usable_mask(active, R)) Py_RETURN_NONE;
+    const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), RM = R * M;
+    if (idx->size(0) != T || T > M || H % 128 != 0 || E <= 0 || E % R != 0 || (fp8 && RM % 4 != 0)) Py_RETURN_NONE;
+    const int64_t L = E / R;
+    const at::Device dev = x->device();
+    at::Tensor recv_x;
+    PyObject* rows = nullptr;
+    if (args[9] != Py_None) {
+        void* p = nullptr;
+        size_t n = 0;
+        if (lib.next_recv_x(s->buf, (int)M, (int)H, (int)E, fp8, &p, &n)) return fail();
+        if (p != nullptr) {
+            rows = PyObject_CallFunction(args[9], "KKLLLOO", (unsigned long long)reinterpret_cast<uintptr_t>(p),
+                                         (unsigned long long)n, (long long)L, (long long)RM, (long long)H,
+                                         fp8 ? Py_True : Py_False, args[0]);
+            if (rows == nullptr) return nullptr;
+            recv_x = *tensor_of(rows);
+        }
+    }
+    if (rows == nullptr) recv_x = empty({L, RM, H}, fp8 ? at::kFloat8_e4m3fn : at::kBFloat16, dev);
+    at::Tensor scales;
+    if (fp8) {  // [L, H/128, R*M] storage seen as [L, R*M, H/128]
+        scales = empty({L, H / 128, RM}, at::kFloat, dev);
+        const int64_t sizes[3] = {L, RM, H / 128}, strides[3] = {H / 128 * RM, 1, RM};
+        scales.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef(sizes), at::IntArrayRef(strides));
+    }
+    Arena small(dev);
+    const int64_t o_count = small.reserve(L * 4), o_range = small.reserve(L * R * 8), o_src = small.reserve(L * RM * 4);
+    small.allocate();
+    mcep_dispatch_args a = {};
+    a.x = x->const_data_ptr(), a.topk_idx = static_cast<const int64_t*>(idx->const_data_ptr());
+    a.active_ranks = static_cast<int32_t*>(active->data_ptr());
+    a.num_tokens = (int)T, a.hidden = (int)H, a.num_topk = (int)K;
+    a.num_max_dispatch_tokens_per_rank = (int)M, a.num_experts = (int)E, a.use_fp8 = fp8, a.timeout_us = timeout;
+    a.packed_recv_x = recv_x.data_ptr();
+    a.packed_recv_x_scales = fp8 ? static_cast<float*>(scales.data_ptr()) : nullptr;
+    a.packed_recv_count = reinterpret_cast<int32_t*>(small.at(o_count));
+    a.packed_recv_layout_range = reinterpret_cast<int64_t*>(small.at(o_range));
+    a.packed_recv_src_info = reinterpret_cast<int32_t*>(small.at(o_src));
+    a.async_finish = async, a.return_recv_hook = hooked, a.compute_stream = current_stream();
+    mcep_event* ev = nullptr;
+    mcep_hook* hk = nullptr;
+    if (call_dispatch(s->buf, &a, &ev, &hk)) {
+        Py_XDECREF(rows);
+        return fail();
+    }
+    return pack({rows ? rows : wrap(std::move(recv_x)), fp8 ? wrap(std::move(scales)) : new_ref(Py_None),
+                 wrap(small.view(o_count, at::kInt, {L})), wrap(small.view(o_src, at::kInt, {L, RM})),
+                 wrap(small.view(o_range, at::kLong, {L, R})), wrap_event(ev), wrap_hook(hk)});
+    END_HANDLE_TH_ERRORS
+}
+
+// combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info, layout_range,
+//                 M, hidden, E, zero_copy, async_finish, return_recv_hook, out or None)
+//   -> (combined_x, event, hook), or None (as above)
+PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    RuntimeObject* s = self_of(self);
+    if (nargs != 14) return PyErr_Format(PyExc_TypeError, "combine_tensors() takes 14 arguments");
+    if (!alive(s)) return nullptr;
+    Reader r{const_cast<PyObject**>(args)};
+    const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *w = tensor_of(args[2]);
+    const at::Tensor *active = tensor_of(args[3]), *src = tensor_of(args[5]), *range = tensor_of(args[6]);
+    const int64_t timeout = r.num(4), M = r.num(7), H = r.num(8), E = r.num(9), R = s->num_ranks;
+    const int zero_copy = r.flag(10), async = r.flag(11), hooked = r.flag(12);
+    if (!r.ok) return nullptr;
+    if (!(x && x->is_cuda() && x->dim() == 3 && x->scalar_type() == at::kBFloat16 && x->is_contiguous()) ||
+        !matrix(idx, at::kLong) || !matrix(w, at::kFloat) || !usable_mask(active, R) || !matrix(src, at::kInt) ||
+        !matrix(range, at::kLong) || E <= 0 || E % R != 0)
+        Py_RETURN_NONE;
+    const int64_t L = E / R, T = w->size(0), K = w->size(1);
+    if (x->size(0) != L || x->size(1) != R * M || x->size(2) != H || H % 128 != 0 || idx->size(0) != T ||
+        idx->size(1) != K || T > M || src->size(0) != L || range->size(0) != L || range->size(1) != R)
+        Py_RETURN_NONE;
+    const at::Tensor* given = tensor_of(args[13]);
+    if (args[13] != Py_None && (!matrix(given, at::kBFloat16) || given->size(0) != T || given->size(1) != H))
+        Py_RETURN_NONE;
+    at::Tensor out = given ? *given : empty({T, H}, at::kBFloat16, x->device());
+    mcep_combine_args a = {};
+    a.x = x->const_data_ptr(), a.topk_idx = static_cast<const int64_t*>(idx->const_data_ptr());
+    a.topk_weights = static_cast<const float*>(w->const_data_ptr());
+    a.src_info = static_cast<const int32_t*>(src->const_data_ptr());
+    a.layout_range = static_cast<const int64_t*>(range->const_data_ptr());
+    a.active_ranks = static_cast<int32_t*>(active->data_ptr());
+    a.num_local_experts = (int)L, a.num_combined_tokens = (int)T, a.hidden = (int)H, a.num_topk = (int)K;
+    a.num_max_dispatch_tokens_per_rank = (int)M, a.num_experts = (int)E, a.timeout_us = timeout;
+    a.zero_copy = zero_copy, a.combined_x = out.data_ptr(), a.async_finish = async, a.return_recv_hook = hooked;
+    a.compute_stream = current_stream();
+    mcep_event* ev = nullptr;
+    mcep_hook* hk = nullptr;
+    if (call_combine(s->buf, &a, &ev, &hk)) return fail();
+    return pack({given ? new_ref(args[13]) : wrap(std::move(out)), wrap_event(ev), wrap_hook(hk)});
+    END_HANDLE_TH_ERRORS
+}
+
+#define MCEP_FAST(fn) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn))
+
+PyMethodDef runtime_methods[] = {
+    {"_adopt", runtime_adopt, METH_VARARGS, "_adopt(handle or None, num_ranks): the mcep_buffer the calls go to."},
+    {"dispatch", MCEP_FAST(runtime_dispatch), METH_FASTCALL | METH_KEYWORDS,
+     "dispatch($self, x_ptr, topk_idx_ptr, active_ranks_ptr, num_tokens, hidden, num_topk, "
+     "num_max_dispatch_tokens_per_rank, num_experts, timeout_us, use_fp8, packed_recv_x_ptr, "
+     "packed_recv_x_scales_ptr, packed_recv_count_ptr, packed_recv_src_info_ptr, packed_recv_layout_range_ptr, "
+     "async_finish, return_recv_hook, compute_stream_ptr)\n--\n\n"
+     "mooncake-ep/include/mooncake_ep_buffer.h:116-124. Returns (event or None, hook or None)."},
+    {"combine", MCEP_FAST(runtime_combine), METH_FASTCALL | METH_KEYWORDS,
+     "combine($self, x_ptr, topk_idx_ptr, topk_weights_ptr, src_info_ptr, layout_range_ptr, active_ranks_ptr, "
+     "num_local_experts, num_combined_tokens, hidden, num_topk, num_max_dispatch_tokens_per_rank, num_experts, "
+     "timeout_us, zero_copy, combined_x_ptr, async_finish, return_recv_hook, compute_stream_ptr)\n--\n\n"
+     "mooncake-ep/include/mooncake_ep_buffer.h:126-133. Returns (event or None, hook or None)."},
+    {"next_recv_x", MCEP_FAST(runtime_next_recv_x), METH_FASTCALL | METH_KEYWORDS,
+     "next_recv_x($self, num_max_dispatch_tokens_per_rank, hidden, num_experts, use_fp8)\n--\n\n"
+     "(device pointer, bytes) of the in-place receive tensor of the next dispatch call, (0, 0) when there is\n"
+     "none (include/mcep.h)."},
+    {"dispatch_tensors", MCEP_FAST(runtime_dispatch_tensors), METH_FASTCALL, "Buffer.dispatch on checked tensors."},
+    {"combine_tensors", MCEP_FAST(runtime_combine_tensors), METH_FASTCALL, "Buffer.combine on checked tensors."},
+    {nullptr, nullptr, 0, nullptr}};
+PyType_Slot runtime_slots[] = {{Py_tp_doc, const_cast<char*>("The calls of an mcep_buffer; base of ep.Buffer.")},
+                               {Py_tp_methods, runtime_methods},
+                               {0, nullptr}};
+PyType_Spec runtime_spec = {"mooncake_b200._mcep_torch.Runtime", sizeof(RuntimeObject), 0,
+                            Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE, runtime_slots};
+
+PyObject* py_adopt_event(PyObject*, PyObject* address) {
+    if (address == Py_None) Py_RETURN_NONE;
+    void* p = PyLong_AsVoidPtr(address);
+    if (PyErr_Occurred()) return nullptr;
+    return wrap_event(static_cast<mcep_event*>(p));
+}
+
+PyMethodDef module_methods[] = {
+    {"adopt_event", py_adopt_event, METH_O, "An EventHandle that owns the mcep_event at this address (None: None)."},
+    {"bind", py_bind, METH_O, "bind({name: address}): the entry points of the loaded libmcep.so."},
+    {"current_stream", py_current_stream, METH_NOARGS, "torch's current CUDA stream as an integer."},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_mcep_torch", "Native binding of libmcep.so for torch tensors.",
+                          -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__mcep_torch(void) {
+    PyObject* m = PyModule_Create(&module_def);
+    if (m == nullptr) return nullptr;
+    event_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&event_spec));
+    hook_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&hook_spec));
+    PyObject* runtime = PyType_FromSpec(&runtime_spec);
+    if (!event_type || !hook_type || !runtime) return nullptr;
+    if (PyModule_AddObjectRef(m, "EventHandle", reinterpret_cast<PyObject*>(event_type)) < 0 ||
+        PyModule_AddObjectRef(m, "Hook", reinterpret_cast<PyObject*>(hook_type)) < 0 ||
+        PyModule_AddObjectRef(m, "Runtime", runtime) < 0)
+        return nullptr;
+    return m;
+}

@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -193,7 +194,48 @@ void fabric_unmap(const DriverApi& d, FabricMapping* m) {
 
 struct mcep_event {
     cudaEvent_t ev = nullptr;
+    int device = 0;
 };
+
+// Completion events come from a small stock per device: creating and destroying
+// one costs more than recording it, and an asynchronous layer needs two. An
+// event may be recorded again while a stream still waits for its previous
+// recording (a wait refers to the recording it saw). The stock is bounded;
+// beyond it events are destroyed as they are freed.
+namespace {
+constexpr size_t kEventStock = 32;
+constexpr int kEventDevices = 64;
+std::mutex g_event_mu;
+std::vector<cudaEvent_t> g_event_stock[kEventDevices];
+
+cudaError_t take_event(mcep_event* e) {
+    cudaError_t err = cudaGetDevice(&e->device);
+    if (err != cudaSuccess) return err;
+    if (e->device < kEventDevices) {
+        std::lock_guard<std::mutex> lk(g_event_mu);
+        auto& stock = g_event_stock[e->device];
+        if (!stock.empty()) {
+            e->ev = stock.back();
+            stock.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaEventCreateWithFlags(&e->ev, cudaEventDisableTiming);
+}
+
+void give_event(mcep_event* e) {
+    if (e->ev == nullptr) return;
+    if (e->device < kEventDevices) {
+        std::lock_guard<std::mutex> lk(g_event_mu);
+        auto& stock = g_event_stock[e->device];
+        if (stock.size() < kEventStock) {
+            stock.push_back(e->ev);
+            return;
+        }
+    }
+    cudaEventDestroy(e->ev);
+}
+}  // namespace
 
 struct mcep_hook {
     std::function<int()> fn;
@@ -812,8 +854,8 @@ static mcep::Words words_of(int dpar, int cpar) {
 
 static int completion_event(cudaStream_t stream, mcep_event** out_event) {
     auto* ev = new mcep_event();
-    if (cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventRecord(ev->ev, stream) != cudaSuccess) {
+    if (take_event(ev) != cudaSuccess || cudaEventRecord(ev->ev, stream) != cudaSuccess) {
+        give_event(ev);
         delete ev;
         return fail(MCEP_ERR_CUDA, "Failed: CUDA error creating the completion event");
     }
@@ -870,7 +912,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     if (a->async_finish)
         if (int rc = order_after(stream, compute, b->ev_a)) return rc;
 
-    const bool pdl = chain_with_pdl(b, stream) && chain_with_pdl(b, compute);
+    const bool pdl = chain_with_pdl(b, stream) && (stream == compute || chain_with_pdl(b, compute));
     const bool chain_first = b->chain_first_once && pdl && !b->defer;
     b->chain_first_once = false;
     mcep::LaunchCtx first{stream, b->num_sms, chain_first};
@@ -1025,7 +1067,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
 
     cudaStream_t compute = reinterpret_cast<cudaStream_t>(a->compute_stream);
     cudaStream_t stream = a->async_finish ? b->comm_stream : compute;
-    const bool pdl = chain_with_pdl(b, stream) && chain_with_pdl(b, compute);
+    const bool pdl = chain_with_pdl(b, stream) && (stream == compute || chain_with_pdl(b, compute));
     const int num_sms = b->num_sms;
 
     if (!group) {
@@ -1246,10 +1288,10 @@ int mcep_launch_deferred(mcep_buffer* const* bufs, int n) {
 int mcep_event_create(uint64_t stream, mcep_event** out) {
     MCEP_REQUIRE(out != nullptr);
     auto* ev = new mcep_event();
-    cudaError_t e = cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming);
+    cudaError_t e = take_event(ev);
     if (e == cudaSuccess) e = cudaEventRecord(ev->ev, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
-        if (ev->ev) cudaEventDestroy(ev->ev);
+        give_event(ev);
         delete ev;
         return fail(MCEP_ERR_CUDA, "Failed: CUDA error '%s' (event create/record)",
                     cudaGetErrorString(e));
@@ -1272,7 +1314,7 @@ int mcep_event_synchronize(mcep_event* ev) {
 
 int mcep_event_free(mcep_event* ev) {
     if (ev == nullptr) return MCEP_OK;
-    if (ev->ev) cudaEventDestroy(ev->ev);
+    give_event(ev);
     delete ev;
     return MCEP_OK;
 }

@@ -1,7 +1,8 @@
 """Native module of the package: the objects the reference exposes as
 `mooncake._ep` / `mooncake.ep` (mooncake-ep/src/ep_py.cpp:14-46,
-mooncake-wheel/mooncake/ep.py:1-26), bound with ctypes to the C ABI of
-`libmcep.so` (include/mcep.h).
+mooncake-wheel/mooncake/ep.py:1-26), over the C ABI of `libmcep.so`
+(include/mcep.h): the calls of the hot path through the native binding
+(csrc/ep_py_torch.cpp), everything else with ctypes.
 
 `Buffer`, `EventHandle`, `get_ep_buffer_size_hint` and `MAX_QP_COUNT` keep the
 reference's names, argument order and return shapes. There is no CPU path:
@@ -11,8 +12,10 @@ import fails.
 from __future__ import annotations
 
 import ctypes
-import os
-from typing import Callable, List, Optional, Tuple
+import importlib.util
+from typing import List, Optional, Tuple
+
+import torch  # noqa: F401  the native binding links against torch's libraries
 
 from . import build as _build
 
@@ -138,6 +141,22 @@ def _load() -> ctypes.CDLL:
 
 _lib = _load()
 
+
+def _load_native():
+    """The compiled part of the binding, told where the entry points of the library are."""
+    spec = importlib.util.spec_from_file_location("mooncake_b200._mcep_torch", _build.build_binding())
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    names = ("mcep_last_error", "mcep_dispatch", "mcep_combine", "mcep_elastic_dispatch", "mcep_elastic_combine",
+             "mcep_buffer_next_recv_x", "mcep_event_create", "mcep_event_current_stream_wait",
+             "mcep_event_synchronize", "mcep_event_free", "mcep_hook_run", "mcep_hook_free")
+    mod.bind({n: _c.cast(getattr(_lib, n), _c.c_void_p).value for n in names})
+    return mod
+
+
+_native = _load_native()
+current_stream = _native.current_stream  # torch's current CUDA stream as an integer
+
 MAX_QP_COUNT = 256  # mooncake-ep/include/mooncake_ep_configs.cuh:5
 
 
@@ -174,46 +193,10 @@ def get_ep_buffer_size_hint(num_max_dispatch_tokens_per_rank: int, hidden: int,
                                                  num_ranks, num_experts))
 
 
-class EventHandle:
-    """mooncake-ep/include/mooncake_ep_event.h:9-44: a CUDA event recorded on
-    `stream_ptr` at construction."""
-
-    def __init__(self, stream_ptr: int = 0, _adopt: Optional[int] = None):
-        if _adopt is not None:
-            self._h = _c.c_void_p(_adopt)
-        else:
-            h = _c.c_void_p()
-            _check(_lib.mcep_event_create(stream_ptr, _c.byref(h)))
-            self._h = h
-
-    def current_stream_wait(self, stream_ptr: int) -> None:
-        _check(_lib.mcep_event_current_stream_wait(self._h, stream_ptr))
-
-    def synchronize(self) -> None:
-        _check(_lib.mcep_event_synchronize(self._h))
-
-    def __del__(self):
-        h, self._h = getattr(self, "_h", None), None
-        if h:
-            _lib.mcep_event_free(h)
+EventHandle = _native.EventHandle  # mooncake-ep/include/mooncake_ep_event.h:9-44
 
 
-class _Hook:
-    """The receive-phase callback (the `std::function<void()>` of the reference)."""
-
-    def __init__(self, handle: int):
-        self._h = _c.c_void_p(handle)
-
-    def __call__(self) -> None:
-        _check(_lib.mcep_hook_run(self._h))
-
-    def __del__(self):
-        h, self._h = getattr(self, "_h", None), None
-        if h:
-            _lib.mcep_hook_free(h)
-
-
-class Buffer:
+class Buffer(_native.Runtime):
     """mooncake-ep/src/ep_py.cpp:28-46 / mooncake-ep/include/mooncake_ep_buffer.h:65-195."""
 
     def __init__(self, rank: int, num_ranks: int, num_ep_buffer_bytes: int,
@@ -222,12 +205,12 @@ class Buffer:
         self.rank, self.num_ranks = rank, num_ranks
         _check(_lib.mcep_buffer_create(rank, num_ranks, num_ep_buffer_bytes,
                                        1 if disable_p2p else 0, _c.byref(self._h)))
-        self._dargs = _DispatchArgs()
-        self._cargs = _CombineArgs()
+        self._adopt(self._h.value, num_ranks)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
-        if h:
+        self._adopt(None, 0)
+        if h and _lib is not None:  # (None while the interpreter shuts down)
             _lib.mcep_buffer_destroy(h)
 
     # -- RDMA surface of the reference: there is no RDMA route here ------------
@@ -316,15 +299,6 @@ class Buffer:
         _check(_lib.mcep_buffer_call_counts(self._h, _c.byref(d), _c.byref(c)))
         return int(d.value), int(c.value)
 
-    def next_recv_x(self, num_max_dispatch_tokens_per_rank: int, hidden: int, num_experts: int,
-                    use_fp8: bool) -> Tuple[int, int]:
-        """(device pointer, bytes) of the in-place receive tensor of the next
-        dispatch call, (0, 0) when there is none (include/mcep.h)."""
-        p, n = _c.c_void_p(), _c.c_size_t()
-        _check(_lib.mcep_buffer_next_recv_x(self._h, num_max_dispatch_tokens_per_rank, hidden,
-                                            num_experts, int(use_fp8), _c.byref(p), _c.byref(n)))
-        return int(p.value or 0), int(n.value)
-
     def next_combine_buffer(self, num_max_dispatch_tokens_per_rank: int, hidden: int,
                             num_experts: int) -> Tuple[int, int]:
         """(device pointer, bytes) of the tensor the next zero-copy combine reads."""
@@ -334,52 +308,7 @@ class Buffer:
                                                     _c.byref(n)))
         return int(p.value or 0), int(n.value)
 
-    # -- the hot path ----------------------------------------------------------
-    def dispatch(self, x_ptr: int, topk_idx_ptr: int, active_ranks_ptr: int, num_tokens: int,
-                 hidden: int, num_topk: int, num_max_dispatch_tokens_per_rank: int,
-                 num_experts: int, timeout_us: int, use_fp8: bool, packed_recv_x_ptr: int,
-                 packed_recv_x_scales_ptr: int, packed_recv_count_ptr: int,
-                 packed_recv_src_info_ptr: int, packed_recv_layout_range_ptr: int,
-                 async_finish: bool, return_recv_hook: bool, compute_stream_ptr: int
-                 ) -> Tuple[Optional[EventHandle], Optional[Callable[[], None]]]:
-        a = self._dargs
-        a.x, a.topk_idx, a.active_ranks = x_ptr, topk_idx_ptr, active_ranks_ptr
-        a.num_tokens, a.hidden, a.num_topk = num_tokens, hidden, num_topk
-        a.num_max_dispatch_tokens_per_rank = num_max_dispatch_tokens_per_rank
-        a.num_experts, a.use_fp8, a.timeout_us = num_experts, int(use_fp8), timeout_us
-        a.packed_recv_x, a.packed_recv_x_scales = packed_recv_x_ptr, packed_recv_x_scales_ptr
-        a.packed_recv_count = packed_recv_count_ptr
-        a.packed_recv_src_info = packed_recv_src_info_ptr
-        a.packed_recv_layout_range = packed_recv_layout_range_ptr
-        a.async_finish, a.return_recv_hook = int(async_finish), int(return_recv_hook)
-        a.compute_stream = compute_stream_ptr
-        ev, hk = _c.c_void_p(), _c.c_void_p()
-        _check(_lib.mcep_dispatch(self._h, _c.byref(a), _c.byref(ev), _c.byref(hk)))
-        return (EventHandle(_adopt=ev.value) if ev.value else None,
-                _Hook(hk.value) if hk.value else None)
-
-    def combine(self, x_ptr: int, topk_idx_ptr: int, topk_weights_ptr: int, src_info_ptr: int,
-                layout_range_ptr: int, active_ranks_ptr: int, num_local_experts: int,
-                num_combined_tokens: int, hidden: int, num_topk: int,
-                num_max_dispatch_tokens_per_rank: int, num_experts: int, timeout_us: int,
-                zero_copy: bool, combined_x_ptr: int, async_finish: bool,
-                return_recv_hook: bool, compute_stream_ptr: int
-                ) -> Tuple[Optional[EventHandle], Optional[Callable[[], None]]]:
-        a = self._cargs
-        a.x, a.topk_idx, a.topk_weights = x_ptr, topk_idx_ptr, topk_weights_ptr
-        a.src_info, a.layout_range, a.active_ranks = src_info_ptr, layout_range_ptr, active_ranks_ptr
-        a.num_local_experts, a.num_combined_tokens = num_local_experts, num_combined_tokens
-        a.hidden, a.num_topk = hidden, num_topk
-        a.num_max_dispatch_tokens_per_rank = num_max_dispatch_tokens_per_rank
-        a.num_experts, a.timeout_us, a.zero_copy = num_experts, timeout_us, int(zero_copy)
-        a.combined_x = combined_x_ptr
-        a.async_finish, a.return_recv_hook = int(async_finish), int(return_recv_hook)
-        a.compute_stream = compute_stream_ptr
-        ev, hk = _c.c_void_p(), _c.c_void_p()
-        _check(_lib.mcep_combine(self._h, _c.byref(a), _c.byref(ev), _c.byref(hk)))
-        return (EventHandle(_adopt=ev.value) if ev.value else None,
-                _Hook(hk.value) if hk.value else None)
-
+    # -- the hot path: `dispatch`, `combine`, `next_recv_x` are methods of the native base ----
 
     # -- elastic-style calls (mooncake-ep/src/mooncake_ep_elastic_buffer.cpp:230-426) -----
     def elastic_dispatch(self, x_ptr: int, x_element_size: int, sf_ptr: int, num_tokens: int,
@@ -412,7 +341,7 @@ class Buffer:
         a.copied_topk_idx = copied_topk_idx_ptr or None
         ev = _c.c_void_p()
         _check(_lib.mcep_elastic_dispatch(self._h, _c.byref(a), _c.byref(ev)))
-        return EventHandle(_adopt=ev.value) if ev.value else None
+        return _native.adopt_event(ev.value)
 
     def elastic_combine(self, x_ptr: int, num_input_tokens: int, hidden: int, topk_idx_ptr: int,
                         num_combined_tokens: int, num_topk: int, topk_weights_ptr: int,
@@ -432,7 +361,7 @@ class Buffer:
         a.combined_x = combined_x_ptr or None
         ev = _c.c_void_p()
         _check(_lib.mcep_elastic_combine(self._h, _c.byref(a), _c.byref(ev)))
-        return EventHandle(_adopt=ev.value) if ev.value else None
+        return _native.adopt_event(ev.value)
 
 
 def elastic_buffer_size_hint(num_max_tokens_per_rank: int, hidden: int, num_ranks: int,

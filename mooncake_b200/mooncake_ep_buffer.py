@@ -35,8 +35,7 @@ import torch.distributed as dist
 from . import ep
 
 
-def _stream_ptr() -> int:
-    return int(torch.cuda.current_stream().cuda_stream)
+_stream_ptr = ep.current_stream
 
 
 class _DeviceBytes:
@@ -173,46 +172,41 @@ class Buffer:
         `[E/R, H/128, R*M]` storage), `recv_count[E/R]` and
         `handle = (src_info, layout_range, M, H, E)`.
         """
+        use_fp8 = True if use_fp8 is None else use_fp8
+        in_place = self._rows_in_place if getattr(self, "recv_in_place", True) else None
+        out = self.runtime.dispatch_tensors(x, topk_idx, active_ranks, num_max_dispatch_tokens_per_rank, num_experts,
+                                            timeout_us, use_fp8, async_finish, return_recv_hook, in_place)
+        if out is None:  # not the plain case: find out what is wrong, or what to put in
+            active_ranks = self._checked_dispatch(x, topk_idx, active_ranks, num_max_dispatch_tokens_per_rank,
+                                                  num_experts, use_fp8)
+            out = self.runtime.dispatch_tensors(x, topk_idx, active_ranks, num_max_dispatch_tokens_per_rank,
+                                                num_experts, timeout_us, use_fp8, async_finish, return_recv_hook,
+                                                in_place)
+            assert out is not None, "dispatch takes CUDA tensors"
+        recv_x, scales, recv_count, src_info, layout_range, event, hook = out
+        handle = (src_info, layout_range, num_max_dispatch_tokens_per_rank, x.size(1), num_experts)
+        keep = (x, topk_idx, recv_x, scales, recv_count, src_info, layout_range) if async_finish else None
+        return ((recv_x, scales) if use_fp8 else recv_x, recv_count, handle, EventOverlap(event, keep), hook)
+
+    def _rows_in_place(self, ptr: int, nbytes: int, L: int, RM: int, H: int, use_fp8: bool,
+                       x: torch.Tensor) -> torch.Tensor:
+        """The symmetric memory in which the next dispatch call of a group lands its rows."""
+        return self._symmetric_tensor(ptr, nbytes, (L, RM, H), torch.float8_e4m3fn if use_fp8 else torch.bfloat16,
+                                      x.device)
+
+    def _checked_dispatch(self, x, topk_idx, active_ranks, M, num_experts, use_fp8) -> torch.Tensor:
+        """The argument checks of the reference's wrapper (:384-404); returns the mask to use."""
         assert x.dim() == 2 and x.is_contiguous()
         assert x.dtype == torch.bfloat16
         assert topk_idx.dim() == 2 and topk_idx.is_contiguous()
         assert topk_idx.dtype == torch.int64
         assert x.size(0) == topk_idx.size(0)
-        assert x.size(0) <= num_max_dispatch_tokens_per_rank
+        assert x.size(0) <= M
         assert x.size(1) % 16 == 0 and x.size(1) % 128 == 0
         assert num_experts % self.group_size == 0
-        active_ranks = self._resolve_active_ranks(active_ranks, x.device)
-        if use_fp8 is None:
-            use_fp8 = True
-        R, M, H = self.group_size, num_max_dispatch_tokens_per_rank, x.size(1)
-        L = num_experts // R
-        dev = x.device
-        rx_dtype = torch.float8_e4m3fn if use_fp8 else torch.bfloat16
-        recv_x = None
-        if getattr(self, "recv_in_place", True):
-            ptr, nbytes = self.runtime.next_recv_x(M, H, num_experts, use_fp8)
-            if ptr:
-                recv_x = self._symmetric_tensor(ptr, nbytes, (L, R * M, H), rx_dtype, dev)
-        if recv_x is None:
-            recv_x = torch.empty((L, R * M, H), device=dev, dtype=rx_dtype)
-        recv_count = torch.empty((L,), dtype=torch.int32, device=dev)
-        src_info = torch.empty((L, R * M), dtype=torch.int32, device=dev)
-        layout_range = torch.empty((L, R), dtype=torch.int64, device=dev)
-        scales = None
         if use_fp8:
-            assert (R * M) % 4 == 0
-            scales = torch.empty((L, H // 128, R * M), dtype=torch.float32,
-                                 device=dev).transpose(1, 2)
-        event, hook = self.runtime.dispatch(
-            x.data_ptr(), topk_idx.data_ptr(), active_ranks.data_ptr(), x.size(0), H,
-            topk_idx.size(1), M, num_experts, timeout_us, use_fp8, recv_x.data_ptr(),
-            0 if scales is None else scales.data_ptr(), recv_count.data_ptr(),
-            src_info.data_ptr(), layout_range.data_ptr(), async_finish, return_recv_hook,
-            _stream_ptr())
-        handle = (src_info, layout_range, M, H, num_experts)
-        keep = (x, topk_idx, recv_x, scales, recv_count, src_info, layout_range)
-        return ((recv_x, scales) if use_fp8 else recv_x, recv_count, handle,
-                EventOverlap(event, keep if async_finish else None), hook)
+            assert (self.group_size * M) % 4 == 0
+        return self._resolve_active_ranks(active_ranks, x.device)
 
     # ------------------------------------------------------------------ combine
     def combine(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor,
@@ -224,6 +218,22 @@ class Buffer:
         (reference :538-678). With `zero_copy` the expert outputs are read from the
         tensor `get_next_combine_buffer(handle)` returned and `x` only gives the
         shape."""
+        src_info, layout_range, M, hidden, num_experts = handle
+        res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info,
+                                           layout_range, M, hidden, num_experts, zero_copy, async_finish,
+                                           return_recv_hook, out)
+        if res is None:  # not the plain case: find out what is wrong, or what to put in
+            active_ranks = self._checked_combine(x, topk_idx, topk_weights, active_ranks, handle, out)
+            res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info,
+                                               layout_range, M, hidden, num_experts, zero_copy, async_finish,
+                                               return_recv_hook, out)
+            assert res is not None, "combine takes CUDA tensors"
+        combined_x, event, hook = res
+        keep = (x, topk_idx, topk_weights, src_info, layout_range, combined_x) if async_finish else None
+        return combined_x, EventOverlap(event, keep), hook
+
+    def _checked_combine(self, x, topk_idx, topk_weights, active_ranks, handle, out) -> torch.Tensor:
+        """The argument checks of the reference's wrapper (:557-603); returns the mask to use."""
         assert x.dim() == 3 and x.is_contiguous()
         assert x.dtype == torch.bfloat16
         assert topk_idx.dim() == 2 and topk_idx.is_contiguous()
@@ -248,17 +258,7 @@ class Buffer:
             assert out.dim() == 2 and out.is_contiguous()
             assert out.size(0) == topk_weights.size(0) and out.size(1) == hidden
             assert out.dtype == x.dtype
-            combined_x = out
-        else:
-            combined_x = torch.empty((topk_weights.size(0), hidden), dtype=x.dtype,
-                                     device=x.device)
-        event, hook = self.runtime.combine(
-            x.data_ptr(), topk_idx.data_ptr(), topk_weights.data_ptr(), src_info.data_ptr(),
-            layout_range.data_ptr(), active_ranks.data_ptr(), x.size(0), topk_weights.size(0),
-            hidden, topk_weights.size(1), M, num_experts, timeout_us, zero_copy,
-            combined_x.data_ptr(), async_finish, return_recv_hook, _stream_ptr())
-        keep = (x, topk_idx, topk_weights, src_info, layout_range, combined_x)
-        return combined_x, EventOverlap(event, keep if async_finish else None), hook
+        return active_ranks
 
     def get_next_combine_buffer(self, handle: tuple) -> torch.Tensor:
         """The tensor `[E/R, R*M, H]` bf16 the next `combine(..., zero_copy=True)`
