@@ -294,8 +294,6 @@ int mcep_elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, m
     da.compute_stream = reinterpret_cast<uint64_t>(stream);
     mcep_event* ev = nullptr;
     mcep_hook* hook = nullptr;
-    // the route kernel lets its dependents start early; the exchange's first kernel waits for it
-    mcep::allow_chained_first_launch(b);
     if (int rc = mcep_dispatch(b, &da, &ev, &hook)) return rc;
 
     auto& rec = s->rec[par];

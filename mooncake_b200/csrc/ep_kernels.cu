@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "ep_device.cuh"
+#include "ep_routing.cuh"
 
 namespace mcep {
 
@@ -104,36 +105,47 @@ namespace kernels {
 constexpr unsigned kFull = 0xffffffffu;
 
 template <typename... KArgs, typename... Args>
-cudaError_t launch(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                   const LaunchCtx& ctx, Args&&... args) {
-    if (g_timing.load()) {
-        TimingRec r{name, nullptr, nullptr};
-        cudaEventCreate(&r.a);
-        cudaEventCreate(&r.b);
-        cudaEventRecord(r.a, ctx.stream);
-        kernel<<<grid, block, smem, ctx.stream>>>(args...);
-        cudaError_t err = cudaGetLastError();
-        cudaEventRecord(r.b, ctx.stream);
-        std::lock_guard<std::mutex> lk(g_timing_mu);
-        g_recs.push_back(r);
-        if (err == cudaSuccess) g_launches.fetch_add(1);
-        return err;
-    }
+cudaError_t launch_clusters(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            int cluster, const LaunchCtx& ctx, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx.stream;
-    cudaLaunchAttribute attr[1];
-    if (ctx.pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
-    cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    const bool timing = g_timing.load();
+    if (ctx.pdl && !timing) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        ++cfg.numAttrs;
+    }
+    TimingRec r{name, nullptr, nullptr};
+    if (timing) {
+        cudaEventCreate(&r.a);
+        cudaEventCreate(&r.b);
+        cudaEventRecord(r.a, ctx.stream);
+    }
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    if (timing) {
+        cudaEventRecord(r.b, ctx.stream);
+        std::lock_guard<std::mutex> lk(g_timing_mu);
+        g_recs.push_back(r);
+    }
     if (err == cudaSuccess) g_launches.fetch_add(1);
     return err;
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                   const LaunchCtx& ctx, Args&&... args) {
+    return launch_clusters(name, kernel, grid, block, smem, 1, ctx, std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
@@ -576,19 +588,104 @@ __global__ void __launch_bounds__(256) ep_layout_slot_kernel(LayoutParams p) {
     }
 }
 
+// ---- the same layout in one launch of one cluster -----------------------------------
+// What dispatch uses for all but the smallest and the largest batches. The blocks
+// of one cluster share the tokens, one lane per token:
+//   bit (expert, token) in the block's shared bitmap, word-major [word][E];
+//   per expert: popcounts of the words -> exclusive prefix over the words, total;
+//   cluster barrier; totals of the lower blocks through distributed shared memory;
+//   slot = lower blocks + lower words + lower bits of the own word.
+// 4096 tokens x 8 of 256: one launch in place of the two above (4 + 10 us).
+constexpr int kLayoutCluster = 8, kLayoutClusterLarge = 16;
+
+template <int KB>
+__device__ __forceinline__ void cluster_layout(const LayoutParams& p, uint32_t* mask, int* pre, int* total) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, words = nthr >> 5;
+    const int rank = blockIdx.x, blocks = gridDim.x;
+    const int t = rank * nthr + tid;
+    for (int i = tid; i < p.E * words; i += nthr) mask[i] = 0;
+    int e[KB];
+#pragma unroll
+    for (int k = 0; k < KB; ++k) e[k] = -1;
+    if (t < p.T) load_choices<KB>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
+    drop_repeats<KB, false>(e);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+        if (e[k] >= 0) atomicOr(&mask[warp * p.E + e[k]], 1u << lane);
+    __syncthreads();
+    for (int x = tid; x < p.E; x += nthr) {
+        int run = 0;
+        for (int w = 0; w < words; ++w) {
+            const int c = __popc(mask[w * p.E + x]);
+            pre[w * p.E + x] = run;
+            run += c;
+        }
+        total[x] = run;
+    }
+    cluster_sync();  // (a block barrier as well)
+    for (int x = tid; x < p.E; x += nthr) {
+        int base = 0;
+#pragma unroll
+        for (int r = 0; r < kLayoutClusterLarge - 1; ++r)
+            if (r < rank) base += ld_cluster_s32(total + x, r);
+        total[p.E + x] = base;
+        if (rank == blocks - 1) {
+            const int c = base + total[x];
+            p.count[x] = c;
+            if (p.recv_count) p.recv_count[x] = c;
+            if (p.layout_range) p.layout_range[x] = c;  // begin 0 | count
+        }
+    }
+    __syncthreads();
+    if (t < p.T) {
+        const unsigned lower = (1u << lane) - 1u;
+        int32_t* out = p.slot + (size_t)t * p.K;
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+            if (k >= p.K) break;
+            int s = -1;
+            if (e[k] >= 0) {
+                const int at = warp * p.E + e[k];
+                s = total[p.E + e[k]] + pre[at] + __popc(mask[at] & lower);
+            }
+            out[k] = s;
+        }
+    }
+    cluster_sync();  // no block leaves while its totals may still be read
+}
+
+__global__ void __launch_bounds__(1024) ep_layout_cluster_kernel(LayoutParams p) {
+    extern __shared__ int smem_i32[];
+    const int words = blockDim.x >> 5;
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem_i32);  // [words][E]
+    int* pre = smem_i32 + words * p.E;                       // [words][E]
+    int* total = smem_i32 + 2 * words * p.E;                 // [E] this block, [E] lower blocks
+    pdl_wait();
+    pdl_launch_dependents();
+    if (p.K <= 4)
+        cluster_layout<4>(p, mask, pre, total);
+    else if (p.K <= 8)
+        cluster_layout<8>(p, mask, pre, total);
+    else
+        cluster_layout<16>(p, mask, pre, total);
+}
+
 // =============================================================================
 // sending token rows (single rank and groups)
 // =============================================================================
-// One block per token (blocks stride over the tokens), one warp per 512-channel
-// tile of the row. The block reads the bf16 row once (32 bytes per lane),
-// quantises it in registers when FP8 is on, and stores it to the row of every
-// selected expert's packed receive area: this GPU's (single rank, or an expert
-// this rank owns) or a peer's, over NVLink.
+// A block takes a batch of `C` consecutive tokens, reads each bf16 row once (32
+// bytes per lane, one warp per 512-channel tile), quantises it in registers when
+// FP8 is on, and stores it to the row of every selected expert's packed receive
+// area: this GPU's (single rank, or an expert this rank owns) or a peer's, over
+// NVLink.
 //
-// kFused: the position of the token among this rank's tokens for each of its
-// experts is counted here instead of read from the layout kernel - every warp
-// takes whole tokens of the (small) index matrix. The host uses it when one
-// block per token fits the machine in one wave.
+// A single rank launches one block per batch, however many there are: the
+// hardware then hands the batches out as SMs come free. Rows of 14 KB to 8
+// experts each, 4096 tokens: 98 us with one resident wave striding over the
+// tokens (the slowest SM decides), 85 us with a block each. Tokens leave in
+// ascending order over the whole grid, which keeps an expert's rows together in
+// time and in HBM pages.
 //
 // What goes where for entry (t, k) with expert e, owner rank o, local expert le,
 // row r = first row of this rank's segment in e + earlier tokens of this rank:
@@ -601,200 +698,152 @@ __global__ void __launch_bounds__(256) ep_layout_slot_kernel(LayoutParams p) {
 struct SendView {
     const char* x;
     const int64_t* topk_idx;
-    const int32_t* slot;
     int T, K, E, R, M, H, rank;
     int L, RM;
+    int C;                    // tokens per batch
+    const int32_t* slot;      // [T*K] position among this rank's tokens for the expert (layout kernel),
+                              // or null: counted here (small batches, one per block)
     int32_t* status;
     // rows this rank owns
     char* recv_x;
     float* recv_scales;
     int32_t* recv_src_info;
     int row_bytes;
+    int32_t* rowmap;
+    // single rank, counted here: the receive layout, written by the block that takes the last batch
+    int32_t* recv_count;
+    int64_t* layout_range;
     // groups only
     const uint64_t* beg;      // local words: first row of this rank's segment per expert
     uint32_t seq;
     WaitCfg wait;
     size_t rx_off, meta_off;
     int meta_stride;
-    int32_t* rowmap;
     char* const* s_peer;      // shared-memory copies of the peer table and the mask
     const int* s_active;
 };
 
-// One pass of all warps over the whole index matrix. With kHist it leaves the
-// whole-batch count per expert in hist[]; with t_own >= 0 it counts, for every
-// expert of token t_own (kmap: expert -> k), the earlier tokens that chose it
-// (s_before[k]). A repeated expert inside a token is counted once (lanes holding
-// the same (token, expert) elect the lowest lane).
-constexpr int kScanAhead = 4;
+constexpr int kBatchEntries = 128;  // (token, k) entries of a batch
 
-template <bool kHist, bool kAhead>
-__device__ __forceinline__ void scan_index_matrix(const int64_t* topk_idx, int T, int K, int E,
-                                                  int* hist, const int* kmap, int* s_before,
-                                                  int t_own, const int (&e_ahead)[kScanAhead]) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int tpw = 32 / K;  // tokens per warp pass (K <= 16)
-    const int sk = lane % K, st = lane / K;
-    const bool lane_used = st < tpw;
-    auto count_pass = [&](int base, int e) {
-        const int t2 = base + st;
-        const bool valid = lane_used && t2 < T;
-        if (!valid || e >= E) e = -1;
-        const unsigned key = e >= 0 ? (((unsigned)st << 16) | (unsigned)e) : (0x80000000u | lane);
-        const unsigned grp = __match_any_sync(kFull, key);
-        if (e >= 0 && (int)(__ffs(grp) - 1) == lane) {
-            if (kHist) atomicAdd(&hist[e], 1);
-            if (t2 < t_own) {
-                const int kk = kmap[e];
-                if (kk >= 0) atomicAdd(&s_before[kk], 1);
-            }
-        }
-    };
-    if (kAhead) {
-#pragma unroll
-        for (int u = 0; u < kScanAhead; ++u) {
-            const int base = (warp + u * nwarps) * tpw;
-            if (base < T) count_pass(base, e_ahead[u]);
-        }
-    }
-    for (int base = (warp + (kAhead ? kScanAhead : 0) * nwarps) * tpw; base < T;
-         base += nwarps * tpw) {
-        const int t2 = base + st;
-        count_pass(base, (lane_used && t2 < T) ? (int)__ldg(topk_idx + (size_t)t2 * K + sk) : -1);
-    }
-}
-
-
-// Requests the first kScanAhead passes of the scan (so the scan does not pay a
-// memory round trip per pass).
-__device__ __forceinline__ void scan_prefetch(const int64_t* topk_idx, int T, int K, bool on,
-                                              int (&e_ahead)[kScanAhead]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int tpw = 32 / K;
-    const int sk = lane % K, st = lane / K;
-#pragma unroll
-    for (int u = 0; u < kScanAhead; ++u) {
-        const int t2 = (warp + u * nwarps) * tpw + st;
-        e_ahead[u] = -1;
-        if (on && st < tpw && t2 < T) e_ahead[u] = (int)__ldg(topk_idx + (size_t)t2 * K + sk);
-    }
-}
-
-template <bool kFP8, bool kGroup, bool kFused>
-__device__ __forceinline__ void send_tokens(const SendView& v, int first_token, int token_stride,
-                                            int* hist /* fused && !group: [E] */,
-                                            int* kmap /* fused: [E] */) {
-    __shared__ char* s_dst[kMaxTopk];
-    __shared__ char* s_meta[kMaxTopk];
-    __shared__ int s_exp[kMaxTopk];
-    __shared__ int s_le[kMaxTopk];
-    __shared__ int s_row[kMaxTopk];
-    __shared__ int s_before[kMaxTopk];
-    __shared__ int s_raw[kMaxTopk];
+// kCount: the positions are counted here, hist: [E] in shared memory; else `slot` has them. All threads of the block call it.
+// What is read before `ready()` is complete when the kernel begins (the rows and the
+// index matrix: the layout kernel ahead has waited for whatever wrote them).
+template <bool kFP8, bool kGroup, bool kCount, typename Ready>
+__device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsend, int* hist, Ready ready) {
+    __shared__ char* s_dst[kBatchEntries];
+    __shared__ char* s_meta[kGroup ? kBatchEntries : 1];
+    __shared__ int s_raw[kBatchEntries];   // expert of the entry, -1: none
+    __shared__ int s_exp[kBatchEntries];   // the same without repeats inside a token
+    __shared__ int s_row[kBatchEntries];
+    __shared__ int s_le[kBatchEntries];
 
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int nchunks = v.H / 16;
     const int ntiles = (v.H + kTileChannels - 1) / kTileChannels;
     const int S = v.H / 128;
+    const int K = v.K;
 
-    for (int t = first_token; t < v.T; t += token_stride) {
-        const char* xrow = v.x + (size_t)t * v.H * 2;
-        V32 first = {};
-        if (warp < ntiles && warp * 32 + lane < nchunks)
-            first = ld32_readonly(xrow + (size_t)(warp * 32 + lane) * 32);
-        // (in production a fused launch has one block per token; blocks that take
-        // several tokens - in-process groups - scan once per token)
-        const bool scan_now = kFused;
-        int e_ahead[kScanAhead];
-        scan_prefetch(v.topk_idx, v.T, v.K, scan_now, e_ahead);
-        int my_slot = -1;
-        if (tid < kMaxTopk) {
-            int e = tid < v.K ? (int)__ldg(v.topk_idx + (size_t)t * v.K + tid) : -1;
-            if (!kFused && tid < v.K) my_slot = __ldg(v.slot + (size_t)t * v.K + tid);
-            s_raw[tid] = (e >= 0 && e < v.E) ? e : -1;
-            s_before[tid] = 0;
-        }
+    // one warp item = one tile of one row of the batch that starts at token t
+    auto load_item = [&](int t, int item) {
+        V32 r = {};
+        const int tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
+        if (tok < v.C && t + tok < v.T && c < nchunks)
+            r = ld32_readonly(v.x + ((size_t)(t + tok) * v.H + (size_t)c * 16) * 2);
+        return r;
+    };
+    int t0 = sid * v.C;
+    V32 ahead = load_item(t0, warp);
+    if (kCount) {
+        for (int e = tid; e < v.E; e += nthr) hist[e] = 0;
+        if (!kGroup && v.T == 0 && sid == 0)
+            for (int e = tid; e < v.E; e += nthr) v.recv_count[e] = 0, v.layout_range[e] = 0;
         __syncthreads();
-        if (tid < kMaxTopk) {
-            int e = s_raw[tid];
-            for (int kk = 0; kk < tid; ++kk)
-                if (s_raw[kk] == e) e = -1;  // a repeat of an earlier entry of this token
+    }
+    int counted = 0;  // tokens that are in hist
+    for (; t0 < v.T;) {
+        const int nt = min(v.C, v.T - t0), ne = nt * K, items = nt * ntiles;
+        const int t1 = t0 + nsend * v.C;
+        int raw = -1, slot = 0;
+        if (tid < ne) raw = (int)__ldg(v.topk_idx + (size_t)t0 * K + tid);
+        if (kCount) {
+            count_tokens<1>(v.topk_idx, counted, t0, K, v.E, choices_in_pairs(v.topk_idx, K), hist);
+        } else {
+            ready();
+            if (tid < ne) slot = __ldg(v.slot + (size_t)t0 * K + tid);
+        }
+        if (raw >= v.E) raw = -1;
+        if (tid < ne) s_raw[tid] = raw;
+        __syncthreads();  // hist holds every token before t0
+        const int tok0 = tid / K * K;  // first entry of this entry's token
+        int e = raw;
+        if (tid < ne) {
+            for (int j = tok0; j < tid; ++j)
+                if (s_raw[j] == raw) e = -1;  // a repeat of an earlier entry of this token
             s_exp[tid] = e;
-            if (scan_now && e >= 0) kmap[e] = tid;
         }
-        __syncthreads();
-        if (scan_now) {
-            if (kGroup)
-                scan_index_matrix<false, true>(v.topk_idx, v.T, v.K, v.E, nullptr, kmap, s_before,
-                                               t, e_ahead);
-            else
-                scan_index_matrix<true, true>(v.topk_idx, v.T, v.K, v.E, hist, kmap, s_before, t,
-                                              e_ahead);
-            __syncthreads();
-        }
-        if (tid < kMaxTopk) {
+        if (nt > 1) __syncthreads();
+        if (tid < ne) {
             char* dst = nullptr;
             char* meta = nullptr;
             int row = -1, le = 0;
-            const int e = s_exp[tid];
             if (e >= 0) {
-                const int s = kFused ? s_before[tid] : my_slot;
+                int s = slot;
+                if (kCount) {
+                    s = hist[e];
+                    for (int j = 0; j < tok0; ++j) s += (s_exp[j] == e);  // earlier tokens of the batch
+                }
                 if (s >= v.M) {
                     atomicOr(v.status, kStatusSlotRange);
-                } else if (s >= 0) {
-                    if (!kGroup) {
-                        le = e;
-                        row = s;
-                        dst = v.recv_x + ((size_t)e * v.RM + s) * (size_t)v.row_bytes;
-                    } else {
-                        const int dr = e / v.L;
-                        le = e - dr * v.L;
-                        if (v.s_active[dr]) {
-                            // the owner's answer: first row of this rank's segment
-                            const uint32_t b = wait_word(v.beg + e, v.seq, v.wait, dr);
-                            if (b) {
-                                row = (int)(b - 1) + s;
-                                if (row >= v.RM) {
-                                    atomicOr(v.status, kStatusSlotRange);
-                                    row = -1;
-                                } else if (dr == v.rank) {
-                                    dst = v.recv_x + ((size_t)le * v.RM + row) * (size_t)v.row_bytes;
-                                } else {
-                                    const size_t r = (size_t)le * v.RM + row;
-                                    dst = v.s_peer[dr] + v.rx_off + r * (size_t)v.row_bytes;
-                                    meta = v.s_peer[dr] + v.meta_off + r * (size_t)v.meta_stride;
-                                }
+                } else if (!kGroup) {
+                    le = e;
+                    row = s;
+                    dst = v.recv_x + ((size_t)e * v.RM + s) * (size_t)v.row_bytes;
+                } else {
+                    const int dr = e / v.L;
+                    le = e - dr * v.L;
+                    if (v.s_active[dr]) {
+                        // the owner's answer: first row of this rank's segment
+                        const uint32_t b = wait_word(v.beg + e, v.seq, v.wait, dr);
+                        if (b) {
+                            row = (int)(b - 1) + s;
+                            if (row >= v.RM) {
+                                atomicOr(v.status, kStatusSlotRange);
+                                row = -1;
+                            } else if (dr == v.rank) {
+                                dst = v.recv_x + ((size_t)le * v.RM + row) * (size_t)v.row_bytes;
+                            } else {
+                                const size_t r = (size_t)le * v.RM + row;
+                                dst = v.s_peer[dr] + v.rx_off + r * (size_t)v.row_bytes;
+                                meta = v.s_peer[dr] + v.meta_off + r * (size_t)v.meta_stride;
                             }
                         }
                     }
                 }
             }
-            if (tid < v.K && v.rowmap != nullptr) v.rowmap[(size_t)t * v.K + tid] = row;
-            if (scan_now && e >= 0) kmap[e] = -1;  // leave the table clean for the next token
+            v.rowmap[(size_t)t0 * K + tid] = row;
             s_dst[tid] = dst;
-            s_meta[tid] = meta;
+            if (kGroup) s_meta[tid] = meta;
             s_le[tid] = le;
             s_row[tid] = row;
         }
-        __syncthreads();
+        __syncthreads();  // the destinations are in place, hist has been read
         if (kGroup) MCEP_TRACE(0, 7);  // the owners' answers are in, rows can go
+        if (kCount && tid < ne && e >= 0) atomicAdd(&hist[e], 1);
         // A repeated expert in a token's list was sent once; combine still adds
         // that row once per listing (mooncake_ep_kernel.cu:734-742 reads the
         // (expert, token) slot for every k), so the repeat records the same row.
-        if (tid < v.K && v.rowmap != nullptr && s_exp[tid] < 0 && s_raw[tid] >= 0) {
-            for (int kk = 0; kk < tid; ++kk)
-                if (s_exp[kk] == s_raw[tid]) v.rowmap[(size_t)t * v.K + tid] = s_row[kk];
-        }
+        if (tid < ne && e < 0 && raw >= 0)
+            for (int j = tok0; j < tid; ++j)
+                if (s_exp[j] == raw) v.rowmap[(size_t)t0 * K + tid] = s_row[j];
 
-        for (int tile = warp; tile < ntiles; tile += nwarps) {
-            const int c = tile * 32 + lane;
+        if (warp >= items && t1 < v.T) ahead = load_item(t1, warp);
+        for (int item = warp; item < items; item += nwarps) {
+            const V32 cur = ahead;
+            ahead = item + nwarps < items ? load_item(t0, item + nwarps) : load_item(t1, warp);
+            const int tok = item / ntiles, tile = item - tok * ntiles;
+            const int c = tile * 32 + lane, k0 = tok * K;
             const bool act = c < nchunks;
-            V32 cur = first;
-            if (tile != warp) {
-                cur = V32{};
-                if (act) cur = ld32_readonly(xrow + (size_t)c * 32);
-            }
             if (kFP8) {
                 float sinv;
                 const uint4 q = quantize16(cur, sinv);
@@ -806,77 +855,67 @@ __device__ __forceinline__ void send_tokens(const SendView& v, int first_token, 
                     sc.w = __shfl_sync(kFull, sinv, 24);
                 }
 #pragma unroll 4
-                for (int k = 0; k < v.K; ++k) {
+                for (int k = k0; k < k0 + K; ++k) {
                     char* d = s_dst[k];
                     if (d == nullptr) continue;
                     if (act) st16(d + (size_t)c * 16, q);
                     char* m = kGroup ? s_meta[k] : nullptr;
                     if (m != nullptr) {
                         if (lane == 0)
-                            st16(m + kMetaHeaderBytes + (size_t)tile * 16,
-                                 *reinterpret_cast<uint4*>(&sc));
+                            st16(m + kMetaHeaderBytes + (size_t)tile * 16, *reinterpret_cast<uint4*>(&sc));
                     } else if (act && (lane & 7) == 0) {
                         v.recv_scales[((size_t)s_le[k] * S + (c >> 3)) * v.RM + s_row[k]] = sinv;
                     }
                 }
             } else {
 #pragma unroll 4
-                for (int k = 0; k < v.K; ++k) {
+                for (int k = k0; k < k0 + K; ++k) {
                     char* d = s_dst[k];
                     if (d == nullptr || !act) continue;
                     st32(d + (size_t)c * 32, cur);
                 }
             }
         }
-        if (tid < v.K && s_dst[tid] != nullptr) {
+        if (tid < ne && s_dst[tid] != nullptr) {
+            const int t = t0 + tid / K;
             if (kGroup && s_meta[tid] != nullptr)
                 st16(s_meta[tid], make_uint4((uint32_t)t, 0u, 0u, 0u));
             else
                 v.recv_src_info[(size_t)s_le[tid] * v.RM + s_row[tid]] = t;
         }
-        __syncthreads();
+        counted = t0 + nt;
+        if (kCount || t1 < v.T) __syncthreads();  // done with the tables of this batch; hist is complete
+        if (!kGroup && kCount && counted == v.T)
+            for (int x = tid; x < v.E; x += nthr) {
+                const int n = hist[x];
+                v.recv_count[x] = n;
+                v.layout_range[x] = n;  // begin 0 | count
+            }
+        t0 = t1;
     }
 }
 
 // =============================================================================
 // single rank: dispatch writes the packed outputs directly
 // =============================================================================
-template <bool kFP8, bool kFused>
-__global__ void __launch_bounds__(512) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
-    extern __shared__ int smem_i32[];
-    int* hist = smem_i32;        // [E] whole-batch counts (fused)
-    int* kmap = smem_i32 + p.E;  // [E] expert -> k of this block's token (fused)
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    pdl_wait();
+// Bound by HBM for large batches (4096 tokens, hidden 7168, top-8, bf16: 529 MB)
+// and by latency for decode (index load -> count -> row stores, one batch per block).
+// Behind a layout kernel the registers are held to 40, so that three blocks of 14
+// warps fit an SM and one block's loads hide behind the stores of the others.
+template <bool kFP8, bool kCount>
+__global__ void __launch_bounds__(512, kCount ? 2 : 3) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
+    extern __shared__ int smem_i32[];  // [E] (kCount)
+    // behind a layout kernel the rows are requested before the wait
+    if (kCount) pdl_wait();
     pdl_launch_dependents();
-    if (kFused)
-        for (int e = tid; e < p.E; e += nthr) hist[e] = 0, kmap[e] = -1;
-    // (the token loop has a barrier before the first use of these tables; a
-    // block without tokens only reads hist after the barrier below)
     SendView v = {};
     v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx, v.slot = p.slot;
     v.T = p.T, v.K = p.K, v.E = p.E, v.R = 1, v.M = p.M, v.H = p.H, v.rank = 0;
-    v.L = p.E, v.RM = p.M, v.status = p.status;
+    v.L = p.E, v.RM = p.M, v.C = p.C, v.status = p.status;
     v.recv_x = reinterpret_cast<char*>(p.recv_x), v.recv_scales = p.recv_scales;
     v.recv_src_info = p.recv_src_info, v.row_bytes = p.H * (kFP8 ? 1 : 2);
-    v.rowmap = p.rowmap;
-    send_tokens<kFP8, false, kFused>(v, blockIdx.x, gridDim.x, hist, kmap);
-    if (kFused) {
-        // the receive layout of a single rank, spread over the grid. A block
-        // without a token has not scanned: it has nothing to add (its share of
-        // the experts is written by... itself, so it scans now).
-        if ((int)blockIdx.x >= p.T) {
-            __syncthreads();
-            const int none[kScanAhead] = {-1, -1, -1, -1};
-            scan_index_matrix<true, false>(p.topk_idx, p.T, p.K, p.E, hist, kmap, nullptr, -1, none);
-            __syncthreads();
-        }
-        for (int e = blockIdx.x * nthr + tid; e < p.E; e += gridDim.x * nthr) {
-            const int c = hist[e];
-            p.recv_count[e] = c;
-            p.layout_range[e] = c;  // begin 0 | count
-        }
-    }
+    v.rowmap = p.rowmap, v.recv_count = p.recv_count, v.layout_range = p.layout_range;
+    send_tokens<kFP8, false, kCount>(v, blockIdx.x, gridDim.x, smem_i32, [] { pdl_wait(); });
 }
 
 // Single rank: rowmap[t][k] = packed row of (token t, expert topk[t][k]) as the
@@ -1037,36 +1076,24 @@ __device__ __forceinline__ void load_peer_tables(void* const* peer_base, const i
 //  3. fix the receive layout (source-rank order), write `layout_range` and
 //     `recv_count`, leave the verdicts for the receive duty, and answer every
 //     source with the first row of its segment in each of this rank's experts.
-template <bool kFused>
+template <bool kCount>
 __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, int* smem_i32,
-                                                 char* const* s_peer, const int* s_active,
-                                                 int (&e)[kMaxTopk]) {
+                                                 char* const* s_peer, const int* s_active) {
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int L = p.E / p.R, n = L * p.R;
-    int* hist = smem_i32;                       // [E] (fused)
-    int* s_cnt = smem_i32 + (kFused ? p.E : 0);  // [L*R]
+    int* hist = smem_i32;         // [E]
+    int* s_cnt = smem_i32 + p.E;  // [L*R]
     MCEP_TRACE(0, 1);
-    if (kFused) {
-        // one lane per token: its choices arrive in one memory round trip
-        // (small batches: T <= 2 x the number of SMs, so one pass)
-        // (the caller requested this thread's token before the peer tables)
+    if (kCount) {
         for (int i = tid; i < p.E; i += nthr) hist[i] = 0;
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kMaxTopk; ++k)
-            if (e[k] >= 0) atomicAdd(&hist[e[k]], 1);
-        for (int t = tid + nthr; t < p.T; t += nthr) {
-            load_token_choices(p.topk_idx, t, p.T, p.K, p.E, e);
-#pragma unroll
-            for (int k = 0; k < kMaxTopk; ++k)
-                if (e[k] >= 0) atomicAdd(&hist[e[k]], 1);
-        }
+        count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), hist);
         __syncthreads();
     }
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
         if (!s_active[dr]) continue;
-        const int c = kFused ? hist[x] : __ldg(p.count + x);
+        const int c = kCount ? hist[x] : __ldg(p.count + x);
         uint64_t* wd = reinterpret_cast<uint64_t*>(s_peer[dr] + p.w.cnt_off) + (p.rank * L + (x - dr * L));
         st_relaxed_sys(wd, ((uint64_t)p.seq << 32) | (uint32_t)(c + 1));
     }
@@ -1247,7 +1274,7 @@ constexpr int kRecvHelpers = 64;
 // kPhases: 1 = control + send; 3 = control + send + receive duty (one launch).
 // `bid` of `nblocks`: the block's place in its rank's share of the grid (the
 // whole grid, except for in-process groups where one launch carries all ranks).
-template <bool kFP8, bool kFused, int kPhases>
+template <bool kFP8, bool kCount, int kPhases>
 __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int bid, int nblocks,
                                               int* smem_i32) {
     __shared__ char* s_peer[kMaxRanks];
@@ -1257,16 +1284,11 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     const int nsend = nblocks - 1;
     const int nh = nsend < kRecvHelpers ? nsend : kRecvHelpers;
     MCEP_TRACE(0, 0);
-    // the control block counts with one lane per token: its token's choices are
-    // requested first, so they travel while the peer tables are read
-    int ctl_choices[kMaxTopk];
-    if (kFused && bid == 0) request_token_choices(p.topk_idx, tid, p.T, p.K, p.E, ctl_choices);
     load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);
-    if (kFused && bid == 0) drop_repeated_choices(ctl_choices);
 
     if (bid == 0) {
         __syncthreads();
-        dispatch_control<kFused>(p, smem_i32, s_peer, s_active, ctl_choices);
+        dispatch_control<kCount>(p, smem_i32, s_peer, s_active);
         if (kPhases == 3) {
             __syncthreads();
             dispatch_recv_duty<kFP8>(p, nh, nh + 1, smem_i32);
@@ -1274,22 +1296,18 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
         return;
     }
 
-    int* kmap = smem_i32;  // [E] (fused)
-    if (kFused)
-        for (int e = tid; e < p.E; e += nthr) kmap[e] = -1;
     const int sid = bid - 1;
-    // (the token loop has barriers of its own before it reads the tables above;
-    // a block without tokens reads them only after the barrier below)
+    __syncthreads();  // the tables above are in place
     SendView v = {};
     v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx, v.slot = p.slot;
     v.T = p.T, v.K = p.K, v.E = p.E, v.R = p.R, v.M = p.M, v.H = p.H, v.rank = p.rank;
-    v.L = p.E / p.R, v.RM = p.R * p.M, v.status = p.wait.status;
+    v.L = p.E / p.R, v.RM = p.R * p.M, v.C = p.C, v.status = p.wait.status;
     v.recv_x = reinterpret_cast<char*>(p.recv_x), v.recv_scales = p.recv_scales;
     v.recv_src_info = p.recv_src_info, v.row_bytes = p.row_bytes;
     v.beg = reinterpret_cast<const uint64_t*>(p.local_base + p.w.beg_off);
     v.seq = p.seq, v.wait = scaled(p.wait, 2), v.rx_off = p.rx_off, v.meta_off = p.meta_off;
     v.meta_stride = p.meta_stride, v.rowmap = p.rowmap, v.s_peer = s_peer, v.s_active = s_active;
-    send_tokens<kFP8, true, kFused>(v, sid, nsend, nullptr, kmap);
+    send_tokens<kFP8, true, kCount>(v, sid, nsend, smem_i32, [] {});
     MCEP_TRACE(0, 5);  // all rows of this block are issued
 
     // Completion. Rows are not fenced one by one: the block issues ONE
@@ -1299,7 +1317,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     // rows are performed system-wide - and tells every peer with one word.
     __syncthreads();
     if (tid == 0) {
-        if (sid < p.T) __threadfence_system();
+        if (sid * p.C < p.T) __threadfence_system();
         s_ticket = (int)atomicAdd(p.ticket, 1u);
     }
     __syncthreads();
@@ -1352,20 +1370,20 @@ __global__ void __launch_bounds__(kMaxRanks) ep_barrier_kernel(BarrierParams p) 
     }
 }
 
-template <bool kFP8, bool kFused, int kPhases>
-__global__ void __launch_bounds__(512) ep_dispatch_kernel(GroupDispatchParams p) {
+template <bool kFP8, bool kCount, int kPhases>
+__global__ void __launch_bounds__(512, 2) ep_dispatch_kernel(GroupDispatchParams p) {
     extern __shared__ int smem_i32[];
     pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
-    dispatch_body<kFP8, kFused, kPhases>(p, blockIdx.x, gridDim.x, smem_i32);
+    dispatch_body<kFP8, kCount, kPhases>(p, blockIdx.x, gridDim.x, smem_i32);
 }
 
 // In-process groups (several logical ranks on one GPU): the ranks' kernels wait
 // for one another, so they cannot be separate launches - nothing would
 // guarantee that they run at the same time. ONE cooperative launch carries all
 // ranks: consecutive runs of `per_rank` blocks do the work of one rank each.
-template <bool kFP8, bool kFused, int kPhases>
+template <bool kFP8, bool kCount, int kPhases>
 __global__ void __launch_bounds__(512)
     ep_dispatch_multi_kernel(const GroupDispatchParams* ps, int per_rank) {
     extern __shared__ int smem_i32[];
@@ -1373,7 +1391,7 @@ __global__ void __launch_bounds__(512)
     const int which = blockIdx.x / per_rank;
     if (threadIdx.x == 0) s_p = ps[which];
     __syncthreads();
-    dispatch_body<kFP8, kFused, kPhases>(s_p, blockIdx.x - which * per_rank, per_rank, smem_i32);
+    dispatch_body<kFP8, kCount, kPhases>(s_p, blockIdx.x - which * per_rank, per_rank, smem_i32);
 }
 
 template <bool kFP8>
@@ -1617,6 +1635,23 @@ using namespace kernels;
 // =============================================================================
 // launchers
 // =============================================================================
+// Kernels are allowed more than 48 KB of dynamic shared memory once per device.
+template <typename K>
+static cudaError_t allow_smem(K kernel, size_t smem) {
+    if (smem <= 40 * 1024) return cudaSuccess;
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& have = allowed[std::make_pair(reinterpret_cast<const void*>(kernel), dev)];
+    if (smem <= have) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) have = smem;
+    return e;
+}
+
 // The chunked route: chunks of up to 256 tokens (fewer when the per-chunk bitmap
 // of all experts would not fit 48 KB of shared memory), at most 128 chunks, and
 // per-chunk histograms that fit the scratch the caller gave.
@@ -1632,7 +1667,36 @@ static bool layout_chunking(const LayoutParams& p, int* chunk_tokens, int* words
     return true;
 }
 
+// Threads per block of the cluster route with clusters of `blocks`: a multiple of
+// 32, one lane per token; 0 when the tables of E experts do not fit shared memory
+// or the batch is too large.
+static int layout_cluster_threads(const LayoutParams& p, int blocks) {
+    if (p.rank_count != nullptr || p.expert_prefix != nullptr) return 0;
+    const int threads = ((p.T + blocks - 1) / blocks + 31) / 32 * 32;
+    if (threads < 32 || threads > 1024) return 0;
+    return (size_t)p.E * (threads / 16 + 2) * sizeof(int) <= 160 * 1024 ? threads : 0;
+}
+
 cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
+    // Sixteen blocks (opt-in cluster size) once eight would have more than 8 warps
+    // each: setting the bits is bound by the shared-memory atomics of a block.
+    static std::atomic<int> large{1};  // 0: the device does not take clusters of 16
+    for (int blocks : {kLayoutClusterLarge, kLayoutCluster}) {
+        if (blocks == kLayoutClusterLarge && (p.T <= kLayoutCluster * 256 || !large.load())) continue;
+        const int threads = layout_cluster_threads(p, blocks);
+        if (threads == 0) continue;
+        const size_t smem = (size_t)p.E * (threads / 16 + 2) * sizeof(int);
+        if (cudaError_t e = allow_smem(ep_layout_cluster_kernel, smem)) return e;
+        if (blocks == kLayoutClusterLarge) {
+            cudaError_t e = cudaFuncSetAttribute(ep_layout_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+        }
+        const cudaError_t e = launch_clusters("ep_layout_cluster", ep_layout_cluster_kernel, dim3(blocks), dim3(threads),
+                                              smem, blocks, ctx, p);
+        if (e == cudaSuccess || blocks == kLayoutCluster) return e;
+        cudaGetLastError();
+        large.store(0);
+    }
     int chunk_tokens = 0, cwords = 0, chunks = 0;
     if (layout_chunking(p, &chunk_tokens, &cwords, &chunks)) {
         cudaError_t e = launch("ep_layout_hist", ep_layout_hist_kernel, dim3(chunks),
@@ -1669,25 +1733,47 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
                   ctx, p, epc, words);
 }
 
-bool can_fuse_layout(int T, int K, int E, int num_sms) {
-    // one block per token, all resident at once even at two blocks per SM, an
-    // index matrix small enough to be scanned by every block, and expert tables
-    // that fit the static shared-memory budget
-    return (long long)T * K <= 4096 && T <= num_sms * 2 && E <= 2048;
+bool counts_in_send_kernel(int T, int num_sms) {
+    // at most two blocks per SM, a token each: each counts the tokens ahead of its
+    // own (up to 0.8 us) in less time than a layout kernel takes
+    return T <= 2 * num_sms;
 }
 
-cudaError_t launch_direct_dispatch(const DirectDispatchParams& p, const LaunchCtx& ctx) {
-    const int threads = block_threads(p.H);
-    const size_t smem = (size_t)(p.fused ? 2 * p.E : 0) * sizeof(int);
+// Tokens per batch and threads per block of the send kernels. Small batches get
+// one block per token (every SM has one or two). Beyond that a batch has enough
+// rows to give every warp of a 14 - 16 warp block one 512-channel tile: rows of 14
+// tiles (hidden 7168) go one by one, rows of 4 tiles in fours.
+static SendShape send_shape(int T, int K, int H, int num_sms, int min_threads) {
+    const int ntiles = (H + kTileChannels - 1) / kTileChannels;
+    SendShape s;
+    s.tokens = 1;
+    if (!counts_in_send_kernel(T, num_sms)) {
+        int c = ntiles >= 16 ? 1 : 16 / ntiles;
+        if (c > 8) c = 8;
+        if (c > kBatchEntries / K) c = kBatchEntries / K;
+        const int most = (T + 2 * num_sms - 1) / (2 * num_sms);
+        s.tokens = c < most ? c : most;
+    }
+    int warps = s.tokens * ntiles;
+    if (warps > 16) warps = 16;
+    if (warps < 4) warps = 4;
+    s.threads = warps * 32 < min_threads ? min_threads : warps * 32;
+    return s;
+}
+
+cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 128);
+    p.C = s.tokens;
+    const size_t smem = p.slot == nullptr ? (size_t)p.E * sizeof(int) : 0;
     void (*k)(DirectDispatchParams) = nullptr;
-    switch ((p.use_fp8 ? 2 : 0) | (p.fused ? 1 : 0)) {
+    switch ((p.use_fp8 ? 2 : 0) | (p.slot == nullptr ? 1 : 0)) {
         case 0: k = ep_dispatch_send_direct_kernel<false, false>; break;
         case 1: k = ep_dispatch_send_direct_kernel<false, true>; break;
         case 2: k = ep_dispatch_send_direct_kernel<true, false>; break;
         default: k = ep_dispatch_send_direct_kernel<true, true>; break;
     }
-    const int grid = p.fused ? (p.T > 0 ? p.T : 1) : persistent_grid(p.T, k, threads, smem, ctx);
-    return launch("ep_dispatch_send_direct", k, dim3(grid), dim3(threads), smem, ctx, p);
+    const int grid = p.T > 0 ? (p.T + p.C - 1) / p.C : 1;
+    return launch("ep_dispatch_send_direct", k, dim3(grid), dim3(s.threads), smem, ctx, p);
 }
 
 cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx& ctx) {
@@ -1714,56 +1800,44 @@ namespace {
 using DispatchKernel = void (*)(GroupDispatchParams);
 
 template <int kPhases>
-DispatchKernel pick_dispatch(bool fp8, bool fused) {
-    switch ((fp8 ? 2 : 0) | (fused ? 1 : 0)) {
-        case 0: return ep_dispatch_kernel<false, false, kPhases>;
-        case 1: return ep_dispatch_kernel<false, true, kPhases>;
-        case 2: return ep_dispatch_kernel<true, false, kPhases>;
-        default: return ep_dispatch_kernel<true, true, kPhases>;
-    }
+DispatchKernel pick_dispatch(bool fp8, bool counting) {
+    if (counting) return fp8 ? ep_dispatch_kernel<true, true, kPhases> : ep_dispatch_kernel<false, true, kPhases>;
+    return fp8 ? ep_dispatch_kernel<true, false, kPhases> : ep_dispatch_kernel<false, false, kPhases>;
 }
 
-size_t dispatch_smem(const GroupDispatchParams& p, bool with_recv) {
-    const size_t n = (size_t)p.E;  // L * R
-    const size_t control = (size_t)(p.fused ? p.E : 0) + 2 * n;
-    const size_t sender = p.fused ? (size_t)p.E : 0;
-    const size_t recv = with_recv ? 2 * n + 1 : 0;
-    size_t m = control > sender ? control : sender;
-    if (recv > m) m = recv;
-    return m * sizeof(int);
-}
+// the control block keeps two tables of E entries, a sender one, the receive duty two and a total
+size_t dispatch_smem(const GroupDispatchParams& p) { return (size_t)(2 * p.E + 1) * sizeof(int); }
 
 }  // namespace
 
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms) {
     // a small batch: one block per token plus the control block (the launcher
     // falls back to two launches when that many blocks are not resident at once)
-    return can_fuse_layout(T, K, E, num_sms) && T + 1 <= 2 * num_sms;
+    return (long long)T * K <= 4096 && E <= 2048 && T + 1 <= 2 * num_sms;
 }
 
-cudaError_t launch_group_dispatch(const GroupDispatchParams& p, const LaunchCtx& ctx) {
-    const int threads = block_threads(p.H, 256);
-    const size_t smem = dispatch_smem(p, true);
-    auto k = pick_dispatch<3>(p.use_fp8 != 0, true);
+cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 256);
+    p.C = s.tokens;
+    const size_t smem = dispatch_smem(p);
+    auto k = pick_dispatch<3>(p.use_fp8 != 0, p.slot == nullptr);
     const int grid = 1 + (p.T > 0 ? p.T : 1);
-    if (grid > resident_blocks(k, threads, smem, ctx)) return cudaErrorInvalidConfiguration;
-    return launch("ep_dispatch", k, dim3(grid), dim3(threads), smem, ctx, p);
+    if (p.C != 1 || grid > resident_blocks(k, s.threads, smem, ctx)) return cudaErrorInvalidConfiguration;
+    return launch("ep_dispatch", k, dim3(grid), dim3(s.threads), smem, ctx, p);
 }
 
-cudaError_t launch_group_dispatch_send(const GroupDispatchParams& p, const LaunchCtx& ctx) {
-    const int threads = block_threads(p.H, 256);
-    const size_t smem = dispatch_smem(p, false);
-    auto k = pick_dispatch<1>(p.use_fp8 != 0, p.fused != 0);
-    // the control block, then one block per token (fused) or a resident wave
-    int senders;
-    if (p.fused) {
-        senders = p.T > 0 ? p.T : 1;
-    } else {
-        long long cap = resident_blocks(k, threads, smem, ctx) - 1;
-        if (cap < 1) cap = 1;
-        senders = (int)(p.T < cap ? (p.T > 0 ? p.T : 1) : cap);
-    }
-    return launch("ep_dispatch_send", k, dim3(1 + senders), dim3(threads), smem, ctx, p);
+cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& ctx) {
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 256);
+    p.C = s.tokens;
+    const size_t smem = dispatch_smem(p);
+    auto k = pick_dispatch<1>(p.use_fp8 != 0, p.slot == nullptr);
+    // the control block, then one block per token (small batches) or a resident wave
+    // (a wave, not a block per batch: every block ends with a system-scope fence)
+    long long cap = resident_blocks(k, s.threads, smem, ctx) - 1;
+    if (cap < 1) cap = 1;
+    const int batches = p.T > 0 ? (p.T + p.C - 1) / p.C : 1;
+    const int senders = (int)(batches < cap ? batches : cap);
+    return launch("ep_dispatch_send", k, dim3(1 + senders), dim3(s.threads), smem, ctx, p);
 }
 
 cudaError_t launch_group_dispatch_recv(const GroupDispatchParams& p, const LaunchCtx& ctx) {
@@ -1851,35 +1925,33 @@ cudaError_t launch_cooperative(const char* name, void (*kernel)(KArgs...), int g
 using DispatchMultiKernel = void (*)(const GroupDispatchParams*, int);
 
 template <int kPhases>
-DispatchMultiKernel pick_dispatch_multi(bool fp8, bool fused) {
-    switch ((fp8 ? 2 : 0) | (fused ? 1 : 0)) {
-        case 0: return ep_dispatch_multi_kernel<false, false, kPhases>;
-        case 1: return ep_dispatch_multi_kernel<false, true, kPhases>;
-        case 2: return ep_dispatch_multi_kernel<true, false, kPhases>;
-        default: return ep_dispatch_multi_kernel<true, true, kPhases>;
-    }
+DispatchMultiKernel pick_dispatch_multi(bool fp8, bool counting) {
+    if (counting)
+        return fp8 ? ep_dispatch_multi_kernel<true, true, kPhases> : ep_dispatch_multi_kernel<false, true, kPhases>;
+    return fp8 ? ep_dispatch_multi_kernel<true, false, kPhases> : ep_dispatch_multi_kernel<false, false, kPhases>;
 }
 
 }  // namespace
 
-cudaError_t launch_group_dispatch_multi(const GroupDispatchParams* params, int n,
+cudaError_t launch_group_dispatch_multi(GroupDispatchParams* params, int n,
                                         GroupDispatchParams* dev_params, int phases,
                                         const LaunchCtx& ctx) {
     if (n < 1) return cudaSuccess;
     int want = 2;
     size_t smem = 0;
     for (int i = 0; i < n; ++i) {
-        if (params[i].use_fp8 != params[0].use_fp8 || params[i].fused != params[0].fused ||
-            params[i].H != params[0].H)
+        if (params[i].use_fp8 != params[0].use_fp8 || params[i].H != params[0].H ||
+            (params[i].slot == nullptr) != (params[0].slot == nullptr))
             return cudaErrorInvalidValue;
+        params[i].C = 1;
         const int blocks = 1 + (params[i].T > 0 ? params[i].T : 1);
         if (blocks > want) want = blocks;
-        const size_t sm = dispatch_smem(params[i], phases == 3);
+        const size_t sm = (size_t)(2 * params[i].E + 4) * sizeof(int);
         if (sm > smem) smem = sm;
     }
     const int threads = block_threads(params[0].H, 256);
-    auto k = phases == 3 ? pick_dispatch_multi<3>(params[0].use_fp8 != 0, params[0].fused != 0)
-                         : pick_dispatch_multi<1>(params[0].use_fp8 != 0, params[0].fused != 0);
+    const bool fp8 = params[0].use_fp8 != 0, counting = params[0].slot == nullptr;
+    auto k = phases == 3 ? pick_dispatch_multi<3>(fp8, counting) : pick_dispatch_multi<1>(fp8, counting);
     const long long cap = resident_blocks(k, threads, smem, ctx) / n;
     if (cap < 2) return cudaErrorInvalidConfiguration;
     const int per_rank = (int)(want < cap ? want : cap);

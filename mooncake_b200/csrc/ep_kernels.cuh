@@ -50,22 +50,25 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx);
 struct DirectDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
-    const int32_t* slot;        // [T*K] from the layout kernel (not fused)
-    const int32_t* count;       // [E]   from the layout kernel (not fused)
+    const int32_t* slot;        // [T*K] from the layout kernel, or null: counted in the send kernel
     int T, K, E, M, H;
     int use_fp8;
-    int fused;                  // count the slots here (slot/count unused) - small batches
+    int C;                      // tokens per batch (set by the launcher)
     int32_t* status;
     void* recv_x;
     float* recv_scales;
     int32_t* recv_src_info;
-    int32_t* recv_count;        // fused: [E]
-    int64_t* layout_range;      // fused: [E]
+    int32_t* recv_count;        // [E], written without `slot`
+    int64_t* layout_range;      // [E], written without `slot`
     int32_t* rowmap;            // [T*K] row of (token, k) inside its expert, kept for combine
 };
-// whether a send kernel may count the slots itself for this problem size
-bool can_fuse_layout(int T, int K, int E, int num_sms);
-cudaError_t launch_direct_dispatch(const DirectDispatchParams& p, const LaunchCtx& ctx);
+// whether the send kernels count the slots themselves for this many tokens
+bool counts_in_send_kernel(int T, int num_sms);
+cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
+
+struct SendShape {
+    int tokens, threads;  // tokens per batch, threads per block
+};
 
 // Single rank: (token, k) -> packed row, inverted from the handle.
 struct CombineInvertParams {
@@ -119,13 +122,13 @@ struct WaitCfg {
 struct GroupDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
-    const int32_t* slot;        // [T*K] from the layout kernel (not fused)
-    const int32_t* count;       // [E]   from the layout kernel (not fused)
+    const int32_t* slot;        // [T*K] and
+    const int32_t* count;       // [E] from the layout kernel, or null: counted in the send kernel
     void* const* peer_base;     // [R] base of every rank's symmetric buffer
     char* local_base;           // this rank's
     int T, K, E, R, M, H, rank;
     int use_fp8;
-    int fused;
+    int C;                      // tokens per batch (set by the launcher)
     Words w;
     size_t rx_off;              // packed receive rows [L][R*M][row_bytes] of this parity
     size_t meta_off;            // side messages [L][R*M][meta_stride] of this parity
@@ -148,9 +151,9 @@ struct GroupDispatchParams {
 };
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms);
 // one launch: control + send + receive duties
-cudaError_t launch_group_dispatch(const GroupDispatchParams& p, const LaunchCtx& ctx);
+cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx);
 // two launches (hook mode, large batches, caller-owned recv_x)
-cudaError_t launch_group_dispatch_send(const GroupDispatchParams& p, const LaunchCtx& ctx);
+cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& ctx);
 cudaError_t launch_group_dispatch_recv(const GroupDispatchParams& p, const LaunchCtx& ctx);
 
 // Combine in a group: expert outputs are made readable in symmetric memory
@@ -184,8 +187,8 @@ cudaError_t launch_group_combine_reduce(const GroupCombineParams& p, const Launc
 // (phases = 1) or the whole call (phases = 3) of `n` ranks as ONE cooperative
 // launch, because kernels that wait for one another must not be separate
 // launches on one GPU. `dev_params` is device memory for `n` parameter blocks.
-// All ranks must agree on payload type, hidden size and `fused`.
-cudaError_t launch_group_dispatch_multi(const GroupDispatchParams* params, int n,
+// All ranks must agree on payload type and hidden size.
+cudaError_t launch_group_dispatch_multi(GroupDispatchParams* params, int n,
                                         GroupDispatchParams* dev_params, int phases,
                                         const LaunchCtx& ctx);
 cudaError_t launch_group_combine_multi(const GroupCombineParams* params, int n,

@@ -1,0 +1,106 @@
+// Reading and counting the index matrix on the device: helpers of the dispatch
+// and layout kernels.
+//
+// Receive order is token order, so the position of a token among the tokens that
+// chose an expert is the number of EARLIER tokens that chose it. For small
+// batches every block of a dispatch kernel counts them itself (count_tokens: one
+// lane per token, shared-memory counters); a warp's 32 counter updates take about
+// 21 cycles, so 296 tokens of 8 choices take 0.8 us, 4096 tokens would take 12 us
+// in every block - larger batches have a layout kernel count once for all.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "ep_kernels.cuh"
+
+namespace mcep {
+
+// The K choices of token t: e[k] = -1 for masked and out-of-range entries (and
+// for k >= K). `vec`: K is even and the matrix 16-byte aligned, two choices per load.
+template <int KB>
+__device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_idx, int t, int K, int E,
+                                             bool vec, int (&e)[KB]) {
+    const int64_t* p = topk_idx + (size_t)t * K;
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < KB; k += 2) {
+            longlong2 v = make_longlong2(-1, -1);
+            if (k < K) v = __ldg(reinterpret_cast<const longlong2*>(p + k));
+            e[k] = (int)v.x, e[k + 1] = (int)v.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < KB; ++k) e[k] = k < K ? (int)__ldg(p + k) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < KB; ++k)
+        if (e[k] >= E) e[k] = -1;  // (negative already means "no expert")
+}
+
+// An expert listed twice by one token counts once: at its first listing, or at
+// its last one (the elastic calls).
+template <int KB, bool kKeepLast>
+__device__ __forceinline__ void drop_repeats(int (&e)[KB]) {
+    if (kKeepLast) {
+#pragma unroll
+        for (int k = 0; k < KB - 1; ++k) {
+            bool dup = false;
+#pragma unroll
+            for (int kk = k + 1; kk < KB; ++kk) dup |= (e[kk] == e[k]);
+            if (dup) e[k] = -1;
+        }
+    } else {
+#pragma unroll
+        for (int k = KB - 1; k > 0; --k) {
+            bool dup = false;
+#pragma unroll
+            for (int kk = 0; kk < k; ++kk) dup |= (e[kk] == e[k]);
+            if (dup) e[k] = -1;
+        }
+    }
+}
+
+// Adds tokens [from, to) to hist[E] (shared memory); all threads of the block
+// share the work, nobody waits. kTokens tokens per lane are requested together.
+template <int KB, int kTokens, bool kKeepLast>
+__device__ __forceinline__ void count_tokens_of(const int64_t* __restrict__ topk_idx, int from, int to, int K,
+                                                int E, bool vec, int* hist) {
+    const int nthr = blockDim.x;
+    for (int t0 = from + threadIdx.x; t0 < to; t0 += nthr * kTokens) {
+        int e[kTokens][KB];
+#pragma unroll
+        for (int u = 0; u < kTokens; ++u) {
+            if (t0 + u * nthr < to) {
+                load_choices<KB>(topk_idx, t0 + u * nthr, K, E, vec, e[u]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < KB; ++k) e[u][k] = -1;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kTokens; ++u) {
+            drop_repeats<KB, kKeepLast>(e[u]);
+#pragma unroll
+            for (int k = 0; k < KB; ++k)
+                if (e[u][k] >= 0) atomicAdd(&hist[e[u][k]], 1);
+        }
+    }
+}
+
+template <int kTokens, bool kKeepLast = false>
+__device__ __forceinline__ void count_tokens(const int64_t* __restrict__ topk_idx, int from, int to, int K, int E,
+                                             bool vec, int* hist) {
+    if (K <= 4)
+        count_tokens_of<4, kTokens, kKeepLast>(topk_idx, from, to, K, E, vec, hist);
+    else if (K <= 8)
+        count_tokens_of<8, kTokens, kKeepLast>(topk_idx, from, to, K, E, vec, hist);
+    else
+        count_tokens_of<16, 1, kKeepLast>(topk_idx, from, to, K, E, vec, hist);
+}
+
+__device__ __forceinline__ bool choices_in_pairs(const int64_t* topk_idx, int K) {
+    return K % 2 == 0 && (reinterpret_cast<uintptr_t>(topk_idx) & 15) == 0;
+}
+
+}  // namespace mcep

@@ -248,7 +248,6 @@ struct mcep_buffer {
     bool all_peers = false;
     bool force_staged = false;
     bool pdl = true;
-    bool fuse_layout = true;
     bool one_kernel = true;
     int64_t hard_timeout_ns = 10ll * 1000 * 1000 * 1000;
     char* base = nullptr;            // symmetric allocation: header region + data area
@@ -291,7 +290,6 @@ struct mcep_buffer {
         mcep::GroupCombineParams c;
     } pending;
     std::function<int()> after_deferred;  // run once the prepared dispatch has been launched
-    bool chain_first_once = false;        // see allow_chained_first_launch
 
     // what combine needs to know about the dispatch call a handle came from
     struct DispatchRecord {
@@ -387,8 +385,6 @@ size_t exchange_bytes(int num_ranks, int num_experts, int M, int hidden) {
 }
 
 void set_after_deferred(mcep_buffer* b, std::function<int()> fn) { b->after_deferred = std::move(fn); }
-
-void allow_chained_first_launch(mcep_buffer* b) { b->chain_first_once = true; }
 
 int report_failure(int code, const char* message) { return fail(code, "%s", message); }
 
@@ -770,7 +766,7 @@ int mcep_buffer_set_option(mcep_buffer* b, const char* name, int64_t value) {
     } else if (!std::strcmp(name, "pdl")) {
         b->pdl = value != 0;
     } else if (!std::strcmp(name, "fuse_layout")) {
-        b->fuse_layout = value != 0;
+        // where the layout is counted follows from the batch size alone
     } else if (!std::strcmp(name, "one_kernel")) {
         b->one_kernel = value != 0;
     } else if (!std::strcmp(name, "defer_launch")) {
@@ -913,13 +909,14 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
         if (int rc = order_after(stream, compute, b->ev_a)) return rc;
 
     const bool pdl = chain_with_pdl(b, stream) && (stream == compute || chain_with_pdl(b, compute));
-    const bool chain_first = b->chain_first_once && pdl && !b->defer;
-    b->chain_first_once = false;
-    mcep::LaunchCtx first{stream, b->num_sms, chain_first};
-    mcep::LaunchCtx next{stream, b->num_sms, pdl};
+    // The first kernel of a call, too, is launched with programmatic stream
+    // serialisation: it waits for everything ahead of it at its top, but its blocks
+    // are in place by then (1 - 2 us of launch latency per call).
+    mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
-    const bool fused = mcep::can_fuse_layout(T, K, E, b->num_sms) && b->fuse_layout;
-    if (!fused) {
+    // Batches of more than two tokens per SM get their layout from a kernel of its own.
+    const bool counting = mcep::counts_in_send_kernel(T, b->num_sms);
+    if (!counting) {
         mcep::LayoutParams lp = {};
         lp.topk_idx = a->topk_idx;
         lp.T = T, lp.K = K, lp.E = E, lp.R = R;
@@ -930,21 +927,23 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
             lp.layout_range = a->packed_recv_layout_range;
         }
         MCEP_CUDA(mcep::launch_layout(lp, first));
+        first.pdl = pdl;  // what follows is chained to the layout kernel
     }
+    const int32_t* slot = counting ? nullptr : sc.slot;
 
     if (!group) {
         // a single rank: the packed outputs are written directly, no words, no waits
         mcep::DirectDispatchParams dp = {};
-        dp.x = a->x, dp.topk_idx = a->topk_idx, dp.slot = sc.slot, dp.count = sc.count;
-        dp.T = T, dp.K = K, dp.E = E, dp.M = M, dp.H = H, dp.use_fp8 = fp8, dp.fused = fused;
-        dp.status = b->status, dp.recv_x = a->packed_recv_x;
+        dp.x = a->x, dp.topk_idx = a->topk_idx;
+        dp.T = T, dp.K = K, dp.E = E, dp.M = M, dp.H = H, dp.use_fp8 = fp8;
+        dp.slot = slot, dp.status = b->status, dp.recv_x = a->packed_recv_x;
         dp.recv_scales = a->packed_recv_x_scales, dp.recv_src_info = a->packed_recv_src_info;
         dp.recv_count = a->packed_recv_count, dp.layout_range = a->packed_recv_layout_range;
         dp.rowmap = sc.rowmap;
         auto& rec = b->record[par];
         rec.key = a->packed_recv_src_info, rec.seq = seq, rec.stamp = ++b->record_clock;
         rec.T = T, rec.K = K, rec.E = E, rec.M = M, rec.H = H;
-        MCEP_CUDA(mcep::launch_direct_dispatch(dp, fused ? first : next));
+        MCEP_CUDA(mcep::launch_direct_dispatch(dp, first));
         if (a->return_recv_hook) {
             auto* h = new mcep_hook();
             h->fn = []() { return MCEP_OK; };
@@ -957,10 +956,10 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
 
     char* area = b->base + kHeaderRegion + (size_t)par * g.parity_bytes;
     mcep::GroupDispatchParams p = {};
-    p.x = a->x, p.topk_idx = a->topk_idx, p.slot = sc.slot, p.count = sc.count;
+    p.x = a->x, p.topk_idx = a->topk_idx, p.slot = slot, p.count = counting ? nullptr : sc.count;
     p.peer_base = b->peer_dev, p.local_base = b->base;
     p.T = T, p.K = K, p.E = E, p.R = R, p.M = M, p.H = H, p.rank = b->rank;
-    p.use_fp8 = fp8, p.fused = fused;
+    p.use_fp8 = fp8;
     p.w = words_of(par, 0);
     p.rx_off = (size_t)(area - b->base), p.meta_off = p.rx_off + g.meta_off;
     p.row_bytes = g.row_bytes, p.meta_stride = g.meta_stride;
@@ -984,7 +983,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
 
     const int num_sms = b->num_sms;
     // Small batches, rows in place, no hook: one launch does it all.
-    bool one_kernel = fused && !p.copy_rows && !a->return_recv_hook && b->one_kernel &&
+    bool one_kernel = !p.copy_rows && !a->return_recv_hook && b->one_kernel &&
                       mcep::group_call_can_be_one_kernel(T, K, E, num_sms);
     if (b->defer) {
         MCEP_REQUIRE(!a->async_finish && !b->graph_mode);
@@ -1011,7 +1010,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
             MCEP_CUDA(e1);
         }
     }
-    if (!one_kernel) MCEP_CUDA(mcep::launch_group_dispatch_send(p, fused ? first : next));
+    if (!one_kernel) MCEP_CUDA(mcep::launch_group_dispatch_send(p, first));
     auto recv = [=](cudaStream_t s, bool chained) -> int {
         mcep::LaunchCtx c0{s, num_sms, chained && pdl};
         if (!one_kernel) MCEP_CUDA(mcep::launch_group_dispatch_recv(p, c0));
@@ -1077,7 +1076,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
         auto& sc = b->scratch[seq & 1];
         if (a->async_finish)
             if (int rc = order_after(stream, compute, b->ev_a)) return rc;
-        mcep::LaunchCtx first{stream, num_sms, false};
+        mcep::LaunchCtx first{stream, num_sms, pdl && !a->async_finish};
         // The rows of (token, k) inside their experts: kept from the dispatch call
         // when the handle is that of one of the last two; otherwise found again
         // in the handle itself - by the reduce kernel (small batches) or by an
@@ -1102,7 +1101,6 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
             MCEP_CUDA(mcep::launch_combine_invert(ip, first));
             rowmap = sc.rowmap_inv;
         }
-        const bool chain = rowmap == sc.rowmap_inv && !search;
         mcep::DirectCombineParams dp = {};
         dp.topk_idx = a->topk_idx, dp.topk_weights = a->topk_weights;
         dp.active_ranks = a->active_ranks;
@@ -1110,8 +1108,9 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
         dp.x = a->x, dp.rowmap = rowmap, dp.search = search;
         dp.src_info = a->src_info, dp.layout_range = a->layout_range;
         dp.combined_x = a->combined_x;
+        const bool chain = pdl && (rowmap == sc.rowmap_inv || !a->async_finish);
         auto reduce = [=](cudaStream_t s, bool chained) -> int {
-            mcep::LaunchCtx c0{s, num_sms, chained && pdl && chain};
+            mcep::LaunchCtx c0{s, num_sms, chained && chain};
             MCEP_CUDA(mcep::launch_direct_combine(dp, c0));
             return MCEP_OK;
         };
@@ -1149,7 +1148,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
     const int par = seq & 1;
     if (a->async_finish)
         if (int rc = order_after(stream, compute, b->ev_a)) return rc;
-    mcep::LaunchCtx first{stream, num_sms, false};
+    mcep::LaunchCtx first{stream, num_sms, pdl && !a->async_finish};
 
     mcep::GroupCombineParams p = {};
     p.x = a->x, p.layout_range = a->layout_range, p.topk_idx = a->topk_idx;

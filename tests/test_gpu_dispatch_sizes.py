@@ -1,0 +1,53 @@
+"""Dispatch at the sizes where its kernels change: the last batch that counts its
+own layout and the first that gets a layout kernel, edges of the layout kernel's
+warps, blocks and cluster, the route beyond it, batches of several rows per
+block and their remainders; odd top-k (index pairs cannot be loaded) and repeats."""
+import pytest
+import torch
+
+from mooncake_b200.mooncake_ep_buffer import Buffer
+from oracle import ep_oracle as ora
+from tests.ep_harness import FakeGroup, make_rank_inputs
+from tests.test_gpu_parity import _check_dispatch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [  # T, H, E, K, fp8
+    (1, 128, 8, 1, True), (2, 8192, 8, 2, False), (3, 8320, 4, 3, True), (296, 512, 16, 3, True), (297, 512, 16, 3, False),
+    (297, 1024, 256, 8, True), (300, 7168, 64, 16, False), (511, 128, 32, 5, True), (513, 2048, 4096, 2, False),
+    (1023, 640, 24, 6, True), (1500, 8320, 8, 2, False), (2049, 384, 128, 8, True), (4096, 128, 4096, 4, False),
+    (8192, 128, 256, 8, True), (8193, 128, 256, 8, True), (9001, 256, 16, 1, False),
+]
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("T,H,E,K,fp8", SIZES)
+def test_dispatch_and_combine(T, H, E, K, fp8, staged):
+    M = (T + 3) // 4 * 4
+    x, idx, w = make_rank_inputs(11, 0, T, H, E, K, "zipf1.2" if T % 2 else "uniform", n_mask=T // 7)
+    if K > 1:
+        idx[::5, K - 1] = idx[::5, 0]  # an expert twice in one token's list
+    if T > 4:
+        idx[T // 2] = -1
+    if staged and Buffer.get_ep_buffer_size_hint(M, H, 1, E) > 40e9:
+        pytest.skip("needs more symmetric memory than a test should hold")
+    buf = Buffer(FakeGroup(0, 1), Buffer.get_ep_buffer_size_hint(M, H, 1, E) if staged else 0)
+    buf.runtime.set_option("force_staged", int(staged))
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    want = ora.dispatch([x], [idx], M, E, fp8)
+    dx, di, dw = x.cuda(), idx.cuda(), w.cuda()
+    for _ in range(2):  # both halves of the scratch
+        recv, cnt, handle, _, _ = buf.dispatch(dx, di, active, M, E, 2_000_000, use_fp8=fp8)
+        torch.cuda.synchronize()
+        got = [dict(recv_x=recv[0] if fp8 else recv, scales=recv[1] if fp8 else None, recv_count=cnt, handle=handle)]
+        if E * M * H <= 1 << 28:
+            _check_dispatch(dict(R=1, E=E, M=M, fp8=fp8), got, want, None)
+        else:
+            assert torch.equal(cnt.cpu(), want[0]["recv_count"])
+        if fp8:
+            continue
+        # the rows went where combine looks for them: x times the sum of the listed weights
+        out, _, _ = buf.combine(recv, di, dw, active, 2_000_000, handle)
+        ref = dx.float() * (dw * (di >= 0)).sum(dim=1, keepdim=True)
+        assert float((out.float() - ref).abs().max() / ref.abs().max()) < 1e-2
+    assert buf.runtime.status() == 0
