@@ -991,9 +991,86 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
     }
 }
 
-template <int kDepth>
-__global__ void __launch_bounds__(512) ep_combine_reduce_direct_kernel(DirectCombineParams p) {
-    static_assert(kMaxTopk % kDepth == 0, "the row batches must tile the top-k table");
+// Single rank, rows known (p.rowmap). No barrier and no shared memory: a warp owns
+// one 512-channel tile of one row of every block's group of tokens, so its loads
+// overlap the sums of the others; the next row's place and weights are requested
+// before this row's data is used. Bound by HBM reads (4096 tokens, hidden 7168,
+// top-8: 470 MB of rows in 90 us, with the last dirty lines of whatever wrote them
+// still leaving L2; 80 us on rows that have been in HBM for a while). The loop runs
+// over groups, alike for all warps of a block: with a loop that the compiler has to
+// take for divergent (a token index that depends on the warp, a loop over tiles) the
+// shuffles cost so many registers that loaded rows spilled, 108 us - so tiles beyond
+// a block's warps are the grid's y. A barrier per token (tokens handed out by a
+// counter) took 111 us.
+// kAbs: rowmap holds rows of the whole tensor and every weight is 1 (elastic calls).
+constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM: nothing spills
+
+template <int kDepth, bool kAbs, int kBlocks>
+__global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_kernel(DirectCombineParams p) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = warp / p.tiles_per_block;  // which token of the group
+    const int c = ((warp - sub * p.tiles_per_block + blockIdx.y * p.tiles_per_block) * 32) + lane;
+    const bool act = c < p.H / 16;
+    pdl_wait();
+    pdl_launch_dependents();
+    const bool on = lane < p.K && ld_volatile_s32(p.active_ranks) != 0;
+    const size_t row_bytes = (size_t)p.H * 2;
+    const char* x = reinterpret_cast<const char*>(p.x) + (size_t)c * 32;
+    char* out = reinterpret_cast<char*>(p.combined_x) + (size_t)c * 32;
+    // a block's groups: every grid-th one, or (p.span) a run of tokens
+    const int step = (p.span ? 1 : gridDim.x) * p.tokens_per_block;
+    const int first = blockIdx.x * (p.span ? p.span : p.tokens_per_block);
+    const int end = p.span ? min(p.T, first + p.span) : p.T;
+
+    int next_row = -1, next_e = -1;
+    float next_w = 1.f;
+    auto request = [&](int tok) {
+        if (on && tok < end) {
+            const size_t at = (size_t)tok * p.K + lane;
+            next_row = __ldg(p.rowmap + at);
+            if (!kAbs) next_e = (int)__ldg(p.topk_idx + at), next_w = __ldg(p.topk_weights + at);
+        } else {
+            next_row = -1;
+        }
+    };
+    request(first + sub);
+    for (int t0 = first; t0 < end; t0 += step) {
+        int row = next_row;
+        if (!kAbs) row = (next_e >= 0 && next_e < p.E && row >= 0 && row < p.M) ? next_e * p.M + row : -1;
+        const float w = next_w;
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (int k0 = 0; k0 < p.K; k0 += kDepth) {
+            V32 v[kDepth];
+#pragma unroll
+            for (int b = 0; b < kDepth; ++b) {
+                const int r = __shfl_sync(kFull, row, k0 + b);
+                if (r >= 0 && act) v[b] = ld32_readonly(x + (size_t)r * row_bytes);
+            }
+            if (k0 == 0) request(t0 + step + sub);
+#pragma unroll
+            for (int b = 0; b < kDepth; ++b) {
+                const int r = __shfl_sync(kFull, row, k0 + b);
+                const float wk = kAbs ? 1.f : __shfl_sync(kFull, w, k0 + b);
+                if (r >= 0) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        acc[2 * i] = fmaf(bf16lo(v[b].w[i]), wk, acc[2 * i]);
+                        acc[2 * i + 1] = fmaf(bf16hi(v[b].w[i]), wk, acc[2 * i + 1]);
+                    }
+                }
+            }
+        }
+        if (act && t0 + sub < end) st32(out + (size_t)(t0 + sub) * row_bytes, pack_bf16x16(acc));
+    }
+}
+
+// Small batches whose rows are not recorded (a handle older than the last two
+// calls, or a copy of one): no separate inversion pass. Warp k looks the token up
+// in the handle itself - the segment of expert topk[t][k] - 32 entries of src_info
+// at a time.
+__global__ void __launch_bounds__(512) ep_combine_search_kernel(DirectCombineParams p) {
     __shared__ const char* s_ptr[kMaxTopk];
     __shared__ float s_w[kMaxTopk];
     __shared__ int s_row[kMaxTopk];
@@ -1002,51 +1079,43 @@ __global__ void __launch_bounds__(512) ep_combine_reduce_direct_kernel(DirectCom
     pdl_wait();
     pdl_launch_dependents();
     for (int t = blockIdx.x; t < p.T; t += gridDim.x) {
-        int e = -1, r = 0;
+        int e = -1;
         float w = 0.f;
         if (tid < p.K) {
             e = (int)__ldg(p.topk_idx + (size_t)t * p.K + tid);
             w = __ldg(p.topk_weights + (size_t)t * p.K + tid);
-            if (!p.search) r = __ldcg(p.rowmap + (size_t)t * p.K + tid);
         }
-        if (p.search) {
-            // Small batches: no separate inversion pass. Warp k looks the token
-            // up in the handle itself - the segment of expert topk[t][k] - 32
-            // entries of src_info at a time.
-            for (int k = warp; k < p.K; k += nwarps) {
-                const int ek = (int)__ldg(p.topk_idx + (size_t)t * p.K + k);
-                int row = -1;
-                if (ek >= 0 && ek < p.E) {
-                    const long long lr = __ldg(p.layout_range + ek);
-                    const int cnt = (int)(lr & 0xffffffffll), begin = (int)(lr >> 32);
-                    for (int j0 = 0; j0 < cnt; j0 += 32) {
-                        const int j = begin + j0 + lane;
-                        const bool hit = j0 + lane < cnt && j < p.M &&
-                                         __ldg(p.src_info + (size_t)ek * p.M + j) == t;
-                        const unsigned m = __ballot_sync(kFull, hit);
-                        if (m) {
-                            row = begin + j0 + __ffs(m) - 1;
-                            break;
-                        }
+        for (int k = warp; k < p.K; k += nwarps) {
+            const int ek = (int)__ldg(p.topk_idx + (size_t)t * p.K + k);
+            int row = -1;
+            if (ek >= 0 && ek < p.E) {
+                const long long lr = __ldg(p.layout_range + ek);
+                const int cnt = (int)(lr & 0xffffffffll), begin = (int)(lr >> 32);
+                for (int j0 = 0; j0 < cnt; j0 += 32) {
+                    const int j = begin + j0 + lane;
+                    const bool hit = j0 + lane < cnt && j < p.M &&
+                                     __ldg(p.src_info + (size_t)ek * p.M + j) == t;
+                    const unsigned m = __ballot_sync(kFull, hit);
+                    if (m) {
+                        row = begin + j0 + __ffs(m) - 1;
+                        break;
                     }
                 }
-                if (lane == 0) s_row[k] = row;
             }
+            if (lane == 0) s_row[k] = row;
         }
         __syncthreads();  // s_row is in place; the previous token's rows are done with s_ptr
         if (tid < kMaxTopk) {
             const char* ptr = nullptr;
-            if (p.search && tid < p.K) r = s_row[tid];
-            if (tid < p.K && e >= 0 && e < p.E) {
-                if (ld_volatile_s32(p.active_ranks) && r >= 0 && r < p.M)
-                    ptr = reinterpret_cast<const char*>(p.x) + ((size_t)e * p.M + r) * p.H * 2;
-            }
+            const int r = tid < p.K ? s_row[tid] : -1;
+            if (e >= 0 && e < p.E && ld_volatile_s32(p.active_ranks) && r >= 0 && r < p.M)
+                ptr = reinterpret_cast<const char*>(p.x) + ((size_t)e * p.M + r) * p.H * 2;
             s_ptr[tid] = ptr;
             s_w[tid] = w;
         }
         __syncthreads();
-        reduce_rows<kDepth, true>(s_ptr, s_w, p.K, p.H,
-                                  reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
+        reduce_rows<8, true>(s_ptr, s_w, p.K, p.H,
+                             reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
     }
 }
 
@@ -1786,12 +1855,42 @@ cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx&
                   ctx, p);
 }
 
-cudaError_t launch_direct_combine(const DirectCombineParams& p, const LaunchCtx& ctx) {
-    const int threads = block_threads(p.H);
-    const bool deep = p.T <= ctx.num_sms;  // one block per SM at most: spend registers on loads in flight
-    auto k = deep ? ep_combine_reduce_direct_kernel<8> : ep_combine_reduce_direct_kernel<4>;
-    const int grid = persistent_grid(p.T, k, threads, 0, ctx);
-    return launch("ep_combine_reduce_direct", k, dim3(grid), dim3(threads), 0, ctx, p);
+cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
+    if (p.search) {
+        const int threads = block_threads(p.H);
+        const int grid = persistent_grid(p.T, ep_combine_search_kernel, threads, 0, ctx);
+        return launch("ep_combine_search", ep_combine_search_kernel, dim3(grid), dim3(threads), 0, ctx, p);
+    }
+    // A block covers as many whole rows as give it 14 to 16 warps once there are more
+    // tokens than SMs; up to one block per SM, registers are spent on loads in flight.
+    const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    const int parts = (ntiles + kReduceWarps - 1) / kReduceWarps;  // blocks that share a row
+    p.tiles_per_block = (ntiles + parts - 1) / parts;
+    p.tokens_per_block = 1;
+    if (p.T > ctx.num_sms) {
+        const int fit = kReduceWarps / p.tiles_per_block, most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
+        p.tokens_per_block = fit < most ? fit : most;
+    }
+    const int threads = 32 * p.tiles_per_block * p.tokens_per_block;
+    const int groups = p.T > 0 ? (p.T + p.tokens_per_block - 1) / p.tokens_per_block : 1;
+    void (*k)(DirectCombineParams) = nullptr;
+    if (p.absolute) {
+        k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, true, 1> : ep_combine_rows_kernel<4, true, 2>;
+    } else {
+        k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, false, 1> : ep_combine_rows_kernel<4, false, 2>;
+    }
+    // How the groups are dealt out, in waves of the blocks that are resident at a time
+    // (two of 16 warps per SM, more of smaller ones). 4 to 16 waves: every block an equal
+    // run of consecutive groups (1024 tokens of 14 KB to 8: 20.5 us; strided 22.5). Fewer:
+    // a full wave striding (equal runs would leave blocks out: 600 tokens 10.6 us against
+    // 12.4). More: runs of four, handed out as blocks finish, so that no SM falls behind
+    // (8192 tokens 166 us; equal runs 176, strided 178).
+    const int resident = ctx.num_sms * (2 * kReduceWarps * 32 / threads) / parts;
+    const int waves = (groups + resident - 1) / resident;
+    const int run = waves < 4 ? 0 : waves <= 16 ? waves : 4;
+    p.span = run * p.tokens_per_block;
+    const int grid = run ? (groups + run - 1) / run : groups < resident ? groups : resident;
+    return launch("ep_combine_reduce_direct", k, dim3(grid, parts), dim3(threads), 0, ctx, p);
 }
 
 // ---- groups -----------------------------------------------------------------------

@@ -88,13 +88,16 @@ struct DirectCombineParams {
     int T, K, E, M, H;
     const void* x;              // rows at x + (expert * M + rowmap[t*K+k]) * 2H
     const int32_t* rowmap;
+    int absolute;               // rowmap names rows of the whole tensor (-1: none), every weight is 1;
+                                // topk_idx and topk_weights are not read
+    int tokens_per_block, tiles_per_block, span;  // set by the launcher (span: tokens a block works through)
     // search: no rowmap; rows are looked up in the handle by the kernel
     int search;
     const int32_t* src_info;
     const int64_t* layout_range;
     void* combined_x;           // [T][H] bf16
 };
-cudaError_t launch_direct_combine(const DirectCombineParams& p, const LaunchCtx& ctx);
+cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx);
 
 // ---- groups: words exchanged through symmetric memory -----------------------------
 // All words are 64-bit: (sequence number of the call << 32) | value, value >= 1.
