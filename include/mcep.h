@@ -369,6 +369,15 @@ typedef struct mcep_elastic_dispatch_args {
 } mcep_elastic_dispatch_args;
 int mcep_elastic_dispatch(mcep_buffer* buf, const mcep_elastic_dispatch_args* args,
                           mcep_event** out_event);
+/* The same call for a caller that needs the counts on the host
+ * (do_cpu_sync, mooncake-wheel/mooncake/mooncake_elastic_buffer.py:640-664): waits for
+ * them and leaves psum_num_recv_tokens_per_scaleup_rank in
+ * host_recv_per_rank[num_ranks] and psum_num_recv_tokens_per_expert in
+ * host_psum_per_expert[num_experts / num_ranks + 1] (host memory). The rows may
+ * still be on their way when it returns, as after any call. */
+int mcep_elastic_dispatch_counted(mcep_buffer* buf, const mcep_elastic_dispatch_args* args,
+                                  int32_t* host_recv_per_rank, int32_t* host_psum_per_expert,
+                                  mcep_event** out_event);
 
 /* Replaces MooncakeElasticBuffer::combine
  * (mooncake-ep/src/mooncake_ep_elastic_buffer.cpp:362-426).

@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.environ.get("MCEP_LIB") or os.path.join(HERE, "libmcep.so")
 SOURCES = ["ep_kernels.cu", "ep_runtime.cu", "ep_noalloc.cu", "ep_elastic_kernels.cu",
            "ep_elastic.cu"]
-HEADERS = ["ep_kernels.cuh", "ep_device.cuh", "ep_routing.cuh", "ep_elastic.cuh", "ep_runtime_internal.h",
+HEADERS = ["ep_kernels.cuh", "ep_device.cuh", "ep_routing.cuh", "ep_launch.cuh", "ep_elastic.cuh", "ep_runtime_internal.h",
            os.path.join("..", "..", "include", "mcep.h")]
 
 

@@ -51,12 +51,44 @@ __device__ __forceinline__ int ld_volatile_s32(const int* p) {
 __device__ __forceinline__ void st_volatile_s32(int* p, int v) {
     asm volatile("st.volatile.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// ---- inputs -----------------------------------------------------------------------
+// Data that the kernel AHEAD may have written and this one only reads. Not __ldg and
+// not ld.global.nc: both promise that the data does not change while the kernel runs,
+// and a kernel that was launched early runs already while it waits for the one
+// ahead - the compiler moved such loads above griddepcontrol.wait, and a copy kernel
+// read the positions of an earlier call. Plain volatile loads stay below it.
+__device__ __forceinline__ int ld_ro(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_ro(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int64_t ld_ro(const int64_t* p) {
+    int64_t v;
+    asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ longlong2 ld_ro(const longlong2* p) {
+    longlong2 v;
+    asm volatile("ld.global.v2.s64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+// The same for words that other blocks of this kernel may be writing (L2).
+__device__ __forceinline__ int ld_l2(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 // ---- 32-byte vector memory ops ----------------------------------------------
-// Read-only inputs that no kernel writes while this one runs (x, expert outputs).
+// Inputs that are read once (x, expert outputs): see above, no .nc; not kept in L1.
 __device__ __forceinline__ V32 ld32_readonly(const void* p) {
     V32 r;
     asm volatile(
-        "ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        "ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]),
           "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7])
         : "l"(p));

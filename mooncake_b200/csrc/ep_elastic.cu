@@ -12,7 +12,9 @@
 // position the row will take inside the source's segment.
 #include "ep_elastic.cuh"
 
+#include <chrono>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -54,6 +56,48 @@ size_t usable_bytes(int64_t num_bytes) { return num_bytes > 0 ? (size_t)num_byte
 int record_stride(int K) { return (int)up(8 * (size_t)K + 4, 16); }
 size_t record_bytes(int R, int M, int K) { return up((size_t)R * M * record_stride(K), 256); }
 
+// Host memory that the device writes the counts of a call into, for callers that wait
+// for them ([0] flag, [1] received rows, [2..] prefix sums per expert). Kept in a
+// small stock: pinning memory costs more than a whole call.
+constexpr size_t kHostCountsBytes = (2 + MCEP_MAX_EXPERTS + 1 + 64) * sizeof(int32_t);
+constexpr size_t kHostCountsStock = 16;
+std::mutex g_counts_mu;
+std::vector<int32_t*> g_counts_stock;
+
+int32_t* take_host_counts() {
+    {
+        std::lock_guard<std::mutex> lk(g_counts_mu);
+        if (!g_counts_stock.empty()) {
+            int32_t* p = g_counts_stock.back();
+            g_counts_stock.pop_back();
+            return p;
+        }
+    }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kHostCountsBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::memset(p, 0, kHostCountsBytes);
+    return static_cast<int32_t*>(p);
+}
+
+void give_host_counts(int32_t* p) {
+    if (p == nullptr) return;
+    p[0] = 0;
+    std::lock_guard<std::mutex> lk(g_counts_mu);
+    if (g_counts_stock.size() < kHostCountsStock)
+        g_counts_stock.push_back(p);
+    else
+        cudaFreeHost(p);
+}
+
+// What a caller that waits for the counts gets.
+struct Counts {
+    int32_t* per_rank;    // [R]
+    int32_t* per_expert;  // [L + 1]
+};
+
 // What the entry points keep per buffer between calls.
 struct ElasticState {
     int R = 0, M = 0, K = 0, L = 0, H = 0;  // capacities of the carve-up below
@@ -76,8 +120,16 @@ struct ElasticState {
     struct Record {
         const void* key = nullptr;  // the handle's recv_src_metadata tensor
         int par = 0, T = 0, K = 0, E = 0, M = 0, H = 0, expand = 0;
+        bool single = false;  // the call took the single-rank path: its rows are in single_rows[par]
         uint64_t stamp = 0;
     } rec[2];
+    // single-rank path: rows kept for combine (per parity), rows of the tokens (scratch)
+    char* single_blob = nullptr;
+    size_t single_entries = 0, single_tokens = 0;
+    int32_t* single_rows[2] = {};
+    int32_t* single_pos = nullptr;
+    int32_t* host_counts = nullptr;
+    uint32_t host_seq = 0;
     uint64_t clock = 0;
     uint32_t calls = 0;
     // The record areas sit at fixed places for the life of the buffer (fixed by its first
@@ -153,6 +205,46 @@ int ensure(ElasticState* s, const mcep::BufferView& v, int M, int K, int L, int 
     return MCEP_OK;
 }
 
+// Scratch of the single-rank path.
+int ensure_single(ElasticState* s, int M, int K) {
+    const size_t entries = (size_t)M * K, tokens = (size_t)M;
+    if (s->single_blob && entries <= s->single_entries && tokens <= s->single_tokens) return MCEP_OK;
+    EL_CUDA(cudaDeviceSynchronize());
+    if (s->single_blob) cudaFree(s->single_blob);
+    s->single_blob = nullptr;
+    s->single_entries = entries > s->single_entries ? entries : s->single_entries;
+    s->single_tokens = tokens > s->single_tokens ? tokens : s->single_tokens;
+    const size_t rows = up(s->single_entries * 4 + 4, 256), pos = up(s->single_tokens * 4 + 4, 256);
+    EL_CUDA(cudaMalloc(&s->single_blob, 2 * rows + pos));
+    s->single_rows[0] = reinterpret_cast<int32_t*>(s->single_blob);
+    s->single_rows[1] = reinterpret_cast<int32_t*>(s->single_blob + rows);
+    s->single_pos = reinterpret_cast<int32_t*>(s->single_blob + 2 * rows);
+    for (auto& r : s->rec)
+        if (r.single) r = ElasticState::Record();
+    if (!s->ev) EL_CUDA(cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming));
+    return MCEP_OK;
+}
+
+// Waits until the device has left the counts of call `seq` in `h`. They are written
+// while the call's rows are still being copied, so this is the time of the counting
+// alone. After some milliseconds (work queued ahead) the stream is waited for instead.
+int wait_for_counts(int32_t* h, int32_t seq, cudaStream_t stream) {
+    const auto start = std::chrono::steady_clock::now();
+    for (unsigned i = 0;; ++i) {
+        if (__atomic_load_n(h, __ATOMIC_ACQUIRE) == seq) return MCEP_OK;
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+        if ((i & 1023u) == 1023u &&
+            std::chrono::steady_clock::now() - start > std::chrono::milliseconds(5))
+            break;
+    }
+    EL_CUDA(cudaStreamSynchronize(stream));
+    if (__atomic_load_n(h, __ATOMIC_ACQUIRE) != seq)
+        return report_failure(MCEP_ERR_CUDA, "Failed: the device did not report the counts of an elastic dispatch");
+    return MCEP_OK;
+}
+
 // Where every rank keeps the records of the call with this parity. In a group:
 // at the end of the data area of the symmetric allocation, same offset on every
 // rank.
@@ -211,11 +303,81 @@ void elastic_release(mcep_buffer* b) {
         g_states.erase(it);
     }
     free_blob(s);
+    if (s->single_blob) cudaFree(s->single_blob);
+    give_host_counts(s->host_counts);
     if (s->ev) cudaEventDestroy(s->ev);
     delete s;
 }
 
 }  // namespace mcep
+
+namespace {
+
+// A single rank: one or two kernels write every output directly.
+int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, const mcep_elastic_dispatch_args* a,
+                    const Counts* counts, mcep_event** out_event) {
+    const int E = a->num_experts, M = a->num_max_tokens_per_rank, T = a->num_tokens, H = a->hidden, K = a->num_topk;
+    EL_REQUIRE(H % 16 == 0 && H % 128 == 0);
+    EL_REQUIRE(reinterpret_cast<uintptr_t>(a->x) % 32 == 0 && reinterpret_cast<uintptr_t>(a->recv_x) % 32 == 0);
+    if (int rc = ensure_single(s, M, K)) return rc;
+    if (counts && s->host_counts == nullptr) {
+        s->host_counts = take_host_counts();
+        EL_REQUIRE(s->host_counts != nullptr);
+    }
+    cudaStream_t stream = nullptr;
+    const bool async = a->async_with_compute_stream != 0;
+    if (int rc = pick_stream(s, v, async, a->compute_stream, &stream)) return rc;
+    const int par = (int)(++s->calls & 1u);
+    const bool expand = a->do_expand != 0;
+    mcep::ElasticSingleParams p = {};
+    p.x = a->x, p.topk_idx = a->topk_idx, p.topk_weights = a->topk_weights;
+    p.T = T, p.K = K, p.E = E, p.H = H, p.alignment = a->expert_alignment;
+    p.max_rows = M * K, p.status = v.status;
+    p.rows = s->single_rows[par], p.token_pos = expand ? s->single_pos : s->single_rows[par];
+    p.recv_x = a->recv_x, p.recv_topk_idx = a->recv_topk_idx, p.recv_topk_weights = a->recv_topk_weights;
+    p.recv_src_metadata = a->recv_src_metadata, p.dst_slot = a->dst_buffer_slot_idx;
+    p.copied_topk_idx = a->copied_topk_idx;
+    p.psum_rank = a->psum_num_recv_tokens_per_scaleup_rank, p.psum_expert = a->psum_num_recv_tokens_per_expert;
+    if (counts) p.host_counts = s->host_counts, p.host_seq = (int32_t)++s->host_seq;
+    const bool chain = mcep::may_chain(b, stream);
+    mcep::LaunchCtx ctx{stream, v.num_sms, chain && !async, chain};
+    EL_CUDA(mcep::launch_elastic_single_dispatch(p, expand, ctx));
+    mcep::count_dispatch_call(b);
+    auto& rec = s->rec[par];
+    rec.key = a->recv_src_metadata, rec.par = par, rec.T = T, rec.K = K, rec.E = E, rec.M = M, rec.H = H;
+    rec.expand = expand, rec.single = true, rec.stamp = ++s->clock;
+    if (async)
+        if (int rc = mcep_event_create(reinterpret_cast<uint64_t>(stream), out_event)) return rc;
+    if (counts) {
+        if (int rc = wait_for_counts(s->host_counts, p.host_seq, stream)) return rc;
+        counts->per_rank[0] = s->host_counts[1];
+        std::memcpy(counts->per_expert, s->host_counts + 2, (size_t)(E + 1) * sizeof(int32_t));
+    }
+    return MCEP_OK;
+}
+
+// Combine of such a call: the rows are gathered from where the dispatch put them.
+int single_combine(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, const ElasticState::Record& rec,
+                   const mcep_elastic_combine_args* a, mcep_event** out_event) {
+    EL_REQUIRE(reinterpret_cast<uintptr_t>(a->x) % 32 == 0 && reinterpret_cast<uintptr_t>(a->combined_x) % 32 == 0);
+    cudaStream_t stream = nullptr;
+    const bool async = a->async_with_compute_stream != 0;
+    if (int rc = pick_stream(s, v, async, a->compute_stream, &stream)) return rc;
+    mcep::DirectCombineParams p = {};
+    p.active_ranks = a->active_ranks;
+    p.T = rec.T, p.K = rec.expand ? rec.K : 1, p.H = rec.H;
+    p.x = a->x, p.rowmap = s->single_rows[rec.par], p.absolute = 1;
+    p.combined_x = a->combined_x;
+    mcep::LaunchCtx ctx{stream, v.num_sms, mcep::may_chain(b, stream) && !async};
+    EL_CUDA(mcep::launch_direct_combine(p, ctx));
+    mcep::count_combine_call(b);
+    if (async) return mcep_event_create(reinterpret_cast<uint64_t>(stream), out_event);
+    return MCEP_OK;
+}
+
+int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const Counts* counts, mcep_event** out_event);
+
+}  // namespace
 
 extern "C" {
 
@@ -225,6 +387,22 @@ uint64_t mcep_elastic_buffer_size_hint(int M, int hidden, int num_ranks, int num
 }
 
 int mcep_elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, mcep_event** out_event) {
+    return elastic_dispatch(b, a, nullptr, out_event);
+}
+
+int mcep_elastic_dispatch_counted(mcep_buffer* b, const mcep_elastic_dispatch_args* a, int32_t* per_rank,
+                                  int32_t* per_expert, mcep_event** out_event) {
+    EL_REQUIRE(per_rank != nullptr && per_expert != nullptr);
+    const Counts counts{per_rank, per_expert};
+    return elastic_dispatch(b, a, &counts, out_event);
+}
+
+}  // extern "C"
+
+namespace {
+
+int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const Counts* counts,
+                     mcep_event** out_event) {
     EL_REQUIRE(b != nullptr && a != nullptr && out_event != nullptr);
     *out_event = nullptr;
     const mcep::BufferView v = mcep::view_of(b);
@@ -242,6 +420,9 @@ int mcep_elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, m
     EL_REQUIRE(a->recv_x != nullptr && a->recv_topk_idx != nullptr && a->recv_src_metadata != nullptr);
     const int L = E / R;
     ElasticState* s = state_of(b);
+    if (!v.group && !v.defer && mcep::elastic_single_fits(T, K, E))
+        return single_dispatch(b, s, v, a, counts, out_event);
+    EL_REQUIRE(counts == nullptr || !v.defer);
     const size_t rec_want = record_bytes(R, M, K);
     const size_t rec_bytes = (v.group && s->record_area_bytes != 0) ? s->record_area_bytes : rec_want;
     if (rec_want > rec_bytes)
@@ -298,7 +479,7 @@ int mcep_elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, m
 
     auto& rec = s->rec[par];
     rec.key = a->recv_src_metadata, rec.par = par, rec.T = T, rec.K = K, rec.E = E, rec.M = M, rec.H = H;
-    rec.expand = a->do_expand != 0, rec.stamp = ++s->clock;
+    rec.expand = a->do_expand != 0, rec.single = false, rec.stamp = ++s->clock;
 
     mcep::ElasticEpilogueParams ep = {};
     ep.layout_range = s->layout_range[par];
@@ -340,9 +521,21 @@ int mcep_elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, m
         return MCEP_OK;
     }
     if (int rc = after()) return rc;
-    if (a->async_with_compute_stream) return mcep_event_create(reinterpret_cast<uint64_t>(stream), out_event);
+    if (a->async_with_compute_stream)
+        if (int rc = mcep_event_create(reinterpret_cast<uint64_t>(stream), out_event)) return rc;
+    if (counts) {
+        EL_CUDA(cudaMemcpyAsync(counts->per_rank, a->psum_num_recv_tokens_per_scaleup_rank, (size_t)R * sizeof(int32_t),
+                                cudaMemcpyDeviceToHost, stream));
+        EL_CUDA(cudaMemcpyAsync(counts->per_expert, a->psum_num_recv_tokens_per_expert,
+                                (size_t)(L + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        EL_CUDA(cudaStreamSynchronize(stream));
+    }
     return MCEP_OK;
 }
+
+}  // namespace
+
+extern "C" {
 
 int mcep_elastic_combine(mcep_buffer* b, const mcep_elastic_combine_args* a, mcep_event** out_event) {
     EL_REQUIRE(b != nullptr && a != nullptr && out_event != nullptr);
@@ -369,6 +562,7 @@ int mcep_elastic_combine(mcep_buffer* b, const mcep_elastic_combine_args* a, mce
         return report_failure(MCEP_ERR_INVALID,
                               "Failed: Assertion error 'elastic combine arguments match the dispatch call of "
                               "the handle'");
+    if (rec->single) return single_combine(b, s, v, *rec, a, out_event);
     const int par = rec->par;
     cudaStream_t stream = nullptr;
     if (int rc = pick_stream(s, v, a->async_with_compute_stream != 0, a->compute_stream, &stream)) return rc;

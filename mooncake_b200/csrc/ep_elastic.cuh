@@ -15,6 +15,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "ep_kernels.cuh"
+
 namespace mcep {
 
 // A record per row a rank is about to receive, stored by the source in the
@@ -82,6 +84,39 @@ struct ElasticLocalReduceParams {
 };
 cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int num_sms,
                                         cudaStream_t stream);
+
+// ---- a single rank ----------------------------------------------------------------------
+// Nothing is exchanged: a received row is the token itself, its position the number
+// of earlier tokens that name any expert, its expanded rows follow from the routing
+// alone. One launch (small batches) or two (layout, copy) write all outputs, the
+// rows go straight to where they end up, and combine gathers from there.
+struct ElasticSingleParams {
+    const void* x;               // [T][H] bf16
+    const int64_t* topk_idx;     // [T][K]
+    const float* topk_weights;   // [T][K] or null
+    int T, K, E, H, alignment;
+    int C;                       // tokens per block of the copy kernel (set by the launcher)
+    int max_rows;                // expanded: rows recv_x has room for
+    int32_t* status;
+    int32_t* rows;               // kept for combine: [T] received row of the token, or (expanded) [T][K] row
+                                 // of the entry; -1: none
+    int32_t* token_pos;          // expanded: [T] scratch, received row of the token (else == rows)
+    void* recv_x;
+    int64_t* recv_topk_idx;      // [n][K]
+    float* recv_topk_weights;    // [n][K], expanded: [rows]; or null
+    int32_t* recv_src_metadata;  // [n][K+2]
+    int32_t* dst_slot;           // [T][K]
+    int64_t* copied_topk_idx;    // [T][K] or null
+    int32_t* psum_rank;          // [1]
+    int32_t* psum_expert;        // [E+1]
+    // a caller that waits for the counts: host memory the device can write,
+    // [0] flag (host_seq once the rest is there), [1] received rows, [2..] psum_expert
+    int32_t* host_counts;
+    int32_t host_seq;
+};
+// whether the kernels below take this problem (else the general path does)
+bool elastic_single_fits(int T, int K, int E);
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx);
 
 // float ones of a given length (the weights of the exchange's reduction)
 cudaError_t launch_elastic_fill_ones(float* w, size_t n, cudaStream_t stream);

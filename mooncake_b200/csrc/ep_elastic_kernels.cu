@@ -2,8 +2,12 @@
 // another GPU; the exchange between the ranks is the group dispatch / combine.
 #include "ep_elastic.cuh"
 
+#include <atomic>
+
 #include "ep_device.cuh"
 #include "ep_kernels.cuh"
+#include "ep_launch.cuh"
+#include "ep_routing.cuh"
 
 namespace mcep {
 namespace {
@@ -78,7 +82,7 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_route_kernel(ElasticRoute
 #pragma unroll
             for (int k = 0; k < kMaxTopk; ++k) {
                 if (k >= p.K) break;
-                const int64_t e = __ldg(p.topk_idx + (size_t)t * p.K + k);
+                const int64_t e = ld_ro(p.topk_idx + (size_t)t * p.K + k);
                 hit = hit || (e >= 0 && e < p.E && (int)e / L == r);
             }
             before += hit ? 1 : 0;
@@ -101,7 +105,7 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_route_kernel(ElasticRoute
         int master = -1;
         if (t < p.T) {
 #pragma unroll
-            for (int k = 0; k < kMaxTopk; ++k) raw[k] = k < p.K ? __ldg(p.topk_idx + (size_t)t * p.K + k) : -1;
+            for (int k = 0; k < kMaxTopk; ++k) raw[k] = k < p.K ? ld_ro(p.topk_idx + (size_t)t * p.K + k) : -1;
 #pragma unroll
             for (int k = 0; k < kMaxTopk; ++k) {
                 rk[k] = (raw[k] >= 0 && raw[k] < p.E) ? (int)raw[k] / L : -1;
@@ -132,7 +136,7 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_route_kernel(ElasticRoute
                 if (k >= p.K) break;
                 reinterpret_cast<int32_t*>(rec)[k] = rk[k] >= 0 ? (int32_t)raw[k] : -1;
                 reinterpret_cast<float*>(rec)[p.K + k] =
-                    p.topk_weights ? __ldg(p.topk_weights + (size_t)t * p.K + k) : 0.f;
+                    p.topk_weights ? ld_ro(p.topk_weights + (size_t)t * p.K + k) : 0.f;
             }
             reinterpret_cast<int32_t*>(rec)[2 * p.K] = t;
         }
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_epilogue_kernel(ElasticEp
             // entry e of the exclusive sum adds the aligned count of expert e - 1
             int c = 0;
             if (e >= 1 && e <= p.L) {
-                c = __ldcg(p.hist + e - 1);
+                c = ld_l2(p.hist + e - 1);
                 c = (c + p.alignment - 1) / p.alignment * p.alignment;
             }
             int v = c;
@@ -336,6 +340,341 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_local_reduce_kernel(Elast
     }
 }
 
+// ---- a single rank ----------------------------------------------------------------------
+__device__ __forceinline__ int aligned_count(int c, int a) { return (c + a - 1) / a * a; }
+
+// In-place exclusive sums of a[0..n), the total in a[n] (shared memory, whole block).
+__device__ void exclusive_sums(int* a, int n) {
+    __shared__ int s_sum[32];
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+    const int per = (n + nthr - 1) / nthr, b = min(tid * per, n), e = min(b + per, n);
+    int sum = 0;
+    for (int i = b; i < e; ++i) sum += a[i];
+    int incl = sum;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(kAll, incl, d);
+        if (lane >= d) incl += u;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    int run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += s_sum[w];
+    for (int i = b; i < e; ++i) {
+        const int c = a[i];
+        a[i] = run;
+        run += c;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int total = 0;
+        for (int w = 0; w < nwarps; ++w) total += s_sum[w];
+        a[n] = total;
+    }
+    __syncthreads();
+}
+
+// What a caller may be waiting for on the host, then the flag that says so.
+__device__ void tell_host(const ElasticSingleParams& p, int n) {
+    if (p.host_counts == nullptr) return;
+    volatile int32_t* h = p.host_counts;
+    __syncthreads();  // psum_expert has been written by this block
+    for (int i = threadIdx.x; i <= p.E; i += blockDim.x) h[2 + i] = p.psum_expert[i];
+    if (threadIdx.x == 0) h[1] = n;
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) h[0] = p.host_seq;
+}
+
+// Layout in one launch of one cluster (as the dispatch calls' layout kernel): a lane
+// per token. Column E of the tables stands for "the token goes anywhere", so a
+// token's received row is found like its rows inside the experts.
+//   kExpand: bit (expert, token) in [word][E + 1], popcounts, prefix over words and
+//   blocks; else only the number of hits per expert and column E are needed.
+// An expert listed twice counts twice in the hit counts and has its row at the last
+// listing (mooncake_ep_elastic_dispatch_copy_epilogue.cuh:114-141).
+constexpr int kSingleCluster = 8, kSingleClusterLarge = 16;
+
+template <bool kExpand, int KB>
+__device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int* smem) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, words = nthr >> 5;
+    const int rank = blockIdx.x, blocks = gridDim.x, E1 = p.E + 1;
+    const int t = rank * nthr + tid;
+    int* total = smem;                  // [E1] hits in this block (column E: tokens received)
+    int* lower = smem + E1;             // [E1] in the lower blocks
+    int* every = smem + 2 * E1;         // [E1 + 1] in all blocks, then the aligned sums
+    int* repeats = smem + 3 * E1 + 1;   // [E1] of the hits, those that have no row (kExpand)
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem + 4 * E1 + 1);  // [words][E1] (kExpand)
+    int* pre = smem + 4 * E1 + 1 + words * E1;                        // [words][E1] (kExpand)
+    __shared__ int s_warp[32];
+    for (int i = tid; i < E1; i += nthr) total[i] = 0, repeats[i] = 0;
+    if (kExpand)
+        for (int i = tid; i < E1 * words; i += nthr) mask[i] = 0;
+    int e[KB];
+#pragma unroll
+    for (int k = 0; k < KB; ++k) e[k] = -1;
+    if (t < p.T) load_choices<KB>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < KB; ++k) any |= e[k] >= 0;
+    const unsigned sent = __ballot_sync(kAll, any);
+    if (lane == 0) s_warp[warp] = __popc(sent);
+    __syncthreads();
+    if (!kExpand) {
+#pragma unroll
+        for (int k = 0; k < KB; ++k)
+            if (e[k] >= 0) atomicAdd(&total[e[k]], 1);
+    } else {
+        int all[KB];
+#pragma unroll
+        for (int k = 0; k < KB; ++k) all[k] = e[k];
+        drop_repeats<KB, true>(e);
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+            if (e[k] >= 0) atomicOr(&mask[warp * E1 + e[k]], 1u << lane);
+            if (all[k] >= 0 && e[k] < 0) atomicAdd(&repeats[all[k]], 1);
+        }
+    }
+    int before_warp = 0, in_block = 0;
+    for (int w = 0; w < words; ++w) {
+        if (w < warp) before_warp += s_warp[w];
+        in_block += s_warp[w];
+    }
+    __syncthreads();
+    if (kExpand)
+        for (int x = tid; x < p.E; x += nthr) {
+            int run = 0;
+            for (int w = 0; w < words; ++w) {
+                const int c = __popc(mask[w * E1 + x]);
+                pre[w * E1 + x] = run;
+                run += c;
+            }
+            total[x] = run;
+        }
+    if (tid == 0) total[p.E] = in_block;
+    cluster_sync();
+    for (int x = tid; x < E1; x += nthr) {
+        int lo = 0, sum = 0, rep = 0;
+#pragma unroll
+        for (int r = 0; r < kSingleClusterLarge; ++r) {
+            if (r >= blocks) break;
+            const int c = ld_cluster_s32(total + x, r);
+            if (kExpand) rep += ld_cluster_s32(repeats + x, r);
+            if (r < rank) lo += c;
+            sum += c;
+        }
+        lower[x] = lo;
+        every[x] = x < p.E ? aligned_count(sum + rep, p.alignment) : sum;
+        if (kExpand && rank == blocks - 1) p.psum_expert[x] = x < p.E ? sum : 0;  // rows of the expert, for below
+    }
+    __syncthreads();
+    const int n = every[p.E];
+    __syncthreads();
+    exclusive_sums(every, p.E);  // where every expert's segment starts
+    if (rank == blocks - 1) {
+        for (int x = tid; x < E1; x += nthr) {
+            const int rows = kExpand && x < p.E ? p.psum_expert[x] : 0;
+            p.psum_expert[x] = every[x] + rows;  // expanded: where it ends
+        }
+        if (tid == 0) p.psum_rank[0] = n;
+        tell_host(p, n);
+    }
+    if (t < p.T) {
+        const unsigned below = (1u << lane) - 1u;
+        p.token_pos[t] = any ? lower[p.E] + before_warp + __popc(sent & below) : -1;
+        if (kExpand) {
+            int32_t* out = p.rows + (size_t)t * p.K;
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+                if (k >= p.K) break;
+                const int at = warp * E1 + e[k];
+                out[k] = e[k] >= 0 ? every[e[k]] + lower[e[k]] + pre[at] + __popc(mask[at] & below) : -1;
+            }
+        }
+    }
+    cluster_sync();  // no block leaves while its totals may still be read
+}
+
+template <bool kExpand>
+__global__ void __launch_bounds__(1024) ep_elastic_single_layout_kernel(ElasticSingleParams p) {
+    extern __shared__ int smem_i32[];
+    pdl_wait();
+    pdl_launch_dependents();
+    if (p.K <= 4)
+        single_layout<kExpand, 4>(p, smem_i32);
+    else if (p.K <= 8)
+        single_layout<kExpand, 8>(p, smem_i32);
+    else
+        single_layout<kExpand, 16>(p, smem_i32);
+}
+
+// Tokens of [0, T) that name any expert, and those of [0, upto) among them; whole block.
+__device__ __forceinline__ int2 count_sent(const ElasticSingleParams& p, int upto) {
+    int n = 0, before = 0;
+    for (int t0 = 0; t0 < p.T; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x;
+        bool any = false;
+        if (t < p.T)
+            for (int k = 0; k < p.K && !any; ++k) {
+                const int e = (int)ld_ro(p.topk_idx + (size_t)t * p.K + k);
+                any = e >= 0 && e < p.E;
+            }
+        n += __syncthreads_count(any);
+        before += __syncthreads_count(any && t < upto);
+    }
+    return make_int2(n, before);
+}
+
+// Every listing of tokens [0, T), repeats included, into hits[E] (whole block, no barrier).
+__device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hits) {
+    for (int i = threadIdx.x; i < p.T * p.K; i += blockDim.x) {
+        const int e = (int)ld_ro(p.topk_idx + i);
+        if (e >= 0 && e < p.E) atomicAdd(&hits[e], 1);
+    }
+}
+
+// Rows and per-entry outputs. A block takes C tokens; C rows of a batch are requested
+// up to four per warp before the first is stored. Bound by HBM (4096 tokens of 14 KB:
+// 117 MB in and out). Behind the layout kernel (kCount false) the rows are requested
+// before its results are waited for. With kCount (small batches, one token per block)
+// there is no layout kernel: every block finds its token's places itself and block 0
+// writes the counts.
+template <bool kExpand, bool kCount>
+__global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
+    extern __shared__ int smem_i32[];  // kCount: [E + 1] hits / starts, [E] earlier tokens (kExpand)
+    constexpr int kEntries = 128;
+    __shared__ int s_exp[kEntries];  // expert of the entry or -1
+    __shared__ int s_row[kEntries];  // expanded row of the entry or -1 (kExpand)
+    __shared__ int s_pos[kEntries];  // received row of token c
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+    const int K = p.K, nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    if (kCount) pdl_wait();
+    pdl_launch_dependents();
+    int bid = blockIdx.x;
+    if (kCount) {
+        if (bid == 0) {  // the counts
+            for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
+            int* rows = smem_i32 + p.E + 1;
+            if (kExpand)
+                for (int i = tid; i < p.E; i += nthr) rows[i] = 0;
+            const int n = count_sent(p, 0).x;
+            __syncthreads();
+            count_hits(p, smem_i32);
+            if (kExpand) count_tokens<1, true>(p.topk_idx, 0, p.T, K, p.E, choices_in_pairs(p.topk_idx, K), rows);
+            __syncthreads();
+            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
+            __syncthreads();
+            exclusive_sums(smem_i32, p.E);
+            for (int i = tid; i <= p.E; i += nthr)
+                p.psum_expert[i] = smem_i32[i] + (kExpand && i < p.E ? rows[i] : 0);
+            if (tid == 0) p.psum_rank[0] = n;
+            tell_host(p, n);
+            return;
+        }
+        bid -= 1;
+    }
+    const int t0 = bid * p.C;
+    if (t0 >= p.T) return;
+    const int nt = min(p.C, p.T - t0), ne = nt * K, items = nt * ntiles;
+    auto load_item = [&](int item) {
+        V32 r = {};
+        const int tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
+        if (item < items && c < nchunks)
+            r = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)(t0 + tok) * p.H + (size_t)c * 16) * 2);
+        return r;
+    };
+    constexpr int kAhead = kExpand ? 1 : 4;
+    V32 v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) v[u] = load_item(warp + u * nwarps);
+    int64_t raw = -1;
+    float w = 0.f;
+    if (tid < ne) {
+        raw = ld_ro(p.topk_idx + (size_t)t0 * K + tid);
+        if (p.topk_weights) w = ld_ro(p.topk_weights + (size_t)t0 * K + tid);
+    }
+    const int e = (int)raw >= 0 && (int)raw < p.E ? (int)raw : -1;
+    if (tid < ne) s_exp[tid] = e;
+    if (kCount) {
+        const int pos = count_sent(p, t0).y;  // (its barriers make s_exp visible as well)
+        bool any = false;
+        for (int k = 0; k < K; ++k) any |= s_exp[k] >= 0;
+        if (tid == 0) s_pos[0] = any ? pos : -1, p.token_pos[t0] = any ? pos : -1;
+        if (kExpand) {
+            int* before = smem_i32 + p.E + 1;
+            for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
+            for (int i = tid; i < p.E; i += nthr) before[i] = 0;
+            __syncthreads();
+            count_hits(p, smem_i32);
+            count_tokens<1, true>(p.topk_idx, 0, t0, K, p.E, choices_in_pairs(p.topk_idx, K), before);
+            __syncthreads();
+            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
+            __syncthreads();
+            exclusive_sums(smem_i32, p.E);
+            if (tid < ne) {
+                bool last = e >= 0;
+                for (int k = tid + 1; k < K; ++k) last = last && s_exp[k] != e;
+                const int row = last ? smem_i32[e] + before[e] : -1;
+                s_row[tid] = row;
+                p.rows[(size_t)t0 * K + tid] = row;
+            }
+        }
+    } else {
+        pdl_wait();
+        if (tid < nt) {
+            const int pos = ld_ro(p.token_pos + t0 + tid);
+            s_pos[tid] = pos < p.T ? pos : -1;
+        }
+        if (kExpand && tid < ne) s_row[tid] = ld_ro(p.rows + (size_t)t0 * K + tid);
+    }
+    if (kExpand && tid < ne && s_row[tid] >= p.max_rows) {  // aligned segments beyond the caller's tensor
+        s_row[tid] = -1;
+        atomicOr(p.status, kStatusSlotRange);
+    }
+    __syncthreads();
+    if (tid < ne) {
+        const int tok = tid / K, k = tid - tok * K, pos = s_pos[tok];
+        int master = 0;
+        for (int j = 0; j < K; ++j)
+            if (s_exp[tok * K + j] >= 0) master = j;
+        const size_t at = (size_t)t0 * K + tid;
+        p.dst_slot[at] = pos >= 0 && k == master ? pos : -1;
+        if (p.copied_topk_idx) p.copied_topk_idx[at] = raw;
+        if (pos >= 0) {
+            p.recv_topk_idx[(size_t)pos * K + k] = e;
+            int32_t* md = p.recv_src_metadata + (size_t)pos * (K + 2);
+            if (k == 0) md[0] = t0 + tok;
+            if (k == 1 % K) md[1] = master;
+            if (kExpand) {
+                const int row = s_row[tid];
+                md[2 + k] = row;
+                if (p.recv_topk_weights && row >= 0) p.recv_topk_weights[row] = w;
+            } else if (p.recv_topk_weights) {
+                p.recv_topk_weights[(size_t)pos * K + k] = w;
+            }
+        }
+    }
+    char* out = static_cast<char*>(p.recv_x);
+    for (int i0 = warp; i0 < items; i0 += nwarps * kAhead) {
+        if (i0 != warp) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) v[u] = load_item(i0 + u * nwarps);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int item = i0 + u * nwarps;
+            if (item >= items) break;
+            const int tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
+            if (c >= nchunks) continue;
+            if (kExpand) {
+                for (int k = tok * K; k < (tok + 1) * K; ++k)
+                    if (s_row[k] >= 0) st32(out + ((size_t)s_row[k] * p.H + (size_t)c * 16) * 2, v[u]);
+            } else if (s_pos[tok] >= 0) {
+                st32(out + ((size_t)s_pos[tok] * p.H + (size_t)c * 16) * 2, v[u]);
+            }
+        }
+    }
+}
+
 __global__ void ep_elastic_fill_ones_kernel(float* w, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         w[i] = 1.0f;
@@ -354,18 +693,10 @@ cudaError_t launch_elastic_epilogue(const ElasticEpilogueParams& p, int num_sms,
                                     bool pdl) {
     const int cap_blocks = (p.R * p.M + kWarps - 1) / kWarps;
     const int grid = max(1, min(2 * num_sms, cap_blocks));
-    LaunchScope scope("ep_elastic_epilogue", stream);
     // with `pdl` the blocks may become resident while the exchange's last kernel drains;
     // they wait for its completion before they read anything
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kThreads), cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    if (pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr, cfg.numAttrs = 1;
-    }
-    return scope.done(cudaLaunchKernelEx(&cfg, ep_elastic_epilogue_kernel, p));
+    return launch_kernel("ep_elastic_epilogue", ep_elastic_epilogue_kernel, dim3(grid), dim3(kThreads), 0, 1,
+                         LaunchCtx{stream, num_sms, pdl}, p);
 }
 
 cudaError_t launch_elastic_expand_scan(const ElasticExpandParams& p, cudaStream_t stream) {
@@ -385,6 +716,68 @@ cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int n
     LaunchScope scope("ep_elastic_local_reduce", stream);
     ep_elastic_local_reduce_kernel<<<4 * num_sms, kThreads, 0, stream>>>(p);
     return scope.done(cudaGetLastError());
+}
+
+namespace {
+// Threads per block of the layout kernel with clusters of `blocks`; 0: does not fit.
+int single_layout_threads(int T, int blocks) {
+    const int threads = ((T + blocks - 1) / blocks + 31) / 32 * 32;
+    return threads >= 32 && threads <= 1024 ? threads : 0;
+}
+size_t single_layout_smem(int E, int threads, bool expand) {
+    return (size_t)(4 * (E + 1) + 1 + (expand ? 2 * (threads / 32) * (E + 1) : 0)) * sizeof(int);
+}
+constexpr size_t kSingleSmemMax = 200 * 1024;
+bool counts_in_copy_kernel(int T, int num_sms) { return T <= 2 * num_sms; }
+}  // namespace
+
+bool elastic_single_fits(int T, int K, int E) {
+    const int threads = single_layout_threads(T < 1 ? 1 : T, kSingleClusterLarge);
+    return K <= kMaxTopk && E <= kMaxExperts && threads != 0 && single_layout_smem(E, threads, true) <= kSingleSmemMax;
+}
+
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx) {
+    const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    if (counts_in_copy_kernel(p.T, ctx.num_sms)) {
+        // one launch: a block per token (every SM has one or two) and the block of the counts
+        p.C = 1;
+        const int warps = ntiles < 8 ? 8 : ntiles < 16 ? ntiles : 16;
+        auto k = expand ? ep_elastic_single_copy_kernel<true, true> : ep_elastic_single_copy_kernel<false, true>;
+        return launch_kernel("ep_elastic_single_copy", k, dim3(1 + p.T), dim3(warps * 32),
+                             (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
+    }
+    // (sixteen blocks, an opt-in cluster size, once eight would have more than 8 warps each)
+    static std::atomic<int> large{1};
+    cudaError_t err = cudaErrorInvalidConfiguration;
+    for (int blocks : {kSingleClusterLarge, kSingleCluster}) {
+        if (blocks == kSingleClusterLarge && (p.T <= kSingleCluster * 256 || !large.load())) continue;
+        const int threads = single_layout_threads(p.T, blocks);
+        const size_t smem = threads ? single_layout_smem(p.E, threads, expand) : 0;
+        if (threads == 0 || smem > kSingleSmemMax) continue;
+        auto k = expand ? ep_elastic_single_layout_kernel<true> : ep_elastic_single_layout_kernel<false>;
+        if ((err = allow_shared_memory(reinterpret_cast<const void*>(k), smem))) return err;
+        if (blocks == kSingleClusterLarge &&
+            (err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
+            return err;
+        err = launch_kernel("ep_elastic_single_layout", k, dim3(blocks), dim3(threads), smem, blocks, ctx, p);
+        if (err == cudaSuccess) break;
+        if (blocks == kSingleCluster) return err;
+        cudaGetLastError();
+        large.store(0);
+    }
+    if (err != cudaSuccess) return err;
+    LaunchCtx chained = ctx;
+    chained.pdl = ctx.chain;
+    // a warp gets about four tiles of plain rows, or one tile that is stored K times
+    int c = (expand ? 16 : 64) / ntiles;
+    if (c > 8) c = 8;
+    if (c > 128 / p.K) c = 128 / p.K;
+    const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
+    p.C = c < 1 ? 1 : c < most ? c : most;
+    int warps = p.C * ntiles;
+    warps = warps > 16 ? 16 : warps < 4 ? 4 : warps;
+    auto k = expand ? ep_elastic_single_copy_kernel<true, false> : ep_elastic_single_copy_kernel<false, false>;
+    return launch_kernel("ep_elastic_single_copy", k, dim3((p.T + p.C - 1) / p.C), dim3(warps * 32), 0, 1, chained, p);
 }
 
 cudaError_t launch_elastic_fill_ones(float* w, size_t n, cudaStream_t stream) {

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "ep_device.cuh"
+#include "ep_launch.cuh"
 #include "ep_routing.cuh"
 
 namespace mcep {
@@ -100,52 +101,31 @@ cudaError_t LaunchScope::done(cudaError_t err) {
     return err;
 }
 
+bool kernel_timing_on() { return g_timing.load(); }
+
+cudaError_t allow_shared_memory(const void* kernel, size_t smem) {
+    if (smem <= 40 * 1024) return cudaSuccess;
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& have = allowed[std::make_pair(kernel, dev)];
+    if (smem <= have) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) have = smem;
+    return e;
+}
+
 namespace kernels {
 
 constexpr unsigned kFull = 0xffffffffu;
 
 template <typename... KArgs, typename... Args>
-cudaError_t launch_clusters(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                            int cluster, const LaunchCtx& ctx, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx.stream;
-    cudaLaunchAttribute attr[2];
-    cfg.attrs = attr;
-    if (cluster > 1) {
-        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-        attr[cfg.numAttrs].val.clusterDim.x = cluster;
-        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
-        ++cfg.numAttrs;
-    }
-    const bool timing = g_timing.load();
-    if (ctx.pdl && !timing) {
-        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
-        ++cfg.numAttrs;
-    }
-    TimingRec r{name, nullptr, nullptr};
-    if (timing) {
-        cudaEventCreate(&r.a);
-        cudaEventCreate(&r.b);
-        cudaEventRecord(r.a, ctx.stream);
-    }
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-    if (timing) {
-        cudaEventRecord(r.b, ctx.stream);
-        std::lock_guard<std::mutex> lk(g_timing_mu);
-        g_recs.push_back(r);
-    }
-    if (err == cudaSuccess) g_launches.fetch_add(1);
-    return err;
-}
-
-template <typename... KArgs, typename... Args>
 cudaError_t launch(const char* name, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                    const LaunchCtx& ctx, Args&&... args) {
-    return launch_clusters(name, kernel, grid, block, smem, 1, ctx, std::forward<Args>(args)...);
+    return launch_kernel(name, kernel, grid, block, smem, 1, ctx, std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
@@ -377,7 +357,7 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             const int i = i0 + u * nthr;
-            ev[u] = i < n ? (int)__ldg(p.topk_idx + i) : -1;
+            ev[u] = i < n ? (int)ld_ro(p.topk_idx + i) : -1;
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -411,7 +391,7 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             const int i = i0 + u * nthr;
-            ev[u] = i < n ? (int)__ldg(p.topk_idx + i) : -2;
+            ev[u] = i < n ? (int)ld_ro(p.topk_idx + i) : -2;
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -420,7 +400,7 @@ __global__ void __launch_bounds__(1024)
             if (e >= e0 && e < e1) {
                 const int t = i / p.K, k = i - t * p.K;
                 bool dup = false;
-                for (int kk = 0; kk < k; ++kk) dup |= ((int)__ldg(p.topk_idx + t * p.K + kk) == e);
+                for (int kk = 0; kk < k; ++kk) dup |= ((int)ld_ro(p.topk_idx + t * p.K + kk) == e);
                 const int o = (e - e0) * words + (t >> 5);
                 p.slot[i] = dup ? -1 : (int)(wpre[o] + __popc(mask[o] & ((1u << (t & 31)) - 1u)));
             } else if (e < 0 && i < n && blockIdx.x == 0) {
@@ -443,7 +423,7 @@ __global__ void __launch_bounds__(1024)
         int carry = 0;
         for (int b = 0; b < L; b += 32) {
             const int le = b + lane;
-            const int c = le < L ? __ldcg(p.count + r * L + le) : 0;
+            const int c = le < L ? ld_l2(p.count + r * L + le) : 0;
             const int incl = warp_inclusive_scan(c, lane);
             if (le < L && p.expert_prefix) p.expert_prefix[r * L + le] = carry + incl - c;
             carry += __shfl_sync(kFull, incl, 31);
@@ -471,7 +451,7 @@ __device__ __forceinline__ void request_token_choices(const int64_t* topk_idx, i
     for (int k = 0; k < kMaxTopk; ++k) {
         e[k] = -1;
         if (t < T && k < K) {
-            const int v = (int)__ldg(topk_idx + (size_t)t * K + k);
+            const int v = (int)ld_ro(topk_idx + (size_t)t * K + k);
             e[k] = (v >= 0 && v < E) ? v : -1;
         }
     }
@@ -540,7 +520,7 @@ __global__ void __launch_bounds__(256) ep_layout_slot_kernel(LayoutParams p) {
             int v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                v[u] = c0 + u < (int)blockIdx.x ? __ldcg(p.chunk_hist + (size_t)(c0 + u) * p.E + i) : 0;
+                v[u] = c0 + u < (int)blockIdx.x ? ld_l2(p.chunk_hist + (size_t)(c0 + u) * p.E + i) : 0;
 #pragma unroll
             for (int u = 0; u < 8; ++u) sum += v[u];
         }
@@ -765,12 +745,12 @@ __device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsen
         const int nt = min(v.C, v.T - t0), ne = nt * K, items = nt * ntiles;
         const int t1 = t0 + nsend * v.C;
         int raw = -1, slot = 0;
-        if (tid < ne) raw = (int)__ldg(v.topk_idx + (size_t)t0 * K + tid);
+        if (tid < ne) raw = (int)ld_ro(v.topk_idx + (size_t)t0 * K + tid);
         if (kCount) {
             count_tokens<1>(v.topk_idx, counted, t0, K, v.E, choices_in_pairs(v.topk_idx, K), hist);
         } else {
             ready();
-            if (tid < ne) slot = __ldg(v.slot + (size_t)t0 * K + tid);
+            if (tid < ne) slot = ld_ro(v.slot + (size_t)t0 * K + tid);
         }
         if (raw >= v.E) raw = -1;
         if (tid < ne) s_raw[tid] = raw;
@@ -928,7 +908,7 @@ __global__ void __launch_bounds__(256) ep_combine_invert_kernel(CombineInvertPar
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         const int le = (int)(i / p.M), j = (int)(i - (long long)le * p.M);
-        const long long lr = __ldg(p.layout_range + le * p.R + p.rank);
+        const long long lr = ld_ro(p.layout_range + le * p.R + p.rank);
         const int cnt = (int)(lr & 0xffffffffll);
         if (j >= cnt) continue;
         const int row = (int)(lr >> 32) + j;
@@ -936,14 +916,14 @@ __global__ void __launch_bounds__(256) ep_combine_invert_kernel(CombineInvertPar
             atomicOr(p.status, kStatusSlotRange);
             continue;
         }
-        const int t = __ldg(p.src_info + (size_t)le * RM + row);
+        const int t = ld_ro(p.src_info + (size_t)le * RM + row);
         if (t < 0 || t >= p.T) {
             atomicOr(p.status, kStatusBadSource);
             continue;
         }
         const int e = p.rank * p.L + le;
         for (int k = 0; k < p.K; ++k)
-            if ((int)__ldg(p.topk_idx + (size_t)t * p.K + k) == e) p.rowmap[(size_t)t * p.K + k] = row;
+            if ((int)ld_ro(p.topk_idx + (size_t)t * p.K + k) == e) p.rowmap[(size_t)t * p.K + k] = row;
     }
 }
 
@@ -1027,8 +1007,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     auto request = [&](int tok) {
         if (on && tok < end) {
             const size_t at = (size_t)tok * p.K + lane;
-            next_row = __ldg(p.rowmap + at);
-            if (!kAbs) next_e = (int)__ldg(p.topk_idx + at), next_w = __ldg(p.topk_weights + at);
+            next_row = ld_ro(p.rowmap + at);
+            if (!kAbs) next_e = (int)ld_ro(p.topk_idx + at), next_w = ld_ro(p.topk_weights + at);
         } else {
             next_row = -1;
         }
@@ -1082,19 +1062,19 @@ __global__ void __launch_bounds__(512) ep_combine_search_kernel(DirectCombinePar
         int e = -1;
         float w = 0.f;
         if (tid < p.K) {
-            e = (int)__ldg(p.topk_idx + (size_t)t * p.K + tid);
-            w = __ldg(p.topk_weights + (size_t)t * p.K + tid);
+            e = (int)ld_ro(p.topk_idx + (size_t)t * p.K + tid);
+            w = ld_ro(p.topk_weights + (size_t)t * p.K + tid);
         }
         for (int k = warp; k < p.K; k += nwarps) {
-            const int ek = (int)__ldg(p.topk_idx + (size_t)t * p.K + k);
+            const int ek = (int)ld_ro(p.topk_idx + (size_t)t * p.K + k);
             int row = -1;
             if (ek >= 0 && ek < p.E) {
-                const long long lr = __ldg(p.layout_range + ek);
+                const long long lr = ld_ro(p.layout_range + ek);
                 const int cnt = (int)(lr & 0xffffffffll), begin = (int)(lr >> 32);
                 for (int j0 = 0; j0 < cnt; j0 += 32) {
                     const int j = begin + j0 + lane;
                     const bool hit = j0 + lane < cnt && j < p.M &&
-                                     __ldg(p.src_info + (size_t)ek * p.M + j) == t;
+                                     ld_ro(p.src_info + (size_t)ek * p.M + j) == t;
                     const unsigned m = __ballot_sync(kFull, hit);
                     if (m) {
                         row = begin + j0 + __ffs(m) - 1;
@@ -1162,7 +1142,7 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
         if (!s_active[dr]) continue;
-        const int c = kCount ? hist[x] : __ldg(p.count + x);
+        const int c = kCount ? hist[x] : ld_ro(p.count + x);
         uint64_t* wd = reinterpret_cast<uint64_t*>(s_peer[dr] + p.w.cnt_off) + (p.rank * L + (x - dr * L));
         st_relaxed_sys(wd, ((uint64_t)p.seq << 32) | (uint32_t)(c + 1));
     }
@@ -1499,7 +1479,7 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
         int* beg = smem_i32 + n + 1;  // [n] first row of each (expert, source) segment
         for (int i = tid; i < n; i += nthr) {
             const int src = i % p.R;
-            const long long lr = __ldg(p.layout_range + i);
+            const long long lr = ld_ro(p.layout_range + i);
             int c = (int)(lr & 0xffffffffll);
             if (src == p.rank || !s_active[src]) c = 0;
             pre[i] = c;
@@ -1591,9 +1571,9 @@ __device__ __forceinline__ void combine_reduce_duty(const GroupCombineParams& p,
             const char* ptr = nullptr;
             float w = 0.f;
             if (tid < p.K) {
-                const int e = (int)__ldg(p.topk_idx + (size_t)t * p.K + tid);
-                w = __ldg(p.topk_weights + (size_t)t * p.K + tid);
-                const int row = __ldcg(p.rowmap + (size_t)t * p.K + tid);
+                const int e = (int)ld_ro(p.topk_idx + (size_t)t * p.K + tid);
+                w = ld_ro(p.topk_weights + (size_t)t * p.K + tid);
+                const int row = ld_l2(p.rowmap + (size_t)t * p.K + tid);
                 if (e >= 0 && e < p.E && row >= 0 && row < RM) {
                     const int o = e / L, le = e - o * L;
                     const size_t off = ((size_t)le * RM + row) * (size_t)p.H * 2;
@@ -1704,23 +1684,6 @@ using namespace kernels;
 // =============================================================================
 // launchers
 // =============================================================================
-// Kernels are allowed more than 48 KB of dynamic shared memory once per device.
-template <typename K>
-static cudaError_t allow_smem(K kernel, size_t smem) {
-    if (smem <= 40 * 1024) return cudaSuccess;
-    static std::mutex mu;
-    static std::map<std::pair<const void*, int>, size_t> allowed;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    size_t& have = allowed[std::make_pair(reinterpret_cast<const void*>(kernel), dev)];
-    if (smem <= have) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) have = smem;
-    return e;
-}
-
 // The chunked route: chunks of up to 256 tokens (fewer when the per-chunk bitmap
 // of all experts would not fit 48 KB of shared memory), at most 128 chunks, and
 // per-chunk histograms that fit the scratch the caller gave.
@@ -1755,13 +1718,13 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
         const int threads = layout_cluster_threads(p, blocks);
         if (threads == 0) continue;
         const size_t smem = (size_t)p.E * (threads / 16 + 2) * sizeof(int);
-        if (cudaError_t e = allow_smem(ep_layout_cluster_kernel, smem)) return e;
+        if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(ep_layout_cluster_kernel), smem)) return e;
         if (blocks == kLayoutClusterLarge) {
             cudaError_t e = cudaFuncSetAttribute(ep_layout_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e != cudaSuccess) return e;
         }
-        const cudaError_t e = launch_clusters("ep_layout_cluster", ep_layout_cluster_kernel, dim3(blocks), dim3(threads),
-                                              smem, blocks, ctx, p);
+        const cudaError_t e = launch_kernel("ep_layout_cluster", ep_layout_cluster_kernel, dim3(blocks), dim3(threads),
+                                            smem, blocks, ctx, p);
         if (e == cudaSuccess || blocks == kLayoutCluster) return e;
         cudaGetLastError();
         large.store(0);

@@ -25,7 +25,8 @@ constexpr int kStatusNoPeer = 8;  // a rank marked active has no mapped buffer
 struct LaunchCtx {
     cudaStream_t stream;
     int num_sms;
-    bool pdl;  // launch with programmatic stream serialisation
+    bool pdl;            // launch with programmatic stream serialisation
+    bool chain = false;  // the same for what follows the first kernel of a call made of several
 };
 
 // ---- routing layout ---------------------------------------------------------

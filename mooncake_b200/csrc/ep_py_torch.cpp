@@ -24,6 +24,7 @@
 #include <cstring>
 #include <initializer_list>
 #include <string>
+#include <vector>
 
 #include "mcep.h"
 
@@ -35,6 +36,7 @@ struct Library {
     decltype(&mcep_dispatch) dispatch;
     decltype(&mcep_combine) combine;
     decltype(&mcep_elastic_dispatch) elastic_dispatch;
+    decltype(&mcep_elastic_dispatch_counted) elastic_dispatch_counted;
     decltype(&mcep_elastic_combine) elastic_combine;
     decltype(&mcep_buffer_next_recv_x) next_recv_x;
     decltype(&mcep_event_create) event_create;
@@ -46,7 +48,7 @@ struct Library {
 } lib;
 
 const char* const kSymbols[] = {"mcep_last_error", "mcep_dispatch", "mcep_combine", "mcep_elastic_dispatch",
-                                "mcep_elastic_combine", "mcep_buffer_next_recv_x", "mcep_event_create",
+                                "mcep_elastic_dispatch_counted", "mcep_elastic_combine", "mcep_buffer_next_recv_x", "mcep_event_create",
                                 "mcep_event_current_stream_wait", "mcep_event_synchronize", "mcep_event_free",
                                 "mcep_hook_run", "mcep_hook_free"};
 constexpr size_t kNumSymbols = sizeof(kSymbols) / sizeof(kSymbols[0]);
@@ -512,6 +514,143 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
     END_HANDLE_TH_ERRORS
 }
 
+// elastic_dispatch_tensors(x, topk_idx, topk_weights or None, active_ranks, kept_idx or None, E, M,
+//                          alignment, do_expand, do_cpu_sync, timeout_us, async, in_place or None)
+//   -> (recv_x, recv_topk_idx, recv_topk_weights or None, recv_src_metadata, psum_rank, psum_expert,
+//       dst_buffer_slot_idx, kept_idx, counts or None, event), or None (as above)
+// `kept_idx`: the cached handle's routing (topk_idx is then that tensor); None: a copy is made.
+// psum_expert is [L + 1] with do_expand and its entries 1.. without, as the wrapper hands it out;
+// `counts` is the list of tokens per local expert (do_cpu_sync), the row tensors are then cut to length.
+PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    RuntimeObject* s = self_of(self);
+    if (nargs != 13) return PyErr_Format(PyExc_TypeError, "elastic_dispatch_tensors() takes 13 arguments");
+    if (!alive(s)) return nullptr;
+    Reader r{const_cast<PyObject**>(args)};
+    const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *w = tensor_of(args[2]);
+    const at::Tensor *active = tensor_of(args[3]), *cached = tensor_of(args[4]);
+    const int64_t E = r.num(5), M = r.num(6), alignment = r.num(7), timeout = r.num(10), R = s->num_ranks;
+    const int expand = r.flag(8), sync = r.flag(9), async = r.flag(11);
+    if (!r.ok) return nullptr;
+    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !usable_mask(active, R) || M < 0 || R < 1 ||
+        (args[2] != Py_None && !matrix(w, at::kFloat)))
+        Py_RETURN_NONE;
+    const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), L = E / R;
+    if (idx->size(0) != T || E < 0 || (w && w->sizes() != idx->sizes())) Py_RETURN_NONE;
+    const int64_t n_cap = M * R, out_cap = expand ? n_cap * K : n_cap;
+    const at::Device dev = x->device();
+
+    at::Tensor recv_x;
+    if (args[12] != Py_None && !expand) {
+        void* p = nullptr;
+        size_t n = 0;
+        if (lib.next_recv_x(s->buf, (int)M, (int)H, (int)R, 0, &p, &n)) return fail();
+        if (p != nullptr) {
+            PyObject* rows = PyObject_CallFunction(args[12], "KKLLO", (unsigned long long)reinterpret_cast<uintptr_t>(p),
+                                                   (unsigned long long)n, (long long)n_cap, (long long)H, args[0]);
+            if (rows == nullptr) return nullptr;
+            recv_x = *tensor_of(rows);
+            Py_DECREF(rows);
+        }
+    }
+    const bool in_place = recv_x.defined();
+    if (!in_place) recv_x = empty({out_cap, H}, at::kBFloat16, dev);
+    Arena small(dev);
+    const int64_t o_rank = small.reserve(R * 4), o_expert = small.reserve((L + 1) * 4), o_slot = small.reserve(T * K * 4);
+    const int64_t o_idx = small.reserve(n_cap * K * 8), o_md = small.reserve(n_cap * (K + 2) * 4);
+    const int64_t o_w = w ? small.reserve((expand ? out_cap : n_cap * K) * 4) : 0;
+    const int64_t o_kept = cached ? 0 : small.reserve(T * K * 8);
+    small.allocate();
+
+    mcep_elastic_dispatch_args a = {};
+    a.x = x->const_data_ptr(), a.x_element_size = 2, a.num_tokens = (int)T, a.hidden = (int)H;
+    a.topk_idx = static_cast<const int64_t*>(idx->const_data_ptr()), a.num_topk = (int)K;
+    a.topk_weights = w ? static_cast<const float*>(w->const_data_ptr()) : nullptr;
+    a.active_ranks = static_cast<int32_t*>(active->data_ptr());
+    a.num_experts = (int)E, a.num_max_tokens_per_rank = (int)M, a.expert_alignment = (int)alignment;
+    a.do_expand = expand, a.cached_mode = cached != nullptr, a.timeout_us = timeout;
+    a.async_with_compute_stream = async, a.compute_stream = current_stream();
+    a.psum_num_recv_tokens_per_scaleup_rank = reinterpret_cast<int32_t*>(small.at(o_rank));
+    a.psum_num_recv_tokens_per_expert = reinterpret_cast<int32_t*>(small.at(o_expert));
+    a.dst_buffer_slot_idx = reinterpret_cast<int32_t*>(small.at(o_slot));
+    a.recv_x = recv_x.data_ptr(), a.recv_topk_idx = reinterpret_cast<int64_t*>(small.at(o_idx));
+    a.recv_topk_weights = w ? reinterpret_cast<float*>(small.at(o_w)) : nullptr;
+    a.recv_src_metadata = reinterpret_cast<int32_t*>(small.at(o_md));
+    a.copied_topk_idx = cached ? nullptr : reinterpret_cast<int64_t*>(small.at(o_kept));
+    mcep_event* ev = nullptr;
+    std::vector<int32_t> host(sync ? R + L + 1 : 0);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = sync ? lib.elastic_dispatch_counted(s->buf, &a, host.data(), host.data() + R, &ev)
+              : lib.elastic_dispatch(s->buf, &a, &ev);
+    Py_END_ALLOW_THREADS
+    if (rc) return fail();
+
+    int64_t n = n_cap, n_out = out_cap;
+    PyObject* counts = sync ? PyList_New(L) : new_ref(Py_None);
+    if (counts == nullptr) return nullptr;
+    if (sync) {
+        const int32_t* psum = host.data() + R;
+        n = host[R - 1];
+        n_out = expand ? (L ? psum[L - 1] : 0) : n;
+        int64_t prev = 0;  // expanded: the entries are where the segments end, unaligned
+        for (int64_t i = 0; i < L; ++i) {
+            const int64_t c = expand ? psum[i] - (prev + alignment - 1) / alignment * alignment : psum[i + 1] - psum[i];
+            prev = psum[i];
+            PyList_SET_ITEM(counts, i, PyLong_FromLongLong(c));
+        }
+        if (n_out != recv_x.size(0)) recv_x = in_place ? recv_x.narrow(0, 0, n_out) : recv_x;
+        if (!in_place) recv_x.unsafeGetTensorImpl()->set_sizes_contiguous({n_out, H});
+    }
+    const int64_t first = expand ? 0 : 1;
+    return pack({wrap(std::move(recv_x)), wrap(small.view(o_idx, at::kLong, {n, K})),
+                 !w ? new_ref(Py_None)
+                    : wrap(expand ? small.view(o_w, at::kFloat, {n_out}) : small.view(o_w, at::kFloat, {n, K})),
+                 wrap(small.view(o_md, at::kInt, {n, K + 2})), wrap(small.view(o_rank, at::kInt, {R})),
+                 wrap(small.view(o_expert + 4 * first, at::kInt, {L + 1 - first})),
+                 wrap(small.view(o_slot, at::kInt, {T, K})),
+                 cached ? new_ref(args[4]) : wrap(small.view(o_kept, at::kLong, {T, K})), counts, wrap_event(ev)});
+    END_HANDLE_TH_ERRORS
+}
+
+// elastic_combine_tensors(x, topk_idx, topk_weights or None, psum_rank, recv_src_metadata, active_ranks,
+//                         E, M, do_expand, timeout_us, async) -> (combined_x, event), or None (as above)
+PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    RuntimeObject* s = self_of(self);
+    if (nargs != 11) return PyErr_Format(PyExc_TypeError, "elastic_combine_tensors() takes 11 arguments");
+    if (!alive(s)) return nullptr;
+    Reader r{const_cast<PyObject**>(args)};
+    const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *w = tensor_of(args[2]);
+    const at::Tensor *psum = tensor_of(args[3]), *md = tensor_of(args[4]), *active = tensor_of(args[5]);
+    const int64_t E = r.num(6), M = r.num(7), timeout = r.num(9);
+    const int expand = r.flag(8), async = r.flag(10);
+    if (!r.ok) return nullptr;
+    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !psum || !md || !usable_mask(active, s->num_ranks))
+        Py_RETURN_NONE;
+    const int64_t T = idx->size(0), K = idx->size(1), H = x->size(1);
+    at::Tensor out = empty({T, H}, at::kBFloat16, x->device());
+    mcep_elastic_combine_args a = {};
+    a.x = x->const_data_ptr(), a.num_input_tokens = (int)x->size(0), a.hidden = (int)H;
+    a.topk_idx = static_cast<const int64_t*>(idx->const_data_ptr());
+    a.num_combined_tokens = (int)T, a.num_topk = (int)K;
+    a.topk_weights = w ? static_cast<const float*>(w->const_data_ptr()) : nullptr;
+    a.psum_num_recv_tokens_per_scaleup_rank = static_cast<const int32_t*>(psum->const_data_ptr());
+    // (the handle's tensor by its address: it stays the same when the host cut it to length)
+    a.recv_src_metadata = reinterpret_cast<const int32_t*>(static_cast<const char*>(md->storage().data()) +
+                                                           md->storage_offset() * (int64_t)sizeof(int32_t));
+    a.active_ranks = static_cast<int32_t*>(active->data_ptr());
+    a.num_experts = (int)E, a.num_max_tokens_per_rank = (int)M, a.do_expand = expand, a.timeout_us = timeout;
+    a.async_with_compute_stream = async, a.compute_stream = current_stream();
+    a.combined_x = out.data_ptr();
+    mcep_event* ev = nullptr;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = lib.elastic_combine(s->buf, &a, &ev);
+    Py_END_ALLOW_THREADS if (rc) return fail();
+    return pack({wrap(std::move(out)), wrap_event(ev)});
+    END_HANDLE_TH_ERRORS
+}
+
 #define MCEP_FAST(fn) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn))
 
 PyMethodDef runtime_methods[] = {
@@ -533,6 +672,10 @@ PyMethodDef runtime_methods[] = {
      "none (include/mcep.h)."},
     {"dispatch_tensors", MCEP_FAST(runtime_dispatch_tensors), METH_FASTCALL, "Buffer.dispatch on checked tensors."},
     {"combine_tensors", MCEP_FAST(runtime_combine_tensors), METH_FASTCALL, "Buffer.combine on checked tensors."},
+    {"elastic_dispatch_tensors", MCEP_FAST(runtime_elastic_dispatch_tensors), METH_FASTCALL,
+     "ElasticBuffer.dispatch on checked tensors."},
+    {"elastic_combine_tensors", MCEP_FAST(runtime_elastic_combine_tensors), METH_FASTCALL,
+     "ElasticBuffer.combine on checked tensors."},
     {nullptr, nullptr, 0, nullptr}};
 PyType_Slot runtime_slots[] = {{Py_tp_doc, const_cast<char*>("The calls of an mcep_buffer; base of ep.Buffer.")},
                                {Py_tp_methods, runtime_methods},

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ep_device.cuh"
 #include "ep_kernels.cuh"
 
 namespace mcep {
@@ -26,12 +27,12 @@ __device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_id
 #pragma unroll
         for (int k = 0; k < KB; k += 2) {
             longlong2 v = make_longlong2(-1, -1);
-            if (k < K) v = __ldg(reinterpret_cast<const longlong2*>(p + k));
+            if (k < K) v = ld_ro(reinterpret_cast<const longlong2*>(p + k));
             e[k] = (int)v.x, e[k + 1] = (int)v.y;
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < KB; ++k) e[k] = k < K ? (int)__ldg(p + k) : -1;
+        for (int k = 0; k < KB; ++k) e[k] = k < K ? (int)ld_ro(p + k) : -1;
     }
 #pragma unroll
     for (int k = 0; k < KB; ++k)

@@ -386,6 +386,10 @@ size_t exchange_bytes(int num_ranks, int num_experts, int M, int hidden) {
 
 void set_after_deferred(mcep_buffer* b, std::function<int()> fn) { b->after_deferred = std::move(fn); }
 
+void count_dispatch_call(mcep_buffer* b) { ++b->dseq; }
+void count_combine_call(mcep_buffer* b) { ++b->cseq; }
+bool may_chain(const mcep_buffer* b, cudaStream_t stream) { return chain_with_pdl(b, stream); }
+
 int report_failure(int code, const char* message) { return fail(code, "%s", message); }
 
 }  // namespace mcep

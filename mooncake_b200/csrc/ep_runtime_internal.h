@@ -32,6 +32,14 @@ size_t exchange_bytes(int num_ranks, int num_experts, int M, int hidden);
 // has been launched (run once, then forgotten).
 void set_after_deferred(mcep_buffer* b, std::function<int()> fn);
 
+// Elastic calls that do not go through mcep_dispatch / mcep_combine count as one of
+// each all the same.
+void count_dispatch_call(mcep_buffer* b);
+void count_combine_call(mcep_buffer* b);
+
+// Whether kernels queued on `stream` may be chained with programmatic launches now.
+bool may_chain(const mcep_buffer* b, cudaStream_t stream);
+
 // Records the message mcep_last_error() returns and hands `code` back.
 int report_failure(int code, const char* message);
 

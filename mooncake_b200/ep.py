@@ -118,6 +118,8 @@ def _load() -> ctypes.CDLL:
         "mcep_dispatch": (i32, [vp, _c.POINTER(_DispatchArgs), _c.POINTER(vp), _c.POINTER(vp)]),
         "mcep_combine": (i32, [vp, _c.POINTER(_CombineArgs), _c.POINTER(vp), _c.POINTER(vp)]),
         "mcep_elastic_dispatch": (i32, [vp, _c.POINTER(_ElasticDispatchArgs), _c.POINTER(vp)]),
+        "mcep_elastic_dispatch_counted": (i32, [vp, _c.POINTER(_ElasticDispatchArgs), _c.POINTER(_c.c_int32),
+                                                _c.POINTER(_c.c_int32), _c.POINTER(vp)]),
         "mcep_elastic_combine": (i32, [vp, _c.POINTER(_ElasticCombineArgs), _c.POINTER(vp)]),
         "mcep_elastic_buffer_size_hint": (u64, [i32, i32, i32, i32]),
         "mcep_event_create": (i32, [u64, _c.POINTER(vp)]),
@@ -147,8 +149,8 @@ def _load_native():
     spec = importlib.util.spec_from_file_location("mooncake_b200._mcep_torch", _build.build_binding())
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
-    names = ("mcep_last_error", "mcep_dispatch", "mcep_combine", "mcep_elastic_dispatch", "mcep_elastic_combine",
-             "mcep_buffer_next_recv_x", "mcep_event_create", "mcep_event_current_stream_wait",
+    names = ("mcep_last_error", "mcep_dispatch", "mcep_combine", "mcep_elastic_dispatch",
+             "mcep_elastic_dispatch_counted", "mcep_elastic_combine", "mcep_buffer_next_recv_x", "mcep_event_create", "mcep_event_current_stream_wait",
              "mcep_event_synchronize", "mcep_event_free", "mcep_hook_run", "mcep_hook_free")
     mod.bind({n: _c.cast(getattr(_lib, n), _c.c_void_p).value for n in names})
     return mod

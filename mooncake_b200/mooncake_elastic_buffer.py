@@ -33,10 +33,6 @@ from . import ep
 from .mooncake_ep_buffer import EventOverlap, _DeviceBytes, _stream_ptr
 
 
-def _ceil_div(x: int, y: int) -> int:
-    return (x + y - 1) // y
-
-
 class EPHandle:
     """What `combine` (and a cached `dispatch`) needs from a `dispatch` call.
     Field names as in the reference (:46-81)."""
@@ -110,6 +106,8 @@ class ElasticBuffer:
         self.num_scaleout_ranks, self.num_scaleup_ranks = 1, self.num_ranks
         self.scaleout_rank_idx, self.scaleup_rank_idx = 0, self.rank_idx
         self.num_rdma_ranks, self.num_nvlink_ranks = 1, self.num_ranks
+        self._num_sms: dict = {}  # per device
+        self._ones: Optional[torch.Tensor] = None
         self.runtime: Optional[ep.Buffer] = ep.Buffer(self.rank_idx, self.num_ranks, num_bytes, False)
         self._connect_native()
         torch.cuda.synchronize()
@@ -161,7 +159,11 @@ class ElasticBuffer:
 
     def get_theoretical_num_sms(self, num_experts: int, num_topk: int) -> int:
         """Accepted for interface parity; the kernels size their own grids."""
-        return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+        dev = torch.cuda.current_device()
+        n = self._num_sms.get(dev)
+        if n is None:
+            n = self._num_sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+        return n
 
     def barrier(self, use_comm_stream: bool = True, with_cpu_sync: bool = False) -> None:
         """A barrier of the group on the device (reference :417-423)."""
@@ -177,6 +179,19 @@ class ElasticBuffer:
             raw = torch.as_tensor(_DeviceBytes(self.runtime, ptr, nbytes), device=device)
             t = self._views[key] = raw.view(torch.bfloat16).view(shape)
         return t
+
+    def _rows_in_place(self, ptr: int, nbytes: int, rows: int, hidden: int, x: torch.Tensor) -> torch.Tensor:
+        """The symmetric memory in which the next dispatch call of a group lands its rows."""
+        return self._symmetric_tensor(ptr, nbytes, (rows, hidden), x.device)
+
+    def _active_ranks(self, device: torch.device) -> torch.Tensor:
+        """All ranks take part. A group's call may clear entries (timeouts), so each gets
+        a mask of its own; a single rank waits for nobody and never writes it."""
+        if self.num_ranks > 1:
+            return torch.ones(self.num_ranks, dtype=torch.int32, device=device)
+        if self._ones is None or self._ones.device != device:
+            self._ones = torch.ones(1, dtype=torch.int32, device=device)
+        return self._ones
 
     def _timeout_us(self) -> int:
         return -1 if self.num_gpu_timeout_secs < 0 else int(self.num_gpu_timeout_secs) * 1_000_000
@@ -213,82 +228,35 @@ class ElasticBuffer:
                 raise AssertionError("topk_idx must be provided when cached handle is not provided")
             expert_alignment = 1 if expert_alignment is None else expert_alignment
             do_cpu_sync = True if do_cpu_sync is None else do_cpu_sync
-        assert x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16
-        assert topk_idx.dtype == torch.int64 and topk_idx.is_contiguous()
         if num_experts is None:
             num_experts = int(torch.max(topk_idx).item()) + 1
         if num_max_tokens_per_rank is None:
             num_max_tokens_per_rank = self.num_max_tokens_per_rank or x.shape[0]
         if num_sms is None:
             num_sms = self.get_theoretical_num_sms(num_experts, topk_idx.shape[1])
-        dev = x.device
-        T, H, K = int(x.shape[0]), int(x.shape[1]), int(topk_idx.shape[1])
-        L = num_experts // self.num_ranks
-        n_cap = num_max_tokens_per_rank * self.num_ranks
-        out_cap = n_cap * K if do_expand else n_cap
-
-        active_ranks = torch.ones(self.num_ranks, dtype=torch.int32, device=dev)
-        psum_expert = torch.empty(L + 1, dtype=torch.int32, device=dev)
-        psum_rank = torch.empty(self.num_scaleup_ranks, dtype=torch.int32, device=dev)
-        dst_buffer_slot_idx = torch.empty((T, K), dtype=torch.int32, device=dev)
-        recv_x = None
-        if self.recv_in_place and not do_expand:
-            # where the exchange lands the rows: the flat tensor itself
-            ptr, nbytes = self.runtime.next_recv_x(num_max_tokens_per_rank, H, self.num_ranks, False)
-            if ptr:
-                recv_x = self._symmetric_tensor(ptr, nbytes, (n_cap, H), dev)
-        if recv_x is None:
-            recv_x = torch.empty((out_cap, H), dtype=x.dtype, device=dev)
-        recv_topk_idx = torch.empty((n_cap, K), dtype=topk_idx.dtype, device=dev)
-        recv_topk_weights = (torch.empty((out_cap,) if do_expand else (n_cap, K), dtype=torch.float32,
-                                         device=dev) if topk_weights is not None else None)
-        recv_src_metadata = torch.empty((n_cap, K + 2), dtype=torch.int32, device=dev)
-        if topk_weights is not None:
-            assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
-        # the handle keeps its own copy of the routing, as the reference's does (:679); the
-        # copy is written by the call's first kernel
-        kept_idx = handle.topk_idx if handle is not None else torch.empty_like(topk_idx)
-        event = self.runtime.elastic_dispatch(
-            x.data_ptr(), x.element_size(), 0, T, H, 0, 0, 0, topk_idx.data_ptr(), K,
-            0 if topk_weights is None else topk_weights.data_ptr(), active_ranks.data_ptr(),
-            num_experts, num_max_tokens_per_rank, expert_alignment, do_expand,
-            async_with_compute_stream, _stream_ptr(), handle is not None, psum_rank.data_ptr(),
-            psum_expert.data_ptr(), dst_buffer_slot_idx.data_ptr(), recv_x.data_ptr(), 0,
-            recv_topk_idx.data_ptr(), 0 if recv_topk_weights is None else recv_topk_weights.data_ptr(),
-            recv_src_metadata.data_ptr(), self._timeout_us(),
-            0 if handle is not None else kept_idx.data_ptr())
-        handle_psum_expert = psum_expert if do_expand else psum_expert[1:]
-
-        counts: List[int] = []
-        if do_cpu_sync:
-            if event is not None:
-                event.synchronize()
-            rank_cpu, expert_cpu = psum_rank.cpu(), psum_expert.cpu()
-            n_recv = int(rank_cpu[self.num_scaleup_ranks - 1])
-            n_out = n_recv
-            if do_expand:
-                prev = 0
-                for i in range(L):
-                    cur = int(expert_cpu[i])
-                    counts.append(cur - _ceil_div(prev, expert_alignment) * expert_alignment)
-                    prev = cur
-                n_out = 0 if L == 0 else int(expert_cpu[L - 1])
-            else:
-                counts = [int(expert_cpu[i + 1] - expert_cpu[i]) for i in range(L)]
-            recv_x = recv_x[:n_out]
-            recv_topk_idx = recv_topk_idx[:n_recv]
-            if recv_topk_weights is not None:
-                recv_topk_weights = recv_topk_weights[:n_out]
-            recv_src_metadata = recv_src_metadata[:n_recv]
-
-        out_handle = EPHandle(do_expand, num_experts, expert_alignment, num_max_tokens_per_rank,
-                              num_sms, kept_idx, counts, psum_rank, handle_psum_expert,
-                              recv_src_metadata, dst_buffer_slot_idx, None, None, native_handle=True)
-        keep = (x, topk_idx, kept_idx, active_ranks, recv_x, recv_topk_idx, psum_rank, psum_expert,
-                recv_src_metadata, dst_buffer_slot_idx) + \
-            (() if topk_weights is None else (topk_weights, recv_topk_weights))
-        return (recv_x, recv_topk_idx, recv_topk_weights, out_handle,
-                EventOverlap(event, keep if async_with_compute_stream else None))
+        active_ranks = self._active_ranks(x.device)
+        # the handle keeps its own copy of the routing, as the reference's does (:679), written by
+        # the call's kernels; a cached handle's is used again
+        out = self.runtime.elastic_dispatch_tensors(
+            x, topk_idx, topk_weights, active_ranks, None if handle is None else handle.topk_idx, num_experts,
+            num_max_tokens_per_rank, expert_alignment, do_expand, do_cpu_sync, self._timeout_us(),
+            async_with_compute_stream, self._rows_in_place if self.recv_in_place else None)
+        if out is None:
+            assert x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16
+            assert topk_idx.dtype == torch.int64 and topk_idx.is_contiguous()
+            assert topk_weights is None or (topk_weights.dtype == torch.float32 and topk_weights.is_contiguous())
+            raise AssertionError("dispatch takes CUDA tensors x [T, H], topk_idx [T, K], topk_weights [T, K]")
+        (recv_x, recv_topk_idx, recv_topk_weights, recv_src_metadata, psum_rank, psum_expert, dst_buffer_slot_idx,
+         kept_idx, counts, event) = out
+        out_handle = EPHandle(do_expand, num_experts, expert_alignment, num_max_tokens_per_rank, num_sms, kept_idx,
+                              counts or [], psum_rank, psum_expert, recv_src_metadata, dst_buffer_slot_idx, None, None,
+                              native_handle=True)
+        keep = None
+        if async_with_compute_stream:
+            keep = (x, topk_idx, kept_idx, active_ranks, recv_x, recv_topk_idx, psum_rank, psum_expert,
+                    recv_src_metadata, dst_buffer_slot_idx) + \
+                (() if topk_weights is None else (topk_weights, recv_topk_weights))
+        return recv_x, recv_topk_idx, recv_topk_weights, out_handle, EventOverlap(event, keep)
 
     # ------------------------------------------------------------------ combine
     def combine(self, x: torch.Tensor, handle: EPHandle, topk_weights: Optional[torch.Tensor] = None,
@@ -298,21 +266,18 @@ class ElasticBuffer:
             raise RuntimeError("ElasticBuffer has been destroyed")
         if handle.native_handle is None:
             raise RuntimeError("EPHandle does not contain a native handle")
-        assert x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16
         if handle.do_expand and topk_weights is not None:
             # the reference asserts the same on the device (combine_official.cuh:70)
             raise AssertionError("topk_weights must be None with an expanded layout")
-        dev = x.device
-        active_ranks = torch.ones(self.num_ranks, dtype=torch.int32, device=dev)
-        T, K = int(handle.topk_idx.shape[0]), int(handle.topk_idx.shape[1])
-        combined_x = torch.empty((T, x.shape[1]), dtype=x.dtype, device=dev)
-        event = self.runtime.elastic_combine(
-            x.data_ptr(), int(x.shape[0]), int(x.shape[1]), handle.topk_idx.data_ptr(), T, K,
-            0 if topk_weights is None else topk_weights.data_ptr(),
-            handle.psum_num_recv_tokens_per_scaleup_rank.data_ptr(),
-            handle.recv_src_metadata.data_ptr(), active_ranks.data_ptr(), handle.num_experts,
-            handle.num_max_tokens_per_rank, handle.do_expand, async_with_compute_stream,
-            _stream_ptr(), combined_x.data_ptr(), self._timeout_us())
-        keep = (x, active_ranks, combined_x, handle.topk_idx, handle.recv_src_metadata) + \
-            (() if topk_weights is None else (topk_weights,))
-        return combined_x, None, EventOverlap(event, keep if async_with_compute_stream else None)
+        active_ranks = self._active_ranks(x.device)
+        res = self.runtime.elastic_combine_tensors(
+            x, handle.topk_idx, topk_weights, handle.psum_num_recv_tokens_per_scaleup_rank, handle.recv_src_metadata,
+            active_ranks, handle.num_experts, handle.num_max_tokens_per_rank, handle.do_expand, self._timeout_us(),
+            async_with_compute_stream)
+        assert res is not None, "combine takes a contiguous [n, H] bf16 CUDA tensor"
+        combined_x, event = res
+        keep = None
+        if async_with_compute_stream:
+            keep = (x, active_ranks, combined_x, handle.topk_idx, handle.recv_src_metadata) + \
+                (() if topk_weights is None else (topk_weights,))
+        return combined_x, None, EventOverlap(event, keep)

@@ -1,0 +1,81 @@
+"""The single-rank path of the elastic calls at the sizes where its kernels change:
+the last batch that is done in one launch and the first with a layout kernel,
+edges of its warps, blocks and cluster sizes, the first batch beyond it (general
+path), several rows per block and their remainders, odd top-k, repeats inside a
+token, padding tokens, an alignment; through `ElasticBuffer` with and without the
+wait for the counts."""
+import pytest
+import torch
+
+from mooncake_b200 import ElasticBuffer
+from oracle import elastic_oracle as eo
+from tests.ep_harness import FakeGroup, make_rank_inputs
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [  # T, H, E, K, expand, alignment
+    (1, 128, 4, 1, False, 1), (1, 8320, 8, 2, True, 4), (33, 512, 256, 8, True, 1), (296, 256, 16, 3, False, 8),
+    (296, 640, 16, 16, True, 2), (297, 256, 16, 3, True, 1), (297, 7168, 8, 4, False, 1), (1023, 128, 4096, 2, True, 1),
+    (1024, 1152, 24, 6, False, 1), (2049, 128, 64, 8, True, 16), (2500, 256, 4096, 1, False, 1),
+    (4097, 128, 8, 5, False, 1), (16385, 128, 4, 1, False, 1), (600, 128, 5000, 2, False, 1),
+]
+
+
+@pytest.mark.parametrize("T,H,E,K,expand,alignment", SIZES)
+def test_dispatch_and_combine(T, H, E, K, expand, alignment):
+    M = T + 3 + (E * (alignment - 1) // K if expand else 0)  # room for the aligned segments
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K, num_gpu_timeout_secs=2)
+    x, idx, w = make_rank_inputs(31, 0, T, H, E, K, "uniform", n_mask=T // 9)
+    if K > 1 and not expand:
+        idx[::4, 0] = idx[::4, K - 1]  # an expert twice in one token's list (the oracle would expand it twice)
+    if T > 2:
+        idx[1], idx[T // 2] = -1, -1   # tokens that go nowhere
+    want = eo.elastic_dispatch([x], [idx], [w], E, M, alignment, expand)[0]
+    n = want["n"]
+    dx, di, dw = x.cuda(), idx.cuda(), w.cuda()
+    for sync in (True, False):
+        recv, ridx, rw, h, _ = buf.dispatch(dx, topk_idx=di, topk_weights=dw, num_experts=E, num_max_tokens_per_rank=M,
+                                            expert_alignment=alignment, do_expand=expand, do_cpu_sync=sync)
+        torch.cuda.synchronize()
+        assert h.psum_num_recv_tokens_per_scaleup_rank.tolist() == [n]
+        psum = want["psum_expert"].tolist()
+        assert h.psum_num_recv_tokens_per_expert.tolist() == (psum if expand else psum[1:])
+        assert torch.equal(h.dst_buffer_slot_idx.cpu(), want["dst_buffer_slot_idx"]) and torch.equal(h.topk_idx, di)
+        if sync:
+            assert ridx.shape[0] == h.num_recv_tokens == n
+            # (what the reference's wrapper makes of the sums, mooncake_elastic_buffer.py:650-662)
+            starts = [-(-v // alignment) * alignment for v in [0] + psum[:E - 1]] if expand else psum[:E]
+            assert h.num_recv_tokens_per_expert_list == [e - s for s, e in zip(starts, psum[:E] if expand else psum[1:])]
+        assert torch.equal(ridx[:n].cpu(), want["recv_topk_idx"])
+        md = h.recv_src_metadata[:n].cpu()
+        assert torch.equal(md if expand else md[:, :2],
+                           want["recv_src_metadata"] if expand else want["recv_src_metadata"][:, :2])
+        used = want["used"] if expand else slice(0, n)
+        rows = want["recv_x"].shape[0] if expand else n
+        got = recv[:min(rows, recv.shape[0])].cpu()
+        keep = want["used"][:got.shape[0]] if expand else used
+        assert torch.equal(got[keep].view(torch.int16), want["recv_x"][:got.shape[0]][keep].view(torch.int16))
+        assert torch.equal(rw[:got.shape[0]].cpu()[keep], want["recv_topk_weights"][:got.shape[0]][keep])
+        y = (recv.float() * 1.25).nan_to_num().to(torch.bfloat16)
+        out, _, _ = buf.combine(y, h)
+        torch.cuda.synchronize()
+        ref = eo.elastic_combine([y.cpu()], [want], [idx], E, expand)[0]
+        assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
+    assert buf.runtime.status() == 0
+
+
+def test_counts_of_back_to_back_calls_and_an_empty_batch():
+    """Every waiting call gets its own counts, also with nothing to send."""
+    T, H, E, K = 700, 128, 8, 2
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    x = torch.zeros((T, H), dtype=torch.bfloat16, device="cuda")
+    for c in range(6):
+        idx = torch.full((T, K), -1, dtype=torch.int64)
+        idx[: 117 * c, 0] = c
+        recv, _, _, h, _ = buf.dispatch(x, topk_idx=idx.cuda(), num_experts=E, num_max_tokens_per_rank=T)
+        assert recv.shape == (117 * c, H)
+        assert h.num_recv_tokens_per_expert_list == [117 * c if e == c else 0 for e in range(E)]
+        out, _, _ = buf.combine(recv, h)
+        assert out.shape == (T, H) and not bool(out.any())
+    recv, _, _, h, _ = buf.dispatch(x[:0], topk_idx=idx[:0].cuda(), num_experts=E, num_max_tokens_per_rank=T)
+    assert recv.shape == (0, H) and h.num_recv_tokens_per_expert_list == [0] * E
