@@ -54,9 +54,9 @@ __device__ __forceinline__ void st_volatile_s32(int* p, int v) {
 // ---- inputs -----------------------------------------------------------------------
 // Data that the kernel AHEAD may have written and this one only reads. Not __ldg and
 // not ld.global.nc: both promise that the data does not change while the kernel runs,
-// and a kernel that was launched early runs already while it waits for the one
-// ahead - the compiler moved such loads above griddepcontrol.wait, and a copy kernel
-// read the positions of an earlier call. Plain volatile loads stay below it.
+// and a kernel that was launched early runs already while the one ahead still writes.
+// With them a copy kernel read the positions of an earlier call although the loads
+// stood behind griddepcontrol.wait; plain volatile loads are ordered by it.
 __device__ __forceinline__ int ld_ro(const int32_t* p) {
     int v;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -151,14 +151,32 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The word at the same place of block `rank`'s shared memory.
+// The word at the same place of block `rank`'s shared memory. (Volatile, but no
+// memory clobber: a run of these loads is in flight together.)
 __device__ __forceinline__ int ld_cluster_s32(const int* p, int rank) {
     const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
     uint32_t remote;
     int v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote));
     return v;
+}
+// The sums of that word over all `blocks` blocks of the cluster and over those below
+// `rank`. One round trip: with the bounds as branches around the loads each of them
+// waited for the one before, 4 of the 9 us of a layout kernel.
+template <int kMaxBlocks>
+__device__ __forceinline__ int cluster_sum(const int* p, int rank, int blocks, int* lower) {
+    int v[kMaxBlocks];
+#pragma unroll
+    for (int r = 0; r < kMaxBlocks; ++r) v[r] = ld_cluster_s32(p, r < blocks ? r : blocks - 1);
+    int sum = 0, lo = 0;
+#pragma unroll
+    for (int r = 0; r < kMaxBlocks; ++r) {
+        if (r < blocks) sum += v[r];
+        if (r < rank) lo += v[r];
+    }
+    *lower = lo;
+    return sum;
 }
 
 // ---- bf16 / fp8 ------------------------------------------------------------------

@@ -347,39 +347,39 @@ __device__ __forceinline__ int aligned_count(int c, int a) { return (c + a - 1) 
 __device__ void exclusive_sums(int* a, int n) {
     __shared__ int s_sum[32];
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-    const int per = (n + nthr - 1) / nthr, b = min(tid * per, n), e = min(b + per, n);
+    const int per = n <= nthr ? 1 : (n + nthr - 1) / nthr, b = min(tid * per, n), e = min(b + per, n);
     int sum = 0;
     for (int i = b; i < e; ++i) sum += a[i];
-    int incl = sum;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int u = __shfl_up_sync(kAll, incl, d);
-        if (lane >= d) incl += u;
-    }
+    auto scan = [&](int v) {
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(kAll, v, d);
+            if (lane >= d) v += u;
+        }
+        return v;
+    };
+    const int incl = scan(sum);
     if (lane == 31) s_sum[warp] = incl;
     __syncthreads();
-    int run = incl - sum;
-    for (int w = 0; w < warp; ++w) run += s_sum[w];
+    // every warp scans the warps' sums for itself: no further barrier for them
+    const int mine = lane < nwarps ? s_sum[lane] : 0, warps = scan(mine);
+    int run = __shfl_sync(kAll, warps - mine, warp) + incl - sum;
     for (int i = b; i < e; ++i) {
         const int c = a[i];
         a[i] = run;
         run += c;
     }
-    __syncthreads();
-    if (tid == 0) {
-        int total = 0;
-        for (int w = 0; w < nwarps; ++w) total += s_sum[w];
-        a[n] = total;
-    }
+    if (tid == nthr - 1) a[n] = run;
     __syncthreads();
 }
 
-// What a caller may be waiting for on the host, then the flag that says so.
-__device__ void tell_host(const ElasticSingleParams& p, int n) {
+// What a caller may be waiting for on the host, then the flag that says so. One block
+// of the copy kernel does it, so that no kernel's completion waits for the bus.
+__device__ void tell_host(const ElasticSingleParams& p) {
     if (p.host_counts == nullptr) return;
     volatile int32_t* h = p.host_counts;
-    __syncthreads();  // psum_expert has been written by this block
-    for (int i = threadIdx.x; i <= p.E; i += blockDim.x) h[2 + i] = p.psum_expert[i];
-    if (threadIdx.x == 0) h[1] = n;
+    for (int i = threadIdx.x; i <= p.E; i += blockDim.x) h[2 + i] = ld_l2(p.psum_expert + i);
+    if (threadIdx.x == 0) h[1] = ld_l2(p.psum_rank);
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) h[0] = p.host_seq;
@@ -403,8 +403,9 @@ __device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int*
     int* lower = smem + E1;             // [E1] in the lower blocks
     int* every = smem + 2 * E1;         // [E1 + 1] in all blocks, then the aligned sums
     int* repeats = smem + 3 * E1 + 1;   // [E1] of the hits, those that have no row (kExpand)
-    uint32_t* mask = reinterpret_cast<uint32_t*>(smem + 4 * E1 + 1);  // [words][E1] (kExpand)
-    int* pre = smem + 4 * E1 + 1 + words * E1;                        // [words][E1] (kExpand)
+    int* rows_of = smem + 4 * E1 + 1;   // [E1] rows of the expert in all blocks (kExpand)
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem + 5 * E1 + 1);  // [words][E1] (kExpand)
+    int* pre = smem + 5 * E1 + 1 + words * E1;                        // [words][E1] (kExpand)
     __shared__ int s_warp[32];
     for (int i = tid; i < E1; i += nthr) total[i] = 0, repeats[i] = 0;
     if (kExpand)
@@ -452,31 +453,29 @@ __device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int*
         }
     if (tid == 0) total[p.E] = in_block;
     cluster_sync();
+    // Every column is needed by the last block (the counts) and, expanded, by all (where
+    // the segments start); else a block needs column E alone.
+    const bool last = rank == blocks - 1;
     for (int x = tid; x < E1; x += nthr) {
-        int lo = 0, sum = 0, rep = 0;
-#pragma unroll
-        for (int r = 0; r < kSingleClusterLarge; ++r) {
-            if (r >= blocks) break;
-            const int c = ld_cluster_s32(total + x, r);
-            if (kExpand) rep += ld_cluster_s32(repeats + x, r);
-            if (r < rank) lo += c;
-            sum += c;
-        }
+        if (!kExpand && !last && x != p.E) continue;
+        int lo, none, rep = 0;
+        const int sum = blocks > kSingleCluster ? cluster_sum<kSingleClusterLarge>(total + x, rank, blocks, &lo)
+                                                : cluster_sum<kSingleCluster>(total + x, rank, blocks, &lo);
+        if (kExpand)
+            rep = blocks > kSingleCluster ? cluster_sum<kSingleClusterLarge>(repeats + x, rank, blocks, &none)
+                                          : cluster_sum<kSingleCluster>(repeats + x, rank, blocks, &none);
         lower[x] = lo;
         every[x] = x < p.E ? aligned_count(sum + rep, p.alignment) : sum;
-        if (kExpand && rank == blocks - 1) p.psum_expert[x] = x < p.E ? sum : 0;  // rows of the expert, for below
+        if (kExpand) rows_of[x] = sum;
     }
     __syncthreads();
-    const int n = every[p.E];
-    __syncthreads();
-    exclusive_sums(every, p.E);  // where every expert's segment starts
-    if (rank == blocks - 1) {
-        for (int x = tid; x < E1; x += nthr) {
-            const int rows = kExpand && x < p.E ? p.psum_expert[x] : 0;
-            p.psum_expert[x] = every[x] + rows;  // expanded: where it ends
-        }
-        if (tid == 0) p.psum_rank[0] = n;
-        tell_host(p, n);
+    if (kExpand || last) {
+        if (last && tid == 0) p.psum_rank[0] = every[p.E];
+        __syncthreads();
+        exclusive_sums(every, p.E);  // where every expert's segment starts
+        if (last)
+            for (int x = tid; x < E1; x += nthr)  // expanded: where it ends
+                p.psum_expert[x] = every[x] + (kExpand && x < p.E ? rows_of[x] : 0);
     }
     if (t < p.T) {
         const unsigned below = (1u << lane) - 1u;
@@ -567,7 +566,8 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
             for (int i = tid; i <= p.E; i += nthr)
                 p.psum_expert[i] = smem_i32[i] + (kExpand && i < p.E ? rows[i] : 0);
             if (tid == 0) p.psum_rank[0] = n;
-            tell_host(p, n);
+            __syncthreads();
+            tell_host(p);
             return;
         }
         bid -= 1;
@@ -620,6 +620,7 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
         }
     } else {
         pdl_wait();
+        if (bid == 0) tell_host(p);
         if (tid < nt) {
             const int pos = ld_ro(p.token_pos + t0 + tid);
             s_pos[tid] = pos < p.T ? pos : -1;
@@ -725,7 +726,7 @@ int single_layout_threads(int T, int blocks) {
     return threads >= 32 && threads <= 1024 ? threads : 0;
 }
 size_t single_layout_smem(int E, int threads, bool expand) {
-    return (size_t)(4 * (E + 1) + 1 + (expand ? 2 * (threads / 32) * (E + 1) : 0)) * sizeof(int);
+    return (size_t)(5 * (E + 1) + 1 + (expand ? 2 * (threads / 32) * (E + 1) : 0)) * sizeof(int);
 }
 constexpr size_t kSingleSmemMax = 200 * 1024;
 bool counts_in_copy_kernel(int T, int num_sms) { return T <= 2 * num_sms; }
@@ -746,11 +747,14 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         return launch_kernel("ep_elastic_single_copy", k, dim3(1 + p.T), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
-    // (sixteen blocks, an opt-in cluster size, once eight would have more than 8 warps each)
-    static std::atomic<int> large{1};
+    // Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
+    // each, or where eight blocks' tables do not fit.
+    static std::atomic<int> large{1};  // 0: the device does not take clusters of 16
     cudaError_t err = cudaErrorInvalidConfiguration;
-    for (int blocks : {kSingleClusterLarge, kSingleCluster}) {
-        if (blocks == kSingleClusterLarge && (p.T <= kSingleCluster * 256 || !large.load())) continue;
+    const bool prefer_large = p.T > kSingleCluster * 256;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        const int blocks = prefer_large == (attempt == 0) ? kSingleClusterLarge : kSingleCluster;
+        if (blocks == kSingleClusterLarge && !large.load()) continue;
         const int threads = single_layout_threads(p.T, blocks);
         const size_t smem = threads ? single_layout_smem(p.E, threads, expand) : 0;
         if (threads == 0 || smem > kSingleSmemMax) continue;

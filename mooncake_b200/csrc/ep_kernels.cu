@@ -605,13 +605,11 @@ __device__ __forceinline__ void cluster_layout(const LayoutParams& p, uint32_t* 
     }
     cluster_sync();  // (a block barrier as well)
     for (int x = tid; x < p.E; x += nthr) {
-        int base = 0;
-#pragma unroll
-        for (int r = 0; r < kLayoutClusterLarge - 1; ++r)
-            if (r < rank) base += ld_cluster_s32(total + x, r);
+        int base;
+        const int c = blocks > kLayoutCluster ? cluster_sum<kLayoutClusterLarge>(total + x, rank, blocks, &base)
+                                              : cluster_sum<kLayoutCluster>(total + x, rank, blocks, &base);
         total[p.E + x] = base;
         if (rank == blocks - 1) {
-            const int c = base + total[x];
             p.count[x] = c;
             if (p.recv_count) p.recv_count[x] = c;
             if (p.layout_range) p.layout_range[x] = c;  // begin 0 | count
