@@ -95,7 +95,8 @@ struct ElasticSingleParams {
     const int64_t* topk_idx;     // [T][K]
     const float* topk_weights;   // [T][K] or null
     int T, K, E, H, alignment;
-    int C;                       // tokens per block of the copy kernel (set by the launcher)
+    int C, early, teller;        // tokens per block of the copy kernel, tokens copied ahead of the layout,
+                                 // block that tells the host (set by the launcher)
     int max_rows;                // expanded: rows recv_x has room for
     int32_t* status;
     int32_t* rows;               // kept for combine: [T] received row of the token, or (expanded) [T][K] row

@@ -523,6 +523,24 @@ __device__ __forceinline__ int2 count_sent(const ElasticSingleParams& p, int upt
     return make_int2(n, before);
 }
 
+// Tokens of [0, upto) that name any expert; whole block.
+__device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upto) {
+    const bool vec = choices_in_pairs(p.topk_idx, p.K);
+    int n = 0;
+    for (int t0 = 0; t0 < upto; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x;
+        bool any = false;
+        if (t < upto) {
+            int e[kMaxTopk];
+            load_choices<kMaxTopk>(p.topk_idx, t, p.K, p.E, vec, e);
+#pragma unroll
+            for (int k = 0; k < kMaxTopk; ++k) any |= e[k] >= 0;
+        }
+        n += __syncthreads_count(any);
+    }
+    return n;
+}
+
 // Every listing of tokens [0, T), repeats included, into hits[E] (whole block, no barrier).
 __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hits) {
     for (int i = threadIdx.x; i < p.T * p.K; i += blockDim.x) {
@@ -618,9 +636,20 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
                 p.rows[(size_t)t0 * K + tid] = row;
             }
         }
+    } else if (!kExpand && t0 < p.early && t0 + p.C < p.T) {
+        // ahead of the layout kernel: the tokens before this batch are counted here
+        // (not the last batch: a block of every launch waits)
+        __syncthreads();
+        int pos = sent_before(p, t0);
+        for (int tok = 0; tok < nt; ++tok) {
+            bool any = false;
+            for (int k = 0; k < K; ++k) any |= s_exp[tok * K + k] >= 0;
+            if (tid == 0) s_pos[tok] = any ? pos : -1;
+            pos += any ? 1 : 0;
+        }
     } else {
         pdl_wait();
-        if (bid == 0) tell_host(p);
+        if (bid == p.teller) tell_host(p);
         if (tid < nt) {
             const int pos = ld_ro(p.token_pos + t0 + tid);
             s_pos[tid] = pos < p.T ? pos : -1;
@@ -778,6 +807,10 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     if (c > 128 / p.K) c = 128 / p.K;
     const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
     p.C = c < 1 ? 1 : c < most ? c : most;
+    // (an expanded row's place depends on all tokens: nothing to send ahead)
+    p.early = expand ? 0 : early_tokens(ctx.num_sms);
+    p.teller = (p.early + p.C - 1) / p.C;  // the first block that waits for the layout kernel
+    if (p.teller > (p.T + p.C - 1) / p.C - 1) p.teller = (p.T + p.C - 1) / p.C - 1;
     int warps = p.C * ntiles;
     warps = warps > 16 ? 16 : warps < 4 ? 4 : warps;
     auto k = expand ? ep_elastic_single_copy_kernel<true, false> : ep_elastic_single_copy_kernel<false, false>;

@@ -54,7 +54,7 @@ struct DirectDispatchParams {
     const int32_t* slot;        // [T*K] from the layout kernel, or null: counted in the send kernel
     int T, K, E, M, H;
     int use_fp8;
-    int C;                      // tokens per batch (set by the launcher)
+    int C, early;               // tokens per batch, tokens sent ahead of the layout (set by the launcher)
     int32_t* status;
     void* recv_x;
     float* recv_scales;
@@ -65,6 +65,9 @@ struct DirectDispatchParams {
 };
 // whether the send kernels count the slots themselves for this many tokens
 bool counts_in_send_kernel(int T, int num_sms);
+// tokens whose rows a kernel behind a layout kernel sends before that one has finished,
+// counting the earlier tokens itself
+int early_tokens(int num_sms);
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
 
 struct SendShape {
