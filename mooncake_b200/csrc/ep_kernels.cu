@@ -704,11 +704,12 @@ struct SendView {
 
 constexpr int kBatchEntries = 128;  // (token, k) entries of a batch
 
+// Returns whether one of this thread's entries went to a peer.
 // kCount: the positions are counted here, hist: [E] in shared memory; else `slot` has them. All threads of the block call it.
 // What is read before `ready()` is complete when the kernel begins (the rows and the
 // index matrix: the layout kernel ahead has waited for whatever wrote them).
 template <bool kFP8, bool kGroup, bool kCount, bool kEarly, typename Ready>
-__device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsend, int* hist, Ready ready) {
+__device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsend, int* hist, Ready ready) {
     __shared__ char* s_dst[kBatchEntries];
     __shared__ char* s_meta[kGroup ? kBatchEntries : 1];
     __shared__ int s_raw[kBatchEntries];   // expert of the entry, -1: none
@@ -740,6 +741,7 @@ __device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsen
         __syncthreads();
     }
     int counted = 0;  // tokens that are in hist
+    bool remote = false;  // (of this thread's entries) something was stored in a peer's memory
     for (; t0 < v.T;) {
         const int nt = min(v.C, v.T - t0), ne = nt * K, items = nt * ntiles;
         const int t1 = t0 + nsend * v.C;
@@ -809,7 +811,7 @@ __device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsen
             }
             v.rowmap[(size_t)t0 * K + tid] = row;
             s_dst[tid] = dst;
-            if (kGroup) s_meta[tid] = meta;
+            if (kGroup) s_meta[tid] = meta, remote |= meta != nullptr;
             s_le[tid] = le;
             s_row[tid] = row;
         }
@@ -879,6 +881,7 @@ __device__ __forceinline__ void send_tokens(const SendView& v, int sid, int nsen
             }
         t0 = t1;
     }
+    return remote;
 }
 
 // =============================================================================
@@ -1111,7 +1114,8 @@ __global__ void __launch_bounds__(512) ep_combine_search_kernel(DirectCombinePar
 __device__ __forceinline__ void load_peer_tables(void* const* peer_base, const int32_t* active_ranks,
                                                  int R, int32_t* status, char** s_peer,
                                                  int* s_active) {
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
+    // (the last threads of the block: in a small batch's control block the others count)
+    for (int r = blockDim.x - 1 - threadIdx.x; r < R; r += blockDim.x) {
         char* pb = reinterpret_cast<char*>(peer_base[r]);
         int a = ld_volatile_s32(active_ranks + r);
         if (a && pb == nullptr) {  // marked active but never mapped: leave it alone
@@ -1139,12 +1143,6 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
     int* hist = smem_i32;         // [E]
     int* s_cnt = smem_i32 + p.E;  // [L*R]
     MCEP_TRACE(0, 1);
-    if (kCount) {
-        for (int i = tid; i < p.E; i += nthr) hist[i] = 0;
-        __syncthreads();
-        count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), hist);
-        __syncthreads();
-    }
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
         if (!s_active[dr]) continue;
@@ -1339,6 +1337,11 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     const int nsend = nblocks - 1;
     const int nh = nsend < kRecvHelpers ? nsend : kRecvHelpers;
     MCEP_TRACE(0, 0);
+    if (kCount && bid == 0) {  // the counts do not wait for the peer tables (0.8 us)
+        for (int i = tid; i < p.E; i += nthr) smem_i32[i] = 0;
+        __syncthreads();
+        count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
+    }
     load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);
 
     if (bid == 0) {
@@ -1362,17 +1365,18 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     v.beg = reinterpret_cast<const uint64_t*>(p.local_base + p.w.beg_off);
     v.seq = p.seq, v.wait = scaled(p.wait, 2), v.rx_off = p.rx_off, v.meta_off = p.meta_off;
     v.meta_stride = p.meta_stride, v.rowmap = p.rowmap, v.s_peer = s_peer, v.s_active = s_active;
-    send_tokens<kFP8, true, kCount, false>(v, sid, nsend, smem_i32, [] {});
+    const bool remote = send_tokens<kFP8, true, kCount, false>(v, sid, nsend, smem_i32, [] {});
     MCEP_TRACE(0, 5);  // all rows of this block are issued
 
-    // Completion. Rows are not fenced one by one: the block issues ONE
-    // system-scope fence for everything it stored (it costs microseconds even
-    // when idle), then takes a ticket. Whoever takes the last ticket has,
-    // through the counter, observed every block's fence - all of this rank's
-    // rows are performed system-wide - and tells every peer with one word.
-    __syncthreads();
+    // Completion. Rows are not fenced one by one: a block that stored something in a
+    // peer's memory issues ONE system-scope fence for all of it (2 - 4 us, even when
+    // idle), then takes a ticket. Whoever takes the last ticket has, through the
+    // counter, observed every such fence - all of this rank's rows are performed
+    // system-wide - and tells every peer with one word. Rows of experts this rank
+    // owns are nobody else's to read: the kernel's end orders them.
+    const bool any_remote = __syncthreads_or(remote ? 1 : 0) != 0;
     if (tid == 0) {
-        if (sid * p.C < p.T) __threadfence_system();
+        if (any_remote) __threadfence_system();
         s_ticket = (int)atomicAdd(p.ticket, 1u);
     }
     __syncthreads();
@@ -1483,6 +1487,7 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
     bool stored = false;
     if (!p.zero_copy) {
         int* beg = smem_i32 + n + 1;  // [n] first row of each (expert, source) segment
+        bool mine = false;
         for (int i = tid; i < n; i += nthr) {
             const int src = i % p.R;
             const long long lr = ld_ro(p.layout_range + i);
@@ -1490,10 +1495,13 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
             if (src == p.rank || !s_active[src]) c = 0;
             pre[i] = c;
             beg[i] = (int)(lr >> 32);
+            mine = mine || c > 0;
         }
-        __syncthreads();
-        block_exclusive_scan(pre, n, s_wt);
-        const int total = pre[n];
+        int total = 0;
+        if (__syncthreads_or(mine ? 1 : 0)) {
+            block_exclusive_scan(pre, n, s_wt);
+            total = pre[n];
+        }
         const char* xb = reinterpret_cast<const char*>(p.x);
         char* cin = p.local_base + p.cin_off;
         // A work item is a run of tiles of one row, sized so that the rows spread

@@ -356,15 +356,15 @@ int check_connected(const mcep_buffer* b) {
 }  // namespace
 
 namespace {
-bool chain_with_pdl(const mcep_buffer* b, cudaStream_t stream) {
-    if (!b->pdl) return false;
+bool is_capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return st == cudaStreamCaptureStatusNone;
+    return st != cudaStreamCaptureStatusNone;
 }
+bool chain_with_pdl(const mcep_buffer* b, cudaStream_t stream) { return b->pdl && !is_capturing(stream); }
 }  // namespace
 
 namespace mcep {
@@ -997,7 +997,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
         if (a->return_recv_hook) {
             auto* h = new mcep_hook();
             h->fn = [=]() {
-                mcep::LaunchCtx c0{compute, num_sms, false};
+                mcep::LaunchCtx c0{compute, num_sms, false};  // (in-process groups)
                 MCEP_CUDA(mcep::launch_group_dispatch_recv(p, c0));
                 return MCEP_OK;
             };
@@ -1025,7 +1025,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
 
     if (a->return_recv_hook) {
         auto* h = new mcep_hook();
-        h->fn = [=]() { return recv(compute, false); };
+        h->fn = [=]() { return recv(compute, !is_capturing(compute)); };
         *out_hook = h;
         return MCEP_OK;
     }
@@ -1120,7 +1120,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
         };
         if (a->return_recv_hook) {
             auto* h = new mcep_hook();
-            h->fn = [=]() { return reduce(compute, false); };
+            h->fn = [=]() { return reduce(compute, !is_capturing(compute)); };
             *out_hook = h;
             return MCEP_OK;
         }
@@ -1196,7 +1196,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
 
     if (a->return_recv_hook) {
         auto* h = new mcep_hook();
-        h->fn = [=]() { return reduce(compute, false); };
+        h->fn = [=]() { return reduce(compute, !is_capturing(compute)); };
         *out_hook = h;
         return MCEP_OK;
     }
