@@ -277,6 +277,8 @@ private:
     char* data_ = nullptr;
 };
 
+constexpr int64_t kScalesInArena = 32 << 20;
+
 PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
 // A new tuple that takes over the references of `items`; null if any is null.
@@ -439,15 +441,19 @@ PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssi
         }
     }
     if (rows == nullptr) recv_x = empty({L, RM, H}, fp8 ? at::kFloat8_e4m3fn : at::kBFloat16, dev);
+    Arena small(dev);
+    const int64_t o_count = small.reserve(L * 4), o_range = small.reserve(L * R * 8), o_src = small.reserve(L * RM * 4);
+    // The scales, too, while they are small (a thirtieth of the rows): the handle then
+    // keeps their memory until combine. Larger ones are freed with their tensor.
+    const bool scales_inside = fp8 && L * H / 128 * RM * 4 <= kScalesInArena;
+    const int64_t o_scales = scales_inside ? small.reserve(L * H / 128 * RM * 4) : 0;
+    small.allocate();
     at::Tensor scales;
     if (fp8) {  // [L, H/128, R*M] storage seen as [L, R*M, H/128]
-        scales = empty({L, H / 128, RM}, at::kFloat, dev);
+        scales = scales_inside ? small.view(o_scales, at::kFloat, {L, H / 128, RM}) : empty({L, H / 128, RM}, at::kFloat, dev);
         const int64_t sizes[3] = {L, RM, H / 128}, strides[3] = {H / 128 * RM, 1, RM};
         scales.unsafeGetTensorImpl()->set_sizes_and_strides(at::IntArrayRef(sizes), at::IntArrayRef(strides));
     }
-    Arena small(dev);
-    const int64_t o_count = small.reserve(L * 4), o_range = small.reserve(L * R * 8), o_src = small.reserve(L * RM * 4);
-    small.allocate();
     mcep_dispatch_args a = {};
     a.x = x->const_data_ptr(), a.topk_idx = static_cast<const int64_t*>(idx->const_data_ptr());
     a.active_ranks = static_cast<int32_t*>(active->data_ptr());

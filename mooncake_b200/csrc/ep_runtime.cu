@@ -918,8 +918,8 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     // are in place by then (1 - 2 us of launch latency per call).
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
-    // Batches of more than two tokens per SM get their layout from a kernel of its own.
-    const bool counting = mcep::counts_in_send_kernel(T, b->num_sms);
+    // Larger batches get their layout from a kernel of its own.
+    const bool counting = mcep::counts_in_send_kernel(T, b->num_sms, group);
     if (!counting) {
         mcep::LayoutParams lp = {};
         lp.topk_idx = a->topk_idx;

@@ -106,7 +106,7 @@ class ElasticBuffer:
         self.num_scaleout_ranks, self.num_scaleup_ranks = 1, self.num_ranks
         self.scaleout_rank_idx, self.scaleup_rank_idx = 0, self.rank_idx
         self.num_rdma_ranks, self.num_nvlink_ranks = 1, self.num_ranks
-        self._num_sms: dict = {}  # per device
+        self._num_sms = 0  # of the buffer's device
         self._ones: Optional[torch.Tensor] = None
         self.runtime: Optional[ep.Buffer] = ep.Buffer(self.rank_idx, self.num_ranks, num_bytes, False)
         self._connect_native()
@@ -159,11 +159,9 @@ class ElasticBuffer:
 
     def get_theoretical_num_sms(self, num_experts: int, num_topk: int) -> int:
         """Accepted for interface parity; the kernels size their own grids."""
-        dev = torch.cuda.current_device()
-        n = self._num_sms.get(dev)
-        if n is None:
-            n = self._num_sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
-        return n
+        if self._num_sms == 0:
+            self._num_sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+        return self._num_sms
 
     def barrier(self, use_comm_stream: bool = True, with_cpu_sync: bool = False) -> None:
         """A barrier of the group on the device (reference :417-423)."""
