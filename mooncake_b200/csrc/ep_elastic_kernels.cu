@@ -539,7 +539,7 @@ __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hi
 // there is no layout kernel: every block finds its token's places itself and block 0
 // writes the counts.
 template <bool kExpand, bool kCount>
-__global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
+__global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
     extern __shared__ int smem_i32[];  // kCount: [E + 1] hits / starts, [E] earlier tokens (kExpand)
     constexpr int kEntries = 128;
     __shared__ int s_exp[kEntries];  // expert of the entry or -1
@@ -790,8 +790,11 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     if (err != cudaSuccess) return err;
     LaunchCtx chained = ctx;
     chained.pdl = ctx.chain;
-    // a warp gets about four tiles of plain rows, or one tile that is stored K times
-    int c = (expand ? 16 : 64) / ntiles;
+    // Plain rows: a warp gets about four tiles, all requested at once, two blocks per SM
+    // (4096 rows of 14 KB: 22 us; one row per block 40, three smaller blocks per SM 31).
+    // Expanded: every row is stored K times; a row per block and three blocks per SM
+    // (1024 rows of 8 KB to 8: 27.8 us per layer; two rows and two blocks 29.2).
+    int c = expand ? 1 : 64 / ntiles;
     if (c > 8) c = 8;
     if (c > 128 / p.K) c = 128 / p.K;
     const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
