@@ -1867,14 +1867,15 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, false, 1> : ep_combine_rows_kernel<4, false, 2>;
     }
     // How the groups are dealt out, in waves of the blocks that are resident at a time
-    // (two of 16 warps per SM, more of smaller ones). 4 to 16 waves: every block an equal
+    // (two of 16 warps per SM, more of smaller ones). 4 to 8 waves: every block an equal
     // run of consecutive groups (1024 tokens of 14 KB to 8: 20.5 us; strided 22.5). Fewer:
     // a full wave striding (equal runs would leave blocks out: 600 tokens 10.6 us against
-    // 12.4). More: runs of four, handed out as blocks finish, so that no SM falls behind
-    // (8192 tokens 166 us; equal runs 176, strided 178).
+    // 12.4). More: runs of two, handed out as blocks finish, so that no SM falls behind
+    // (4096 tokens after a write of 512 MB, whose last lines are still leaving L2: 96 us,
+    // equal runs and strided 100; 8192 tokens 168 against 184 and 181).
     const int resident = ctx.num_sms * (2 * kReduceWarps * 32 / threads) / parts;
     const int waves = (groups + resident - 1) / resident;
-    const int run = waves < 4 ? 0 : waves <= 16 ? waves : 4;
+    const int run = waves < 4 ? 0 : waves <= 8 ? waves : 2;
     p.span = run * p.tokens_per_block;
     const int grid = run ? (groups + run - 1) / run : groups < resident ? groups : resident;
     return launch("ep_combine_reduce_direct", k, dim3(grid, parts), dim3(threads), 0, ctx, p);
