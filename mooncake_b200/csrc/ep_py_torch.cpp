@@ -17,7 +17,10 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <structmember.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -193,6 +196,84 @@ PyType_Slot event_slots[] = {
 PyType_Spec event_spec = {"mooncake_b200._mcep_torch.EventHandle", sizeof(EventObject), 0,
                           Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE, event_slots};
 
+// The state of `EventOverlap` (mooncake_ep_buffer.py derives from it): an event and the
+// tensors that must outlive it.
+struct OverlapObject {
+    PyObject_HEAD
+    PyObject* event;
+    PyObject* extra_tensors;
+};
+PyTypeObject* overlap_type = nullptr;  // the derived class once it has been registered
+
+int overlap_init(PyObject* self, PyObject* args, PyObject* kw) {
+    static const char* names[] = {"event", "extra_tensors", nullptr};
+    PyObject *event = Py_None, *extra = Py_None;
+    if (!PyArg_ParseTupleAndKeywords(args, kw, "|OO", const_cast<char**>(names), &event, &extra)) return -1;
+    OverlapObject* o = reinterpret_cast<OverlapObject*>(self);
+    Py_INCREF(event), Py_INCREF(extra);
+    Py_XSETREF(o->event, event);
+    Py_XSETREF(o->extra_tensors, extra);
+    return 0;
+}
+int overlap_traverse(PyObject* self, visitproc visit, void* arg) {
+    OverlapObject* o = reinterpret_cast<OverlapObject*>(self);
+    Py_VISIT(o->event);
+    Py_VISIT(o->extra_tensors);
+    Py_VISIT(Py_TYPE(self));
+    return 0;
+}
+int overlap_clear(PyObject* self) {
+    OverlapObject* o = reinterpret_cast<OverlapObject*>(self);
+    Py_CLEAR(o->event);
+    Py_CLEAR(o->extra_tensors);
+    return 0;
+}
+void overlap_dealloc(PyObject* self) {
+    PyTypeObject* type = Py_TYPE(self);
+    PyObject_GC_UnTrack(self);
+    overlap_clear(self);
+    type->tp_free(self);
+    Py_DECREF(type);
+}
+PyMemberDef overlap_members[] = {
+    {"event", T_OBJECT, offsetof(OverlapObject, event), 0, nullptr},
+    {"extra_tensors", T_OBJECT, offsetof(OverlapObject, extra_tensors), 0, nullptr},
+    {nullptr, 0, 0, 0, nullptr}};
+PyType_Slot overlap_slots[] = {
+    {Py_tp_doc, const_cast<char*>("An event plus the tensors that must outlive it.")},
+    {Py_tp_new, reinterpret_cast<void*>(PyType_GenericNew)},
+    {Py_tp_init, reinterpret_cast<void*>(overlap_init)},
+    {Py_tp_traverse, reinterpret_cast<void*>(overlap_traverse)},
+    {Py_tp_clear, reinterpret_cast<void*>(overlap_clear)},
+    {Py_tp_dealloc, reinterpret_cast<void*>(overlap_dealloc)},
+    {Py_tp_members, overlap_members},
+    {0, nullptr}};
+PyType_Spec overlap_spec = {"mooncake_b200._mcep_torch.EventOverlapBase", sizeof(OverlapObject), 0,
+                            Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC, overlap_slots};
+
+// Takes over the references of both; null if one of them is.
+PyObject* wrap_overlap(PyObject* event, PyObject* extra) {
+    PyObject* self = event && extra ? overlap_type->tp_alloc(overlap_type, 0) : nullptr;
+    if (self == nullptr) {
+        Py_XDECREF(event);
+        Py_XDECREF(extra);
+        return nullptr;
+    }
+    reinterpret_cast<OverlapObject*>(self)->event = event;
+    reinterpret_cast<OverlapObject*>(self)->extra_tensors = extra;
+    return self;
+}
+
+PyObject* py_register_overlap(PyObject*, PyObject* cls) {
+    PyTypeObject* base = overlap_type;
+    while (base->tp_base != nullptr && base->tp_base != &PyBaseObject_Type) base = base->tp_base;
+    if (!PyType_Check(cls) || !PyType_IsSubtype(reinterpret_cast<PyTypeObject*>(cls), base))
+        return PyErr_Format(PyExc_TypeError, "a class derived from EventOverlapBase is wanted");
+    Py_INCREF(cls);
+    overlap_type = reinterpret_cast<PyTypeObject*>(cls);
+    Py_RETURN_NONE;
+}
+
 struct HookObject {
     PyObject_HEAD
     mcep_hook* hook;
@@ -242,8 +323,20 @@ bool usable_mask(const at::Tensor* t, int64_t ranks) {
     return t && t->is_cuda() && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
 }
 
+// torch.empty without the way through the tensor factory (0.2 us per tensor).
 at::Tensor empty(at::IntArrayRef size, at::ScalarType type, at::Device dev) {
-    return at::detail::empty_cuda(size, type, dev, std::nullopt);
+    if (c10::cuda::current_device() != dev.index()) return at::detail::empty_cuda(size, type, dev, std::nullopt);
+    const auto meta = c10::scalarTypeToTypeMeta(type);
+    size_t bytes = meta.itemsize();
+    for (const int64_t n : size) {
+        TORCH_CHECK(n >= 0, "negative size");
+        bytes *= (size_t)n;
+    }
+    c10::Allocator* allocator = c10::cuda::CUDACachingAllocator::get();
+    c10::Storage storage(c10::Storage::use_byte_size_t(), bytes, allocator->allocate(bytes), allocator, true);
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(std::move(storage), c10::DispatchKeySet(c10::DispatchKey::CUDA), meta);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(size);
+    return t;
 }
 
 // Several small output tensors cut out of one allocation: the caching allocator
@@ -409,7 +502,8 @@ PyObject* runtime_next_recv_x(PyObject* self, PyObject* const* args, Py_ssize_t 
 //                  return_recv_hook, in_place or None)
 // `in_place`(pointer, bytes, L, R*M, H, use_fp8, x) makes the tensor over the symmetric memory in
 // which a group's rows land; without it, or for a single rank, the rows get a tensor of their own.
-//   -> (recv_x, scales or None, recv_count, src_info, layout_range, event, hook)
+//   -> what Buffer.dispatch returns: (recv_x or (recv_x, scales), recv_count,
+//       (src_info, layout_range, M, H, E), EventOverlap, hook or None),
 // or None when an argument is not what the call takes (the wrapper then says which).
 PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
@@ -471,25 +565,44 @@ PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssi
         Py_XDECREF(rows);
         return fail();
     }
-    return pack({rows ? rows : wrap(std::move(recv_x)), fp8 ? wrap(std::move(scales)) : new_ref(Py_None),
-                 wrap(small.view(o_count, at::kInt, {L})), wrap(small.view(o_src, at::kInt, {L, RM})),
-                 wrap(small.view(o_range, at::kLong, {L, R})), wrap_event(ev), wrap_hook(hk)});
+    PyObject* p_rows = rows ? rows : wrap(std::move(recv_x));
+    PyObject* p_scales = fp8 ? wrap(std::move(scales)) : new_ref(Py_None);
+    PyObject* p_count = wrap(small.view(o_count, at::kInt, {L}));
+    PyObject* p_src = wrap(small.view(o_src, at::kInt, {L, RM}));
+    PyObject* p_range = wrap(small.view(o_range, at::kLong, {L, R}));
+    PyObject* keep = Py_None;
+    if (async) {
+        keep = PyTuple_Pack(7, args[0], args[1], p_rows, p_scales, p_count, p_src, p_range);
+    } else {
+        Py_INCREF(keep);
+    }
+    PyObject* handle = pack({p_src, p_range, new_ref(args[3]), PyLong_FromLongLong(H), new_ref(args[4])});
+    PyObject* got = p_rows;
+    if (fp8) {
+        got = pack({p_rows, p_scales});
+    } else {
+        Py_DECREF(p_scales);
+    }
+    return pack({got, p_count, handle, wrap_overlap(wrap_event(ev), keep), wrap_hook(hk)});
     END_HANDLE_TH_ERRORS
 }
 
-// combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info, layout_range,
-//                 M, hidden, E, zero_copy, async_finish, return_recv_hook, out or None)
-//   -> (combined_x, event, hook), or None (as above)
+// combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, handle, zero_copy,
+//                 async_finish, return_recv_hook, out or None)
+//   -> what Buffer.combine returns: (combined_x, EventOverlap, hook or None), or None (as above)
 PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     RuntimeObject* s = self_of(self);
-    if (nargs != 14) return PyErr_Format(PyExc_TypeError, "combine_tensors() takes 14 arguments");
+    if (nargs != 10) return PyErr_Format(PyExc_TypeError, "combine_tensors() takes 10 arguments");
     if (!alive(s)) return nullptr;
-    Reader r{const_cast<PyObject**>(args)};
+    if (!PyTuple_Check(args[5]) || PyTuple_GET_SIZE(args[5]) != 5) Py_RETURN_NONE;
+    PyObject* const* h = &PyTuple_GET_ITEM(args[5], 0);  // (src_info, layout_range, M, H, E)
+    Reader r{const_cast<PyObject**>(args)}, hr{const_cast<PyObject**>(h)};
     const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *w = tensor_of(args[2]);
-    const at::Tensor *active = tensor_of(args[3]), *src = tensor_of(args[5]), *range = tensor_of(args[6]);
-    const int64_t timeout = r.num(4), M = r.num(7), H = r.num(8), E = r.num(9), R = s->num_ranks;
-    const int zero_copy = r.flag(10), async = r.flag(11), hooked = r.flag(12);
+    const at::Tensor *active = tensor_of(args[3]), *src = tensor_of(h[0]), *range = tensor_of(h[1]);
+    const int64_t timeout = r.num(4), M = hr.num(2), H = hr.num(3), E = hr.num(4), R = s->num_ranks;
+    const int zero_copy = r.flag(6), async = r.flag(7), hooked = r.flag(8);
+    if (!hr.ok) return nullptr;
     if (!r.ok) return nullptr;
     if (!(x && x->is_cuda() && x->dim() == 3 && x->scalar_type() == at::kBFloat16 && x->is_contiguous()) ||
         !matrix(idx, at::kLong) || !matrix(w, at::kFloat) || !usable_mask(active, R) || !matrix(src, at::kInt) ||
@@ -499,8 +612,8 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
     if (x->size(0) != L || x->size(1) != R * M || x->size(2) != H || H % 128 != 0 || idx->size(0) != T ||
         idx->size(1) != K || T > M || src->size(0) != L || range->size(0) != L || range->size(1) != R)
         Py_RETURN_NONE;
-    const at::Tensor* given = tensor_of(args[13]);
-    if (args[13] != Py_None && (!matrix(given, at::kBFloat16) || given->size(0) != T || given->size(1) != H))
+    const at::Tensor* given = tensor_of(args[9]);
+    if (args[9] != Py_None && (!matrix(given, at::kBFloat16) || given->size(0) != T || given->size(1) != H))
         Py_RETURN_NONE;
     at::Tensor out = given ? *given : empty({T, H}, at::kBFloat16, x->device());
     mcep_combine_args a = {};
@@ -516,7 +629,14 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
     mcep_event* ev = nullptr;
     mcep_hook* hk = nullptr;
     if (call_combine(s->buf, &a, &ev, &hk)) return fail();
-    return pack({given ? new_ref(args[13]) : wrap(std::move(out)), wrap_event(ev), wrap_hook(hk)});
+    PyObject* p_out = given ? new_ref(args[9]) : wrap(std::move(out));
+    PyObject* keep = Py_None;
+    if (async) {
+        keep = PyTuple_Pack(6, args[0], args[1], args[2], h[0], h[1], p_out);
+    } else {
+        Py_INCREF(keep);
+    }
+    return pack({p_out, wrap_overlap(wrap_event(ev), keep), wrap_hook(hk)});
     END_HANDLE_TH_ERRORS
 }
 
@@ -699,6 +819,7 @@ PyObject* py_adopt_event(PyObject*, PyObject* address) {
 PyMethodDef module_methods[] = {
     {"adopt_event", py_adopt_event, METH_O, "An EventHandle that owns the mcep_event at this address (None: None)."},
     {"bind", py_bind, METH_O, "bind({name: address}): the entry points of the loaded libmcep.so."},
+    {"register_overlap", py_register_overlap, METH_O, "The class (derived from EventOverlapBase) that calls return."},
     {"current_stream", py_current_stream, METH_NOARGS, "torch's current CUDA stream as an integer."},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_mcep_torch", "Native binding of libmcep.so for torch tensors.",
@@ -711,9 +832,11 @@ PyMODINIT_FUNC PyInit__mcep_torch(void) {
     if (m == nullptr) return nullptr;
     event_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&event_spec));
     hook_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&hook_spec));
+    overlap_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&overlap_spec));
     PyObject* runtime = PyType_FromSpec(&runtime_spec);
-    if (!event_type || !hook_type || !runtime) return nullptr;
+    if (!event_type || !hook_type || !overlap_type || !runtime) return nullptr;
     if (PyModule_AddObjectRef(m, "EventHandle", reinterpret_cast<PyObject*>(event_type)) < 0 ||
+        PyModule_AddObjectRef(m, "EventOverlapBase", reinterpret_cast<PyObject*>(overlap_type)) < 0 ||
         PyModule_AddObjectRef(m, "Hook", reinterpret_cast<PyObject*>(hook_type)) < 0 ||
         PyModule_AddObjectRef(m, "Runtime", runtime) < 0)
         return nullptr;

@@ -49,14 +49,10 @@ class _DeviceBytes:
                                          "data": (ptr, False), "version": 3}
 
 
-class EventOverlap:
-    """An event plus the tensors that must outlive it (reference :34-90)."""
-
-    def __init__(self, event: Optional["ep.EventHandle"] = None,
-                 extra_tensors: Optional[Tuple[torch.Tensor, ...]] = None) -> None:
-        self.event = event
-        # kept alive here rather than via record_stream, which CUDA graphs reject
-        self.extra_tensors = extra_tensors
+class EventOverlap(ep.EventOverlapBase):
+    """An event plus the tensors that must outlive it (reference :34-90):
+    `EventOverlap(event=None, extra_tensors=None)`. The tensors are kept alive here
+    rather than via record_stream, which CUDA graphs reject."""
 
     def current_stream_wait(self) -> None:
         assert self.event is not None
@@ -70,7 +66,12 @@ class EventOverlap:
             self.event.current_stream_wait(_stream_ptr())
 
 
+ep.register_overlap(EventOverlap)
+
+
 class Buffer:
+    recv_in_place = True  # a group's rows stay in symmetric memory (module docstring)
+
     def __init__(self, group: dist.ProcessGroup, num_ep_buffer_bytes: int = 0,
                  disable_p2p: bool = False, recv_in_place: bool = True):
         self.recv_in_place = recv_in_place
@@ -173,7 +174,7 @@ class Buffer:
         `handle = (src_info, layout_range, M, H, E)`.
         """
         use_fp8 = True if use_fp8 is None else use_fp8
-        in_place = self._rows_in_place if getattr(self, "recv_in_place", True) else None
+        in_place = self._rows_in_place if self.recv_in_place else None
         out = self.runtime.dispatch_tensors(x, topk_idx, active_ranks, num_max_dispatch_tokens_per_rank, num_experts,
                                             timeout_us, use_fp8, async_finish, return_recv_hook, in_place)
         if out is None:  # not the plain case: find out what is wrong, or what to put in
@@ -183,10 +184,7 @@ class Buffer:
                                                 num_experts, timeout_us, use_fp8, async_finish, return_recv_hook,
                                                 in_place)
             assert out is not None, "dispatch takes CUDA tensors"
-        recv_x, scales, recv_count, src_info, layout_range, event, hook = out
-        handle = (src_info, layout_range, num_max_dispatch_tokens_per_rank, x.size(1), num_experts)
-        keep = (x, topk_idx, recv_x, scales, recv_count, src_info, layout_range) if async_finish else None
-        return ((recv_x, scales) if use_fp8 else recv_x, recv_count, handle, EventOverlap(event, keep), hook)
+        return out
 
     def _rows_in_place(self, ptr: int, nbytes: int, L: int, RM: int, H: int, use_fp8: bool,
                        x: torch.Tensor) -> torch.Tensor:
@@ -218,19 +216,14 @@ class Buffer:
         (reference :538-678). With `zero_copy` the expert outputs are read from the
         tensor `get_next_combine_buffer(handle)` returned and `x` only gives the
         shape."""
-        src_info, layout_range, M, hidden, num_experts = handle
-        res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info,
-                                           layout_range, M, hidden, num_experts, zero_copy, async_finish,
-                                           return_recv_hook, out)
+        res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, handle, zero_copy,
+                                           async_finish, return_recv_hook, out)
         if res is None:  # not the plain case: find out what is wrong, or what to put in
             active_ranks = self._checked_combine(x, topk_idx, topk_weights, active_ranks, handle, out)
-            res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, src_info,
-                                               layout_range, M, hidden, num_experts, zero_copy, async_finish,
-                                               return_recv_hook, out)
+            res = self.runtime.combine_tensors(x, topk_idx, topk_weights, active_ranks, timeout_us, tuple(handle),
+                                               zero_copy, async_finish, return_recv_hook, out)
             assert res is not None, "combine takes CUDA tensors"
-        combined_x, event, hook = res
-        keep = (x, topk_idx, topk_weights, src_info, layout_range, combined_x) if async_finish else None
-        return combined_x, EventOverlap(event, keep), hook
+        return res
 
     def _checked_combine(self, x, topk_idx, topk_weights, active_ranks, handle, out) -> torch.Tensor:
         """The argument checks of the reference's wrapper (:557-603); returns the mask to use."""
