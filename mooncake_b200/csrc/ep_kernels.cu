@@ -1055,6 +1055,60 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     }
 }
 
+// One row per token (top-1, and every flat elastic combine of a single rank): a gather.
+// The kernel above would have a single load per lane in flight; here a warp requests
+// up to four tiles of its block's `tokens_per_block` rows before it uses the first.
+template <bool kAbs>
+__global__ void __launch_bounds__(512, 2) ep_combine_one_row_kernel(DirectCombineParams p) {
+    constexpr int kAhead = 4, kMost = 16;
+    __shared__ int s_row[kMost];
+    __shared__ float s_w[kMost];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    const int t0 = blockIdx.x * p.tokens_per_block, nt = min(p.tokens_per_block, p.T - t0), items = nt * ntiles;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (tid < nt) {
+        int row = ld_ro(p.rowmap + t0 + tid);
+        float w = 1.f;
+        if (!kAbs) {
+            const int e = (int)ld_ro(p.topk_idx + t0 + tid);
+            w = ld_ro(p.topk_weights + t0 + tid);
+            row = (e >= 0 && e < p.E && row >= 0 && row < p.M) ? e * p.M + row : -1;
+        }
+        s_row[tid] = ld_volatile_s32(p.active_ranks) != 0 ? row : -1;
+        s_w[tid] = w;
+    }
+    __syncthreads();
+    const size_t row_bytes = (size_t)p.H * 2;
+    for (int i0 = warp; i0 < items; i0 += nwarps * kAhead) {
+        V32 v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int item = i0 + u * nwarps, tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
+            const int r = item < items && c < nchunks ? s_row[tok] : -1;
+            if (r >= 0) v[u] = ld32_readonly(reinterpret_cast<const char*>(p.x) + (size_t)r * row_bytes + (size_t)c * 32);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int item = i0 + u * nwarps, tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
+            if (item >= items || c >= nchunks) continue;
+            float acc[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+            if (s_row[tok] >= 0) {
+                const float w = kAbs ? 1.f : s_w[tok];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    acc[2 * i] = fmaf(bf16lo(v[u].w[i]), w, 0.f);
+                    acc[2 * i + 1] = fmaf(bf16hi(v[u].w[i]), w, 0.f);
+                }
+            }
+            st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + tok) * row_bytes + (size_t)c * 32, pack_bf16x16(acc));
+        }
+    }
+}
+
 // Small batches whose rows are not recorded (a handle older than the last two
 // calls, or a copy of one): no separate inversion pass. Warp k looks the token up
 // in the handle itself - the segment of expert topk[t][k] - 32 entries of src_info
@@ -1848,9 +1902,22 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         const int grid = persistent_grid(p.T, ep_combine_search_kernel, threads, 0, ctx);
         return launch("ep_combine_search", ep_combine_search_kernel, dim3(grid), dim3(threads), 0, ctx, p);
     }
+    const int row_tiles = (p.H + kTileChannels - 1) / kTileChannels;
+    if (p.K == 1) {
+        // two rounds of four tiles per warp (4096 rows of 14 KB: 21.0 us, 29 - 32 with the
+        // kernel for more rows; four rows per block 21.5, two 25.6)
+        int c = 112 / row_tiles;
+        if (c > 16) c = 16;
+        const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
+        p.tokens_per_block = c < 1 ? 1 : c < most ? c : most < 1 ? 1 : most;
+        const int warps = p.tokens_per_block * row_tiles;
+        auto k = p.absolute ? ep_combine_one_row_kernel<true> : ep_combine_one_row_kernel<false>;
+        const int grid = p.T > 0 ? (p.T + p.tokens_per_block - 1) / p.tokens_per_block : 1;
+        return launch("ep_combine_reduce_direct", k, dim3(grid), dim3(32 * (warps < 16 ? warps : 16)), 0, ctx, p);
+    }
     // A block covers as many whole rows as give it 14 to 16 warps once there are more
     // tokens than SMs; up to one block per SM, registers are spent on loads in flight.
-    const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    const int ntiles = row_tiles;
     const int parts = (ntiles + kReduceWarps - 1) / kReduceWarps;  // blocks that share a row
     p.tiles_per_block = (ntiles + parts - 1) / parts;
     p.tokens_per_block = 1;
@@ -1867,15 +1934,16 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, false, 1> : ep_combine_rows_kernel<4, false, 2>;
     }
     // How the groups are dealt out, in waves of the blocks that are resident at a time
-    // (two of 16 warps per SM, more of smaller ones). 4 to 8 waves: every block an equal
-    // run of consecutive groups (1024 tokens of 14 KB to 8: 20.5 us; strided 22.5). Fewer:
-    // a full wave striding (equal runs would leave blocks out: 600 tokens 10.6 us against
-    // 12.4). More: runs of two, handed out as blocks finish, so that no SM falls behind
-    // (4096 tokens after a write of 512 MB, whose last lines are still leaving L2: 96 us,
-    // equal runs and strided 100; 8192 tokens 168 against 184 and 181).
+    // (two of 16 warps per SM, more of smaller ones). Fewer than 8 rows per token, or
+    // fewer than 4 waves: a full wave striding (4096 tokens of 14 KB to 4: 45.7 us, runs
+    // 47.5; 600 to 8: 10.6, equal runs, which leave blocks out, 12.4). Else, 4 to 8 waves:
+    // every block an equal run of consecutive groups (1024 tokens to 8: 20.5 us, strided
+    // 22.5). More: runs of two, handed out as blocks finish, so that no SM falls behind
+    // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
+    // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181).
     const int resident = ctx.num_sms * (2 * kReduceWarps * 32 / threads) / parts;
     const int waves = (groups + resident - 1) / resident;
-    const int run = waves < 4 ? 0 : waves <= 8 ? waves : 2;
+    const int run = p.K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
     p.span = run * p.tokens_per_block;
     const int grid = run ? (groups + run - 1) / run : groups < resident ? groups : resident;
     return launch("ep_combine_reduce_direct", k, dim3(grid, parts), dim3(threads), 0, ctx, p);
