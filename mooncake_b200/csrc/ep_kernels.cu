@@ -1269,13 +1269,15 @@ __device__ __forceinline__ void dispatch_recv_duty(const GroupDispatchParams& p,
     for (int r = tid; r < p.R; r += nthr) s_tot[r] = 0;
     __syncthreads();
     // the control block's verdicts: what every source sends to every local expert
+    bool from_peers = false;
     for (int i = tid; i < n; i += nthr) {
         const uint32_t v = wait_local_word(p.res_cnt + i, p.seq, scaled(p.wait, 2));
         const int c = v ? (int)v - 1 : 0;
         pre[i] = c;
         if (c) atomicAdd(&s_tot[i % p.R], c);
+        from_peers |= c != 0 && i % p.R != p.rank;
     }
-    __syncthreads();
+    if (!__syncthreads_or(from_peers ? 1 : 0)) return;  // only rows this rank sent to itself
     for (int le = tid; le < L; le += nthr) {
         int run = 0;
         for (int src = 0; src < p.R; ++src) {
@@ -1693,6 +1695,110 @@ __global__ void __launch_bounds__(512) ep_combine_kernel(GroupCombineParams p) {
     combine_body<kPhases>(p, blockIdx.x, gridDim.x, smem_i32);
 }
 
+// The reduce duty of batches with more tokens than SMs, in a launch of its own: as
+// ep_combine_rows_kernel, no barrier per token, a warp owns one tile of one row of every
+// group of tokens. What a group adds: a row lies in its owner's memory, readable once
+// the owner's word is here. A warp asks for an owner's word once - when a token of it
+// first needs that owner - and keeps the verdict. One rank on this path, 2048 tokens of
+// 14 KB to 8: 47 us, with a barrier per token and the words looked at for every one 59
+// (512 tokens 16.7 and 18.9).
+template <int kDepth>
+__global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel(GroupCombineParams p) {
+    __shared__ char* s_peer[kMaxRanks];
+    __shared__ int s_active[kMaxRanks];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = warp / p.tiles_per_block;
+    const int c = ((warp - sub * p.tiles_per_block + blockIdx.y * p.tiles_per_block) * 32) + lane;
+    const bool act = c < p.H / 16;
+    pdl_wait();
+    pdl_launch_dependents();
+    resolve_seq(p);
+    const int L = p.E / p.R, RM = p.R * p.M;
+    const size_t row_bytes = (size_t)p.H * 2;
+    const int step = (p.span ? 1 : gridDim.x) * p.tokens_per_block;
+    const int first = blockIdx.x * (p.span ? p.span : p.tokens_per_block);
+    const int end = p.span ? min(p.T, first + p.span) : p.T;
+
+    int next_row = -1, next_e = -1;
+    float next_w = 0.f;
+    auto request = [&](int tok) {
+        if (lane < p.K && tok < end) {
+            const size_t at = (size_t)tok * p.K + lane;
+            next_row = ld_l2(p.rowmap + at);
+            next_e = (int)ld_ro(p.topk_idx + at), next_w = ld_ro(p.topk_weights + at);
+        } else {
+            next_row = -1;
+        }
+    };
+    request(first + sub);
+    load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);
+    __syncthreads();
+    const char* own = p.zero_copy ? p.local_base + p.cin_off : reinterpret_cast<const char*>(p.x);
+    const uint64_t* flags = reinterpret_cast<const uint64_t*>(p.local_base + p.w.cflag_off);
+    unsigned known[2] = {0, 0}, good[2] = {0, 0};  // owners whose word has been asked for / whose rows count
+    for (int t0 = first; t0 < end; t0 += step) {
+        int owner = -1;
+        const char* row = nullptr;
+        if (next_e >= 0 && next_e < p.E && next_row >= 0 && next_row < RM) {
+            owner = next_e / L;
+            const size_t off = ((size_t)(next_e - owner * L) * RM + next_row) * row_bytes;
+            row = (owner == p.rank ? own : s_peer[owner] + p.cin_off) + off;
+        }
+        const float w = next_w;
+        const bool ask = owner >= 0 && !((known[owner >> 5] >> (owner & 31)) & 1u);
+        if (__any_sync(kFull, ask)) {
+            bool ok = false;
+            if (ask && ld_volatile_s32(p.wait.active_ranks + owner)) {
+                if (owner == p.rank)
+                    ok = true;
+                else if (s_peer[owner] != nullptr)
+                    ok = resolve_flag(flags, p.res_cflag, owner, p.seq, p.wait, owner,
+                                      ((blockIdx.x + owner) & 7) == 0 && warp == 0) != 0 &&
+                         ld_volatile_s32(p.wait.active_ranks + owner) != 0;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const unsigned bit = ask && (owner >> 5) == h ? 1u << (owner & 31) : 0u;
+                known[h] |= __reduce_or_sync(kFull, bit);
+                good[h] |= __reduce_or_sync(kFull, ok ? bit : 0u);
+            }
+            __syncwarp();  // the acquire of one lane orders the loads of all
+        }
+        if (owner < 0 || !((good[owner >> 5] >> (owner & 31)) & 1u)) row = nullptr;
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (int k0 = 0; k0 < p.K; k0 += kDepth) {
+            V32 v[kDepth];
+            unsigned there = 0;
+#pragma unroll
+            for (int b = 0; b < kDepth; ++b) {
+                const char* r = reinterpret_cast<const char*>(
+                    __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(row), k0 + b));
+                if (r != nullptr) {
+                    there |= 1u << b;
+                    if (act) v[b] = ld32_coherent(r + (size_t)c * 32);
+                }
+            }
+            if (k0 == 0) request(t0 + step + sub);
+#pragma unroll
+            for (int b = 0; b < kDepth; ++b) {
+                const float wk = __shfl_sync(kFull, w, k0 + b);
+                if (there & (1u << b)) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        acc[2 * i] = fmaf(bf16lo(v[b].w[i]), wk, acc[2 * i]);
+                        acc[2 * i + 1] = fmaf(bf16hi(v[b].w[i]), wk, acc[2 * i + 1]);
+                    }
+                }
+            }
+        }
+        if (act && t0 + sub < end)
+            st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + sub) * row_bytes + (size_t)c * 32,
+                 pack_bf16x16(acc));
+    }
+}
+
 // All logical ranks of an in-process group in one cooperative launch (see
 // ep_dispatch_multi_kernel).
 __global__ void __launch_bounds__(512)
@@ -1896,6 +2002,41 @@ cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx&
                   ctx, p);
 }
 
+// How the kernels that give a warp one tile of a row per token are laid out.
+struct ReduceShape {
+    int tiles_per_block, tokens_per_block, span, threads;
+    dim3 grid;
+};
+static ReduceShape reduce_shape(int T, int K, int H, int num_sms) {
+    ReduceShape s;
+    // A block covers as many whole rows as give it 14 to 16 warps once there are more
+    // tokens than SMs; up to one block per SM, registers are spent on loads in flight.
+    const int ntiles = (H + kTileChannels - 1) / kTileChannels;
+    const int parts = (ntiles + kReduceWarps - 1) / kReduceWarps;  // blocks that share a row
+    s.tiles_per_block = (ntiles + parts - 1) / parts;
+    s.tokens_per_block = 1;
+    if (T > num_sms) {
+        const int fit = kReduceWarps / s.tiles_per_block, most = (T + 2 * num_sms - 1) / (2 * num_sms);
+        s.tokens_per_block = fit < most ? fit : most;
+    }
+    s.threads = 32 * s.tiles_per_block * s.tokens_per_block;
+    const int groups = T > 0 ? (T + s.tokens_per_block - 1) / s.tokens_per_block : 1;
+    // How the groups are dealt out, in waves of the blocks that are resident at a time
+    // (two of 16 warps per SM, more of smaller ones). Fewer than 8 rows per token, or
+    // fewer than 4 waves: a full wave striding (4096 tokens of 14 KB to 4: 45.7 us, runs
+    // 47.5; 600 to 8: 10.6, equal runs, which leave blocks out, 12.4). Else, 4 to 8 waves:
+    // every block an equal run of consecutive groups (1024 tokens to 8: 20.5 us, strided
+    // 22.5). More: runs of two, handed out as blocks finish, so that no SM falls behind
+    // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
+    // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181).
+    const int resident = num_sms * (2 * kReduceWarps * 32 / s.threads) / parts;
+    const int waves = (groups + resident - 1) / resident;
+    const int run = K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
+    s.span = run * s.tokens_per_block;
+    s.grid = dim3(run ? (groups + run - 1) / run : groups < resident ? groups : resident, parts);
+    return s;
+}
+
 cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
     if (p.search) {
         const int threads = block_threads(p.H);
@@ -1915,38 +2056,15 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         const int grid = p.T > 0 ? (p.T + p.tokens_per_block - 1) / p.tokens_per_block : 1;
         return launch("ep_combine_reduce_direct", k, dim3(grid), dim3(32 * (warps < 16 ? warps : 16)), 0, ctx, p);
     }
-    // A block covers as many whole rows as give it 14 to 16 warps once there are more
-    // tokens than SMs; up to one block per SM, registers are spent on loads in flight.
-    const int ntiles = row_tiles;
-    const int parts = (ntiles + kReduceWarps - 1) / kReduceWarps;  // blocks that share a row
-    p.tiles_per_block = (ntiles + parts - 1) / parts;
-    p.tokens_per_block = 1;
-    if (p.T > ctx.num_sms) {
-        const int fit = kReduceWarps / p.tiles_per_block, most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
-        p.tokens_per_block = fit < most ? fit : most;
-    }
-    const int threads = 32 * p.tiles_per_block * p.tokens_per_block;
-    const int groups = p.T > 0 ? (p.T + p.tokens_per_block - 1) / p.tokens_per_block : 1;
+    const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
+    p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
     void (*k)(DirectCombineParams) = nullptr;
     if (p.absolute) {
         k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, true, 1> : ep_combine_rows_kernel<4, true, 2>;
     } else {
         k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, false, 1> : ep_combine_rows_kernel<4, false, 2>;
     }
-    // How the groups are dealt out, in waves of the blocks that are resident at a time
-    // (two of 16 warps per SM, more of smaller ones). Fewer than 8 rows per token, or
-    // fewer than 4 waves: a full wave striding (4096 tokens of 14 KB to 4: 45.7 us, runs
-    // 47.5; 600 to 8: 10.6, equal runs, which leave blocks out, 12.4). Else, 4 to 8 waves:
-    // every block an equal run of consecutive groups (1024 tokens to 8: 20.5 us, strided
-    // 22.5). More: runs of two, handed out as blocks finish, so that no SM falls behind
-    // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
-    // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181).
-    const int resident = ctx.num_sms * (2 * kReduceWarps * 32 / threads) / parts;
-    const int waves = (groups + resident - 1) / resident;
-    const int run = p.K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
-    p.span = run * p.tokens_per_block;
-    const int grid = run ? (groups + run - 1) / run : groups < resident ? groups : resident;
-    return launch("ep_combine_reduce_direct", k, dim3(grid, parts), dim3(threads), 0, ctx, p);
+    return launch("ep_combine_reduce_direct", k, shape.grid, dim3(shape.threads), 0, ctx, p);
 }
 
 // ---- groups -----------------------------------------------------------------------
@@ -2036,7 +2154,13 @@ cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const Laun
     return launch("ep_combine_publish", k, dim3(grid), dim3(threads), smem, ctx, p);
 }
 
-cudaError_t launch_group_combine_reduce(const GroupCombineParams& p, const LaunchCtx& ctx) {
+cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx) {
+    // (rows of 8 tiles and more: 2000 tokens of 4 tiles to 4 took 10.1 us with it, 9.0 without)
+    if (p.T > ctx.num_sms && p.H >= 8 * kTileChannels) {
+        const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
+        p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
+        return launch("ep_combine_reduce", ep_combine_gather_kernel<4>, shape.grid, dim3(shape.threads), 0, ctx, p);
+    }
     const int threads = block_threads(p.H);
     auto k = ep_combine_kernel<2>;
     const int grid = persistent_grid(p.T, k, threads, 0, ctx);

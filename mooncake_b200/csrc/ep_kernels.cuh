@@ -185,10 +185,11 @@ struct GroupCombineParams {
     uint64_t* res_cflag;        // [R]
     unsigned* ticket;
     void* combined_x;           // [T][H] bf16
+    int tokens_per_block, tiles_per_block, span;  // set by the launcher (reduce phase of large batches)
 };
 cudaError_t launch_group_combine(const GroupCombineParams& p, const LaunchCtx& ctx);
 cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const LaunchCtx& ctx);
-cudaError_t launch_group_combine_reduce(const GroupCombineParams& p, const LaunchCtx& ctx);
+cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx);
 
 // In-process groups (several logical ranks on one GPU, tests): the send phase
 // (phases = 1) or the whole call (phases = 3) of `n` ranks as ONE cooperative
