@@ -889,10 +889,11 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
 // =============================================================================
 // Bound by HBM for large batches (4096 tokens, hidden 7168, top-8, bf16: 529 MB)
 // and by latency for decode (index load -> count -> row stores, one batch per block).
-// Behind a layout kernel the registers are held to 40, so that three blocks of 14
-// warps fit an SM and one block's loads hide behind the stores of the others.
+// Behind a layout kernel the registers are held to 40, so that six blocks of 8 warps
+// fit an SM and one block's loads hide behind the stores of the others (2001 rows of
+// 8 KB to 8, us per layer: 64 registers 51.4, 48 51.1, 40 48.7, 36 52.3).
 template <bool kFP8, bool kCount>
-__global__ void __launch_bounds__(512, kCount ? 2 : 3) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
+__global__ void __launch_bounds__(kCount ? 512 : 256, kCount ? 2 : 6) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
     extern __shared__ int smem_i32[];  // [E] (kCount)
     // behind a layout kernel the rows are requested before the wait
     if (kCount) pdl_wait();
@@ -1941,39 +1942,49 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
 
 int early_tokens(int num_sms) { return 3 * num_sms; }
 
-bool counts_in_send_kernel(int T, int num_sms, bool group) {
-    // A group's sender blocks are one resident wave, a token each. A single rank has a
-    // block per batch, however many: up to 3.5 tokens per SM every block counts the
-    // tokens ahead of its own in less time than a layout kernel adds (512 tokens: 8.1 us
-    // per layer against 10.2 for top-2 of 4096 channels, 15.7 against 16.9 for top-8;
-    // 700 tokens: 23.4 against 21.9 for top-8).
-    return group ? T <= 2 * num_sms : 2 * T <= 7 * num_sms;
+bool counts_in_send_kernel(int T, int K, int num_sms, bool group) {
+    // A group's sender blocks are one resident wave, a token each. A single rank counts
+    // in one resident wave of blocks with as many tokens each as that takes. Up to two
+    // choices per token that beats a layout kernel as far as it was measured (us per
+    // layer, rows of 8 KB to 2: 1000 tokens 11.9 against 13.2, 4000 34.3 against 36.8; to
+    // 1: 8192 tokens 48.3 against 53.1). From three on the rows of the third token of a
+    // block cost more than the layout kernel does (8 KB to 8: 520 tokens 15.4 against
+    // 16.2, 580 16.0 against 16.5, 600 18.5 against 17.9).
+    if (group) return T <= 2 * num_sms;
+    return K <= 2 ? T <= 8192 / K : T <= 4 * num_sms;
 }
 
-// Tokens per batch and threads per block of the send kernels. Small batches get
-// one block per token (every SM has one or two). Beyond that a batch has enough
-// rows to give every warp of a 14 - 16 warp block one 512-channel tile: rows of 14
-// tiles (hidden 7168) go one by one, rows of 4 tiles in fours.
-static SendShape send_shape(int T, int K, int H, int num_sms, int min_threads) {
+// Tokens per batch and threads per block of the send kernels.
+// A single rank that counts: one resident wave of up to 16 warps, each with a tile at a
+// time (1000 rows of 8 KB to 2: 11.9 us per layer, two waves 14.0).
+// Behind a layout kernel it is the number of independent blocks that hides the chain
+// index -> slot -> stores: a single rank's have one token and up to 8 warps (2048 rows of
+// 14 KB to 4 in FP8: 47.4 us per layer with 8 warps, 51.9 with 14; 2000 rows of 4 KB to 8:
+// 25.6 with one token per block, 26.9 with four).
+// A group's sender blocks are one resident wave that strides: batches of 16 warp tiles,
+// 8 warps once there are more tokens than blocks (2000 rows of 8 KB to 8: 64.0 us per
+// layer, 16 warps 67.3; one token per batch 64.6, rows of 2 KB 30.7 against 27.0), a warp
+// per tile before (256 tokens of 14 KB to 8: 20.9 us, 8 warps 23.4).
+static SendShape send_shape(int T, int K, int H, int num_sms, bool counting, bool group) {
     const int ntiles = (H + kTileChannels - 1) / kTileChannels;
+    const int wave = (T + 2 * num_sms - 1) / (2 * num_sms);  // tokens per batch: two blocks per SM
     SendShape s;
     s.tokens = 1;
-    if (T > 2 * num_sms) {
-        int c = ntiles >= 16 ? 1 : 16 / ntiles;
-        if (c > 8) c = 8;
-        if (c > kBatchEntries / K) c = kBatchEntries / K;
-        const int most = (T + 2 * num_sms - 1) / (2 * num_sms);
-        s.tokens = c < most ? c : most;
-    }
+    if (group || counting) s.tokens = wave;
+    if (group && s.tokens > 16 / ntiles) s.tokens = 16 / ntiles;
+    if (group && s.tokens > 8) s.tokens = 8;
+    if (s.tokens > kBatchEntries / K) s.tokens = kBatchEntries / K;
+    if (s.tokens < 1) s.tokens = 1;
+    const int most = (group ? T > 2 * num_sms : !counting) ? 8 : 16, least = group ? 8 : 4;
     int warps = s.tokens * ntiles;
-    if (warps > 16) warps = 16;
-    if (warps < 4) warps = 4;
-    s.threads = warps * 32 < min_threads ? min_threads : warps * 32;
+    if (warps > most) warps = most;
+    if (warps < least) warps = least;
+    s.threads = 32 * warps;
     return s;
 }
 
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 128);
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, false);
     p.C = s.tokens;
     // About the first wave of blocks: their rows leave while the layout kernel runs, for
     // up to 1.5 us of counting (2001 tokens FP8: 52.9 us per layer without, 52.3 with one
@@ -2090,7 +2101,7 @@ bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms) {
 }
 
 cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 256);
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
     auto k = pick_dispatch<3>(p.use_fp8 != 0, p.slot == nullptr);
@@ -2100,7 +2111,7 @@ cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
 }
 
 cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, 256);
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
     auto k = pick_dispatch<1>(p.use_fp8 != 0, p.slot == nullptr);

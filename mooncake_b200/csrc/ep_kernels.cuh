@@ -64,7 +64,7 @@ struct DirectDispatchParams {
     int32_t* rowmap;            // [T*K] row of (token, k) inside its expert, kept for combine
 };
 // whether the send kernels count the slots themselves for this many tokens
-bool counts_in_send_kernel(int T, int num_sms, bool group);
+bool counts_in_send_kernel(int T, int K, int num_sms, bool group);
 // tokens whose rows a kernel behind a layout kernel sends before that one has finished,
 // counting the earlier tokens itself
 int early_tokens(int num_sms);

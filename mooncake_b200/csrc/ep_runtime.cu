@@ -919,7 +919,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
     // Larger batches get their layout from a kernel of its own.
-    const bool counting = mcep::counts_in_send_kernel(T, b->num_sms, group);
+    const bool counting = mcep::counts_in_send_kernel(T, K, b->num_sms, group);
     if (!counting) {
         mcep::LayoutParams lp = {};
         lp.topk_idx = a->topk_idx;
