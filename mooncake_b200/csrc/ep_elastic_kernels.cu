@@ -506,21 +506,24 @@ __global__ void __launch_bounds__(1024) ep_elastic_single_layout_kernel(ElasticS
         single_layout<kExpand, 16>(p, smem_i32);
 }
 
-// Tokens of [0, upto) that name any expert; whole block.
+// Tokens of [0, upto) that name any expert; whole block, once per kernel.
 __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upto) {
+    __shared__ int s_sent[32];
     const bool vec = choices_in_pairs(p.topk_idx, p.K);
     int n = 0;
-    for (int t0 = 0; t0 < upto; t0 += blockDim.x) {
-        const int t = t0 + threadIdx.x;
+    for (int t = threadIdx.x; t < upto; t += blockDim.x) {
+        int e[kMaxTopk];
+        load_choices<kMaxTopk>(p.topk_idx, t, p.K, p.E, vec, e);
         bool any = false;
-        if (t < upto) {
-            int e[kMaxTopk];
-            load_choices<kMaxTopk>(p.topk_idx, t, p.K, p.E, vec, e);
 #pragma unroll
-            for (int k = 0; k < kMaxTopk; ++k) any |= e[k] >= 0;
-        }
-        n += __syncthreads_count(any);
+        for (int k = 0; k < kMaxTopk; ++k) any |= e[k] >= 0;
+        n += any;
     }
+    n = __reduce_add_sync(kAll, n);
+    if ((threadIdx.x & 31) == 0) s_sent[threadIdx.x >> 5] = n;
+    __syncthreads();
+    n = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) n += s_sent[w];
     return n;
 }
 
@@ -535,9 +538,9 @@ __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hi
 // Rows and per-entry outputs. A block takes C tokens; C rows of a batch are requested
 // up to four per warp before the first is stored. Bound by HBM (4096 tokens of 14 KB:
 // 117 MB in and out). Behind the layout kernel (kCount false) the rows are requested
-// before its results are waited for. With kCount (small batches, one token per block)
-// there is no layout kernel: every block finds its token's places itself and block 0
-// writes the counts.
+// before its results are waited for. With kCount (small batches; kExpand: one token per
+// block) there is no layout kernel: every block finds its tokens' places itself and block
+// 0 writes the counts.
 template <bool kExpand, bool kCount>
 __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
     extern __shared__ int smem_i32[];  // kCount: [E + 1] hits / starts, [E] earlier tokens (kExpand)
@@ -597,10 +600,13 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
     if (tid < ne) s_exp[tid] = e;
     if (kCount) {
         __syncthreads();
-        const int pos = sent_before(p, t0);
-        bool any = false;
-        for (int k = 0; k < K; ++k) any |= s_exp[k] >= 0;
-        if (tid == 0) s_pos[0] = any ? pos : -1, p.token_pos[t0] = any ? pos : -1;
+        int pos = sent_before(p, t0);
+        for (int tok = 0; tok < nt; ++tok) {
+            bool any = false;
+            for (int k = 0; k < K; ++k) any |= s_exp[tok * K + k] >= 0;
+            if (tid == 0) s_pos[tok] = any ? pos : -1, p.token_pos[t0 + tok] = any ? pos : -1;
+            pos += any ? 1 : 0;
+        }
         if (kExpand) {
             int* before = smem_i32 + p.E + 1;
             for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
@@ -742,11 +748,12 @@ size_t single_layout_smem(int E, int threads, bool expand) {
     return (size_t)(5 * (E + 1) + 1 + (expand ? 2 * (threads / 32) * (E + 1) : 0)) * sizeof(int);
 }
 constexpr size_t kSingleSmemMax = 200 * 1024;
-// One launch: flat rows up to 3.5 tokens per SM (400 tokens of top-8: 9.0 us per layer
-// against 11.1, 512: 10.6 against 11.1, 700: 14.4 against 11.7); expanded rows, where
-// every block counts all choices, up to two.
-bool counts_in_copy_kernel(int T, int num_sms, bool expand) {
-    return expand ? T <= 2 * num_sms : 2 * T <= 7 * num_sms;
+// One launch. Flat rows: up to 4096 choices and seven tokens per SM, in one resident wave
+// (us per layer: 500 tokens of 14 KB to 8 10.3, behind a layout kernel 12.5; 1000 of 8 KB
+// to 2 10.2 against 11.5; 700 to 8 11.2 against 10.6, 2000 to 2 14.3 against 14.2).
+// Expanded rows, where every block counts all choices, up to two tokens per SM.
+bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand) {
+    return expand ? T <= 2 * num_sms : T * K <= 4096 && T <= 7 * num_sms;
 }
 }  // namespace
 
@@ -757,12 +764,16 @@ bool elastic_single_fits(int T, int K, int E) {
 
 cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx) {
     const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-    if (counts_in_copy_kernel(p.T, ctx.num_sms, expand)) {
-        // one launch: a block per token and the block of the counts
-        p.C = 1;
-        const int warps = ntiles < 8 ? 8 : ntiles < 16 ? ntiles : 16;
+    if (counts_in_copy_kernel(p.T, p.K, ctx.num_sms, expand)) {
+        // one launch: the block of the counts, and a block per token or (flat) per as many
+        // tokens as make one resident wave
+        p.C = expand ? 1 : (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
+        if (p.C > 128 / p.K) p.C = 128 / p.K;
+        if (p.C < 1) p.C = 1;
+        const int items = p.C * ntiles;
+        const int warps = items < 8 ? 8 : items < 16 ? items : 16;
         auto k = expand ? ep_elastic_single_copy_kernel<true, true> : ep_elastic_single_copy_kernel<false, true>;
-        return launch_kernel("ep_elastic_single_copy", k, dim3(1 + p.T), dim3(warps * 32),
+        return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
     // Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
@@ -790,11 +801,11 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     if (err != cudaSuccess) return err;
     LaunchCtx chained = ctx;
     chained.pdl = ctx.chain;
-    // Plain rows: a warp gets about four tiles, all requested at once, two blocks per SM
-    // (4096 rows of 14 KB: 22 us; one row per block 40, three smaller blocks per SM 31).
-    // Expanded: every row is stored K times; a row per block and three blocks per SM
-    // (1024 rows of 8 KB to 8: 27.8 us per layer; two rows and two blocks 29.2).
-    int c = expand ? 1 : 64 / ntiles;
+    // Blocks of up to 8 warps. Plain rows: a warp gets about four tiles, all requested at
+    // once (4096 rows of 4 KB: 15.0 us per layer, 16 warps 16.3). Expanded: every row is
+    // stored K times; a row per block (1024 rows of 8 KB to 8: 27.8 us per layer, two rows
+    // 29.2; 4096 rows of 14 KB to 2: 66.9, 14 warps 74.7).
+    int c = expand ? 1 : 32 / ntiles;
     if (c > 8) c = 8;
     if (c > 128 / p.K) c = 128 / p.K;
     const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
@@ -804,7 +815,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     p.teller = (p.early + p.C - 1) / p.C;  // the first block that waits for the layout kernel
     if (p.teller > (p.T + p.C - 1) / p.C - 1) p.teller = (p.T + p.C - 1) / p.C - 1;
     int warps = p.C * ntiles;
-    warps = warps > 16 ? 16 : warps < 4 ? 4 : warps;
+    warps = warps > 8 ? 8 : warps < 4 ? 4 : warps;
     auto k = expand ? ep_elastic_single_copy_kernel<true, false> : ep_elastic_single_copy_kernel<false, false>;
     return launch_kernel("ep_elastic_single_copy", k, dim3((p.T + p.C - 1) / p.C), dim3(warps * 32), 0, 1, chained, p);
 }
