@@ -893,7 +893,7 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
 // fit an SM and one block's loads hide behind the stores of the others (2001 rows of
 // 8 KB to 8, us per layer: 64 registers 51.4, 48 51.1, 40 48.7, 36 52.3).
 template <bool kFP8, bool kCount>
-__global__ void __launch_bounds__(kCount ? 512 : 256, kCount ? 2 : 6) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
+__global__ void __launch_bounds__(512, kCount ? 2 : 3) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
     extern __shared__ int smem_i32[];  // [E] (kCount)
     // behind a layout kernel the rows are requested before the wait
     if (kCount) pdl_wait();
@@ -1960,12 +1960,15 @@ bool counts_in_send_kernel(int T, int K, int num_sms, bool group) {
 // Behind a layout kernel it is the number of independent blocks that hides the chain
 // index -> slot -> stores: a single rank's have one token and up to 8 warps (2048 rows of
 // 14 KB to 4 in FP8: 47.4 us per layer with 8 warps, 51.9 with 14; 2000 rows of 4 KB to 8:
-// 25.6 with one token per block, 26.9 with four).
+// 25.6 with one token per block, 26.9 with four). A warp per tile again where twice the
+// L2 and more of bf16 rows is written, 8 per token: the stores alone are the bound then
+// and fewer rows at a time suit HBM (4096 rows of 14 KB to 8 after a large write: 91.6
+// us, 8 warps 93.1; to 4, us per layer: 97.4 with 8 warps, 104.3 with 14).
 // A group's sender blocks are one resident wave that strides: batches of 16 warp tiles,
 // 8 warps once there are more tokens than blocks (2000 rows of 8 KB to 8: 64.0 us per
 // layer, 16 warps 67.3; one token per batch 64.6, rows of 2 KB 30.7 against 27.0), a warp
 // per tile before (256 tokens of 14 KB to 8: 20.9 us, 8 warps 23.4).
-static SendShape send_shape(int T, int K, int H, int num_sms, bool counting, bool group) {
+static SendShape send_shape(int T, int K, int H, bool fp8, int num_sms, bool counting, bool group) {
     const int ntiles = (H + kTileChannels - 1) / kTileChannels;
     const int wave = (T + 2 * num_sms - 1) / (2 * num_sms);  // tokens per batch: two blocks per SM
     SendShape s;
@@ -1975,7 +1978,8 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool counting, boo
     if (group && s.tokens > 8) s.tokens = 8;
     if (s.tokens > kBatchEntries / K) s.tokens = kBatchEntries / K;
     if (s.tokens < 1) s.tokens = 1;
-    const int most = (group ? T > 2 * num_sms : !counting) ? 8 : 16, least = group ? 8 : 4;
+    const bool stores = !group && !fp8 && K >= 8 && (long long)T * K * H * 2 > 256ll << 20;
+    const int most = (group ? T > 2 * num_sms : !counting && !stores) ? 8 : 16, least = group ? 8 : 4;
     int warps = s.tokens * ntiles;
     if (warps > most) warps = most;
     if (warps < least) warps = least;
@@ -1984,7 +1988,7 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool counting, boo
 }
 
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, false);
+    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, false);
     p.C = s.tokens;
     // About the first wave of blocks: their rows leave while the layout kernel runs, for
     // up to 1.5 us of counting (2001 tokens FP8: 52.9 us per layer without, 52.3 with one
@@ -2103,7 +2107,7 @@ bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms) {
 }
 
 cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, true);
+    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
     auto k = pick_dispatch<3>(p.use_fp8 != 0, p.slot == nullptr);
@@ -2113,7 +2117,7 @@ cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
 }
 
 cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, p.slot == nullptr, true);
+    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
     auto k = pick_dispatch<1>(p.use_fp8 != 0, p.slot == nullptr);

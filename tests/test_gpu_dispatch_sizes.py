@@ -16,7 +16,7 @@ SIZES = [  # T, H, E, K, fp8
     (1, 128, 8, 1, True), (1, 8320, 8, 1, False), (17, 640, 8, 1, False), (1001, 8320, 16, 1, False), (2, 8192, 8, 2, False), (3, 8320, 4, 3, True), (296, 512, 16, 3, True), (297, 512, 16, 3, False),
     (297, 1024, 256, 8, True), (300, 7168, 64, 16, False), (511, 128, 32, 5, True), (513, 2048, 4096, 2, False),
     (1023, 640, 24, 6, True), (1500, 8320, 8, 2, False), (2049, 384, 128, 8, True), (4096, 128, 4096, 4, False),
-    (592, 4096, 16, 3, True), (593, 4096, 16, 3, False), (4096, 1024, 8, 2, True), (4097, 640, 8, 2, False), (8192, 128, 8, 1, True),
+    (2341, 7168, 8, 8, False), (592, 4096, 16, 3, True), (593, 4096, 16, 3, False), (4096, 1024, 8, 2, True), (4097, 640, 8, 2, False), (8192, 128, 8, 1, True),
     (8192, 128, 256, 8, True), (8193, 128, 256, 8, True), (9001, 256, 16, 1, False),
 ]
 
