@@ -24,6 +24,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstring>
 #include <initializer_list>
 #include <string>
@@ -717,8 +718,10 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
     if (counts == nullptr) return nullptr;
     if (sync) {
         const int32_t* psum = host.data() + R;
-        n = host[R - 1];
-        n_out = expand ? (L ? psum[L - 1] : 0) : n;
+        // (never beyond what was allocated: aligned segments can end further on than the
+        // expanded rows have room for, and those rows are dropped)
+        n = std::min<int64_t>(host[R - 1], n_cap);
+        n_out = expand ? std::min<int64_t>(L ? psum[L - 1] : 0, out_cap) : n;
         int64_t prev = 0;  // expanded: the entries are where the segments end, unaligned
         for (int64_t i = 0; i < L; ++i) {
             const int64_t c = expand ? psum[i] - (prev + alignment - 1) / alignment * alignment : psum[i + 1] - psum[i];
