@@ -13,6 +13,7 @@
 #include "ep_elastic.cuh"
 
 #include <chrono>
+#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -367,6 +368,8 @@ int single_combine(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, c
     p.active_ranks = a->active_ranks;
     p.T = rec.T, p.K = rec.expand ? rec.K : 1, p.H = rec.H;
     p.x = a->x, p.rowmap = s->single_rows[rec.par], p.absolute = 1;
+    // rows beyond the caller's are not read (0 with a tensor: not said how many)
+    p.M = a->num_input_tokens > 0 || a->x == nullptr ? a->num_input_tokens : INT_MAX;
     p.combined_x = a->combined_x;
     mcep::LaunchCtx ctx{stream, v.num_sms, mcep::may_chain(b, stream) && !async};
     EL_CUDA(mcep::launch_direct_combine(p, ctx));

@@ -343,6 +343,14 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_local_reduce_kernel(Elast
 // ---- a single rank ----------------------------------------------------------------------
 __device__ __forceinline__ int aligned_count(int c, int a) { return (c + a - 1) / a * a; }
 
+// An expanded row, or -1 where aligned segments reach beyond the caller's tensors: the row
+// is dropped, in the copy, in the metadata and in the rows that combine gathers.
+__device__ __forceinline__ int row_with_room(const ElasticSingleParams& p, int row) {
+    if (row < p.max_rows) return row;
+    atomicOr(p.status, kStatusSlotRange);
+    return -1;
+}
+
 // In-place exclusive sums of a[0..n), the total in a[n] (shared memory, whole block).
 __device__ void exclusive_sums(int* a, int n) {
     __shared__ int s_sum[32];
@@ -486,7 +494,7 @@ __device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int*
             for (int k = 0; k < KB; ++k) {
                 if (k >= p.K) break;
                 const int at = warp * E1 + e[k];
-                out[k] = e[k] >= 0 ? every[e[k]] + lower[e[k]] + pre[at] + __popc(mask[at] & below) : -1;
+                out[k] = e[k] < 0 ? -1 : row_with_room(p, every[e[k]] + lower[e[k]] + pre[at] + __popc(mask[at] & below));
             }
         }
     }
@@ -622,7 +630,7 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
             if (tid < ne) {
                 bool last = e >= 0;
                 for (int k = tid + 1; k < K; ++k) last = last && s_exp[k] != e;
-                const int row = last ? smem_i32[e] + before[e] : -1;
+                const int row = last ? row_with_room(p, smem_i32[e] + before[e]) : -1;
                 s_row[tid] = row;
                 p.rows[(size_t)t0 * K + tid] = row;
             }
@@ -646,10 +654,6 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
             s_pos[tid] = pos < p.T ? pos : -1;
         }
         if (kExpand && tid < ne) s_row[tid] = ld_ro(p.rows + (size_t)t0 * K + tid);
-    }
-    if (kExpand && tid < ne && s_row[tid] >= p.max_rows) {  // aligned segments beyond the caller's tensor
-        s_row[tid] = -1;
-        atomicOr(p.status, kStatusSlotRange);
     }
     __syncthreads();
     if (tid < ne) {

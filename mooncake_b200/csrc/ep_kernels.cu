@@ -1025,8 +1025,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     };
     request(first + sub);
     for (int t0 = first; t0 < end; t0 += step) {
-        int row = next_row;
-        if (!kAbs) row = (next_e >= 0 && next_e < p.E && row >= 0 && row < p.M) ? next_e * p.M + row : -1;
+        int row = next_row < p.M ? next_row : -1;
+        if (!kAbs) row = (next_e >= 0 && next_e < p.E && row >= 0) ? next_e * p.M + row : -1;
         const float w = next_w;
         float acc[16];
 #pragma unroll
@@ -1076,6 +1076,8 @@ __global__ void __launch_bounds__(512, 2) ep_combine_one_row_kernel(DirectCombin
             const int e = (int)ld_ro(p.topk_idx + t0 + tid);
             w = ld_ro(p.topk_weights + t0 + tid);
             row = (e >= 0 && e < p.E && row >= 0 && row < p.M) ? e * p.M + row : -1;
+        } else if (row >= p.M) {
+            row = -1;
         }
         s_row[tid] = ld_volatile_s32(p.active_ranks) != 0 ? row : -1;
         s_w[tid] = w;

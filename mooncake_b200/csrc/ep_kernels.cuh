@@ -92,8 +92,8 @@ struct DirectCombineParams {
     int T, K, E, M, H;
     const void* x;              // rows at x + (expert * M + rowmap[t*K+k]) * 2H
     const int32_t* rowmap;
-    int absolute;               // rowmap names rows of the whole tensor (-1: none), every weight is 1;
-                                // topk_idx and topk_weights are not read
+    int absolute;               // rowmap names rows of the whole tensor, which has M of them (-1: none), every
+                                // weight is 1; topk_idx and topk_weights are not read
     int tokens_per_block, tiles_per_block, span;  // set by the launcher (span: tokens a block works through)
     // search: no rowmap; rows are looked up in the handle by the kernel
     int search;

@@ -56,3 +56,23 @@ def test_dispatch_stays_inside_its_tensors(T, H, E, K, alignment):
         md[:, 2:][md[:, 2:] >= room] = -1
         assert torch.equal(h.recv_src_metadata[:n].cpu(), md)
         assert buf.runtime.status() == 1  # rows out of range, nothing else
+
+
+@pytest.mark.parametrize("T,H,E,K,alignment", SIZES)
+def test_combine_adds_the_rows_that_there_was_room_for(T, H, E, K, alignment):
+    x, idx, w = _inputs(T, H, E, K)
+    want = eo.elastic_dispatch([x], [idx], [w], E, T, alignment, True)[0]
+    room = T * K
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    for sync in (True, False):
+        recv, _, _, h, _ = buf.dispatch(x.cuda(), topk_idx=idx.cuda(), num_experts=E, num_max_tokens_per_rank=T,
+                                        expert_alignment=alignment, do_expand=True, do_cpu_sync=sync)
+        y = torch.randn((room, H), generator=torch.Generator().manual_seed(T)).to(torch.bfloat16)
+        for rows in (room, room // 2):  # a tensor with fewer rows is not read beyond them either
+            out, _, _ = buf.combine(y[:rows].cuda(), h)
+            ref = torch.zeros((T, H), dtype=torch.bfloat16)
+            for (_, t), md in zip(want["rows"], want["recv_src_metadata"][:, 2:].tolist()):
+                there = [y[v] for v in md if 0 <= v < rows]
+                if there:
+                    ref[t] = eo.bf16_sum(there)
+            assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
