@@ -357,6 +357,11 @@ int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, 
     return MCEP_OK;
 }
 
+// Rows of combine's input; none beyond them is read (0 with a tensor: not said how many).
+int rows_of_x(const mcep_elastic_combine_args* a) {
+    return a->num_input_tokens > 0 || a->x == nullptr ? a->num_input_tokens : INT_MAX;
+}
+
 // Combine of such a call: the rows are gathered from where the dispatch put them.
 int single_combine(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, const ElasticState::Record& rec,
                    const mcep_elastic_combine_args* a, mcep_event** out_event) {
@@ -368,8 +373,7 @@ int single_combine(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, c
     p.active_ranks = a->active_ranks;
     p.T = rec.T, p.K = rec.expand ? rec.K : 1, p.H = rec.H;
     p.x = a->x, p.rowmap = s->single_rows[rec.par], p.absolute = 1;
-    // rows beyond the caller's are not read (0 with a tensor: not said how many)
-    p.M = a->num_input_tokens > 0 || a->x == nullptr ? a->num_input_tokens : INT_MAX;
+    p.M = rows_of_x(a);
     p.combined_x = a->combined_x;
     mcep::LaunchCtx ctx{stream, v.num_sms, mcep::may_chain(b, stream) && !async};
     EL_CUDA(mcep::launch_direct_combine(p, ctx));
@@ -506,6 +510,7 @@ int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const 
     xp.psum_start = s->psum_start, xp.psum_expert = a->psum_num_recv_tokens_per_expert;
     xp.recv_src_metadata = a->recv_src_metadata, xp.recv_x = a->recv_x;
     xp.recv_topk_weights = a->recv_topk_weights;
+    xp.max_rows = R * M * K, xp.status = v.status;
 
     const int num_sms = v.num_sms;
     const bool expand = a->do_expand != 0;
@@ -582,7 +587,7 @@ int mcep_elastic_combine(mcep_buffer* b, const mcep_elastic_combine_args* a, mce
         }
         mcep::ElasticLocalReduceParams lp = {};
         lp.layout_range = s->layout_range[par], lp.recv_src_metadata = a->recv_src_metadata;
-        lp.x = a->x, lp.R = R, lp.K = K, lp.H = H, lp.y = y;
+        lp.x = a->x, lp.R = R, lp.K = K, lp.H = H, lp.x_rows = rows_of_x(a), lp.y = y;
         EL_CUDA(mcep::launch_elastic_local_reduce(lp, v.num_sms, stream));
         x = y;
     }

@@ -66,20 +66,22 @@ struct ElasticExpandParams {
     const int32_t* psum_start;    // [L+1]
     int32_t* psum_expert;         // [L+1]: entries < L become the ends of the segments
     int32_t* recv_src_metadata;   // [n][K+2], columns 2.. written here
-    void* recv_x;                 // [rows][row_bytes]
-    float* recv_topk_weights;     // [rows] or null
+    void* recv_x;                 // [max_rows][row_bytes]
+    float* recv_topk_weights;     // [max_rows] or null
+    int max_rows;                 // rows that aligned segments push beyond are dropped (metadata -1, status)
+    int32_t* status;
 };
 cudaError_t launch_elastic_expand_scan(const ElasticExpandParams& p, cudaStream_t stream);
 cudaError_t launch_elastic_expand_copy(const ElasticExpandParams& p, int num_sms, cudaStream_t stream);
 
 // Expanded layout, combine side: the rows of one received token are summed into
 // one row before they travel (1 row: copied; more: fp32 accumulation in listing
-// order, rounded to bf16 once).
+// order, rounded to bf16 once; none, all dropped by the dispatch call: zeros).
 struct ElasticLocalReduceParams {
     const int64_t* layout_range;      // [R]
     const int32_t* recv_src_metadata; // [n][K+2]
-    const void* x;                    // [rows][H] bf16
-    int R, K, H;
+    const void* x;                    // [x_rows][H] bf16
+    int R, K, H, x_rows;
     void* y;                          // [n][H] bf16
 };
 cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int num_sms,

@@ -257,7 +257,10 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_expand_scan_kernel(Elasti
             for (int k = 0; k < p.K; ++k)
                 if (p.recv_topk_idx[(size_t)i * p.K + k] == e) k_hit = k;
         const int pos = block_position(k_hit >= 0, s_warp, &s_base);
-        if (k_hit >= 0) p.recv_src_metadata[(size_t)i * md_stride + 2 + k_hit] = start + pos;
+        if (k_hit >= 0 && start + pos < p.max_rows)
+            p.recv_src_metadata[(size_t)i * md_stride + 2 + k_hit] = start + pos;
+        else if (k_hit >= 0)  // (the entry stays -1: dropped)
+            atomicOr(p.status, kStatusSlotRange);
     }
     if (threadIdx.x == 0) p.psum_expert[e] = start + s_base;
 }
@@ -297,10 +300,13 @@ __global__ void __launch_bounds__(kThreads) ep_elastic_local_reduce_kernel(Elast
     const int row_bytes = p.H * 2;
     for (int i = blockIdx.x * kWarps + warp; i < n; i += gridDim.x * kWarps) {
         const int slot = lane < p.K ? p.recv_src_metadata[(size_t)i * md_stride + 2 + lane] : -1;
-        const unsigned valid = __ballot_sync(kAll, slot >= 0);
+        const unsigned valid = __ballot_sync(kAll, slot >= 0 && slot < p.x_rows);
         const int cnt = __popc(valid);
         char* dst = static_cast<char*>(p.y) + (size_t)i * row_bytes;
-        if (cnt == 0) continue;
+        if (cnt == 0) {
+            for (int c = lane * 32; c < row_bytes; c += 32 * 32) st32(dst + c, V32{});
+            continue;
+        }
         if (cnt == 1) {
             const int s = __shfl_sync(kAll, slot, __ffs(valid) - 1);
             for (int c = lane * 32; c < row_bytes; c += 32 * 32)

@@ -7,6 +7,7 @@ import torch
 from mooncake_b200 import ElasticBuffer
 from oracle import elastic_oracle as eo
 from tests.ep_harness import FakeGroup, make_rank_inputs
+from tests.test_gpu_elastic import _combine, _dispatch, _group
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +77,42 @@ def test_combine_adds_the_rows_that_there_was_room_for(T, H, E, K, alignment):
                 if there:
                     ref[t] = eo.bf16_sum(there)
             assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
+
+
+@pytest.mark.parametrize("Ts,M,H,E,K,alignment,staged", [
+    ([33, 20], 40, 256, 32, 4, 128, True), ([64, 0], 64, 128, 8, 2, 256, True), ([9, 9], 9, 640, 4, 1, 64, True),
+    ([40], 40, 256, 64, 8, 128, True), ([16385], 16385, 128, 4, 1, 8192, False)])
+def test_general_path(Ts, M, H, E, K, alignment, staged):
+    """Groups, and the batches that a single rank's own kernels do not take."""
+    R, room = len(Ts), len(Ts) * M * K
+    ins = [make_rank_inputs(89, r, Ts[r], H, E, K, "uniform", n_mask=3) for r in range(R)]
+    xs, idxs, ws = [i[0] for i in ins], [i[1] for i in ins], [i[2] for i in ins]
+    want = eo.elastic_dispatch(xs, idxs, ws, E, M, alignment, True)
+    assert any(o["n_expanded"] > room for o in want)
+    bufs = _group(R, M, H, K, staged)
+    keep = []
+    outs = _dispatch(bufs, xs, idxs, ws, E, M, alignment, True, keep)
+    g = torch.Generator().manual_seed(M)
+    ys = [torch.randn((room, H), generator=g).to(torch.bfloat16) for _ in range(R)]
+    back = [{} for _ in range(R)]  # what a rank sends back for (source, token)
+    for r, (d, o) in enumerate(zip(outs, want)):
+        used = o["used"][:room]
+        assert d["psum_expert"].tolist() == o["psum_expert"].tolist()
+        assert torch.equal(d["recv_x"].cpu()[:used.shape[0]][used].view(torch.int16),
+                           o["recv_x"][:room][used].view(torch.int16))
+        assert torch.equal(d["recv_w"].cpu()[:used.shape[0]][used], o["recv_topk_weights"][:room][used])
+        md = o["recv_src_metadata"].clone()
+        md[:, 2:][md[:, 2:] >= room] = -1
+        assert torch.equal(d["md"][:o["n"]].cpu(), md)
+        assert bufs[r].runtime.status() == int(bool((o["recv_src_metadata"][:, 2:] >= room).any()))
+        for key, rows in zip(o["rows"], md[:, 2:].tolist()):
+            there = [ys[r][v] for v in rows if v >= 0]
+            back[r][key] = eo.bf16_sum(there) if there else torch.zeros(H, dtype=torch.bfloat16)
+    got = _combine(bufs, [y.cuda() for y in ys], outs, E, M, True)
+    for s in range(R):
+        for t in range(Ts[s]):
+            lanes = eo.rank_lanes(idxs[s][t], E // R, E)
+            order = [d for d, _ in sorted(lanes.items(), key=lambda kv: kv[1])]
+            ref = eo.bf16_sum([back[d][(s, t)] for d in order]) if order else torch.zeros(H, dtype=torch.bfloat16)
+            if t % max(1, Ts[s] // 200) == 0 or not order:
+                assert torch.equal(got[s][t].cpu().view(torch.int16), ref.view(torch.int16)), (s, t)
