@@ -114,9 +114,10 @@ class ElasticBuffer:
         self.scaleout_rank_idx, self.scaleup_rank_idx = 0, self.rank_idx
         self.num_rdma_ranks, self.num_nvlink_ranks = 1, self.num_ranks
         self._num_sms = 0  # of the buffer's device
-        self._ones: Optional[torch.Tensor] = None
         self.runtime: Optional[ep.Buffer] = ep.Buffer(self.rank_idx, self.num_ranks, num_bytes, False)
         self._connect_native()
+        # the mask of a single rank's calls, complete before any stream can read it
+        self._ones = torch.ones(self.num_ranks, dtype=torch.int32, device="cuda")
         torch.cuda.synchronize()
         if self.num_ranks > 1:
             dist.barrier(group)
@@ -192,10 +193,8 @@ class ElasticBuffer:
     def _active_ranks(self, device: torch.device) -> torch.Tensor:
         """All ranks take part. A group's call may clear entries (timeouts), so each gets
         a mask of its own; a single rank waits for nobody and never writes it."""
-        if self.num_ranks > 1:
+        if self.num_ranks > 1 or self._ones.device != device:
             return torch.ones(self.num_ranks, dtype=torch.int32, device=device)
-        if self._ones is None or self._ones.device != device:
-            self._ones = torch.ones(1, dtype=torch.int32, device=device)
         return self._ones
 
     def _timeout_us(self) -> int:

@@ -80,3 +80,21 @@ def test_counts_of_back_to_back_calls_and_an_empty_batch():
         assert out.shape == (T, H) and not bool(out.any())
     recv, _, _, h, _ = buf.dispatch(x[:0], topk_idx=idx[:0].cuda(), num_experts=E, num_max_tokens_per_rank=T)
     assert recv.shape == (0, H) and h.num_recv_tokens_per_expert_list == [0] * E
+
+
+def test_a_first_call_inside_a_failed_capture_leaves_nothing_behind():
+    """The first call sizes the scratch, which no stream capture allows. The calls after
+    it see a mask of ones all the same, on whatever stream they run."""
+    T, H, E, K = 40, 256, 8, 2
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    x, idx, w = (t.cuda() for t in make_rank_inputs(3, 0, T, H, E, K))
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode="thread_local"):
+            buf.dispatch(x, topk_idx=idx, num_experts=E, num_max_tokens_per_rank=T, do_cpu_sync=False)
+    assert buf._active_ranks(x.device).tolist() == [1]
+    with torch.cuda.stream(torch.cuda.Stream()):
+        recv, _, _, h, _ = buf.dispatch(x, topk_idx=idx, num_experts=E, num_max_tokens_per_rank=T)
+        out, _, _ = buf.combine(recv, h)
+        torch.cuda.synchronize()
+    assert torch.equal(out, x)
