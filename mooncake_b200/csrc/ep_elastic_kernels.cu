@@ -427,7 +427,7 @@ __device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int*
     int e[KB];
 #pragma unroll
     for (int k = 0; k < KB; ++k) e[k] = -1;
-    if (t < p.T) load_choices<KB>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
+    if (t < p.T) load_choices<KB, true>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
     bool any = false;
 #pragma unroll
     for (int k = 0; k < KB; ++k) any |= e[k] >= 0;
@@ -527,7 +527,7 @@ __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upt
     int n = 0;
     for (int t = threadIdx.x; t < upto; t += blockDim.x) {
         int e[kMaxTopk];
-        load_choices<kMaxTopk>(p.topk_idx, t, p.K, p.E, vec, e);
+        load_choices<kMaxTopk, true>(p.topk_idx, t, p.K, p.E, vec, e);
         bool any = false;
 #pragma unroll
         for (int k = 0; k < kMaxTopk; ++k) any |= e[k] >= 0;
@@ -545,8 +545,8 @@ __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upt
 // Every listing of tokens [0, T), repeats included, into hits[E] (whole block, no barrier).
 __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hits) {
     for (int i = threadIdx.x; i < p.T * p.K; i += blockDim.x) {
-        const int e = (int)ld_ro(p.topk_idx + i);
-        if (e >= 0 && e < p.E) atomicAdd(&hits[e], 1);
+        const int e = expert_of(ld_ro(p.topk_idx + i), p.E);
+        if (e >= 0) atomicAdd(&hits[e], 1);
     }
 }
 
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
         raw = ld_ro(p.topk_idx + (size_t)t0 * K + tid);
         if (p.topk_weights) w = ld_ro(p.topk_weights + (size_t)t0 * K + tid);
     }
-    const int e = (int)raw >= 0 && (int)raw < p.E ? (int)raw : -1;
+    const int e = expert_of(raw, p.E);
     if (tid < ne) s_exp[tid] = e;
     if (kCount) {
         __syncthreads();

@@ -587,7 +587,7 @@ __device__ __forceinline__ void cluster_layout(const LayoutParams& p, uint32_t* 
     int e[KB];
 #pragma unroll
     for (int k = 0; k < KB; ++k) e[k] = -1;
-    if (t < p.T) load_choices<KB>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
+    if (t < p.T) load_choices<KB, false>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
     drop_repeats<KB, false>(e);
     __syncthreads();
 #pragma unroll

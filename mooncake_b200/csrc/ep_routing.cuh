@@ -17,9 +17,14 @@
 
 namespace mcep {
 
+// An entry of the index matrix as the elastic calls read it: all 64 bits decide
+// whether it names an expert (-1: it does not). The legacy calls look at the low 32 bits.
+__device__ __forceinline__ int expert_of(int64_t v, int E) { return v >= 0 && v < E ? (int)v : -1; }
+
 // The K choices of token t: e[k] = -1 for masked and out-of-range entries (and
 // for k >= K). `vec`: K is even and the matrix 16-byte aligned, two choices per load.
-template <int KB>
+// kWide: as expert_of.
+template <int KB, bool kWide>
 __device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_idx, int t, int K, int E,
                                              bool vec, int (&e)[KB]) {
     const int64_t* p = topk_idx + (size_t)t * K;
@@ -28,19 +33,22 @@ __device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_id
         for (int k = 0; k < KB; k += 2) {
             longlong2 v = make_longlong2(-1, -1);
             if (k < K) v = ld_ro(reinterpret_cast<const longlong2*>(p + k));
-            e[k] = (int)v.x, e[k + 1] = (int)v.y;
+            e[k] = kWide ? expert_of(v.x, E) : (int)v.x, e[k + 1] = kWide ? expert_of(v.y, E) : (int)v.y;
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < KB; ++k) e[k] = k < K ? (int)ld_ro(p + k) : -1;
+        for (int k = 0; k < KB; ++k) {
+            const int64_t v = k < K ? ld_ro(p + k) : -1;
+            e[k] = kWide ? expert_of(v, E) : (int)v;
+        }
     }
 #pragma unroll
     for (int k = 0; k < KB; ++k)
-        if (e[k] >= E) e[k] = -1;  // (negative already means "no expert")
+        if (!kWide && e[k] >= E) e[k] = -1;  // (negative already means "no expert")
 }
 
 // An expert listed twice by one token counts once: at its first listing, or at
-// its last one (the elastic calls).
+// its last one (the elastic calls: kKeepLast).
 template <int KB, bool kKeepLast>
 __device__ __forceinline__ void drop_repeats(int (&e)[KB]) {
     if (kKeepLast) {
@@ -73,7 +81,7 @@ __device__ __forceinline__ void count_tokens_of(const int64_t* __restrict__ topk
 #pragma unroll
         for (int u = 0; u < kTokens; ++u) {
             if (t0 + u * nthr < to) {
-                load_choices<KB>(topk_idx, t0 + u * nthr, K, E, vec, e[u]);
+                load_choices<KB, kKeepLast>(topk_idx, t0 + u * nthr, K, E, vec, e[u]);
             } else {
 #pragma unroll
                 for (int k = 0; k < KB; ++k) e[u][k] = -1;

@@ -98,3 +98,24 @@ def test_a_first_call_inside_a_failed_capture_leaves_nothing_behind():
         out, _, _ = buf.combine(recv, h)
         torch.cuda.synchronize()
     assert torch.equal(out, x)
+
+
+@pytest.mark.parametrize("T,K,expand", [(40, 2, False), (40, 3, True), (297, 2, True), (700, 8, False), (2000, 3, False)])
+def test_all_64_bits_of_an_entry_decide(T, K, expand):
+    """Entries whose low 32 bits look like an expert name none."""
+    H, E = 128, 8
+    x, idx, w = make_rank_inputs(7, 0, T, H, E, K)
+    g = torch.Generator().manual_seed(T)
+    far = torch.randint(0, 6, (T, K), generator=g)
+    idx += torch.tensor([0, 0, 0, 1 << 32, -(1 << 32), 1 << 62])[far]
+    want = eo.elastic_dispatch([x], [idx], [w], E, T, 1, expand)[0]
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    recv, ridx, _, h, _ = buf.dispatch(x.cuda(), topk_idx=idx.cuda(), topk_weights=w.cuda(), num_experts=E,
+                                       num_max_tokens_per_rank=T, do_expand=expand)
+    assert torch.equal(h.topk_idx.cpu(), idx) and h.num_recv_tokens_per_expert_list == want["hits"]
+    assert torch.equal(ridx.cpu(), want["recv_topk_idx"])
+    assert torch.equal(h.dst_buffer_slot_idx.cpu(), want["dst_buffer_slot_idx"])
+    assert torch.equal(recv.cpu().view(torch.int16), want["recv_x"].view(torch.int16))
+    out, _, _ = buf.combine(recv, h)
+    ref = eo.elastic_combine([want["recv_x"]], [want], [idx], E, expand)[0]
+    assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
