@@ -396,7 +396,11 @@ PyObject* new_ref(PyObject* o) {
 
 uint64_t current_stream() { return reinterpret_cast<uint64_t>(c10::cuda::getCurrentCUDAStream().stream()); }
 
-PyObject* py_current_stream(PyObject*, PyObject*) { return PyLong_FromUnsignedLongLong(current_stream()); }
+PyObject* py_current_stream(PyObject*, PyObject*) {
+    HANDLE_TH_ERRORS  // (no device, no driver)
+    return PyLong_FromUnsignedLongLong(current_stream());
+    END_HANDLE_TH_ERRORS
+}
 
 // ---- the runtime object -----------------------------------------------------------------
 struct RuntimeObject {
