@@ -320,6 +320,10 @@ const at::Tensor* tensor_of(PyObject* o) { return o && THPVariable_Check(o) ? &T
 bool matrix(const at::Tensor* t, at::ScalarType type) {
     return t && t->is_cuda() && t->dim() == 2 && t->scalar_type() == type && t->is_contiguous();
 }
+// At least `n` entries in a row, whatever the tensor's shape.
+bool entries(const at::Tensor* t, at::ScalarType type, int64_t n) {
+    return t && t->is_cuda() && t->scalar_type() == type && t->is_contiguous() && t->numel() >= n;
+}
 bool usable_mask(const at::Tensor* t, int64_t ranks) {
     return t && t->is_cuda() && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
 }
@@ -663,11 +667,11 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
     const int64_t E = r.num(5), M = r.num(6), alignment = r.num(7), timeout = r.num(10), R = s->num_ranks;
     const int expand = r.flag(8), sync = r.flag(9), async = r.flag(11);
     if (!r.ok) return nullptr;
-    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !usable_mask(active, R) || M < 0 || R < 1 ||
-        (args[2] != Py_None && !matrix(w, at::kFloat)))
+    if (!matrix(x, at::kBFloat16) || !idx || idx->dim() < 2 || !usable_mask(active, R) || M < 0 || R < 1 || E < 0)
         Py_RETURN_NONE;
     const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), L = E / R;
-    if (idx->size(0) != T || E < 0 || (w && w->sizes() != idx->sizes())) Py_RETURN_NONE;
+    // [T][K] entries of each are read; their shapes beyond that are the caller's
+    if (!entries(idx, at::kLong, T * K) || (args[2] != Py_None && !entries(w, at::kFloat, T * K))) Py_RETURN_NONE;
     const int64_t n_cap = M * R, out_cap = expand ? n_cap * K : n_cap;
     const at::Device dev = x->device();
 
@@ -690,7 +694,7 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
     const int64_t o_rank = small.reserve(R * 4), o_expert = small.reserve((L + 1) * 4), o_slot = small.reserve(T * K * 4);
     const int64_t o_idx = small.reserve(n_cap * K * 8), o_md = small.reserve(n_cap * (K + 2) * 4);
     const int64_t o_w = w ? small.reserve((expand ? out_cap : n_cap * K) * 4) : 0;
-    const int64_t o_kept = cached ? 0 : small.reserve(T * K * 8);
+    const int64_t o_kept = cached ? 0 : small.reserve(idx->numel() * 8);
     small.allocate();
 
     mcep_elastic_dispatch_args a = {};
@@ -742,7 +746,7 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
                  wrap(small.view(o_md, at::kInt, {n, K + 2})), wrap(small.view(o_rank, at::kInt, {R})),
                  wrap(small.view(o_expert + 4 * first, at::kInt, {L + 1 - first})),
                  wrap(small.view(o_slot, at::kInt, {T, K})),
-                 cached ? new_ref(args[4]) : wrap(small.view(o_kept, at::kLong, {T, K})), counts, wrap_event(ev)});
+                 cached ? new_ref(args[4]) : wrap(small.view(o_kept, at::kLong, idx->sizes())), counts, wrap_event(ev)});
     END_HANDLE_TH_ERRORS
 }
 
@@ -759,7 +763,8 @@ PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args,
     const int64_t E = r.num(6), M = r.num(7), timeout = r.num(9);
     const int expand = r.flag(8), async = r.flag(10);
     if (!r.ok) return nullptr;
-    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !psum || !md || !usable_mask(active, s->num_ranks))
+    if (!matrix(x, at::kBFloat16) || !idx || idx->dim() < 2 || !entries(idx, at::kLong, 0) || !psum || !md ||
+        !usable_mask(active, s->num_ranks) || (args[2] != Py_None && !w))
         Py_RETURN_NONE;
     const int64_t T = idx->size(0), K = idx->size(1), H = x->size(1);
     at::Tensor out = empty({T, H}, at::kBFloat16, x->device());

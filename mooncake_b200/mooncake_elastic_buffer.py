@@ -249,7 +249,7 @@ class ElasticBuffer:
             assert x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16
             assert topk_idx.dtype == torch.int64 and topk_idx.is_contiguous()
             assert topk_weights is None or (topk_weights.dtype == torch.float32 and topk_weights.is_contiguous())
-            raise AssertionError("dispatch takes CUDA tensors x [T, H], topk_idx [T, K], topk_weights [T, K]")
+            raise AssertionError("dispatch takes CUDA tensors: x [T, H], T * K entries of topk_idx and topk_weights")
         (recv_x, recv_topk_idx, recv_topk_weights, recv_src_metadata, psum_rank, psum_expert, dst_buffer_slot_idx,
          kept_idx, counts, event) = out
         out_handle = EPHandle._of(
@@ -282,7 +282,7 @@ class ElasticBuffer:
             x, handle.topk_idx, topk_weights, handle.psum_num_recv_tokens_per_scaleup_rank, handle.recv_src_metadata,
             active_ranks, handle.num_experts, handle.num_max_tokens_per_rank, handle.do_expand, self._timeout_us(),
             async_with_compute_stream)
-        assert res is not None, "combine takes a contiguous [n, H] bf16 CUDA tensor"
+        assert res is not None, "combine takes a contiguous [n, H] bf16 CUDA tensor (and topk_weights as a tensor)"
         combined_x, event = res
         keep = None
         if async_with_compute_stream:

@@ -119,3 +119,32 @@ def test_all_64_bits_of_an_entry_decide(T, K, expand):
     out, _, _ = buf.combine(recv, h)
     ref = eo.elastic_combine([want["recv_x"]], [want], [idx], E, expand)[0]
     assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
+
+
+def test_shapes_of_the_routing_are_the_callers():
+    """T * K entries of topk_idx and topk_weights are read, whatever their shapes: flat weights,
+    matrices made for the largest batch, a trailing dimension of one."""
+    T, M, H, E, K = 40, 64, 128, 8, 3
+    x, idx, w = make_rank_inputs(9, 0, T, H, E, K)
+    want = eo.elastic_dispatch([x], [idx], [w], E, M)[0]
+    more = torch.full((M, K), -1, dtype=torch.int64)
+    more[:T] = idx
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K)
+    for i, wt in ((idx, w.reshape(-1)), (idx, torch.cat([w, w[:M - T]])), (idx, w.reshape(K, T)), (more, w),
+                  (idx.unsqueeze(2), w), (idx, w.unsqueeze(0))):
+        recv, ridx, rw, h, _ = buf.dispatch(x.cuda(), topk_idx=i.cuda(), topk_weights=wt.contiguous().cuda(),
+                                            num_experts=E, num_max_tokens_per_rank=M)
+        assert torch.equal(recv.cpu().view(torch.int16), want["recv_x"].view(torch.int16))
+        assert torch.equal(ridx.cpu(), want["recv_topk_idx"]) and torch.equal(rw.cpu(), want["recv_topk_weights"])
+        assert h.topk_idx.shape == i.shape and torch.equal(h.topk_idx.reshape(-1)[:T * K].cpu(), idx.reshape(-1))
+        if i.shape[0] == T:
+            out, _, _ = buf.combine(recv, h)
+            assert torch.equal(out.cpu(), x)
+    for bad in (w.half(), w[:T // 2], w.tolist()):
+        with pytest.raises((AssertionError, AttributeError)):
+            buf.dispatch(x.cuda(), topk_idx=idx.cuda(), topk_weights=bad if isinstance(bad, list) else bad.cuda(),
+                         num_experts=E, num_max_tokens_per_rank=M)
+    with pytest.raises(AssertionError):
+        buf.dispatch(x.cuda(), topk_idx=idx[:T // 2].cuda(), num_experts=E, num_max_tokens_per_rank=M)
+    with pytest.raises(AssertionError):
+        buf.combine(recv, h, topk_weights=w.tolist())
