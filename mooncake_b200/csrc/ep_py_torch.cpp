@@ -317,15 +317,18 @@ PyType_Spec hook_spec = {"mooncake_b200._mcep_torch.Hook", sizeof(HookObject), 0
 // ---- tensors -------------------------------------------------------------------------
 const at::Tensor* tensor_of(PyObject* o) { return o && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
+// The device can read and write it where it is: its own memory, or pinned host memory.
+bool reachable(const at::Tensor* t) { return t->is_cuda() || (t->is_cpu() && t->is_pinned()); }
+
 bool matrix(const at::Tensor* t, at::ScalarType type) {
-    return t && t->is_cuda() && t->dim() == 2 && t->scalar_type() == type && t->is_contiguous();
+    return t && reachable(t) && t->dim() == 2 && t->scalar_type() == type && t->is_contiguous();
 }
 // At least `n` entries in a row, whatever the tensor's shape.
 bool entries(const at::Tensor* t, at::ScalarType type, int64_t n) {
-    return t && t->is_cuda() && t->scalar_type() == type && t->is_contiguous() && t->numel() >= n;
+    return t && reachable(t) && t->scalar_type() == type && t->is_contiguous() && t->numel() >= n;
 }
 bool usable_mask(const at::Tensor* t, int64_t ranks) {
-    return t && t->is_cuda() && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
+    return t && reachable(t) && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
 }
 
 // torch.empty without the way through the tensor factory (0.2 us per tensor).
@@ -524,7 +527,7 @@ PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssi
     const int64_t M = r.num(3), E = r.num(4), timeout = r.num(5), R = s->num_ranks;
     const int fp8 = r.flag(6), async = r.flag(7), hooked = r.flag(8);
     if (!r.ok) return nullptr;
-    if (!matrix(x, at::kBFloat16) || !matrix(idx, at::kLong) || !usable_mask(active, R)) Py_RETURN_NONE;
+    if (!matrix(x, at::kBFloat16) || !x->is_cuda() || !matrix(idx, at::kLong) || !usable_mask(active, R)) Py_RETURN_NONE;
     const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), RM = R * M;
     if (idx->size(0) != T || T > M || H % 128 != 0 || E <= 0 || E % R != 0 || (fp8 && RM % 4 != 0)) Py_RETURN_NONE;
     const int64_t L = E / R;
@@ -613,7 +616,10 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
     const int zero_copy = r.flag(6), async = r.flag(7), hooked = r.flag(8);
     if (!hr.ok) return nullptr;
     if (!r.ok) return nullptr;
-    if (!(x && x->is_cuda() && x->dim() == 3 && x->scalar_type() == at::kBFloat16 && x->is_contiguous()) ||
+    // (without `out` the result is where x is; with zero copy a group looks only at x's shape)
+    const bool own_out = args[9] != Py_None;
+    if (!(x && (x->is_cuda() || (own_out && ((zero_copy && R > 1) || reachable(x)))) && x->dim() == 3 &&
+          x->scalar_type() == at::kBFloat16 && x->is_contiguous()) ||
         !matrix(idx, at::kLong) || !matrix(w, at::kFloat) || !usable_mask(active, R) || !matrix(src, at::kInt) ||
         !matrix(range, at::kLong) || E <= 0 || E % R != 0)
         Py_RETURN_NONE;
@@ -622,7 +628,7 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
         idx->size(1) != K || T > M || src->size(0) != L || range->size(0) != L || range->size(1) != R)
         Py_RETURN_NONE;
     const at::Tensor* given = tensor_of(args[9]);
-    if (args[9] != Py_None && (!matrix(given, at::kBFloat16) || given->size(0) != T || given->size(1) != H))
+    if (own_out && (!matrix(given, at::kBFloat16) || given->size(0) != T || given->size(1) != H))
         Py_RETURN_NONE;
     at::Tensor out = given ? *given : empty({T, H}, at::kBFloat16, x->device());
     mcep_combine_args a = {};
@@ -667,7 +673,8 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
     const int64_t E = r.num(5), M = r.num(6), alignment = r.num(7), timeout = r.num(10), R = s->num_ranks;
     const int expand = r.flag(8), sync = r.flag(9), async = r.flag(11);
     if (!r.ok) return nullptr;
-    if (!matrix(x, at::kBFloat16) || !idx || idx->dim() < 2 || !usable_mask(active, R) || M < 0 || R < 1 || E < 0)
+    if (!matrix(x, at::kBFloat16) || !x->is_cuda() || !idx || idx->dim() < 2 || !usable_mask(active, R) || M < 0 ||
+        R < 1 || E < 0)
         Py_RETURN_NONE;
     const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), L = E / R;
     // [T][K] entries of each are read; their shapes beyond that are the caller's
@@ -763,7 +770,7 @@ PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args,
     const int64_t E = r.num(6), M = r.num(7), timeout = r.num(9);
     const int expand = r.flag(8), async = r.flag(10);
     if (!r.ok) return nullptr;
-    if (!matrix(x, at::kBFloat16) || !idx || idx->dim() < 2 || !entries(idx, at::kLong, 0) || !psum || !md ||
+    if (!matrix(x, at::kBFloat16) || !x->is_cuda() || !idx || idx->dim() < 2 || !entries(idx, at::kLong, 0) || !psum || !md ||
         !usable_mask(active, s->num_ranks) || (args[2] != Py_None && !w))
         Py_RETURN_NONE;
     const int64_t T = idx->size(0), K = idx->size(1), H = x->size(1);

@@ -60,3 +60,33 @@ def test_wrong_arguments_raise_assertion_errors():
     with pytest.raises(TypeError, match="unexpected"):
         buf.runtime.dispatch(*([0] * 17), wrong=1)
     assert buf.runtime.status() == 0
+
+
+def test_tensors_in_pinned_host_memory():
+    """Everything but the rows of dispatch may lie in host memory that the device can reach."""
+    from mooncake_b200 import ElasticBuffer
+    ins = make_rank_inputs(6, 0, T, H, E, K, n_mask=2)
+    x, (idx, w) = ins[0].cuda(), [t.pin_memory() for t in ins[1:]]
+    active = torch.ones(1, dtype=torch.int32).pin_memory()
+    mine = torch.empty((T, H), dtype=torch.bfloat16).pin_memory()
+    buf = Buffer(FakeGroup(0, 1), 0)
+    recv, cnt, handle, _, _ = buf.dispatch(x, idx, active, M, E, 200_000, use_fp8=False)
+    y = torch.nan_to_num(recv.float()).to(torch.bfloat16)
+    want = ora.dispatch([ins[0]], [ins[1]], M, E, False)[0]
+    assert torch.equal(cnt.cpu(), want["recv_count"])
+    ref = ora.combine([y.cpu()], [ins[1]], [ins[2]],
+                      [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)[0]
+    held = tuple(t.cpu().pin_memory() for t in handle[:2]) + handle[2:]
+    for rows, h, out in ((y, handle, None), (y.cpu().pin_memory(), held, mine)):
+        got, _, _ = buf.combine(rows, idx, w, active, 200_000, h, out=out)
+        torch.cuda.synchronize()
+        assert torch.equal(got.cpu().view(torch.int16), ref.view(torch.int16))
+    for bad in ((x, ins[1], active), (ins[0], idx, active), (x, idx, torch.ones(1, dtype=torch.int32))):
+        with pytest.raises(AssertionError):  # memory that the device cannot reach
+            buf.dispatch(*bad, M, E, 200_000, use_fp8=False)
+    ebuf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K)
+    erecv, _, ew, eh, _ = ebuf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, num_max_tokens_per_rank=M)
+    there = (ins[1] >= 0).any(dim=1)
+    assert torch.equal(erecv.cpu(), ins[0][there]) and torch.equal(ew.cpu(), ins[2][there])
+    out, _, _ = ebuf.combine(erecv, eh)
+    assert torch.equal(out.cpu(), ins[0] * there.unsqueeze(1))
