@@ -75,6 +75,8 @@ PyObject* py_bind(PyObject*, PyObject* table) {
     Py_RETURN_NONE;
 }
 
+#define MCEP_FAST(fn) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn))
+
 // ---- arguments -----------------------------------------------------------------------
 // Positional and keyword arguments of a call into `out[0..n)` (borrowed; null = not given).
 bool collect(const char* const* names, int n, int required, PyObject* const* args, Py_ssize_t nargs,
@@ -108,21 +110,20 @@ bool collect(const char* const* names, int n, int required, PyObject* const* arg
 struct Reader {
     PyObject** v;
     bool ok = true;
-    long long num(int i, long long dflt = 0) {
-        if (v[i] == nullptr || v[i] == Py_None) return dflt;
+    long long num(int i) {
         const long long r = PyLong_AsLongLong(v[i]);
         if (r == -1 && PyErr_Occurred()) ok = false;
         return r;
     }
-    int i32(int i, int dflt = 0) { return (int)num(i, dflt); }
+    int i32(int i) { return (int)num(i); }
     int flag(int i) {
-        if (v[i] == nullptr) return 0;
-        const int r = PyObject_IsTrue(v[i]);
+        if (v[i] == Py_None) PyErr_SetString(PyExc_TypeError, "a truth value is wanted, not None");
+        const int r = v[i] == Py_None ? -1 : PyObject_IsTrue(v[i]);
         if (r < 0) ok = false;
         return r > 0;
     }
     void* ptr(int i) {
-        if (v[i] == nullptr || v[i] == Py_None) return nullptr;
+        if (v[i] == Py_None) return nullptr;
         void* r = PyLong_AsVoidPtr(v[i]);
         if (r == nullptr && PyErr_Occurred()) ok = false;
         return r;
@@ -169,7 +170,10 @@ void event_dealloc(PyObject* self) {
     Py_DECREF(type);
 }
 
-PyObject* event_stream_wait(PyObject* self, PyObject* stream) {
+PyObject* event_stream_wait(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+    static const char* const names[] = {"stream_ptr"};
+    PyObject* stream;
+    if (!collect(names, 1, 1, args, nargs, kwnames, &stream, "current_stream_wait")) return nullptr;
     const unsigned long long s = PyLong_AsUnsignedLongLong(stream);
     if (PyErr_Occurred()) return nullptr;
     if (lib.event_wait(reinterpret_cast<EventObject*>(self)->ev, s)) return fail();
@@ -184,7 +188,8 @@ PyObject* event_sync(PyObject* self, PyObject*) {
 }
 
 PyMethodDef event_methods[] = {
-    {"current_stream_wait", event_stream_wait, METH_O, "Make the stream (a cudaStream_t as an integer) wait."},
+    {"current_stream_wait", MCEP_FAST(event_stream_wait), METH_FASTCALL | METH_KEYWORDS,
+     "current_stream_wait($self, stream_ptr)\n--\n\nMake the stream (a cudaStream_t as an integer) wait."},
     {"synchronize", event_sync, METH_NOARGS, "Wait for the event on the host."},
     {nullptr, nullptr, 0, nullptr}};
 PyType_Slot event_slots[] = {
@@ -299,7 +304,9 @@ void hook_dealloc(PyObject* self) {
     Py_DECREF(type);
 }
 
-PyObject* hook_call(PyObject* self, PyObject*, PyObject*) {
+PyObject* hook_call(PyObject* self, PyObject* args, PyObject* kw) {
+    if (PyTuple_GET_SIZE(args) != 0 || (kw != nullptr && PyDict_GET_SIZE(kw) != 0))
+        return PyErr_Format(PyExc_TypeError, "the receive hook takes no arguments");
     int rc;
     Py_BEGIN_ALLOW_THREADS rc = lib.hook_run(reinterpret_cast<HookObject*>(self)->hook);
     Py_END_ALLOW_THREADS if (rc) return fail();
@@ -463,7 +470,7 @@ PyObject* runtime_dispatch(PyObject* self, PyObject* const* args, Py_ssize_t nar
     a.packed_recv_count = static_cast<int32_t*>(r.ptr(12)), a.packed_recv_src_info = static_cast<int32_t*>(r.ptr(13));
     a.packed_recv_layout_range = static_cast<int64_t*>(r.ptr(14));
     a.async_finish = r.flag(15), a.return_recv_hook = r.flag(16);
-    a.compute_stream = reinterpret_cast<uint64_t>(r.ptr(17));
+    a.compute_stream = (uint64_t)r.num(17);
     if (!r.ok) return nullptr;
     mcep_event* ev = nullptr;
     mcep_hook* hk = nullptr;
@@ -488,7 +495,7 @@ PyObject* runtime_combine(PyObject* self, PyObject* const* args, Py_ssize_t narg
     a.num_combined_tokens = r.i32(7), a.hidden = r.i32(8), a.num_topk = r.i32(9);
     a.num_max_dispatch_tokens_per_rank = r.i32(10), a.num_experts = r.i32(11), a.timeout_us = r.num(12);
     a.zero_copy = r.flag(13), a.combined_x = r.ptr(14), a.async_finish = r.flag(15), a.return_recv_hook = r.flag(16);
-    a.compute_stream = reinterpret_cast<uint64_t>(r.ptr(17));
+    a.compute_stream = (uint64_t)r.num(17);
     if (!r.ok) return nullptr;
     mcep_event* ev = nullptr;
     mcep_hook* hk = nullptr;
@@ -795,8 +802,6 @@ PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args,
     return pack({wrap(std::move(out)), wrap_event(ev)});
     END_HANDLE_TH_ERRORS
 }
-
-#define MCEP_FAST(fn) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(fn))
 
 PyMethodDef runtime_methods[] = {
     {"_adopt", runtime_adopt, METH_VARARGS, "_adopt(handle or None, num_ranks): the mcep_buffer the calls go to."},

@@ -90,3 +90,31 @@ def test_tensors_in_pinned_host_memory():
     assert torch.equal(erecv.cpu(), ins[0][there]) and torch.equal(ew.cpu(), ins[2][there])
     out, _, _ = ebuf.combine(erecv, eh)
     assert torch.equal(out.cpu(), ins[0] * there.unsqueeze(1))
+
+
+def test_what_is_not_a_number_or_a_flag_is_refused():
+    x, idx, w = [t.cuda() for t in make_rank_inputs(5, 0, T, H, E, K)]
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    buf = Buffer(FakeGroup(0, 1), 0)
+    for bad in (dict(timeout_us=None), dict(num_max_dispatch_tokens_per_rank=None), dict(num_experts=None),
+                dict(async_finish=None)):
+        kw = dict(dict(num_max_dispatch_tokens_per_rank=M, num_experts=E, timeout_us=200_000, async_finish=False), **bad)
+        with pytest.raises(TypeError):
+            buf.dispatch(x, idx, active, use_fp8=False, **kw)
+    for at in (3, 8, 9, 15, 17):
+        args = [0] * 18
+        args[at] = None
+        with pytest.raises(TypeError):
+            buf.runtime.dispatch(*args)
+        with pytest.raises(TypeError):
+            buf.runtime.combine(*(args if at in (8, 15, 17) else [0] * 13 + [None] + [0] * 4))
+    recv, _, handle, _, hook = buf.dispatch(x, idx, active, M, E, 200_000, use_fp8=False, return_recv_hook=True)
+    for bad in ((1,), dict(again=True)):
+        with pytest.raises(TypeError):
+            hook(*bad) if isinstance(bad, tuple) else hook(**bad)
+    hook()
+    _, event, _ = buf.combine(recv, idx, w, active, 200_000, handle, async_finish=True)
+    event.event.current_stream_wait(stream_ptr=torch.cuda.current_stream().cuda_stream)
+    with pytest.raises(TypeError):
+        event.event.current_stream_wait()
+    torch.cuda.synchronize()
