@@ -374,7 +374,8 @@ int mcep_elastic_dispatch(mcep_buffer* buf, const mcep_elastic_dispatch_args* ar
  * them and leaves psum_num_recv_tokens_per_scaleup_rank in
  * host_recv_per_rank[num_ranks] and psum_num_recv_tokens_per_expert in
  * host_psum_per_expert[num_experts / num_ranks + 1] (host memory). The rows may
- * still be on their way when it returns, as after any call. */
+ * still be on their way on compute_stream when it returns, as after any call; with
+ * async_with_compute_stream they have arrived. */
 int mcep_elastic_dispatch_counted(mcep_buffer* buf, const mcep_elastic_dispatch_args* args,
                                   int32_t* host_recv_per_rank, int32_t* host_psum_per_expert,
                                   mcep_event** out_event);

@@ -351,6 +351,9 @@ int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, 
         if (int rc = mcep_event_create(reinterpret_cast<uint64_t>(stream), out_event)) return rc;
     if (counts) {
         if (int rc = wait_for_counts(s->host_counts, p.host_seq, stream)) return rc;
+        // on the communication stream nothing but the event orders the rows before the
+        // caller's streams: a caller that waits for the counts need not wait again
+        if (async) EL_CUDA(cudaStreamSynchronize(stream));
         counts->per_rank[0] = s->host_counts[1];
         std::memcpy(counts->per_expert, s->host_counts + 2, (size_t)(E + 1) * sizeof(int32_t));
     }

@@ -148,3 +148,22 @@ def test_shapes_of_the_routing_are_the_callers():
         buf.dispatch(x.cuda(), topk_idx=idx[:T // 2].cuda(), num_experts=E, num_max_tokens_per_rank=M)
     with pytest.raises(AssertionError):
         buf.combine(recv, h, topk_weights=w.tolist())
+
+
+def test_an_asynchronous_call_with_counts_returns_with_its_rows():
+    """do_cpu_sync waits for the whole call where only an event orders its rows: another
+    stream reads them without waiting for that event."""
+    T, H, E, K = 16384, 7168, 8, 2
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    idx = torch.randn((T, E), generator=g, device="cuda").topk(K, dim=-1)[1].contiguous()
+    other = torch.cuda.Stream()
+    for _ in range(4):
+        x = torch.randn((T, H), generator=g, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        recv, _, _, h, event = buf.dispatch(x, topk_idx=idx, num_experts=E, num_max_tokens_per_rank=T,
+                                            do_cpu_sync=True, async_with_compute_stream=True)
+        with torch.cuda.stream(other):
+            got = recv[-64:].clone()  # (written last)
+        torch.cuda.synchronize()
+        assert torch.equal(got, x[-64:]) and torch.equal(recv, x)
