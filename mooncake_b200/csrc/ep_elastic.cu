@@ -430,7 +430,7 @@ int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const 
     EL_REQUIRE(a->recv_x != nullptr && a->recv_topk_idx != nullptr && a->recv_src_metadata != nullptr);
     const int L = E / R;
     ElasticState* s = state_of(b);
-    if (!v.group && !v.defer && mcep::elastic_single_fits(T, K, E))
+    if (!v.group && !v.defer && mcep::elastic_single_fits(T, K, E, a->do_expand != 0, v.num_sms))
         return single_dispatch(b, s, v, a, counts, out_event);
     EL_REQUIRE(counts == nullptr || !v.defer);
     const size_t rec_want = record_bytes(R, M, K);

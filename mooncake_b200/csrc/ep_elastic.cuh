@@ -118,7 +118,7 @@ struct ElasticSingleParams {
     int32_t host_seq;
 };
 // whether the kernels below take this problem (else the general path does)
-bool elastic_single_fits(int T, int K, int E);
+bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms);
 cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx);
 
 // float ones of a given length (the weights of the exchange's reduction)

@@ -2,8 +2,6 @@
 // another GPU; the exchange between the ranks is the group dispatch / combine.
 #include "ep_elastic.cuh"
 
-#include <atomic>
-
 #include "ep_device.cuh"
 #include "ep_kernels.cuh"
 #include "ep_launch.cuh"
@@ -766,11 +764,42 @@ constexpr size_t kSingleSmemMax = 200 * 1024;
 bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand) {
     return expand ? T <= 2 * num_sms : T * K <= 4096 && T <= 7 * num_sms;
 }
+
+struct SingleLayout {
+    const void* kernel;
+    int blocks, threads;  // blocks 0: none that the device takes
+    size_t smem;
+};
+// Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
+// each, or where eight blocks' tables do not fit.
+cudaError_t pick_single_layout(int T, int E, bool expand, SingleLayout* l) {
+    l->blocks = 0;
+    l->kernel = expand ? reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<true>)
+                       : reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<false>);
+    const bool prefer_large = T > kSingleCluster * 256;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        const int blocks = prefer_large == (attempt == 0) ? kSingleClusterLarge : kSingleCluster;
+        l->threads = single_layout_threads(T, blocks);
+        l->smem = l->threads ? single_layout_smem(E, l->threads, expand) : 0;
+        if (l->threads == 0 || l->smem > kSingleSmemMax) continue;
+        bool fits = false;
+        if (cudaError_t e = cluster_fits(l->kernel, blocks, l->threads, l->smem, &fits)) return e;
+        if (fits) {
+            l->blocks = blocks;
+            break;
+        }
+    }
+    return cudaSuccess;
+}
 }  // namespace
 
-bool elastic_single_fits(int T, int K, int E) {
+bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms) {
     const int threads = single_layout_threads(T < 1 ? 1 : T, kSingleClusterLarge);
-    return K <= kMaxTopk && E <= kMaxExperts && threads != 0 && single_layout_smem(E, threads, true) <= kSingleSmemMax;
+    if (K > kMaxTopk || E > kMaxExperts || threads == 0 || single_layout_smem(E, threads, true) > kSingleSmemMax)
+        return false;
+    if (counts_in_copy_kernel(T, K, num_sms, expand)) return true;
+    SingleLayout l;
+    return pick_single_layout(T, E, expand, &l) == cudaSuccess && l.blocks != 0;
 }
 
 cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx) {
@@ -787,29 +816,13 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
-    // Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
-    // each, or where eight blocks' tables do not fit.
-    static std::atomic<int> large{1};  // 0: the device does not take clusters of 16
-    cudaError_t err = cudaErrorInvalidConfiguration;
-    const bool prefer_large = p.T > kSingleCluster * 256;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        const int blocks = prefer_large == (attempt == 0) ? kSingleClusterLarge : kSingleCluster;
-        if (blocks == kSingleClusterLarge && !large.load()) continue;
-        const int threads = single_layout_threads(p.T, blocks);
-        const size_t smem = threads ? single_layout_smem(p.E, threads, expand) : 0;
-        if (threads == 0 || smem > kSingleSmemMax) continue;
-        auto k = expand ? ep_elastic_single_layout_kernel<true> : ep_elastic_single_layout_kernel<false>;
-        if ((err = allow_shared_memory(reinterpret_cast<const void*>(k), smem))) return err;
-        if (blocks == kSingleClusterLarge &&
-            (err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)))
-            return err;
-        err = launch_kernel("ep_elastic_single_layout", k, dim3(blocks), dim3(threads), smem, blocks, ctx, p);
-        if (err == cudaSuccess) break;
-        if (blocks == kSingleCluster) return err;
-        cudaGetLastError();
-        large.store(0);
-    }
-    if (err != cudaSuccess) return err;
+    SingleLayout l;
+    if (cudaError_t err = pick_single_layout(p.T, p.E, expand, &l)) return err;
+    if (l.blocks == 0) return cudaErrorInvalidConfiguration;  // (elastic_single_fits said so)
+    auto layout = expand ? ep_elastic_single_layout_kernel<true> : ep_elastic_single_layout_kernel<false>;
+    if (cudaError_t err = launch_kernel("ep_elastic_single_layout", layout, dim3(l.blocks), dim3(l.threads), l.smem,
+                                        l.blocks, ctx, p))
+        return err;
     LaunchCtx chained = ctx;
     chained.pdl = ctx.chain;
     // Blocks of up to 8 warps. Plain rows: a warp gets about four tiles, all requested at

@@ -118,6 +118,37 @@ cudaError_t allow_shared_memory(const void* kernel, size_t smem) {
     return e;
 }
 
+cudaError_t cluster_fits(const void* kernel, int blocks, int threads, size_t smem, bool* fits) {
+    *fits = false;
+    static std::mutex mu;
+    static std::map<std::tuple<const void*, int, int, int, size_t>, bool> known;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if ((e = allow_shared_memory(kernel, smem))) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    const auto key = std::make_tuple(kernel, dev, blocks, threads, smem);
+    const auto it = known.find(key);
+    if (it != known.end()) {
+        *fits = it->second;
+        return cudaSuccess;
+    }
+    if (blocks > 8 && (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks), cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+    if (e != cudaSuccess && e != cudaErrorInvalidClusterSize) return e;
+    if (e != cudaSuccess) cudaGetLastError();
+    *fits = known[key] = e == cudaSuccess && clusters > 0;
+    return cudaSuccess;
+}
+
 namespace kernels {
 
 constexpr unsigned kFull = 0xffffffffu;
@@ -1889,22 +1920,17 @@ static int layout_cluster_threads(const LayoutParams& p, int blocks) {
 cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
     // Sixteen blocks (opt-in cluster size) once eight would have more than 8 warps
     // each: setting the bits is bound by the shared-memory atomics of a block.
-    static std::atomic<int> large{1};  // 0: the device does not take clusters of 16
+    const void* k = reinterpret_cast<const void*>(ep_layout_cluster_kernel);
     for (int blocks : {kLayoutClusterLarge, kLayoutCluster}) {
-        if (blocks == kLayoutClusterLarge && (p.T <= kLayoutCluster * 256 || !large.load())) continue;
+        if (blocks == kLayoutClusterLarge && p.T <= kLayoutCluster * 256) continue;
         const int threads = layout_cluster_threads(p, blocks);
         if (threads == 0) continue;
         const size_t smem = (size_t)p.E * (threads / 16 + 2) * sizeof(int);
-        if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(ep_layout_cluster_kernel), smem)) return e;
-        if (blocks == kLayoutClusterLarge) {
-            cudaError_t e = cudaFuncSetAttribute(ep_layout_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return e;
-        }
-        const cudaError_t e = launch_kernel("ep_layout_cluster", ep_layout_cluster_kernel, dim3(blocks), dim3(threads),
-                                            smem, blocks, ctx, p);
-        if (e == cudaSuccess || blocks == kLayoutCluster) return e;
-        cudaGetLastError();
-        large.store(0);
+        bool fits = false;
+        if (cudaError_t e = cluster_fits(k, blocks, threads, smem, &fits)) return e;
+        if (fits)
+            return launch_kernel("ep_layout_cluster", ep_layout_cluster_kernel, dim3(blocks), dim3(threads), smem,
+                                 blocks, ctx, p);
     }
     int chunk_tokens = 0, cwords = 0, chunks = 0;
     if (layout_chunking(p, &chunk_tokens, &cwords, &chunks)) {

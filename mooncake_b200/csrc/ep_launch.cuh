@@ -13,6 +13,10 @@ namespace mcep {
 // (asked of the runtime once per kernel, device and larger size).
 cudaError_t allow_shared_memory(const void* kernel, size_t smem);
 
+// Prepares `kernel` for clusters of `blocks` blocks of this shape; `fits`: whether the
+// current device can run them (asked of the runtime once per device and shape).
+cudaError_t cluster_fits(const void* kernel, int blocks, int threads, size_t smem, bool* fits);
+
 // While per-kernel timing is on, kernels run one after the other.
 bool kernel_timing_on();
 

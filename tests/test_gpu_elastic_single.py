@@ -167,3 +167,28 @@ def test_an_asynchronous_call_with_counts_returns_with_its_rows():
             got = recv[-64:].clone()  # (written last)
         torch.cuda.synchronize()
         assert torch.equal(got, x[-64:]) and torch.equal(recv, x)
+
+
+def test_a_launch_that_fails_changes_nothing_for_later_calls():
+    """A launch into a stream whose capture has become invalid fails. The large cluster of the
+    layout kernel, without which 9000 tokens have no layout, is used afterwards as before."""
+    H, E, K = 128, 8, 8
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=9000, hidden=H, num_topk=K)
+    x, idx, w = make_rank_inputs(21, 0, 9000, H, E, K)
+    x, idx = x.cuda(), idx.cuda()
+
+    def layer(T):
+        recv, _, _, h, _ = buf.dispatch(x[:T], topk_idx=idx[:T], num_experts=E, num_max_tokens_per_rank=9000,
+                                        do_cpu_sync=False)
+        return buf.combine(recv, h)[0]
+
+    layer(5000)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode="thread_local"):
+            with pytest.raises(RuntimeError):
+                torch.cuda.current_stream().synchronize()  # not allowed here: ends the capture
+            with pytest.raises(RuntimeError):
+                layer(5000)
+    for T in (5000, 9000):
+        assert torch.equal(layer(T), x[:T])
