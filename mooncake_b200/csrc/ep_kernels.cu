@@ -2263,18 +2263,18 @@ cudaError_t launch_group_dispatch_multi(GroupDispatchParams* params, int n,
     if (n < 1) return cudaSuccess;
     int want = 2;
     size_t smem = 0;
+    bool counting = false;  // one rank that has no layout: all count (a layout is then left unused)
     for (int i = 0; i < n; ++i) {
-        if (params[i].use_fp8 != params[0].use_fp8 || params[i].H != params[0].H ||
-            (params[i].slot == nullptr) != (params[0].slot == nullptr))
-            return cudaErrorInvalidValue;
+        if (params[i].use_fp8 != params[0].use_fp8 || params[i].H != params[0].H) return cudaErrorInvalidValue;
         params[i].C = 1;
+        counting = counting || params[i].slot == nullptr;
         const int blocks = 1 + (params[i].T > 0 ? params[i].T : 1);
         if (blocks > want) want = blocks;
         const size_t sm = (size_t)(2 * params[i].E + 4) * sizeof(int);
         if (sm > smem) smem = sm;
     }
     const int threads = block_threads(params[0].H, 256);
-    const bool fp8 = params[0].use_fp8 != 0, counting = params[0].slot == nullptr;
+    const bool fp8 = params[0].use_fp8 != 0;
     auto k = phases == 3 ? pick_dispatch_multi<3>(fp8, counting) : pick_dispatch_multi<1>(fp8, counting);
     const long long cap = resident_blocks(k, threads, smem, ctx) / n;
     if (cap < 2) return cudaErrorInvalidConfiguration;

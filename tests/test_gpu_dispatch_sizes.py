@@ -8,7 +8,7 @@ import torch
 from mooncake_b200.mooncake_ep_buffer import Buffer
 from oracle import ep_oracle as ora
 from tests.ep_harness import FakeGroup, make_rank_inputs
-from tests.test_gpu_parity import _check_dispatch
+from tests.test_gpu_parity import _check_dispatch, _run_case
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,10 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
         ref = dx.float() * (dw * (di >= 0)).sum(dim=1, keepdim=True)
         assert float((out.float() - ref).abs().max() / ref.abs().max()) < 1e-2
     assert buf.runtime.status() == 0
+
+
+@pytest.mark.parametrize("mode", ["hook", "sync"])
+@pytest.mark.parametrize("T,fp8", [((280, 320), True), ((320, 280, 257), False), ((296, 297), False)])
+def test_ranks_on_either_side_of_the_counting_limit(T, fp8, mode):
+    """In-process groups: one rank counts its layout in the send kernel, another has a layout kernel."""
+    _run_case(dict(R=len(T), tokens=list(T), M=320, H=128, E=8 * len(T), K=16, fp8=fp8, seed=3), mode=mode)
