@@ -154,9 +154,8 @@ int mcep_launch_deferred(mcep_buffer* const* bufs, int n);
  *                     timeout_us is -1 (default 10000)
  *   "pdl"             1 = kernels of one call are chained with programmatic
  *                     dependent launch (default 1)
- *   "fuse_layout"     accepted, without effect: whether a dispatch call counts its
- *                     routing layout inside the send kernel follows from the
- *                     batch size alone
+ *   "fuse_layout"     1 = small batches count their routing layout inside the
+ *                     send kernel instead of in a kernel of its own (default 1)
  *   "one_kernel"      1 = small batches in a group run the send and the receive
  *                     phase of a call in one launch (default 1)
  *   "defer_launch"    1 = in-process groups: prepare calls, launch them together

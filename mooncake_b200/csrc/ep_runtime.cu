@@ -248,6 +248,7 @@ struct mcep_buffer {
     bool all_peers = false;
     bool force_staged = false;
     bool pdl = true;
+    bool fuse_layout = true;
     bool one_kernel = true;
     int64_t hard_timeout_ns = 10ll * 1000 * 1000 * 1000;
     char* base = nullptr;            // symmetric allocation: header region + data area
@@ -770,7 +771,7 @@ int mcep_buffer_set_option(mcep_buffer* b, const char* name, int64_t value) {
     } else if (!std::strcmp(name, "pdl")) {
         b->pdl = value != 0;
     } else if (!std::strcmp(name, "fuse_layout")) {
-        // where the layout is counted follows from the batch size alone
+        b->fuse_layout = value != 0;
     } else if (!std::strcmp(name, "one_kernel")) {
         b->one_kernel = value != 0;
     } else if (!std::strcmp(name, "defer_launch")) {
@@ -919,7 +920,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
     // Larger batches get their layout from a kernel of its own.
-    const bool counting = mcep::counts_in_send_kernel(T, K, b->num_sms, group);
+    const bool counting = (b->fuse_layout || T == 0) && mcep::counts_in_send_kernel(T, K, b->num_sms, group);
     if (!counting) {
         mcep::LayoutParams lp = {};
         lp.topk_idx = a->topk_idx;
@@ -987,7 +988,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
 
     const int num_sms = b->num_sms;
     // Small batches, rows in place, no hook: one launch does it all.
-    bool one_kernel = !p.copy_rows && !a->return_recv_hook && b->one_kernel &&
+    bool one_kernel = counting && !p.copy_rows && !a->return_recv_hook && b->one_kernel &&
                       mcep::group_call_can_be_one_kernel(T, K, E, num_sms);
     if (b->defer) {
         MCEP_REQUIRE(!a->async_finish && !b->graph_mode);

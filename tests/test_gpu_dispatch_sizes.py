@@ -5,6 +5,7 @@ block and their remainders; odd top-k (index pairs cannot be loaded) and repeats
 import pytest
 import torch
 
+from mooncake_b200 import ep
 from mooncake_b200.mooncake_ep_buffer import Buffer
 from oracle import ep_oracle as ora
 from tests.ep_harness import FakeGroup, make_rank_inputs
@@ -59,3 +60,31 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
 def test_ranks_on_either_side_of_the_counting_limit(T, fp8, mode):
     """In-process groups: one rank counts its layout in the send kernel, another has a layout kernel."""
     _run_case(dict(R=len(T), tokens=list(T), M=320, H=128, E=8 * len(T), K=16, fp8=fp8, seed=3), mode=mode)
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("T", [0, 1, 40, 296])
+def test_a_layout_kernel_for_small_batches(T, staged):
+    """Option "fuse_layout" 0: the layout comes from a kernel of its own, with the same results."""
+    H, E, K, M = 640, 16, 3, 300
+    x, idx, w = make_rank_inputs(13, 0, T, H, E, K, n_mask=T // 7)
+    buf = Buffer(FakeGroup(0, 1), Buffer.get_ep_buffer_size_hint(M, H, 1, E) if staged else 0)
+    buf.runtime.set_option("force_staged", int(staged))
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    want = ora.dispatch([x], [idx], M, E, True)
+    for fuse in (1, 0):
+        buf.runtime.set_option("fuse_layout", fuse)
+        ep.set_kernel_timing(True)
+        try:
+            recv, cnt, handle, _, _ = buf.dispatch(x.cuda(), idx.cuda(), active, M, E, 2_000_000)
+        finally:
+            ep.set_kernel_timing(False)
+        torch.cuda.synchronize()
+        assert any("layout" in name for name in ep.drain_kernel_times()) == (not fuse and T > 0)
+        _check_dispatch(dict(R=1, E=E, M=M, fp8=True),
+                        [dict(recv_x=recv[0], scales=recv[1], recv_count=cnt, handle=handle)], want, None)
+        y = torch.randn((E, M, H), device="cuda").to(torch.bfloat16)
+        out, _, _ = buf.combine(y, idx.cuda(), w.cuda(), active, 2_000_000, handle)
+        ref = ora.combine([y.cpu()], [idx], [w], [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)
+        assert torch.equal(out.cpu().view(torch.int16), ref[0].view(torch.int16))
+    assert buf.runtime.status() == 0
