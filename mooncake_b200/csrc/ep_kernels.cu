@@ -27,6 +27,7 @@
 //     and are never cleaned.
 #include "ep_kernels.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -2074,7 +2075,7 @@ static ReduceShape reduce_shape(int T, int K, int H, int num_sms) {
     // 22.5). More: runs of two, handed out as blocks finish, so that no SM falls behind
     // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
     // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181).
-    const int resident = num_sms * (2 * kReduceWarps * 32 / s.threads) / parts;
+    const int resident = std::max(1, num_sms * (2 * kReduceWarps * 32 / s.threads) / parts);
     const int waves = (groups + resident - 1) / resident;
     const int run = K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
     s.span = run * s.tokens_per_block;

@@ -88,3 +88,17 @@ def test_a_layout_kernel_for_small_batches(T, staged):
         ref = ora.combine([y.cpu()], [idx], [w], [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)
         assert torch.equal(out.cpu().view(torch.int16), ref[0].view(torch.int16))
     assert buf.runtime.status() == 0
+
+
+@pytest.mark.parametrize("T", [2, 150])
+def test_rows_of_more_blocks_than_are_resident(T):
+    """Rows so long that one alone is shared by more combine blocks than the device holds at a time."""
+    H, E, K = 128 * 18952, 2, 2
+    x = torch.randn((T, H), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
+    idx = torch.tensor([[0, 1]] * T, device="cuda")
+    w = torch.full((T, K), 0.5, device="cuda")
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    buf = Buffer(FakeGroup(0, 1), 0)
+    recv, _, handle, _, _ = buf.dispatch(x, idx, active, T, E, 2_000_000, use_fp8=False)
+    out, _, _ = buf.combine(recv, idx, w, active, 2_000_000, handle)
+    assert torch.equal(recv[0], x) and torch.equal(recv[1], x) and torch.equal(out, x)
