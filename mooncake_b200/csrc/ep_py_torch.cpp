@@ -338,8 +338,12 @@ bool usable_mask(const at::Tensor* t, int64_t ranks) {
     return t && reachable(t) && t->dim() == 1 && t->numel() == ranks && t->scalar_type() == at::kInt && t->is_contiguous();
 }
 
-// torch.empty without the way through the tensor factory (0.2 us per tensor).
+// torch.empty without the way through the tensor factory (0.2 us per tensor), except where
+// torch has been asked to fill what is not initialised.
 at::Tensor empty(at::IntArrayRef size, at::ScalarType type, at::Device dev) {
+    const at::Context& context = at::globalContext();
+    if (context.deterministicAlgorithms() && context.deterministicFillUninitializedMemory())
+        return at::empty(size, at::TensorOptions(type).device(dev));
     if (c10::cuda::current_device() != dev.index()) return at::detail::empty_cuda(size, type, dev, std::nullopt);
     const auto meta = c10::scalarTypeToTypeMeta(type);
     size_t bytes = meta.itemsize();

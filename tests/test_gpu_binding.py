@@ -118,3 +118,24 @@ def test_what_is_not_a_number_or_a_flag_is_refused():
     with pytest.raises(TypeError):
         event.event.current_stream_wait()
     torch.cuda.synchronize()
+
+
+def test_outputs_are_filled_where_torch_is_asked_to():
+    """Under deterministic algorithms torch.empty fills its tensors; so do the calls' outputs."""
+    from mooncake_b200 import ElasticBuffer
+    x, idx, w = [t.cuda() for t in make_rank_inputs(5, 0, T, H, E, K)]
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    buf = Buffer(FakeGroup(0, 1), 0)
+    ebuf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K)
+    zeros = [torch.zeros(1 << 20, device="cuda") for _ in range(8)]
+    del zeros  # (blocks that the outputs may get: what is not written reads as zeros)
+    torch.use_deterministic_algorithms(True)
+    try:
+        recv, cnt, handle, _, _ = buf.dispatch(x, idx, active, M, E, 200_000, use_fp8=False)
+        erecv, eidx, ew, eh, _ = ebuf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E,
+                                               num_max_tokens_per_rank=M, do_cpu_sync=False)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    n = cnt.tolist()
+    assert all(bool(recv[e, n[e]:].isnan().all()) and bool((handle[0][e, n[e]:] == -1).all()) for e in range(E))
+    assert torch.equal(erecv[:T], x) and bool(erecv[T:].isnan().all()) and bool(ew[T:].isnan().all())
