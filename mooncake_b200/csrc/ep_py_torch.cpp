@@ -540,7 +540,7 @@ PyObject* runtime_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssi
     if (!r.ok) return nullptr;
     if (!matrix(x, at::kBFloat16) || !x->is_cuda() || !matrix(idx, at::kLong) || !usable_mask(active, R)) Py_RETURN_NONE;
     const int64_t T = x->size(0), H = x->size(1), K = idx->size(1), RM = R * M;
-    if (idx->size(0) != T || T > M || H % 128 != 0 || E <= 0 || E % R != 0 || (fp8 && RM % 4 != 0)) Py_RETURN_NONE;
+    if (idx->size(0) != T || T > M || H % 128 != 0 || E < 0 || E % R != 0 || (fp8 && RM % 4 != 0)) Py_RETURN_NONE;
     const int64_t L = E / R;
     const at::Device dev = x->device();
     at::Tensor recv_x;

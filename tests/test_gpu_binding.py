@@ -49,6 +49,8 @@ def test_wrong_arguments_raise_assertion_errors():
             buf.dispatch(*bad, E, 200_000, use_fp8=False)
     with pytest.raises(AssertionError):
         buf.dispatch(x, idx, active, 15, E, 200_000)  # FP8: the rows of an expert come in fours
+    with pytest.raises(RuntimeError, match="E > 0"):
+        buf.dispatch(x, idx, active, M, 0, 200_000)
     with pytest.raises(RuntimeError, match="async_finish"):
         buf.dispatch(x, idx, active, M, E, 200_000, async_finish=True, return_recv_hook=True)
     y, _, handle, _ = _layer(buf, dev, active)
