@@ -4,6 +4,10 @@ edges of its warps, blocks and cluster sizes, the first batch beyond it (general
 path), several rows per block and their remainders, odd top-k, repeats inside a
 token, padding tokens, an alignment; through `ElasticBuffer` with and without the
 wait for the counts."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -82,7 +86,16 @@ def test_counts_of_back_to_back_calls_and_an_empty_batch():
     assert recv.shape == (0, H) and h.num_recv_tokens_per_expert_list == [0] * E
 
 
-def test_a_first_call_inside_a_failed_capture_leaves_nothing_behind():
+@pytest.mark.parametrize("body", ["_first_call_inside_a_failed_capture", "_launch_that_fails"])
+def test_failed_captures(body):
+    """In a process of its own: a capture that fails leaves torch's default generator in use."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    got = subprocess.run([sys.executable, "-c", f"from tests import test_gpu_elastic_single as t; t.{body}()"],
+                         cwd=root, capture_output=True, text=True, timeout=300)
+    assert got.returncode == 0, got.stderr[-3000:]
+
+
+def _first_call_inside_a_failed_capture():
     """The first call sizes the scratch, which no stream capture allows. The calls after
     it see a mask of ones all the same, on whatever stream they run."""
     T, H, E, K = 40, 256, 8, 2
@@ -169,7 +182,7 @@ def test_an_asynchronous_call_with_counts_returns_with_its_rows():
         assert torch.equal(got, x[-64:]) and torch.equal(recv, x)
 
 
-def test_a_launch_that_fails_changes_nothing_for_later_calls():
+def _launch_that_fails():
     """A launch into a stream whose capture has become invalid fails. The large cluster of the
     layout kernel, without which 9000 tokens have no layout, is used afterwards as before."""
     H, E, K = 128, 8, 8
