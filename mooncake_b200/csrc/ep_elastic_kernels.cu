@@ -518,18 +518,34 @@ __global__ void __launch_bounds__(1024) ep_elastic_single_layout_kernel(ElasticS
         single_layout<kExpand, 16>(p, smem_i32);
 }
 
+// Whether any of the `n` entries from `q` on names an expert; n <= 8, requested together.
+__device__ __forceinline__ bool names_any(const int64_t* q, int n, int E, bool vec) {
+    bool any = false;
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+            longlong2 v = make_longlong2(-1, -1);
+            if (k < n) v = ld_ro(reinterpret_cast<const longlong2*>(q + k));
+            any |= (uint64_t)v.x < (uint64_t)E || (uint64_t)v.y < (uint64_t)E;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int64_t v = k < n ? ld_ro(q + k) : -1;
+            any |= (uint64_t)v < (uint64_t)E;
+        }
+    }
+    return any;
+}
+
 // Tokens of [0, upto) that name any expert; whole block, once per kernel.
 __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upto) {
     __shared__ int s_sent[32];
     const bool vec = choices_in_pairs(p.topk_idx, p.K);
     int n = 0;
     for (int t = threadIdx.x; t < upto; t += blockDim.x) {
-        int e[kMaxTopk];
-        load_choices<kMaxTopk, true>(p.topk_idx, t, p.K, p.E, vec, e);
-        bool any = false;
-#pragma unroll
-        for (int k = 0; k < kMaxTopk; ++k) any |= e[k] >= 0;
-        n += any;
+        const int64_t* q = p.topk_idx + (size_t)t * p.K;
+        n += names_any(q, min(p.K, 8), p.E, vec) || (p.K > 8 && names_any(q + 8, p.K - 8, p.E, vec));
     }
     if (upto <= (int)blockDim.x) return __syncthreads_count(n);  // one pass (128 tokens: 0.3 us less)
     n = __reduce_add_sync(kAll, n);
@@ -543,8 +559,8 @@ __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upt
 // Every listing of tokens [0, T), repeats included, into hits[E] (whole block, no barrier).
 __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hits) {
     for (int i = threadIdx.x; i < p.T * p.K; i += blockDim.x) {
-        const int e = expert_of(ld_ro(p.topk_idx + i), p.E);
-        if (e >= 0) atomicAdd(&hits[e], 1);
+        const int e = all_bits(ld_ro(p.topk_idx + i));
+        if (e >= 0 && e < p.E) atomicAdd(&hits[e], 1);
     }
 }
 
@@ -609,7 +625,7 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
         raw = ld_ro(p.topk_idx + (size_t)t0 * K + tid);
         if (p.topk_weights) w = ld_ro(p.topk_weights + (size_t)t0 * K + tid);
     }
-    const int e = expert_of(raw, p.E);
+    const int e = all_bits(raw) < p.E ? all_bits(raw) : -1;
     if (tid < ne) s_exp[tid] = e;
     if (kCount) {
         __syncthreads();

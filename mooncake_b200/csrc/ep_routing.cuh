@@ -17,13 +17,13 @@
 
 namespace mcep {
 
-// An entry of the index matrix as the elastic calls read it: all 64 bits decide
-// whether it names an expert (-1: it does not). The legacy calls look at the low 32 bits.
-__device__ __forceinline__ int expert_of(int64_t v, int E) { return v >= 0 && v < E ? (int)v : -1; }
+// An entry of the index matrix as the elastic calls read it: all 64 bits decide whether it
+// names an expert (negative: it does not). The legacy calls look at the low 32 bits.
+__device__ __forceinline__ int all_bits(int64_t v) { return (int)(v >> 32) == 0 ? (int)v : -1; }
 
 // The K choices of token t: e[k] = -1 for masked and out-of-range entries (and
 // for k >= K). `vec`: K is even and the matrix 16-byte aligned, two choices per load.
-// kWide: as expert_of.
+// kWide: as all_bits.
 template <int KB, bool kWide>
 __device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_idx, int t, int K, int E,
                                              bool vec, int (&e)[KB]) {
@@ -33,18 +33,18 @@ __device__ __forceinline__ void load_choices(const int64_t* __restrict__ topk_id
         for (int k = 0; k < KB; k += 2) {
             longlong2 v = make_longlong2(-1, -1);
             if (k < K) v = ld_ro(reinterpret_cast<const longlong2*>(p + k));
-            e[k] = kWide ? expert_of(v.x, E) : (int)v.x, e[k + 1] = kWide ? expert_of(v.y, E) : (int)v.y;
+            e[k] = kWide ? all_bits(v.x) : (int)v.x, e[k + 1] = kWide ? all_bits(v.y) : (int)v.y;
         }
     } else {
 #pragma unroll
         for (int k = 0; k < KB; ++k) {
             const int64_t v = k < K ? ld_ro(p + k) : -1;
-            e[k] = kWide ? expert_of(v, E) : (int)v;
+            e[k] = kWide ? all_bits(v) : (int)v;
         }
     }
 #pragma unroll
     for (int k = 0; k < KB; ++k)
-        if (!kWide && e[k] >= E) e[k] = -1;  // (negative already means "no expert")
+        if (e[k] >= E) e[k] = -1;  // (negative already means "no expert")
 }
 
 // An expert listed twice by one token counts once: at its first listing, or at
