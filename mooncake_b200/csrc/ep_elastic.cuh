@@ -117,9 +117,16 @@ struct ElasticSingleParams {
     int32_t* host_counts;
     int32_t host_seq;
 };
-// whether the kernels below take this problem (else the general path does)
-bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms);
-cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx);
+// The layout kernel's cluster; blocks 0: no launch of its own, the copy kernel counts.
+struct SingleLayout {
+    const void* kernel = nullptr;
+    int blocks = 0, threads = 0;
+    size_t smem = 0;
+};
+// whether the kernels below take this problem (else the general path does), and with which layout
+bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms, SingleLayout* layout);
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleLayout& layout,
+                                           const LaunchCtx& ctx);
 
 // float ones of a given length (the weights of the exchange's reduction)
 cudaError_t launch_elastic_fill_ones(float* w, size_t n, cudaStream_t stream);

@@ -781,15 +781,9 @@ bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand) {
     return expand ? T <= 2 * num_sms : T * K <= 4096 && T <= 7 * num_sms;
 }
 
-struct SingleLayout {
-    const void* kernel;
-    int blocks, threads;  // blocks 0: none that the device takes
-    size_t smem;
-};
 // Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
 // each, or where eight blocks' tables do not fit.
-cudaError_t pick_single_layout(int T, int E, bool expand, SingleLayout* l) {
-    l->blocks = 0;
+bool pick_single_layout(int T, int E, bool expand, SingleLayout* l) {
     l->kernel = expand ? reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<true>)
                        : reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<false>);
     const bool prefer_large = T > kSingleCluster * 256;
@@ -799,28 +793,26 @@ cudaError_t pick_single_layout(int T, int E, bool expand, SingleLayout* l) {
         l->smem = l->threads ? single_layout_smem(E, l->threads, expand) : 0;
         if (l->threads == 0 || l->smem > kSingleSmemMax) continue;
         bool fits = false;
-        if (cudaError_t e = cluster_fits(l->kernel, blocks, l->threads, l->smem, &fits)) return e;
-        if (fits) {
+        if (cluster_fits(l->kernel, blocks, l->threads, l->smem, &fits) == cudaSuccess && fits) {
             l->blocks = blocks;
-            break;
+            return true;
         }
     }
-    return cudaSuccess;
+    return false;
 }
 }  // namespace
 
-bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms) {
+bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms, SingleLayout* layout) {
     const int threads = single_layout_threads(T < 1 ? 1 : T, kSingleClusterLarge);
     if (K > kMaxTopk || E > kMaxExperts || threads == 0 || single_layout_smem(E, threads, true) > kSingleSmemMax)
         return false;
-    if (counts_in_copy_kernel(T, K, num_sms, expand)) return true;
-    SingleLayout l;
-    return pick_single_layout(T, E, expand, &l) == cudaSuccess && l.blocks != 0;
+    return counts_in_copy_kernel(T, K, num_sms, expand) || pick_single_layout(T, E, expand, layout);
 }
 
-cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const LaunchCtx& ctx) {
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleLayout& l,
+                                           const LaunchCtx& ctx) {
     const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-    if (counts_in_copy_kernel(p.T, p.K, ctx.num_sms, expand)) {
+    if (l.blocks == 0) {
         // one launch: the block of the counts, and a block per token or (flat) per as many
         // tokens as make one resident wave
         p.C = expand ? 1 : (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
@@ -832,9 +824,6 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
-    SingleLayout l;
-    if (cudaError_t err = pick_single_layout(p.T, p.E, expand, &l)) return err;
-    if (l.blocks == 0) return cudaErrorInvalidConfiguration;  // (elastic_single_fits said so)
     auto layout = expand ? ep_elastic_single_layout_kernel<true> : ep_elastic_single_layout_kernel<false>;
     if (cudaError_t err = launch_kernel("ep_elastic_single_layout", layout, dim3(l.blocks), dim3(l.threads), l.smem,
                                         l.blocks, ctx, p))

@@ -126,7 +126,6 @@ cudaError_t cluster_fits(const void* kernel, int blocks, int threads, size_t sme
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if ((e = allow_shared_memory(kernel, smem))) return e;
     std::lock_guard<std::mutex> lk(mu);
     const auto key = std::make_tuple(kernel, dev, blocks, threads, smem);
     const auto it = known.find(key);
@@ -134,6 +133,7 @@ cudaError_t cluster_fits(const void* kernel, int blocks, int threads, size_t sme
         *fits = it->second;
         return cudaSuccess;
     }
+    if ((e = allow_shared_memory(kernel, smem))) return e;
     if (blocks > 8 && (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks), cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem;
