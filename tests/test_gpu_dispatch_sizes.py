@@ -19,6 +19,7 @@ SIZES = [  # T, H, E, K, fp8
     (1023, 640, 24, 6, True), (1500, 8320, 8, 2, False), (2049, 384, 128, 8, True), (4096, 128, 4096, 4, False),
     (2341, 7168, 8, 8, False), (592, 4096, 16, 3, True), (593, 4096, 16, 3, False), (4096, 1024, 8, 2, True), (4097, 640, 8, 2, False), (8192, 128, 8, 1, True),
     (8192, 128, 256, 8, True), (8193, 128, 256, 8, True), (9001, 256, 16, 1, False),
+    (400, 12416, 8, 8, False), (4800, 4096, 8, 8, False),
 ]
 
 
@@ -46,6 +47,14 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
             _check_dispatch(dict(R=1, E=E, M=M, fp8=fp8), got, want, None)
         else:
             assert torch.equal(cnt.cpu(), want[0]["recv_count"])
+        if E * M * H <= 1 << 28:
+            # combine, bit for bit: weights in listing order, every row from its own place
+            y = torch.randn((E, M, H), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda",
+                            dtype=torch.bfloat16)
+            out, _, _ = buf.combine(y, di, dw, active, 2_000_000, handle)
+            ref = ora.combine([y.cpu()], [idx], [w],
+                              [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)[0]
+            assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
         if fp8:
             continue
         # the rows went where combine looks for them: x times the sum of the listed weights
