@@ -336,7 +336,9 @@ int mcep_combine(mcep_buffer* buf, const mcep_combine_args* args,
  *   recv_topk_weights [n][K] fp32 (do_expand: [rows], the weight of that choice); optional
  *   recv_src_metadata [n][K+2] int32: source rank * M + token, source rank * K +
  *       last lane that names a local expert, and with do_expand the row of each lane
- * Rows beyond the received count are left untouched. Only bf16 payloads
+ * Rows beyond the received count are left untouched. Expanded rows that aligned
+ * segments push beyond n_cap * num_topk are dropped: -1 in recv_src_metadata,
+ * status bit 1, nothing added for them in combine. Only bf16 payloads
  * (x_element_size 2, no scale packs); the reference's pre-quantised (x, sf)
  * input is not built. `cached_mode` (dispatch again with the routing of an
  * earlier handle) recomputes the same layout from `topk_idx` - pass the
@@ -381,7 +383,7 @@ int mcep_elastic_dispatch_counted(mcep_buffer* buf, const mcep_elastic_dispatch_
 
 /* Replaces MooncakeElasticBuffer::combine
  * (mooncake-ep/src/mooncake_ep_elastic_buffer.cpp:362-426).
- * x: [n][H] bf16, one row per received token (do_expand: the expanded rows,
+ * x: [num_input_tokens][H] bf16, one row per received token (do_expand: the expanded rows,
  * summed per received token before they travel - one row copied, two added as
  * one bf16 addition, more accumulated in fp32 and rounded once:
  * mooncake-ep/include/elastic/mooncake_ep_elastic_combine_official.cuh:146-216

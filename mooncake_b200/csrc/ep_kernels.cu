@@ -1025,7 +1025,7 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
 // a block's warps are the grid's y. A barrier per token (tokens handed out by a
 // counter) took 111 us.
 // kAbs: rowmap holds rows of the whole tensor and every weight is 1 (elastic calls).
-constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM: nothing spills
+constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM (with kAbs 12 bytes spill, without none)
 
 template <int kDepth, bool kAbs, int kBlocks>
 __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_kernel(DirectCombineParams p) {
@@ -1991,8 +1991,12 @@ bool counts_in_send_kernel(int T, int K, int num_sms, bool group) {
 // 14 KB to 4 in FP8: 47.4 us per layer with 8 warps, 51.9 with 14; 2000 rows of 4 KB to 8:
 // 25.6 with one token per block, 26.9 with four). A warp per tile again where twice the
 // L2 and more of bf16 rows is written, 8 per token: the stores alone are the bound then
-// and fewer rows at a time suit HBM (4096 rows of 14 KB to 8 after a large write: 91.6
-// us, 8 warps 93.1; to 4, us per layer: 97.4 with 8 warps, 104.3 with 14).
+// and fewer rows at a time suit HBM (to 4, 4096 rows of 14 KB: 97.4 us per layer with 8
+// warps, 104.3 with 14; to 8, a warp per tile | 8 warps, rows of 14 KB: 2600 114.9 | 115.3,
+// 3000 131.5 | 132.0, 4096 173.8 | 174.9, 8192 331.0 | 332.3; 6000 of 12 KB 214.0 | 214.9;
+// 2600 of 16 KB 129.0 | 129.4, 4096 195.7 | 197.2; to 16, 4096 of 14 KB 319.9 | 322.8; runs
+// of one side differ by 0.1 %. Below the limit, 2048 and 2300 of 14 KB, no difference; rows
+// of 10 KB lose 0.3 %, 8000 237.7 | 237.2; up to 8 KB there are 8 warps either way).
 // A group's sender blocks are one resident wave that strides: batches of 16 warp tiles,
 // 8 warps once there are more tokens than blocks (2000 rows of 8 KB to 8: 64.0 us per
 // layer, 16 warps 67.3; one token per batch 64.6, rows of 2 KB 30.7 against 27.0), a warp
@@ -2151,7 +2155,8 @@ cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& c
     const size_t smem = dispatch_smem(p);
     auto k = pick_dispatch<1>(p.use_fp8 != 0, p.slot == nullptr);
     // the control block, then one block per token (small batches) or a resident wave
-    // (a wave, not a block per batch: every block ends with a system-scope fence)
+    // (a wave, not a block per batch: a block that stored rows in a peer's memory, nearly
+    // every one in a group of several GPUs, ends with a system-scope fence)
     long long cap = resident_blocks(k, s.threads, smem, ctx) - 1;
     if (cap < 1) cap = 1;
     const int batches = p.T > 0 ? (p.T + p.C - 1) / p.C : 1;
@@ -2201,7 +2206,12 @@ cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const Laun
 }
 
 cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx) {
-    // (rows of 8 tiles and more: 2000 tokens of 4 tiles to 4 took 10.1 us with it, 9.0 without)
+    // Rows of 8 tiles and more (one rank on this path, us per layer with it | without; 2000
+    // tokens of 4 tiles to 4, the kernel alone 10.1 | 9.0): 8 tiles to 8, 2000 tokens 63.9 |
+    // 69.7, 1024 38.9 | 38.9, 600 30.0 | 28.6, 300 25.6 | 24.5, to 2 2000 32.7 | 33.4; 10
+    // tiles 2000 78.1 | 95.3, 1024 46.2 | 50.4, 300 25.5 | 25.5; 14 tiles 2000 103.8 | 115.8,
+    // 600 39.9 | 40.8, 300 28.2 | 28.6; 16 tiles 1024 63.2 | 71.4. At 8 tiles alone the line
+    // lies too low for fewer than about 1000 tokens.
     if (p.T > ctx.num_sms && p.H >= 8 * kTileChannels) {
         const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
         p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;

@@ -208,7 +208,12 @@ class ElasticBuffer:
                  expert_alignment: Optional[int] = None, handle: Optional[EPHandle] = None,
                  do_expand: bool = False, do_cpu_sync: Optional[bool] = None,
                  num_sms: Optional[int] = None, async_with_compute_stream: bool = False):
-        """Reference :437-714. Returns (recv_x, recv_topk_idx, recv_topk_weights, handle, event)."""
+        """Reference :437-714. Returns (recv_x, recv_topk_idx, recv_topk_weights, handle, event).
+
+        With `do_cpu_sync` the host waits for the counts; the rows are ordered on the current stream
+        as after any call, and have arrived where the call is asynchronous. Expanded rows that
+        `expert_alignment` pushes beyond ranks * num_max_tokens_per_rank * top-k are dropped (row -1
+        in the handle's metadata, status bit 1)."""
         if self.runtime is None:
             raise RuntimeError("ElasticBuffer has been destroyed")
         if isinstance(x, tuple):
