@@ -1025,7 +1025,7 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
 // a block's warps are the grid's y. A barrier per token (tokens handed out by a
 // counter) took 111 us.
 // kAbs: rowmap holds rows of the whole tensor and every weight is 1 (elastic calls).
-constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM (with kAbs 12 bytes spill, without none)
+constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM: nothing spills in the kernel below
 
 template <int kDepth, bool kAbs, int kBlocks>
 __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_kernel(DirectCombineParams p) {
@@ -1044,6 +1044,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     const int first = blockIdx.x * (p.span ? p.span : p.tokens_per_block);
     const int end = p.span ? min(p.T, first + p.span) : p.T;
 
+    // rows that there are (kAbs: a dispatch may have kept some beyond the caller's tensor)
+    const unsigned rows = kAbs ? (unsigned)p.M : 1u << 31;
     int next_row = -1, next_e = -1;
     float next_w = 1.f;
     auto request = [&](int tok) {
@@ -1057,8 +1059,8 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     };
     request(first + sub);
     for (int t0 = first; t0 < end; t0 += step) {
-        int row = next_row < p.M ? next_row : -1;
-        if (!kAbs) row = (next_e >= 0 && next_e < p.E && row >= 0) ? next_e * p.M + row : -1;
+        int row = next_row;
+        if (!kAbs) row = (next_e >= 0 && next_e < p.E && row >= 0 && row < p.M) ? next_e * p.M + row : -1;
         const float w = next_w;
         float acc[16];
 #pragma unroll
@@ -1068,14 +1070,14 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
 #pragma unroll
             for (int b = 0; b < kDepth; ++b) {
                 const int r = __shfl_sync(kFull, row, k0 + b);
-                if (r >= 0 && act) v[b] = ld32_readonly(x + (size_t)r * row_bytes);
+                if ((unsigned)r < rows && act) v[b] = ld32_readonly(x + (size_t)r * row_bytes);
             }
             if (k0 == 0) request(t0 + step + sub);
 #pragma unroll
             for (int b = 0; b < kDepth; ++b) {
                 const int r = __shfl_sync(kFull, row, k0 + b);
                 const float wk = kAbs ? 1.f : __shfl_sync(kFull, w, k0 + b);
-                if (r >= 0) {
+                if ((unsigned)r < rows) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         acc[2 * i] = fmaf(bf16lo(v[b].w[i]), wk, acc[2 * i]);
