@@ -77,6 +77,11 @@ __device__ __forceinline__ longlong2 ld_ro(const longlong2* p) {
     asm volatile("ld.global.v2.s64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ uint4 ld_ro(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 // The same for words that other blocks of this kernel may be writing (L2).
 __device__ __forceinline__ int ld_l2(const int32_t* p) {
     int v;

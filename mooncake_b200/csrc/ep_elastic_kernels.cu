@@ -840,7 +840,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
     p.C = c < 1 ? 1 : c < most ? c : most;
     // (an expanded row's place depends on all tokens: nothing to send ahead)
-    p.early = expand ? 0 : early_tokens(ctx.num_sms);
+    p.early = expand ? 0 : 3 * ctx.num_sms;
     p.teller = (p.early + p.C - 1) / p.C;  // the first block that waits for the layout kernel
     if (p.teller > (p.T + p.C - 1) / p.C - 1) p.teller = (p.T + p.C - 1) / p.C - 1;
     int warps = p.C * ntiles;

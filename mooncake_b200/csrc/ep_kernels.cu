@@ -601,8 +601,8 @@ __global__ void __launch_bounds__(256) ep_layout_slot_kernel(LayoutParams p) {
 }
 
 // ---- the same layout in one launch of one cluster -----------------------------------
-// What dispatch uses for all but the smallest and the largest batches. The blocks
-// of one cluster share the tokens, one lane per token:
+// For callers that want finished positions and up to 16384 tokens. The blocks of one
+// cluster share the tokens, one lane per token:
 //   bit (expert, token) in the block's shared bitmap, word-major [word][E];
 //   per expert: popcounts of the words -> exclusive prefix over the words, total;
 //   cluster barrier; totals of the lower blocks through distributed shared memory;
@@ -681,6 +681,52 @@ __global__ void __launch_bounds__(1024) ep_layout_cluster_kernel(LayoutParams p)
         cluster_layout<16>(p, mask, pre, total);
 }
 
+// ---- the layout as bits, for kernels that look positions up themselves -------------
+// What dispatch uses between the smallest and the largest batches. Every chunk of 128
+// tokens is a block of its own and nothing is summed here: per expert the chunk's bits
+// (RouteBits) and their number, one load, one store. A sender finds its position from them
+// in one round trip more than it would read a finished one (bits_before), but a finished
+// one costs a cluster barrier, remote totals and a prefix over all experts before it
+// exists: from the kernel's start to its end 5.7 us for 2001 tokens to 8 of 128, 9.3 for
+// 4096 to 8 of 256; here 2.4 and 2.
+constexpr int kBitsThreads = 256;
+
+template <int KB>
+__device__ __forceinline__ void set_bits(const LayoutParams& p, uint32_t* mask) {
+    const int t = blockIdx.x * kChunkTokens + threadIdx.x;
+    int e[KB];
+#pragma unroll
+    for (int k = 0; k < KB; ++k) e[k] = -1;
+    if (threadIdx.x < kChunkTokens && t < p.T)
+        load_choices<KB, false>(p.topk_idx, t, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), e);
+#pragma unroll
+    for (int k = 0; k < KB; ++k)  // (a repeated expert sets its bit twice)
+        if (e[k] >= 0) atomicOr(&mask[e[k] * 4 + (threadIdx.x >> 5)], 1u << (threadIdx.x & 31));
+}
+
+__global__ void __launch_bounds__(kBitsThreads) ep_layout_bits_kernel(LayoutParams p) {
+    extern __shared__ uint4 smem_u128[];  // [E] bits of this chunk
+    const int tid = threadIdx.x;
+    for (int i = tid; i < p.E; i += kBitsThreads) smem_u128[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem_u128);
+    if (p.K <= 4)
+        set_bits<4>(p, mask);
+    else if (p.K <= 8)
+        set_bits<8>(p, mask);
+    else
+        set_bits<16>(p, mask);
+    __syncthreads();
+    for (int e = tid; e < p.E; e += kBitsThreads) {
+        const uint4 m = smem_u128[e];
+        p.bits.words[(size_t)e * p.bits.chunks + blockIdx.x] = m;
+        p.bits.counts[(size_t)e * p.bits.stride + blockIdx.x] =
+            (uint8_t)(__popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w));
+    }
+}
+
 // =============================================================================
 // sending token rows (single rank and groups)
 // =============================================================================
@@ -711,7 +757,7 @@ struct SendView {
     int T, K, E, R, M, H, rank;
     int L, RM;
     int C;                    // tokens per batch
-    int early;                // kEarly: batches that begin below this token count for themselves
+    RouteBits bits;           // the layout kernel's bits (words null: none), or
     const int32_t* slot;      // [T*K] position among this rank's tokens for the expert (layout kernel),
                               // or null: counted here (small batches, one per block)
     int32_t* status;
@@ -737,11 +783,10 @@ struct SendView {
 constexpr int kBatchEntries = 128;  // (token, k) entries of a batch
 
 // Returns whether one of this thread's entries went to a peer.
-// kCount: the positions are counted here, hist: [E] in shared memory; else `slot` has them. All threads of the block call it.
-// What is read before `ready()` is complete when the kernel begins (the rows and the
-// index matrix: the layout kernel ahead has waited for whatever wrote them).
-template <bool kFP8, bool kGroup, bool kCount, bool kEarly, typename Ready>
-__device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsend, int* hist, Ready ready) {
+// kCount: the positions are counted here, hist: [E] in shared memory; else `bits` or `slot`
+// have them. All threads of the block call it.
+template <bool kFP8, bool kGroup, bool kCount>
+__device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsend, int* hist) {
     __shared__ char* s_dst[kBatchEntries];
     __shared__ char* s_meta[kGroup ? kBatchEntries : 1];
     __shared__ int s_raw[kBatchEntries];   // expert of the entry, -1: none
@@ -779,18 +824,12 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
         const int t1 = t0 + nsend * v.C;
         int raw = -1, slot = 0;
         if (tid < ne) raw = (int)ld_ro(v.topk_idx + (size_t)t0 * K + tid);
-        // (not the last batch: a block of every launch waits for the layout kernel)
-        const bool early = kEarly && t0 < v.early && t0 + v.C < v.T;
-        const bool counting = kCount || early;
-        if (counting) {
-            if (kEarly) {
-                for (int i = tid; i < v.E; i += nthr) hist[i] = 0;
-                __syncthreads();
-            }
+        if (kCount) {
             count_tokens<1>(v.topk_idx, counted, t0, K, v.E, choices_in_pairs(v.topk_idx, K), hist);
-        } else {
-            ready();
-            if (tid < ne) slot = ld_ro(v.slot + (size_t)t0 * K + tid);
+        } else if (v.bits.words != nullptr) {
+            if (raw >= 0 && raw < v.E) slot = bits_before(v.bits, raw, t0 + tid / K);
+        } else if (tid < ne) {
+            slot = ld_ro(v.slot + (size_t)t0 * K + tid);
         }
         if (raw >= v.E) raw = -1;
         if (tid < ne) s_raw[tid] = raw;
@@ -809,7 +848,7 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
             int row = -1, le = 0;
             if (e >= 0) {
                 int s = slot;
-                if (counting) {
+                if (kCount) {
                     s = hist[e];
                     for (int j = 0; j < tok0; ++j) s += (s_exp[j] == e);  // earlier tokens of the batch
                 }
@@ -921,23 +960,101 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
 // =============================================================================
 // Bound by HBM for large batches (4096 tokens, hidden 7168, top-8, bf16: 529 MB)
 // and by latency for decode (index load -> count -> row stores, one batch per block).
-// Behind a layout kernel the registers are held to 40, so that six blocks of 8 warps
-// fit an SM and one block's loads hide behind the stores of the others (2001 rows of
-// 8 KB to 8, us per layer: 64 registers 51.4, 48 51.1, 40 48.7, 36 52.3).
-template <bool kFP8, bool kCount>
-__global__ void __launch_bounds__(512, kCount ? 2 : 3) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
-    extern __shared__ int smem_i32[];  // [E] (kCount)
-    // behind a layout kernel the rows are requested before the wait
-    if (kCount) pdl_wait();
+template <bool kFP8>
+__global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
+    extern __shared__ int smem_i32[];  // [E]
+    pdl_wait();
     pdl_launch_dependents();
     SendView v = {};
-    v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx, v.slot = p.slot;
+    v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx;
     v.T = p.T, v.K = p.K, v.E = p.E, v.R = 1, v.M = p.M, v.H = p.H, v.rank = 0;
-    v.L = p.E, v.RM = p.M, v.C = p.C, v.early = p.early, v.status = p.status;
+    v.L = p.E, v.RM = p.M, v.C = p.C, v.status = p.status;
     v.recv_x = reinterpret_cast<char*>(p.recv_x), v.recv_scales = p.recv_scales;
     v.recv_src_info = p.recv_src_info, v.row_bytes = p.H * (kFP8 ? 1 : 2);
     v.rowmap = p.rowmap, v.recv_count = p.recv_count, v.layout_range = p.layout_range;
-    send_tokens<kFP8, false, kCount, !kCount>(v, blockIdx.x, gridDim.x, smem_i32, [] { pdl_wait(); });
+    send_tokens<kFP8, false, true>(v, blockIdx.x, gridDim.x, smem_i32);
+}
+
+// Single rank, behind a layout kernel: a warp owns one tile of one token and needs no
+// other: lane k finds the token's k-th row, the tile goes to each. Nothing is shared and
+// nobody waits at a barrier. Blocks are small because it is the turnover of independent
+// warps that hides the chain index -> bits -> stores: with a block per token that met at
+// three barriers a block lived 6 us, 2001 of them behind one another were bound by that
+// and not by HBM (2001 rows of 8 KB to 8 in FP8, the layer 50.1 us, now 46.7; 2000 of 4 KB
+// in bf16 26.2, now 24.9; 4000 of 1 KB 25.0, now 20.2).
+// FP8 wants many warps per SM (quantising is their time; 40 registers, 2048 rows of 14 KB
+// to 4: 46.1 us, with 64 registers 48.1), large bf16 rows few, as the rows that are written
+// at a time then lie closer together in HBM (4096 rows of 14 KB to 8: 172.9 us with 32 warps
+// per SM, 175.1 with 40, 176.1 with 48; 174.6 before). The blocks of a row are neighbours
+// in the grid (parts of a row one after the other over all rows: 175.9).
+constexpr int kRowsWarpsFP8 = 7, kRowsWarps = 4;
+
+template <bool kFP8>
+__global__ void __launch_bounds__((kFP8 ? kRowsWarpsFP8 : kRowsWarps) * 32, kFP8 ? 6 : 8)
+    ep_dispatch_rows_kernel(DirectDispatchParams p) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = warp / p.tiles_per_block;  // which token of the block
+    const int group = blockIdx.x / p.parts, part = blockIdx.x - group * p.parts;
+    const int tile = warp - sub * p.tiles_per_block + part * p.tiles_per_block;
+    const int t = group * p.tokens_per_block + sub, c = tile * 32 + lane;
+    const int K = p.K, M = p.M;
+    const bool act = t < p.T && c < p.H / 16, mine = t < p.T && lane < K;
+    pdl_launch_dependents();
+    // (the rows and the index matrix are complete: the layout kernel has waited for them)
+    V32 row = {};
+    int e = -1;
+    if (act) row = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+    if (mine) e = (int)ld_ro(p.topk_idx + (size_t)t * K + lane);
+    pdl_wait();
+    if (p.bits.words != nullptr && blockIdx.x == gridDim.x - 1) {
+        for (int x = threadIdx.x; x < p.E; x += blockDim.x) {
+            const int n = bits_total(p.bits, x);
+            p.recv_count[x] = n;
+            p.layout_range[x] = n;  // begin 0 | count
+        }
+    }
+    // (a repeated expert has the same row and gets the same bytes twice)
+    int s = -1;
+    if (p.bits.words != nullptr) {
+        if (e >= 0 && e < p.E) s = bits_before(p.bits, e, t);
+    } else {
+        if (mine) s = ld_ro(p.slot + (size_t)t * K + lane);
+        for (int k = 0; k < K; ++k) {  // (that layout kernel leaves a repeat without a position)
+            const int ek = __shfl_sync(kFull, e, k), sk = __shfl_sync(kFull, s, k);
+            if (s < 0 && e >= 0 && ek == e) s = sk;
+        }
+    }
+    if (s >= M) {
+        atomicOr(p.status, kStatusSlotRange);
+        s = -1;
+    }
+    // (32 bits: a device has no room for 2^31 rows of 128 bytes, nor for as many scales of theirs)
+    const int to = s >= 0 ? e * M + s : -1;
+    if (tile == 0 && mine) {
+        p.rowmap[(size_t)t * K + lane] = s;
+        if (s >= 0) p.recv_src_info[to] = t;
+    }
+    if (kFP8) {
+        float sinv;
+        const uint4 q = quantize16(row, sinv);
+        const int at = s >= 0 ? e * (p.H / 128) * M + s : 0;
+        char* out = static_cast<char*>(p.recv_x) + (size_t)c * 16;
+        float* scales = p.recv_scales + (size_t)(c >> 3) * M;
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = __shfl_sync(kFull, to, k), sr = __shfl_sync(kFull, at, k);
+            if (r < 0 || !act) continue;
+            st16(out + (size_t)r * p.H, q);
+            if ((lane & 7) == 0) scales[sr] = sinv;
+        }
+    } else {
+        char* out = static_cast<char*>(p.recv_x) + (size_t)c * 32;
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = __shfl_sync(kFull, to, k);
+            if (r >= 0 && act) st32(out + (size_t)r * p.H * 2, row);
+        }
+    }
 }
 
 // Single rank: rowmap[t][k] = packed row of (token t, expert topk[t][k]) as the
@@ -1237,7 +1354,7 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
         if (!s_active[dr]) continue;
-        const int c = kCount ? hist[x] : ld_ro(p.count + x);
+        const int c = kCount ? hist[x] : p.bits.words != nullptr ? bits_total(p.bits, x) : ld_ro(p.count + x);
         uint64_t* wd = reinterpret_cast<uint64_t*>(s_peer[dr] + p.w.cnt_off) + (p.rank * L + (x - dr * L));
         st_relaxed_sys(wd, ((uint64_t)p.seq << 32) | (uint32_t)(c + 1));
     }
@@ -1450,7 +1567,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     const int sid = bid - 1;
     __syncthreads();  // the tables above are in place
     SendView v = {};
-    v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx, v.slot = p.slot;
+    v.x = reinterpret_cast<const char*>(p.x), v.topk_idx = p.topk_idx, v.slot = p.slot, v.bits = p.bits;
     v.T = p.T, v.K = p.K, v.E = p.E, v.R = p.R, v.M = p.M, v.H = p.H, v.rank = p.rank;
     v.L = p.E / p.R, v.RM = p.R * p.M, v.C = p.C, v.status = p.wait.status;
     v.recv_x = reinterpret_cast<char*>(p.recv_x), v.recv_scales = p.recv_scales;
@@ -1458,7 +1575,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     v.beg = reinterpret_cast<const uint64_t*>(p.local_base + p.w.beg_off);
     v.seq = p.seq, v.wait = scaled(p.wait, 2), v.rx_off = p.rx_off, v.meta_off = p.meta_off;
     v.meta_stride = p.meta_stride, v.rowmap = p.rowmap, v.s_peer = s_peer, v.s_active = s_active;
-    const bool remote = send_tokens<kFP8, true, kCount, false>(v, sid, nsend, smem_i32, [] {});
+    const bool remote = send_tokens<kFP8, true, kCount>(v, sid, nsend, smem_i32);
     MCEP_TRACE(0, 5);  // all rows of this block are issued
 
     // Completion. Rows are not fenced one by one: a block that stored something in a
@@ -1920,7 +2037,23 @@ static int layout_cluster_threads(const LayoutParams& p, int blocks) {
     return (size_t)p.E * (threads / 16 + 2) * sizeof(int) <= 160 * 1024 ? threads : 0;
 }
 
+RouteBits route_bits(void* memory, size_t capacity, int T, int E) {
+    RouteBits b = {};
+    const int chunks = (T + kChunkTokens - 1) / kChunkTokens;
+    const int stride = (chunks + 15) / 16 * 16;
+    if (chunks < 1 || chunks > 128 || (size_t)E * (chunks * sizeof(uint4) + stride) > capacity) return b;
+    b.words = static_cast<uint4*>(memory);
+    b.counts = reinterpret_cast<uint8_t*>(b.words + (size_t)E * chunks);
+    b.chunks = chunks, b.stride = stride;
+    return b;
+}
+
 cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
+    if (p.bits.words != nullptr) {
+        const size_t smem = (size_t)p.E * sizeof(uint4);
+        if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(ep_layout_bits_kernel), smem)) return e;
+        return launch("ep_layout_bits", ep_layout_bits_kernel, dim3(p.bits.chunks), dim3(kBitsThreads), smem, ctx, p);
+    }
     // Sixteen blocks (opt-in cluster size) once eight would have more than 8 warps
     // each: setting the bits is bound by the shared-memory atomics of a block.
     const void* k = reinterpret_cast<const void*>(ep_layout_cluster_kernel);
@@ -1971,50 +2104,40 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
                   ctx, p, epc, words);
 }
 
-int early_tokens(int num_sms) { return 3 * num_sms; }
-
-bool counts_in_send_kernel(int T, int K, int num_sms, bool group) {
-    // A group's sender blocks are one resident wave, a token each. A single rank counts
-    // in one resident wave of blocks with as many tokens each as that takes. Up to two
-    // choices per token that beats a layout kernel as far as it was measured (us per
-    // layer, rows of 8 KB to 2: 1000 tokens 11.9 against 13.2, 4000 34.3 against 36.8; to
-    // 1: 8192 tokens 48.3 against 53.1). From three on the rows of the third token of a
-    // block cost more than the layout kernel does (8 KB to 8: 520 tokens 15.4 against
-    // 16.2, 580 16.0 against 16.5, 600 18.5 against 17.9).
+bool counts_in_send_kernel(int T, int K, int row_bytes, int num_sms, bool group) {
+    // A group's sender blocks are one resident wave, a token each (one rank on this path,
+    // us per layer, counting | layout kernel: rows of 8 KB in bf16 to 8, 200 tokens 17.6 |
+    // 17.2, 290 19.0 | 18.4, 400 30.8 | 26.4; of 7 KB in FP8, 290 23.9 | 26.9).
     if (group) return T <= 2 * num_sms;
-    return K <= 2 ? T <= 8192 / K : T <= 4 * num_sms;
+    // A single rank counts in one resident wave of blocks with as many tokens each as that
+    // takes. Up to two choices per token that is as good as a layout kernel (us per layer,
+    // counting | layout kernel, rows of 8 KB to 2: 1000 tokens 14.6 | 14.4, 4000 39.2 | 38.3;
+    // in FP8 35.7 | 36.2; of 14 KB to 1, 4000 44.3 | 48.0) and saves a launch.
+    if (K <= 2) return T <= 8192 / K;
+    // From three on the layout kernel is the faster one on the device at every size (rows
+    // of 14 KB to 8: 160 tokens 15.2 | 13.8, 300 24.8 | 21.1, 590 32.6 | 31.7; of 4 KB in FP8
+    // to 8: 200 10.0 | 9.6, 400 16.3 | 14.9, 590 20.8 | 20.0; of 4 KB to 4, 590 9.1 | 8.5), but
+    // a layer of three launches takes the host 12.5 us and one of two 10: it is used where
+    // the rows are more than the device moves in that time.
+    return T <= num_sms || (T <= 4 * num_sms && (long long)T * K * row_bytes < 12 << 20);
 }
 
-// Tokens per batch and threads per block of the send kernels.
+// Tokens per batch and threads per block of the kernels that work through batches.
 // A single rank that counts: one resident wave of up to 16 warps, each with a tile at a
 // time (1000 rows of 8 KB to 2: 11.9 us per layer, two waves 14.0).
-// Behind a layout kernel it is the number of independent blocks that hides the chain
-// index -> slot -> stores: a single rank's have one token and up to 8 warps (2048 rows of
-// 14 KB to 4 in FP8: 47.4 us per layer with 8 warps, 51.9 with 14; 2000 rows of 4 KB to 8:
-// 25.6 with one token per block, 26.9 with four). A warp per tile again where twice the
-// L2 and more of bf16 rows is written, 8 per token: the stores alone are the bound then
-// and fewer rows at a time suit HBM (to 4, 4096 rows of 14 KB: 97.4 us per layer with 8
-// warps, 104.3 with 14; to 8, a warp per tile | 8 warps, rows of 14 KB: 2600 114.9 | 115.3,
-// 3000 131.5 | 132.0, 4096 173.8 | 174.9, 8192 331.0 | 332.3; 6000 of 12 KB 214.0 | 214.9;
-// 2600 of 16 KB 129.0 | 129.4, 4096 195.7 | 197.2; to 16, 4096 of 14 KB 319.9 | 322.8; runs
-// of one side differ by 0.1 %. Below the limit, 2048 and 2300 of 14 KB, no difference; rows
-// of 10 KB lose 0.3 %, 8000 237.7 | 237.2; up to 8 KB there are 8 warps either way).
 // A group's sender blocks are one resident wave that strides: batches of 16 warp tiles,
 // 8 warps once there are more tokens than blocks (2000 rows of 8 KB to 8: 64.0 us per
 // layer, 16 warps 67.3; one token per batch 64.6, rows of 2 KB 30.7 against 27.0), a warp
 // per tile before (256 tokens of 14 KB to 8: 20.9 us, 8 warps 23.4).
-static SendShape send_shape(int T, int K, int H, bool fp8, int num_sms, bool counting, bool group) {
+static SendShape send_shape(int T, int K, int H, int num_sms, bool group) {
     const int ntiles = (H + kTileChannels - 1) / kTileChannels;
-    const int wave = (T + 2 * num_sms - 1) / (2 * num_sms);  // tokens per batch: two blocks per SM
     SendShape s;
-    s.tokens = 1;
-    if (group || counting) s.tokens = wave;
+    s.tokens = (T + 2 * num_sms - 1) / (2 * num_sms);  // two blocks per SM
     if (group && s.tokens > 16 / ntiles) s.tokens = 16 / ntiles;
     if (group && s.tokens > 8) s.tokens = 8;
     if (s.tokens > kBatchEntries / K) s.tokens = kBatchEntries / K;
     if (s.tokens < 1) s.tokens = 1;
-    const bool stores = !group && !fp8 && K >= 8 && (long long)T * K * H * 2 > 256ll << 20;
-    const int most = (group ? T > 2 * num_sms : !counting && !stores) ? 8 : 16, least = group ? 8 : 4;
+    const int most = group && T > 2 * num_sms ? 8 : 16, least = group ? 8 : 4;
     int warps = s.tokens * ntiles;
     if (warps > most) warps = most;
     if (warps < least) warps = least;
@@ -2023,23 +2146,22 @@ static SendShape send_shape(int T, int K, int H, bool fp8, int num_sms, bool cou
 }
 
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, false);
-    p.C = s.tokens;
-    // About the first wave of blocks: their rows leave while the layout kernel runs, for
-    // up to 1.5 us of counting (2001 tokens FP8: 52.9 us per layer without, 52.3 with one
-    // token per SM, 50.4 with two, 50.5 with three, 49.9 with six; 4096 tokens bf16: 180.4,
-    // 178.4, 177.8, 177.3, 179.2).
-    p.early = early_tokens(ctx.num_sms);
-    const size_t smem = (size_t)p.E * sizeof(int);
-    void (*k)(DirectDispatchParams) = nullptr;
-    switch ((p.use_fp8 ? 2 : 0) | (p.slot == nullptr ? 1 : 0)) {
-        case 0: k = ep_dispatch_send_direct_kernel<false, false>; break;
-        case 1: k = ep_dispatch_send_direct_kernel<false, true>; break;
-        case 2: k = ep_dispatch_send_direct_kernel<true, false>; break;
-        default: k = ep_dispatch_send_direct_kernel<true, true>; break;
+    if (!p.counting()) {
+        const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+        const int most = p.use_fp8 ? kRowsWarpsFP8 : kRowsWarps;
+        p.parts = (ntiles + most - 1) / most;
+        p.tiles_per_block = (ntiles + p.parts - 1) / p.parts;
+        p.tokens_per_block = most / p.tiles_per_block;
+        const int groups = (p.T + p.tokens_per_block - 1) / p.tokens_per_block;
+        auto k = p.use_fp8 ? ep_dispatch_rows_kernel<true> : ep_dispatch_rows_kernel<false>;
+        return launch("ep_dispatch_send_direct", k, dim3(groups * p.parts),
+                      dim3(32 * p.tiles_per_block * p.tokens_per_block), 0, ctx, p);
     }
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, false);
+    p.C = s.tokens;
+    auto k = p.use_fp8 ? ep_dispatch_send_direct_kernel<true> : ep_dispatch_send_direct_kernel<false>;
     const int grid = p.T > 0 ? (p.T + p.C - 1) / p.C : 1;
-    return launch("ep_dispatch_send_direct", k, dim3(grid), dim3(s.threads), smem, ctx, p);
+    return launch("ep_dispatch_send_direct", k, dim3(grid), dim3(s.threads), (size_t)p.E * sizeof(int), ctx, p);
 }
 
 cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx& ctx) {
@@ -2142,20 +2264,20 @@ bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms) {
 }
 
 cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, true);
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
-    auto k = pick_dispatch<3>(p.use_fp8 != 0, p.slot == nullptr);
+    auto k = pick_dispatch<3>(p.use_fp8 != 0, p.counting());
     const int grid = 1 + (p.T > 0 ? p.T : 1);
     if (p.C != 1 || grid > resident_blocks(k, s.threads, smem, ctx)) return cudaErrorInvalidConfiguration;
     return launch("ep_dispatch", k, dim3(grid), dim3(s.threads), smem, ctx, p);
 }
 
 cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& ctx) {
-    const SendShape s = send_shape(p.T, p.K, p.H, p.use_fp8 != 0, ctx.num_sms, p.slot == nullptr, true);
+    const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
-    auto k = pick_dispatch<1>(p.use_fp8 != 0, p.slot == nullptr);
+    auto k = pick_dispatch<1>(p.use_fp8 != 0, p.counting());
     // the control block, then one block per token (small batches) or a resident wave
     // (a wave, not a block per batch: a block that stored rows in a peer's memory, nearly
     // every one in a group of several GPUs, ends with a system-scope fence)
@@ -2280,7 +2402,7 @@ cudaError_t launch_group_dispatch_multi(GroupDispatchParams* params, int n,
     for (int i = 0; i < n; ++i) {
         if (params[i].use_fp8 != params[0].use_fp8 || params[i].H != params[0].H) return cudaErrorInvalidValue;
         params[i].C = 1;
-        counting = counting || params[i].slot == nullptr;
+        counting = counting || params[i].counting();
         const int blocks = 1 + (params[i].T > 0 ? params[i].T : 1);
         if (blocks > want) want = blocks;
         const size_t sm = (size_t)(2 * params[i].E + 4) * sizeof(int);

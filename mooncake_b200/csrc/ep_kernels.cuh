@@ -30,9 +30,23 @@ struct LaunchCtx {
 };
 
 // ---- routing layout ---------------------------------------------------------
+// The routing as bits: which tokens of a chunk chose an expert, and how many. A token's
+// position among the tokens of its expert is the sum of the counts of the chunks ahead
+// and of the lower bits of its own (bits_before, ep_routing.cuh).
+constexpr int kChunkTokens = 128;
+struct RouteBits {
+    uint4* words;     // [E][chunks], bit t % 128 of chunk t / 128; null: not there
+    uint8_t* counts;  // [E][stride], padding undefined
+    int chunks, stride;
+};
+// Such bits in `capacity` bytes at `memory` (256-byte aligned); words null where they do
+// not fit or where the batch has more than 128 chunks.
+RouteBits route_bits(void* memory, size_t capacity, int T, int E);
+
 struct LayoutParams {
     const int64_t* topk_idx;  // [T][K]
     int T, K, E, R;
+    RouteBits bits;           // words not null: these are written, and nothing below
     int32_t* count;           // [E]
     int32_t* slot;            // [T*K]
     int32_t* rank_count;      // [R] or null
@@ -51,10 +65,13 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx);
 struct DirectDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
-    const int32_t* slot;        // [T*K] from the layout kernel, or null: counted in the send kernel
+    RouteBits bits;             // from the layout kernel (words null: none), or
+    const int32_t* slot;        // [T*K] from another layout kernel, or null: counted in the send kernel
     int T, K, E, M, H;
     int use_fp8;
-    int C, early;               // tokens per batch, tokens sent ahead of the layout (set by the launcher)
+    int C;                      // counting: tokens per batch (set by the launcher)
+    int tiles_per_block, tokens_per_block, parts;  // else: how a block's warps are dealt out, blocks that share
+                                                   // a row (set by the launcher)
     int32_t* status;
     void* recv_x;
     float* recv_scales;
@@ -62,12 +79,10 @@ struct DirectDispatchParams {
     int32_t* recv_count;        // [E], written without `slot`
     int64_t* layout_range;      // [E], written without `slot`
     int32_t* rowmap;            // [T*K] row of (token, k) inside its expert, kept for combine
+    bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 // whether the send kernels count the slots themselves for this many tokens
-bool counts_in_send_kernel(int T, int K, int num_sms, bool group);
-// tokens whose rows a kernel behind a layout kernel sends before that one has finished,
-// counting the earlier tokens itself
-int early_tokens(int num_sms);
+bool counts_in_send_kernel(int T, int K, int row_bytes, int num_sms, bool group);
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
 
 struct SendShape {
@@ -129,8 +144,9 @@ struct WaitCfg {
 struct GroupDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
+    RouteBits bits;             // from the layout kernel (words null: none), or
     const int32_t* slot;        // [T*K] and
-    const int32_t* count;       // [E] from the layout kernel, or null: counted in the send kernel
+    const int32_t* count;       // [E] from another layout kernel, or null: counted in the send kernel
     void* const* peer_base;     // [R] base of every rank's symmetric buffer
     char* local_base;           // this rank's
     int T, K, E, R, M, H, rank;
@@ -155,6 +171,7 @@ struct GroupDispatchParams {
     int32_t* recv_count;        // [L]
     int64_t* layout_range;      // [L][R]
     int copy_rows;              // recv_x is a tensor of the caller's: copy the rows out
+    bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms);
 // one launch: control + send + receive duties

@@ -112,4 +112,38 @@ __device__ __forceinline__ bool choices_in_pairs(const int64_t* topk_idx, int K)
     return K % 2 == 0 && (reinterpret_cast<uintptr_t>(topk_idx) & 15) == 0;
 }
 
+// ---- positions from the layout kernel's bits (RouteBits) ------------------------------
+// Sum of the first `n` counts of a row of bytes, sixteen per load.
+__device__ __forceinline__ int sum_counts(const uint8_t* row, int n) {
+    int sum = 0;
+    for (int c0 = 0; c0 < n; c0 += 16) {
+        const uint4 v = ld_ro(reinterpret_cast<const uint4*>(row + c0));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int there = n - c0 - 4 * j;  // bytes of this word that count
+            const uint32_t keep = there >= 4 ? 0xffffffffu : there > 0 ? (1u << (8 * there)) - 1u : 0u;
+            sum = (int)__dp4a(w[j] & keep, 0x01010101u, (unsigned)sum);
+        }
+    }
+    return sum;
+}
+// Tokens before t that chose expert e.
+__device__ __forceinline__ int bits_before(const RouteBits& b, int e, int t) {
+    const int chunk = t / kChunkTokens, bit = t % kChunkTokens;
+    const uint4 v = ld_ro(b.words + (size_t)e * b.chunks + chunk);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    int n = sum_counts(b.counts + (size_t)e * b.stride, chunk);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int lower = bit - 32 * j;  // bits of this word that are lower
+        n += __popc(w[j] & (lower >= 32 ? 0xffffffffu : lower > 0 ? (1u << lower) - 1u : 0u));
+    }
+    return n;
+}
+// Tokens that chose expert e.
+__device__ __forceinline__ int bits_total(const RouteBits& b, int e) {
+    return sum_counts(b.counts + (size_t)e * b.stride, b.chunks);
+}
+
 }  // namespace mcep

@@ -920,11 +920,14 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
     // Larger batches get their layout from a kernel of its own.
-    const bool counting = (b->fuse_layout || T == 0) && mcep::counts_in_send_kernel(T, K, b->num_sms, group);
+    const bool counting = (b->fuse_layout || T == 0) && 
+                          mcep::counts_in_send_kernel(T, K, g.row_bytes, b->num_sms, group);
+    mcep::RouteBits bits = {};
     if (!counting) {
         mcep::LayoutParams lp = {};
         lp.topk_idx = a->topk_idx;
         lp.T = T, lp.K = K, lp.E = E, lp.R = R;
+        lp.bits = bits = mcep::route_bits(sc.slot, b->scratch_entries * sizeof(int32_t), T, E);
         lp.count = sc.count, lp.slot = sc.slot, lp.ticket = sc.layout_ticket;
         lp.chunk_hist = sc.chunk_hist, lp.chunk_hist_entries = kChunkHistBytes / sizeof(int32_t);
         if (!group) {
@@ -934,14 +937,14 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
         MCEP_CUDA(mcep::launch_layout(lp, first));
         first.pdl = pdl;  // what follows is chained to the layout kernel
     }
-    const int32_t* slot = counting ? nullptr : sc.slot;
+    const int32_t* slot = counting || bits.words != nullptr ? nullptr : sc.slot;
 
     if (!group) {
         // a single rank: the packed outputs are written directly, no words, no waits
         mcep::DirectDispatchParams dp = {};
         dp.x = a->x, dp.topk_idx = a->topk_idx;
         dp.T = T, dp.K = K, dp.E = E, dp.M = M, dp.H = H, dp.use_fp8 = fp8;
-        dp.slot = slot, dp.status = b->status, dp.recv_x = a->packed_recv_x;
+        dp.bits = bits, dp.slot = slot, dp.status = b->status, dp.recv_x = a->packed_recv_x;
         dp.recv_scales = a->packed_recv_x_scales, dp.recv_src_info = a->packed_recv_src_info;
         dp.recv_count = a->packed_recv_count, dp.layout_range = a->packed_recv_layout_range;
         dp.rowmap = sc.rowmap;
@@ -961,7 +964,8 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
 
     char* area = b->base + kHeaderRegion + (size_t)par * g.parity_bytes;
     mcep::GroupDispatchParams p = {};
-    p.x = a->x, p.topk_idx = a->topk_idx, p.slot = slot, p.count = counting ? nullptr : sc.count;
+    p.x = a->x, p.topk_idx = a->topk_idx;
+    p.bits = bits, p.slot = slot, p.count = slot ? sc.count : nullptr;
     p.peer_base = b->peer_dev, p.local_base = b->base;
     p.T = T, p.K = K, p.E = E, p.R = R, p.M = M, p.H = H, p.rank = b->rank;
     p.use_fp8 = fp8;

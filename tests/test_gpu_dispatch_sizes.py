@@ -64,6 +64,30 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
     assert buf.runtime.status() == 0
 
 
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("T,H,E,K", [  # edges of the layout's words, chunks and loads of counts, and where it ends
+    (31, 128, 8, 3), (33, 640, 8, 3), (127, 3584, 8, 5), (128, 4096, 300, 2), (129, 8320, 24, 16), (149, 7168, 8, 8),
+    (2047, 128, 8, 4), (2049, 384, 64, 3), (600, 128, 2600, 1), (16384, 128, 8, 3), (16385, 128, 8, 3)])
+def test_positions_from_the_layout_kernel(T, H, E, K, fp8):
+    """Positions looked up in bits and counts (or read, beyond them), repeats and empty tokens among them."""
+    M = (T + 3) // 4 * 4
+    x, idx, w = make_rank_inputs(17, 0, T, H, E, K, "zipf1.2", n_mask=T // 7)
+    if K > 1:
+        idx[::5, K - 1] = idx[::5, 0]
+    buf = Buffer(FakeGroup(0, 1), 0)
+    buf.runtime.set_option("fuse_layout", 0)
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    recv, cnt, handle, _, _ = buf.dispatch(x.cuda(), idx.cuda(), active, M, E, 2_000_000, use_fp8=fp8)
+    got = [dict(recv_x=recv[0] if fp8 else recv, scales=recv[1] if fp8 else None, recv_count=cnt, handle=handle)]
+    torch.cuda.synchronize()
+    _check_dispatch(dict(R=1, E=E, M=M, fp8=fp8), got, ora.dispatch([x], [idx], M, E, fp8), None)
+    y = torch.randn((E, M, H), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
+    out, _, _ = buf.combine(y, idx.cuda(), w.cuda(), active, 2_000_000, handle)
+    ref = ora.combine([y.cpu()], [idx], [w], [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)
+    assert torch.equal(out.cpu().view(torch.int16), ref[0].view(torch.int16))
+    assert buf.runtime.status() == 0
+
+
 @pytest.mark.parametrize("mode", ["hook", "sync"])
 @pytest.mark.parametrize("T,fp8", [((280, 320), True), ((320, 280, 257), False), ((296, 297), False)])
 def test_ranks_on_either_side_of_the_counting_limit(T, fp8, mode):
