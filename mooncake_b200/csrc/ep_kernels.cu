@@ -982,28 +982,35 @@ __global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectD
 // three barriers a block lived 6 us, 2001 of them behind one another were bound by that
 // and not by HBM (2001 rows of 8 KB to 8 in FP8, the layer 50.1 us, now 46.7; 2000 of 4 KB
 // in bf16 26.2, now 24.9; 4000 of 1 KB 25.0, now 20.2).
-// FP8 wants many warps per SM (quantising is their time; 40 registers, 2048 rows of 14 KB
-// to 4: 46.1 us, with 64 registers 48.1), large bf16 rows few, as the rows that are written
-// at a time then lie closer together in HBM (4096 rows of 14 KB to 8: 172.9 us with 32 warps
-// per SM, 175.1 with 40, 176.1 with 48; 174.6 before). The blocks of a row are neighbours
-// in the grid (parts of a row one after the other over all rows: 175.9).
-constexpr int kRowsWarpsFP8 = 7, kRowsWarps = 4;
-
-template <bool kFP8>
-__global__ void __launch_bounds__((kFP8 ? kRowsWarpsFP8 : kRowsWarps) * 32, kFP8 ? 6 : 8)
+// How many warps and tiles of each (us per layer; launch_direct_dispatch chooses): many warps per SM where the
+// time is that of the loads and of quantising (FP8 to 4, 2048 rows of 14 KB: 46.1 with 42
+// warps, 48.1 with 32; bf16 to 8, 1500 rows of 8 KB: 42.0 | 42.9); with few copies per row
+// and long rows in FP8 two tiles per warp (4096 rows of 14 KB to 3: 68.5, one tile 73.0;
+// before 72.7); fewer warps for large bf16 outputs, as the rows that are written at a time
+// then lie closer together in HBM (4096 rows of 14 KB to 8: 172.9 with 32 warps, 174.7 with
+// 42, 176.1 with 48; 174.6 before). The blocks of a row are neighbours in the grid (parts of
+// a row one after the other over all rows: 175.9).
+template <bool kFP8, int kTiles, int kWarps, int kBlocks>
+__global__ void __launch_bounds__(kWarps * 32, kBlocks)
     ep_dispatch_rows_kernel(DirectDispatchParams p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sub = warp / p.tiles_per_block;  // which token of the block
+    const int sub = warp / p.warps_per_row;  // which token of the block
     const int group = blockIdx.x / p.parts, part = blockIdx.x - group * p.parts;
-    const int tile = warp - sub * p.tiles_per_block + part * p.tiles_per_block;
-    const int t = group * p.tokens_per_block + sub, c = tile * 32 + lane;
+    const int tile = (warp - sub * p.warps_per_row + part * p.warps_per_row) * kTiles;  // the first
+    const int t = group * p.tokens_per_block + sub, nchunks = p.H / 16;
     const int K = p.K, M = p.M;
-    const bool act = t < p.T && c < p.H / 16, mine = t < p.T && lane < K;
+    const bool mine = t < p.T && lane < K;
     pdl_launch_dependents();
     // (the rows and the index matrix are complete: the layout kernel has waited for them)
-    V32 row = {};
+    V32 row[kTiles];
     int e = -1;
-    if (act) row = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+#pragma unroll
+    for (int u = 0; u < kTiles; ++u) {
+        const int c = (tile + u) * 32 + lane;
+        row[u] = V32{};
+        if (t < p.T && c < nchunks)
+            row[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+    }
     if (mine) e = (int)ld_ro(p.topk_idx + (size_t)t * K + lane);
     pdl_wait();
     if (p.bits.words != nullptr && blockIdx.x == gridDim.x - 1) {
@@ -1034,25 +1041,35 @@ __global__ void __launch_bounds__((kFP8 ? kRowsWarpsFP8 : kRowsWarps) * 32, kFP8
         p.rowmap[(size_t)t * K + lane] = s;
         if (s >= 0) p.recv_src_info[to] = t;
     }
+    char* out = static_cast<char*>(p.recv_x);
     if (kFP8) {
-        float sinv;
-        const uint4 q = quantize16(row, sinv);
-        const int at = s >= 0 ? e * (p.H / 128) * M + s : 0;
-        char* out = static_cast<char*>(p.recv_x) + (size_t)c * 16;
-        float* scales = p.recv_scales + (size_t)(c >> 3) * M;
+        const int S = p.H / 128, at = s >= 0 ? e * S * M + s : 0;
+        float sinv[kTiles];
+        uint4 q[kTiles];
+#pragma unroll
+        for (int u = 0; u < kTiles; ++u) q[u] = quantize16(row[u], sinv[u]);
 #pragma unroll 4
         for (int k = 0; k < K; ++k) {
             const int r = __shfl_sync(kFull, to, k), sr = __shfl_sync(kFull, at, k);
-            if (r < 0 || !act) continue;
-            st16(out + (size_t)r * p.H, q);
-            if ((lane & 7) == 0) scales[sr] = sinv;
+            if (r < 0) continue;
+#pragma unroll
+            for (int u = 0; u < kTiles; ++u) {
+                const int c = (tile + u) * 32 + lane;
+                if (c >= nchunks) continue;
+                st16(out + (size_t)r * p.H + (size_t)c * 16, q[u]);
+                if ((lane & 7) == 0) p.recv_scales[(size_t)sr + (size_t)(c >> 3) * M] = sinv[u];
+            }
         }
     } else {
-        char* out = static_cast<char*>(p.recv_x) + (size_t)c * 32;
 #pragma unroll 4
         for (int k = 0; k < K; ++k) {
             const int r = __shfl_sync(kFull, to, k);
-            if (r >= 0 && act) st32(out + (size_t)r * p.H * 2, row);
+            if (r < 0) continue;
+#pragma unroll
+            for (int u = 0; u < kTiles; ++u) {
+                const int c = (tile + u) * 32 + lane;
+                if (c < nchunks) st32(out + (size_t)r * p.H * 2 + (size_t)c * 32, row[u]);
+            }
         }
     }
 }
@@ -2148,14 +2165,26 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool group) {
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
     if (!p.counting()) {
         const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-        const int most = p.use_fp8 ? kRowsWarpsFP8 : kRowsWarps;
-        p.parts = (ntiles + most - 1) / most;
-        p.tiles_per_block = (ntiles + p.parts - 1) / p.parts;
-        p.tokens_per_block = most / p.tiles_per_block;
+        void (*k)(DirectDispatchParams) = ep_dispatch_rows_kernel<true, 1, 7, 6>;
+        int tiles = 1, most = 7;
+        if (p.use_fp8) {
+            // two tiles | one: 4096 rows of 14 KB to 3 68.5 | 73.0, to 4 82.4 | 85.5, to 8 145.9 |
+            // 145.8; 4000 of 4 KB to 4 29.2 | 29.8; 1500 of 8 KB to 8 37.6 | 36.5
+            if (p.K <= 4 && ntiles >= 4) k = ep_dispatch_rows_kernel<true, 2, 4, 10>, tiles = 2, most = 4;
+        } else if ((long long)p.T * p.K * p.H * 2 < 256 << 20) {
+            // 42 warps per SM | 32: to 3, 4096 rows of 14 KB (168 MB) 78.4 | 79.8; to 4 (224 MB) 97.4 |
+            // 97.2, to 6 135.8 | 135.5, to 8 174.7 | 173.7
+            k = ep_dispatch_rows_kernel<false, 1, 7, 6>;
+        } else {
+            k = ep_dispatch_rows_kernel<false, 1, 4, 8>, most = 4;
+        }
+        const int warps = (ntiles + tiles - 1) / tiles;  // of a row
+        p.parts = (warps + most - 1) / most;
+        p.warps_per_row = (warps + p.parts - 1) / p.parts;
+        p.tokens_per_block = most / p.warps_per_row;
         const int groups = (p.T + p.tokens_per_block - 1) / p.tokens_per_block;
-        auto k = p.use_fp8 ? ep_dispatch_rows_kernel<true> : ep_dispatch_rows_kernel<false>;
-        return launch("ep_dispatch_send_direct", k, dim3(groups * p.parts),
-                      dim3(32 * p.tiles_per_block * p.tokens_per_block), 0, ctx, p);
+        return launch("ep_dispatch_send_direct", k, dim3(groups * p.parts), dim3(32 * p.warps_per_row * p.tokens_per_block),
+                      0, ctx, p);
     }
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, false);
     p.C = s.tokens;

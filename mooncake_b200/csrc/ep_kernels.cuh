@@ -70,8 +70,8 @@ struct DirectDispatchParams {
     int T, K, E, M, H;
     int use_fp8;
     int C;                      // counting: tokens per batch (set by the launcher)
-    int tiles_per_block, tokens_per_block, parts;  // else: how a block's warps are dealt out, blocks that share
-                                                   // a row (set by the launcher)
+    int warps_per_row, tokens_per_block, parts;  // else: how a block's warps are dealt out, blocks that share a row
+                                                 // (set by the launcher)
     int32_t* status;
     void* recv_x;
     float* recv_scales;
