@@ -88,6 +88,11 @@ __device__ __forceinline__ int ld_l2(const int32_t* p) {
     asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ uint4 ld_l2(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 // ---- 32-byte vector memory ops ----------------------------------------------
 // Inputs that are read once (x, expert outputs): see above, no .nc; not kept in L1.
 __device__ __forceinline__ V32 ld32_readonly(const void* p) {

@@ -316,7 +316,7 @@ namespace {
 
 // A single rank: one or two kernels write every output directly.
 int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, const mcep_elastic_dispatch_args* a,
-                    const mcep::SingleLayout& layout, const Counts* counts, mcep_event** out_event) {
+                    const mcep::SingleTables& tables, const Counts* counts, mcep_event** out_event) {
     const int E = a->num_experts, M = a->num_max_tokens_per_rank, T = a->num_tokens, H = a->hidden, K = a->num_topk;
     EL_REQUIRE(H % 16 == 0 && H % 128 == 0);
     EL_REQUIRE(reinterpret_cast<uintptr_t>(a->x) % 32 == 0 && reinterpret_cast<uintptr_t>(a->recv_x) % 32 == 0);
@@ -342,7 +342,7 @@ int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, 
     if (counts) p.host_counts = s->host_counts, p.host_seq = (int32_t)++s->host_seq;
     const bool chain = mcep::may_chain(b, stream);
     mcep::LaunchCtx ctx{stream, v.num_sms, chain && !async, chain};
-    EL_CUDA(mcep::launch_elastic_single_dispatch(p, expand, layout, ctx));
+    EL_CUDA(mcep::launch_elastic_single_dispatch(p, expand, tables, ctx));
     mcep::count_dispatch_call(b);
     auto& rec = s->rec[par];
     rec.key = a->recv_src_metadata, rec.par = par, rec.T = T, rec.K = K, rec.E = E, rec.M = M, rec.H = H;
@@ -430,9 +430,12 @@ int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const 
     EL_REQUIRE(a->recv_x != nullptr && a->recv_topk_idx != nullptr && a->recv_src_metadata != nullptr);
     const int L = E / R;
     ElasticState* s = state_of(b);
-    mcep::SingleLayout layout;
-    if (!v.group && !v.defer && mcep::elastic_single_fits(T, K, E, a->do_expand != 0, v.num_sms, &layout))
-        return single_dispatch(b, s, v, a, layout, counts, out_event);
+    mcep::SingleTables tables;
+    const mcep::LayoutScratch scratch = mcep::next_layout_scratch(b);
+    if (!v.group && !v.defer &&
+        mcep::elastic_single_tables(T, K, E, a->do_expand != 0, v.num_sms, scratch.memory, scratch.bytes,
+                                    scratch.ticket, &tables))
+        return single_dispatch(b, s, v, a, tables, counts, out_event);
     EL_REQUIRE(counts == nullptr || !v.defer);
     const size_t rec_want = record_bytes(R, M, K);
     const size_t rec_bytes = (v.group && s->record_area_bytes != 0) ? s->record_area_bytes : rec_want;

@@ -97,8 +97,13 @@ struct ElasticSingleParams {
     const int64_t* topk_idx;     // [T][K]
     const float* topk_weights;   // [T][K] or null
     int T, K, E, H, alignment;
-    int C, early, teller;        // tokens per block of the copy kernel, tokens copied ahead of the layout,
-                                 // block that tells the host (set by the launcher)
+    int C;                       // tokens per block of the copy kernel, and behind a layout kernel
+    int warps_per_row, parts;    // the warps and the blocks that share a row (set by the launcher)
+    RouteBits bits;              // behind a layout kernel: row 0 all tokens that name an expert, 1 + e (expanded)
+                                 // those that name e
+    uint16_t* hits;              // [E][bits.stride] listings per chunk
+    int32_t* starts;             // [E + 1] expanded: where the experts' segments start
+    unsigned* ticket;            // expanded: chunks that are done
     int max_rows;                // expanded: rows recv_x has room for
     int32_t* status;
     int32_t* rows;               // kept for combine: [T] received row of the token, or (expanded) [T][K] row
@@ -117,15 +122,18 @@ struct ElasticSingleParams {
     int32_t* host_counts;
     int32_t host_seq;
 };
-// The layout kernel's cluster; blocks 0: no launch of its own, the copy kernel counts.
-struct SingleLayout {
-    const void* kernel = nullptr;
-    int blocks = 0, threads = 0;
-    size_t smem = 0;
+// The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
+struct SingleTables {
+    RouteBits bits = {};
+    uint16_t* hits = nullptr;
+    int32_t* starts = nullptr;
+    unsigned* ticket = nullptr;
 };
-// whether the kernels below take this problem (else the general path does), and with which layout
-bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms, SingleLayout* layout);
-cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleLayout& layout,
+// Whether the kernels below take this problem (else the general path does), and its tables,
+// in `bytes` bytes at `scratch` (256-byte aligned).
+bool elastic_single_tables(int T, int K, int E, bool expand, int num_sms, void* scratch, size_t bytes, unsigned* ticket,
+                           SingleTables* tables);
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleTables& tables,
                                            const LaunchCtx& ctx);
 
 // float ones of a given length (the weights of the exchange's reduction)

@@ -397,31 +397,20 @@ __device__ void tell_host(const ElasticSingleParams& p) {
     if (threadIdx.x == 0) h[0] = p.host_seq;
 }
 
-// Layout in one launch of one cluster (as the dispatch calls' layout kernel): a lane
-// per token. Column E of the tables stands for "the token goes anywhere", so a
-// token's received row is found like its rows inside the experts.
-//   kExpand: bit (expert, token) in [word][E + 1], popcounts, prefix over words and
-//   blocks; else only the number of hits per expert and column E are needed.
-// An expert listed twice counts twice in the hit counts and has its row at the last
-// listing (mooncake_ep_elastic_dispatch_copy_epilogue.cuh:114-141).
-constexpr int kSingleCluster = 8, kSingleClusterLarge = 16;
+// The layout as bits (RouteBits), a block per 128 tokens, as ep_layout_bits_kernel. Row 0 of
+// the table stands for "the token goes anywhere", from which its received row is found; rows
+// 1 + e (kExpand) are the experts'. `hits` are listings: an expert listed twice counts twice
+// in them and has its row at the last listing
+// (mooncake_ep_elastic_dispatch_copy_epilogue.cuh:114-141).
+// An expanded row's place depends on the hits of all experts below its own: the block that
+// finishes last sums them up (kExpand). For flat rows they are results only, and a block of
+// the copy kernel sums them, so that no row waits.
+constexpr int kBitsThreads = 256;
 
 template <bool kExpand, int KB>
-__device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int* smem) {
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, words = nthr >> 5;
-    const int rank = blockIdx.x, blocks = gridDim.x, E1 = p.E + 1;
-    const int t = rank * nthr + tid;
-    int* total = smem;                  // [E1] hits in this block (column E: tokens received)
-    int* lower = smem + E1;             // [E1] in the lower blocks
-    int* every = smem + 2 * E1;         // [E1 + 1] in all blocks, then the aligned sums
-    int* repeats = smem + 3 * E1 + 1;   // [E1] of the hits, those that have no row (kExpand)
-    int* rows_of = smem + 4 * E1 + 1;   // [E1] rows of the expert in all blocks (kExpand)
-    uint32_t* mask = reinterpret_cast<uint32_t*>(smem + 5 * E1 + 1);  // [words][E1] (kExpand)
-    int* pre = smem + 5 * E1 + 1 + words * E1;                        // [words][E1] (kExpand)
-    __shared__ int s_warp[32];
-    for (int i = tid; i < E1; i += nthr) total[i] = 0, repeats[i] = 0;
-    if (kExpand)
-        for (int i = tid; i < E1 * words; i += nthr) mask[i] = 0;
+__device__ __forceinline__ void single_bits(const ElasticSingleParams& p, uint32_t* mask, int* extra) {
+    const int t = blockIdx.x * kChunkTokens + threadIdx.x, lane = threadIdx.x & 31, word = threadIdx.x >> 5;
+    if (threadIdx.x >= kChunkTokens) return;
     int e[KB];
 #pragma unroll
     for (int k = 0; k < KB; ++k) e[k] = -1;
@@ -430,92 +419,76 @@ __device__ __forceinline__ void single_layout(const ElasticSingleParams& p, int*
 #pragma unroll
     for (int k = 0; k < KB; ++k) any |= e[k] >= 0;
     const unsigned sent = __ballot_sync(kAll, any);
-    if (lane == 0) s_warp[warp] = __popc(sent);
-    __syncthreads();
-    if (!kExpand) {
+    if (lane == 0) mask[word] = sent;
+    int all[KB];
 #pragma unroll
-        for (int k = 0; k < KB; ++k)
-            if (e[k] >= 0) atomicAdd(&total[e[k]], 1);
-    } else {
-        int all[KB];
+    for (int k = 0; k < KB; ++k) all[k] = e[k];
+    if (kExpand) drop_repeats<KB, true>(e);
 #pragma unroll
-        for (int k = 0; k < KB; ++k) all[k] = e[k];
-        drop_repeats<KB, true>(e);
+    for (int k = 0; k < KB; ++k) {
+        if (kExpand && e[k] >= 0) atomicOr(&mask[(1 + e[k]) * 4 + word], 1u << lane);
+        if (all[k] >= 0 && (!kExpand || e[k] < 0)) atomicAdd(&extra[all[k]], 1);
+    }
+}
+
+// Hits of expert e in all chunks.
+__device__ __forceinline__ int sum_hits(const ElasticSingleParams& p, int e) {
+    int sum = 0;
+    for (int c0 = 0; c0 < p.bits.chunks; c0 += 8) {
+        const uint4 v = ld_l2(reinterpret_cast<const uint4*>(p.hits + (size_t)e * p.bits.stride + c0));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int k = 0; k < KB; ++k) {
-            if (e[k] >= 0) atomicOr(&mask[warp * E1 + e[k]], 1u << lane);
-            if (all[k] >= 0 && e[k] < 0) atomicAdd(&repeats[all[k]], 1);
-        }
+        for (int j = 0; j < 8; ++j)
+            if (c0 + j < p.bits.chunks) sum += (w[j / 2] >> (16 * (j & 1))) & 0xffff;
     }
-    int before_warp = 0, in_block = 0;
-    for (int w = 0; w < words; ++w) {
-        if (w < warp) before_warp += s_warp[w];
-        in_block += s_warp[w];
-    }
-    __syncthreads();
-    if (kExpand)
-        for (int x = tid; x < p.E; x += nthr) {
-            int run = 0;
-            for (int w = 0; w < words; ++w) {
-                const int c = __popc(mask[w * E1 + x]);
-                pre[w * E1 + x] = run;
-                run += c;
-            }
-            total[x] = run;
-        }
-    if (tid == 0) total[p.E] = in_block;
-    cluster_sync();
-    // Every column is needed by the last block (the counts) and, expanded, by all (where
-    // the segments start); else a block needs column E alone.
-    const bool last = rank == blocks - 1;
-    for (int x = tid; x < E1; x += nthr) {
-        if (!kExpand && !last && x != p.E) continue;
-        int lo, none, rep = 0;
-        const int sum = blocks > kSingleCluster ? cluster_sum<kSingleClusterLarge>(total + x, rank, blocks, &lo)
-                                                : cluster_sum<kSingleCluster>(total + x, rank, blocks, &lo);
-        if (kExpand)
-            rep = blocks > kSingleCluster ? cluster_sum<kSingleClusterLarge>(repeats + x, rank, blocks, &none)
-                                          : cluster_sum<kSingleCluster>(repeats + x, rank, blocks, &none);
-        lower[x] = lo;
-        every[x] = x < p.E ? aligned_count(sum + rep, p.alignment) : sum;
-        if (kExpand) rows_of[x] = sum;
-    }
-    __syncthreads();
-    if (kExpand || last) {
-        if (last && tid == 0) p.psum_rank[0] = every[p.E];
-        __syncthreads();
-        exclusive_sums(every, p.E);  // where every expert's segment starts
-        if (last)
-            for (int x = tid; x < E1; x += nthr)  // expanded: where it ends
-                p.psum_expert[x] = every[x] + (kExpand && x < p.E ? rows_of[x] : 0);
-    }
-    if (t < p.T) {
-        const unsigned below = (1u << lane) - 1u;
-        p.token_pos[t] = any ? lower[p.E] + before_warp + __popc(sent & below) : -1;
-        if (kExpand) {
-            int32_t* out = p.rows + (size_t)t * p.K;
-#pragma unroll
-            for (int k = 0; k < KB; ++k) {
-                if (k >= p.K) break;
-                const int at = warp * E1 + e[k];
-                out[k] = e[k] < 0 ? -1 : row_with_room(p, every[e[k]] + lower[e[k]] + pre[at] + __popc(mask[at] & below));
-            }
-        }
-    }
-    cluster_sync();  // no block leaves while its totals may still be read
+    return sum;
 }
 
 template <bool kExpand>
-__global__ void __launch_bounds__(1024) ep_elastic_single_layout_kernel(ElasticSingleParams p) {
-    extern __shared__ int smem_i32[];
+__global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSingleParams p) {
+    extern __shared__ uint4 smem_u128[];  // [1 or 1 + E] bits of this chunk, then [E + 1] listings beyond them
+    __shared__ bool s_last;
+    const int tid = threadIdx.x, rows = kExpand ? 1 + p.E : 1;
+    int* extra = reinterpret_cast<int*>(smem_u128 + rows);
+    for (int i = tid; i < rows; i += kBitsThreads) smem_u128[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i <= p.E; i += kBitsThreads) extra[i] = 0;
+    __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem_u128);
     if (p.K <= 4)
-        single_layout<kExpand, 4>(p, smem_i32);
+        single_bits<kExpand, 4>(p, mask, extra);
     else if (p.K <= 8)
-        single_layout<kExpand, 8>(p, smem_i32);
+        single_bits<kExpand, 8>(p, mask, extra);
     else
-        single_layout<kExpand, 16>(p, smem_i32);
+        single_bits<kExpand, 16>(p, mask, extra);
+    __syncthreads();
+    for (int x = tid; x < rows; x += kBitsThreads) {
+        const uint4 m = smem_u128[x];
+        const int n = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+        p.bits.words[(size_t)x * p.bits.chunks + blockIdx.x] = m;
+        p.bits.counts[(size_t)x * p.bits.stride + blockIdx.x] = (uint8_t)n;
+        if (kExpand && x > 0) p.hits[(size_t)(x - 1) * p.bits.stride + blockIdx.x] = (uint16_t)(n + extra[x - 1]);
+    }
+    if (!kExpand) {
+        for (int x = tid; x < p.E; x += kBitsThreads)
+            p.hits[(size_t)x * p.bits.stride + blockIdx.x] = (uint16_t)extra[x];
+        return;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicInc(p.ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int x = tid; x < p.E; x += kBitsThreads) extra[x] = aligned_count(sum_hits(p, x), p.alignment);
+    __syncthreads();
+    exclusive_sums(extra, p.E);  // where every expert's segment starts
+    for (int x = tid; x <= p.E; x += kBitsThreads) {
+        p.starts[x] = extra[x];
+        p.psum_expert[x] = extra[x] + (x < p.E ? bits_total<true>(p.bits, 1 + x) : 0);  // where it ends
+    }
+    if (tid == 0) p.psum_rank[0] = bits_total<true>(p.bits, 0);
 }
 
 // Whether any of the `n` entries from `q` on names an expert; n <= 8, requested together.
@@ -564,47 +537,41 @@ __device__ __forceinline__ void count_hits(const ElasticSingleParams& p, int* hi
     }
 }
 
-// Rows and per-entry outputs. A block takes C tokens; C rows of a batch are requested
-// up to four per warp before the first is stored. Bound by HBM (4096 tokens of 14 KB:
-// 117 MB in and out). Behind the layout kernel (kCount false) the rows are requested
-// before its results are waited for. With kCount (small batches; kExpand: one token per
-// block) there is no layout kernel: every block finds its tokens' places itself and block
-// 0 writes the counts.
-template <bool kExpand, bool kCount>
-__global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
-    extern __shared__ int smem_i32[];  // kCount: [E + 1] hits / starts, [E] earlier tokens (kExpand)
+// Small batches, without a layout kernel: rows and per-entry outputs. A block takes C
+// tokens (kExpand: one), finds their places itself and copies the rows, up to four of a
+// batch per warp requested before the first is stored; block 0 writes the counts.
+template <bool kExpand>
+__global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticSingleParams p) {
+    extern __shared__ int smem_i32[];  // [E + 1] hits / starts, [E] earlier tokens (kExpand)
     constexpr int kEntries = 128;
     __shared__ int s_exp[kEntries];  // expert of the entry or -1
     __shared__ int s_row[kEntries];  // expanded row of the entry or -1 (kExpand)
     __shared__ int s_pos[kEntries];  // received row of token c
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int K = p.K, nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-    if (kCount) pdl_wait();
+    pdl_wait();
     pdl_launch_dependents();
-    int bid = blockIdx.x;
-    if (kCount) {
-        if (bid == 0) {  // the counts
-            for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
-            int* rows = smem_i32 + p.E + 1;
-            if (kExpand)
-                for (int i = tid; i < p.E; i += nthr) rows[i] = 0;
-            const int n = sent_before(p, p.T);
-            __syncthreads();
-            count_hits(p, smem_i32);
-            if (kExpand) count_tokens<1, true>(p.topk_idx, 0, p.T, K, p.E, choices_in_pairs(p.topk_idx, K), rows);
-            __syncthreads();
-            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
-            __syncthreads();
-            exclusive_sums(smem_i32, p.E);
-            for (int i = tid; i <= p.E; i += nthr)
-                p.psum_expert[i] = smem_i32[i] + (kExpand && i < p.E ? rows[i] : 0);
-            if (tid == 0) p.psum_rank[0] = n;
-            __syncthreads();
-            tell_host(p);
-            return;
-        }
-        bid -= 1;
+    if (blockIdx.x == 0) {  // the counts
+        for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
+        int* rows = smem_i32 + p.E + 1;
+        if (kExpand)
+            for (int i = tid; i < p.E; i += nthr) rows[i] = 0;
+        const int n = sent_before(p, p.T);
+        __syncthreads();
+        count_hits(p, smem_i32);
+        if (kExpand) count_tokens<1, true>(p.topk_idx, 0, p.T, K, p.E, choices_in_pairs(p.topk_idx, K), rows);
+        __syncthreads();
+        for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
+        __syncthreads();
+        exclusive_sums(smem_i32, p.E);
+        for (int i = tid; i <= p.E; i += nthr)
+            p.psum_expert[i] = smem_i32[i] + (kExpand && i < p.E ? rows[i] : 0);
+        if (tid == 0) p.psum_rank[0] = n;
+        __syncthreads();
+        tell_host(p);
+        return;
     }
+    const int bid = blockIdx.x - 1;
     const int t0 = bid * p.C;
     if (t0 >= p.T) return;
     const int nt = min(p.C, p.T - t0), ne = nt * K, items = nt * ntiles;
@@ -627,53 +594,32 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
     }
     const int e = all_bits(raw) < p.E ? all_bits(raw) : -1;
     if (tid < ne) s_exp[tid] = e;
-    if (kCount) {
+    __syncthreads();
+    int pos = sent_before(p, t0);
+    for (int tok = 0; tok < nt; ++tok) {
+        bool any = false;
+        for (int k = 0; k < K; ++k) any |= s_exp[tok * K + k] >= 0;
+        if (tid == 0) s_pos[tok] = any ? pos : -1, p.token_pos[t0 + tok] = any ? pos : -1;
+        pos += any ? 1 : 0;
+    }
+    if (kExpand) {
+        int* before = smem_i32 + p.E + 1;
+        for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
+        for (int i = tid; i < p.E; i += nthr) before[i] = 0;
         __syncthreads();
-        int pos = sent_before(p, t0);
-        for (int tok = 0; tok < nt; ++tok) {
-            bool any = false;
-            for (int k = 0; k < K; ++k) any |= s_exp[tok * K + k] >= 0;
-            if (tid == 0) s_pos[tok] = any ? pos : -1, p.token_pos[t0 + tok] = any ? pos : -1;
-            pos += any ? 1 : 0;
-        }
-        if (kExpand) {
-            int* before = smem_i32 + p.E + 1;
-            for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
-            for (int i = tid; i < p.E; i += nthr) before[i] = 0;
-            __syncthreads();
-            count_hits(p, smem_i32);
-            count_tokens<1, true>(p.topk_idx, 0, t0, K, p.E, choices_in_pairs(p.topk_idx, K), before);
-            __syncthreads();
-            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
-            __syncthreads();
-            exclusive_sums(smem_i32, p.E);
-            if (tid < ne) {
-                bool last = e >= 0;
-                for (int k = tid + 1; k < K; ++k) last = last && s_exp[k] != e;
-                const int row = last ? row_with_room(p, smem_i32[e] + before[e]) : -1;
-                s_row[tid] = row;
-                p.rows[(size_t)t0 * K + tid] = row;
-            }
-        }
-    } else if (!kExpand && t0 < p.early && t0 + p.C < p.T) {
-        // ahead of the layout kernel: the tokens before this batch are counted here
-        // (not the last batch: a block of every launch waits)
+        count_hits(p, smem_i32);
+        count_tokens<1, true>(p.topk_idx, 0, t0, K, p.E, choices_in_pairs(p.topk_idx, K), before);
         __syncthreads();
-        int pos = sent_before(p, t0);
-        for (int tok = 0; tok < nt; ++tok) {
-            bool any = false;
-            for (int k = 0; k < K; ++k) any |= s_exp[tok * K + k] >= 0;
-            if (tid == 0) s_pos[tok] = any ? pos : -1;
-            pos += any ? 1 : 0;
+        for (int i = tid; i < p.E; i += nthr) smem_i32[i] = aligned_count(smem_i32[i], p.alignment);
+        __syncthreads();
+        exclusive_sums(smem_i32, p.E);
+        if (tid < ne) {
+            bool last = e >= 0;
+            for (int k = tid + 1; k < K; ++k) last = last && s_exp[k] != e;
+            const int row = last ? row_with_room(p, smem_i32[e] + before[e]) : -1;
+            s_row[tid] = row;
+            p.rows[(size_t)t0 * K + tid] = row;
         }
-    } else {
-        pdl_wait();
-        if (bid == p.teller) tell_host(p);
-        if (tid < nt) {
-            const int pos = ld_ro(p.token_pos + t0 + tid);
-            s_pos[tid] = pos < p.T ? pos : -1;
-        }
-        if (kExpand && tid < ne) s_row[tid] = ld_ro(p.rows + (size_t)t0 * K + tid);
     }
     __syncthreads();
     if (tid < ne) {
@@ -716,6 +662,108 @@ __global__ void __launch_bounds__(512, kExpand && !kCount ? 3 : 2) ep_elastic_si
             } else if (s_pos[tok] >= 0) {
                 st32(out + ((size_t)s_pos[tok] * p.H + (size_t)c * 16) * 2, v[u]);
             }
+        }
+    }
+}
+
+// Behind ep_elastic_bits_kernel: as ep_dispatch_rows_kernel, a warp owns tiles of one token,
+// finds the token's place itself and needs no other warp; the warp of a token's first tile
+// writes what there is per entry. Block 0 writes and passes on the counts.
+// Two tiles per warp and 40 warps per SM: a row is stored once (or K times, few in general),
+// so it is the bytes requested at a time that matter. Flat, 4096 rows of 14 KB, dispatch
+// alone: 20.4 us, one tile and 32 warps 29.0, 48 warps 25.6, four tiles and 32 warps 20.8 (a
+// block per eight tokens and a layout kernel of one cluster before: 23.5). Expanded, the
+// layer, 4096 rows of 14 KB to 2 and to 8: 64.8 and 176.9 us, one tile and 40 warps 74.9 and
+// 178.3, 42 warps in blocks of seven 71.7 and 176.4, four tiles and 32 warps 67.5 and 182.1
+// (a block per token before: 65.1 and 179.2).
+constexpr int kElasticWarps = 4, kElasticTiles = 2;
+
+template <bool kExpand>
+__global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel(ElasticSingleParams p) {
+    extern __shared__ int smem_i32[];  // flat: [E + 1] hits / sums (block 0)
+    constexpr int kTiles = kElasticTiles;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    if (blockIdx.x == 0) {
+        pdl_wait();
+        if (!kExpand) {
+            for (int x = tid; x < p.E; x += blockDim.x) smem_i32[x] = aligned_count(sum_hits(p, x), p.alignment);
+            __syncthreads();
+            exclusive_sums(smem_i32, p.E);
+            for (int x = tid; x <= p.E; x += blockDim.x) p.psum_expert[x] = smem_i32[x];
+            if (tid == 0) p.psum_rank[0] = bits_total<false>(p.bits, 0);
+            __syncthreads();
+        }
+        tell_host(p);
+        return;
+    }
+    const int sub = warp / p.warps_per_row;
+    const int group = (blockIdx.x - 1) / p.parts, part = (blockIdx.x - 1) - group * p.parts;
+    const int first = (part * p.warps_per_row + warp - sub * p.warps_per_row) * kTiles;  // tile
+    const int t = group * p.C + sub, K = p.K;
+    const bool mine = t < p.T && lane < K;
+    V32 v[kTiles];
+#pragma unroll
+    for (int u = 0; u < kTiles; ++u) {
+        const int c = (first + u) * 32 + lane;
+        if (t < p.T && c < p.H / 16)
+            v[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+    }
+    int64_t raw = -1;
+    float w = 0.f;
+    if (mine) {
+        raw = ld_ro(p.topk_idx + (size_t)t * K + lane);
+        if (first == 0 && p.topk_weights) w = ld_ro(p.topk_weights + (size_t)t * K + lane);
+    }
+    const int e = (uint64_t)raw < (uint64_t)p.E ? (int)raw : -1;
+    const unsigned named = __ballot_sync(kAll, e >= 0);
+    pdl_wait();
+    const int pos = named ? bits_before(p.bits, 0, t) : -1;
+    int row = -1;
+    // (a repeat's earlier listings find the last one's row and store the same bytes)
+    if (kExpand && e >= 0) row = row_with_room(p, ld_ro(p.starts + e) + bits_before(p.bits, 1 + e, t));
+    if (first == 0 && t < p.T) {
+        const int master = 31 - __clz(named);
+        const unsigned same = __match_any_sync(kAll, e);
+        const int kept = 31 - __clz(same) == lane ? row : -1;  // the entry's row: at its last listing
+        const size_t at = (size_t)t * K + lane;
+        if (mine) {
+            p.dst_slot[at] = named && lane == master ? pos : -1;
+            if (p.copied_topk_idx) p.copied_topk_idx[at] = raw;
+            if (kExpand) p.rows[at] = kept;
+            if (named) {
+                p.recv_topk_idx[(size_t)pos * K + lane] = e;
+                int32_t* md = p.recv_src_metadata + (size_t)pos * (K + 2);
+                if (lane == 0) md[0] = t;
+                if (lane == 1 % K) md[1] = master;
+                if (kExpand) {
+                    md[2 + lane] = kept;
+                    if (p.recv_topk_weights && kept >= 0) p.recv_topk_weights[kept] = w;
+                } else if (p.recv_topk_weights) {
+                    p.recv_topk_weights[(size_t)pos * K + lane] = w;
+                }
+            }
+        }
+        if (!kExpand && lane == 0) p.token_pos[t] = pos;
+    }
+    char* out = static_cast<char*>(p.recv_x);
+    const size_t row_bytes = (size_t)p.H * 2;
+    if (kExpand) {
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = __shfl_sync(kAll, row, k);
+            if (r < 0) continue;
+#pragma unroll
+            for (int u = 0; u < kTiles; ++u) {
+                const int c = (first + u) * 32 + lane;
+                if (c < p.H / 16) st32(out + (size_t)r * row_bytes + (size_t)c * 32, v[u]);
+            }
+        }
+    } else if (named) {
+#pragma unroll
+        for (int u = 0; u < kTiles; ++u) {
+            const int c = (first + u) * 32 + lane;
+            if (c < p.H / 16) st32(out + (size_t)pos * row_bytes + (size_t)c * 32, v[u]);
         }
     }
 }
@@ -764,15 +812,6 @@ cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int n
 }
 
 namespace {
-// Threads per block of the layout kernel with clusters of `blocks`; 0: does not fit.
-int single_layout_threads(int T, int blocks) {
-    const int threads = ((T + blocks - 1) / blocks + 31) / 32 * 32;
-    return threads >= 32 && threads <= 1024 ? threads : 0;
-}
-size_t single_layout_smem(int E, int threads, bool expand) {
-    return (size_t)(5 * (E + 1) + 1 + (expand ? 2 * (threads / 32) * (E + 1) : 0)) * sizeof(int);
-}
-constexpr size_t kSingleSmemMax = 200 * 1024;
 // One launch. Flat rows: up to 4096 choices and seven tokens per SM, in one resident wave
 // (us per layer: 500 tokens of 14 KB to 8 10.3, behind a layout kernel 12.5; 1000 of 8 KB
 // to 2 10.2 against 11.5; 700 to 8 11.2 against 10.6, 2000 to 2 14.3 against 14.2).
@@ -780,39 +819,28 @@ constexpr size_t kSingleSmemMax = 200 * 1024;
 bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand) {
     return expand ? T <= 2 * num_sms : T * K <= 4096 && T <= 7 * num_sms;
 }
-
-// Sixteen blocks (an opt-in cluster size) once eight would have more than 8 warps
-// each, or where eight blocks' tables do not fit.
-bool pick_single_layout(int T, int E, bool expand, SingleLayout* l) {
-    l->kernel = expand ? reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<true>)
-                       : reinterpret_cast<const void*>(ep_elastic_single_layout_kernel<false>);
-    const bool prefer_large = T > kSingleCluster * 256;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        const int blocks = prefer_large == (attempt == 0) ? kSingleClusterLarge : kSingleCluster;
-        l->threads = single_layout_threads(T, blocks);
-        l->smem = l->threads ? single_layout_smem(E, l->threads, expand) : 0;
-        if (l->threads == 0 || l->smem > kSingleSmemMax) continue;
-        bool fits = false;
-        if (cluster_fits(l->kernel, blocks, l->threads, l->smem, &fits) == cudaSuccess && fits) {
-            l->blocks = blocks;
-            return true;
-        }
-    }
-    return false;
-}
 }  // namespace
 
-bool elastic_single_fits(int T, int K, int E, bool expand, int num_sms, SingleLayout* layout) {
-    const int threads = single_layout_threads(T < 1 ? 1 : T, kSingleClusterLarge);
-    if (K > kMaxTopk || E > kMaxExperts || threads == 0 || single_layout_smem(E, threads, true) > kSingleSmemMax)
-        return false;
-    return counts_in_copy_kernel(T, K, num_sms, expand) || pick_single_layout(T, E, expand, layout);
+bool elastic_single_tables(int T, int K, int E, bool expand, int num_sms, void* scratch, size_t bytes, unsigned* ticket,
+                           SingleTables* tables) {
+    *tables = SingleTables();
+    if (K > kMaxTopk || E > kMaxExperts) return false;
+    if (counts_in_copy_kernel(T, K, num_sms, expand)) return true;
+    const size_t starts = ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
+    const size_t hits = (size_t)E * (((T + kChunkTokens - 1) / kChunkTokens + 15) / 16 * 16) * sizeof(uint16_t);
+    if (starts + hits > bytes) return false;
+    char* at = static_cast<char*>(scratch);
+    tables->starts = reinterpret_cast<int32_t*>(at);
+    tables->hits = reinterpret_cast<uint16_t*>(at + starts);
+    tables->bits = route_bits(at + starts + hits, bytes - starts - hits, T, expand ? 1 + E : 1);
+    tables->ticket = ticket;
+    return tables->bits.words != nullptr;
 }
 
-cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleLayout& l,
+cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleTables& tables,
                                            const LaunchCtx& ctx) {
     const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-    if (l.blocks == 0) {
+    if (tables.bits.words == nullptr) {
         // one launch: the block of the counts, and a block per token or (flat) per as many
         // tokens as make one resident wave
         p.C = expand ? 1 : (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
@@ -820,33 +848,26 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         if (p.C < 1) p.C = 1;
         const int items = p.C * ntiles;
         const int warps = items < 8 ? 8 : items < 16 ? items : 16;
-        auto k = expand ? ep_elastic_single_copy_kernel<true, true> : ep_elastic_single_copy_kernel<false, true>;
+        auto k = expand ? ep_elastic_single_copy_kernel<true> : ep_elastic_single_copy_kernel<false>;
         return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
-    auto layout = expand ? ep_elastic_single_layout_kernel<true> : ep_elastic_single_layout_kernel<false>;
-    if (cudaError_t err = launch_kernel("ep_elastic_single_layout", layout, dim3(l.blocks), dim3(l.threads), l.smem,
-                                        l.blocks, ctx, p))
-        return err;
+    p.bits = tables.bits, p.hits = tables.hits, p.starts = tables.starts, p.ticket = tables.ticket;
+    auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
+    const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
+    if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;
+    if (cudaError_t e = launch_kernel("ep_elastic_single_layout", layout, dim3(p.bits.chunks), dim3(kBitsThreads), smem,
+                                      1, ctx, p))
+        return e;
     LaunchCtx chained = ctx;
     chained.pdl = ctx.chain;
-    // Blocks of up to 8 warps. Plain rows: a warp gets about four tiles, all requested at
-    // once (4096 rows of 4 KB: 15.0 us per layer, 16 warps 16.3). Expanded: every row is
-    // stored K times; a row per block (1024 rows of 8 KB to 8: 27.8 us per layer, two rows
-    // 29.2; 4096 rows of 14 KB to 2: 66.9, 14 warps 74.7).
-    int c = expand ? 1 : 32 / ntiles;
-    if (c > 8) c = 8;
-    if (c > 128 / p.K) c = 128 / p.K;
-    const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
-    p.C = c < 1 ? 1 : c < most ? c : most;
-    // (an expanded row's place depends on all tokens: nothing to send ahead)
-    p.early = expand ? 0 : 3 * ctx.num_sms;
-    p.teller = (p.early + p.C - 1) / p.C;  // the first block that waits for the layout kernel
-    if (p.teller > (p.T + p.C - 1) / p.C - 1) p.teller = (p.T + p.C - 1) / p.C - 1;
-    int warps = p.C * ntiles;
-    warps = warps > 8 ? 8 : warps < 4 ? 4 : warps;
-    auto k = expand ? ep_elastic_single_copy_kernel<true, false> : ep_elastic_single_copy_kernel<false, false>;
-    return launch_kernel("ep_elastic_single_copy", k, dim3((p.T + p.C - 1) / p.C), dim3(warps * 32), 0, 1, chained, p);
+    const int warps = (ntiles + kElasticTiles - 1) / kElasticTiles;  // of a row
+    p.parts = (warps + kElasticWarps - 1) / kElasticWarps;
+    p.warps_per_row = (warps + p.parts - 1) / p.parts;
+    p.C = kElasticWarps / p.warps_per_row;
+    auto k = expand ? ep_elastic_rows_kernel<true> : ep_elastic_rows_kernel<false>;
+    return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C * p.parts),
+                         dim3(p.C * p.warps_per_row * 32), expand ? 0 : ((size_t)p.E + 1) * sizeof(int), 1, chained, p);
 }
 
 cudaError_t launch_elastic_fill_ones(float* w, size_t n, cudaStream_t stream) {

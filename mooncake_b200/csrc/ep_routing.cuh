@@ -113,11 +113,14 @@ __device__ __forceinline__ bool choices_in_pairs(const int64_t* topk_idx, int K)
 }
 
 // ---- positions from the layout kernel's bits (RouteBits) ------------------------------
-// Sum of the first `n` counts of a row of bytes, sixteen per load.
+// Sum of the first `n` counts of a row of bytes, sixteen per load. kHere: written by other
+// blocks of this kernel.
+template <bool kHere>
 __device__ __forceinline__ int sum_counts(const uint8_t* row, int n) {
     int sum = 0;
     for (int c0 = 0; c0 < n; c0 += 16) {
-        const uint4 v = ld_ro(reinterpret_cast<const uint4*>(row + c0));
+        const uint4* at = reinterpret_cast<const uint4*>(row + c0);
+        const uint4 v = kHere ? ld_l2(at) : ld_ro(at);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -133,7 +136,7 @@ __device__ __forceinline__ int bits_before(const RouteBits& b, int e, int t) {
     const int chunk = t / kChunkTokens, bit = t % kChunkTokens;
     const uint4 v = ld_ro(b.words + (size_t)e * b.chunks + chunk);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    int n = sum_counts(b.counts + (size_t)e * b.stride, chunk);
+    int n = sum_counts<false>(b.counts + (size_t)e * b.stride, chunk);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int lower = bit - 32 * j;  // bits of this word that are lower
@@ -142,8 +145,9 @@ __device__ __forceinline__ int bits_before(const RouteBits& b, int e, int t) {
     return n;
 }
 // Tokens that chose expert e.
+template <bool kHere = false>
 __device__ __forceinline__ int bits_total(const RouteBits& b, int e) {
-    return sum_counts(b.counts + (size_t)e * b.stride, b.chunks);
+    return sum_counts<kHere>(b.counts + (size_t)e * b.stride, b.chunks);
 }
 
 }  // namespace mcep

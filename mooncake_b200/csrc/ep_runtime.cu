@@ -389,6 +389,10 @@ void set_after_deferred(mcep_buffer* b, std::function<int()> fn) { b->after_defe
 
 void count_dispatch_call(mcep_buffer* b) { ++b->dseq; }
 void count_combine_call(mcep_buffer* b) { ++b->cseq; }
+LayoutScratch next_layout_scratch(mcep_buffer* b) {
+    const auto& sc = b->scratch[(b->dseq + 1) & 1];
+    return {sc.slot, b->scratch_entries * sizeof(int32_t), sc.layout_ticket};
+}
 bool may_chain(const mcep_buffer* b, cudaStream_t stream) { return chain_with_pdl(b, stream); }
 
 int report_failure(int code, const char* message) { return fail(code, "%s", message); }

@@ -37,6 +37,14 @@ void set_after_deferred(mcep_buffer* b, std::function<int()> fn);
 void count_dispatch_call(mcep_buffer* b);
 void count_combine_call(mcep_buffer* b);
 
+// Where the next dispatch call of the buffer keeps its layout (of that call's parity).
+struct LayoutScratch {
+    void* memory;  // 256-byte aligned
+    size_t bytes;
+    unsigned* ticket;  // zero between calls
+};
+LayoutScratch next_layout_scratch(mcep_buffer* b);
+
 // Whether kernels queued on `stream` may be chained with programmatic launches now.
 bool may_chain(const mcep_buffer* b, cudaStream_t stream);
 

@@ -69,6 +69,32 @@ def test_dispatch_and_combine(T, H, E, K, expand, alignment):
     assert buf.runtime.status() == 0
 
 
+@pytest.mark.parametrize("T,H,E,K,expand,alignment", [  # words, chunks and loads of counts; rows of odd tiles and parts
+    (16384, 128, 8, 2, True, 1), (16384, 128, 300, 1, False, 3), (4225, 640, 24, 5, True, 8), (4224, 1152, 9, 7, False, 1),
+    (1153, 4224, 8, 3, True, 2), (2049, 8320, 8, 2, False, 1), (384, 128, 4096, 4, True, 1)])
+def test_layout_in_bits(T, H, E, K, expand, alignment):
+    test_dispatch_and_combine(T, H, E, K, expand, alignment)
+
+
+def test_a_repeat_has_its_expanded_row_at_its_last_listing():
+    """An expert listed twice takes two rows of its segment and fills one; the first listing names none."""
+    T, H, E, K = 700, 1152, 8, 3
+    x, idx, w = make_rank_inputs(41, 0, T, H, E, K)
+    idx[::3, 0] = idx[::3, 2]
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    recv, _, rw, h, _ = buf.dispatch(x.cuda(), topk_idx=idx.cuda(), topk_weights=w.cuda(), num_experts=E,
+                                     num_max_tokens_per_rank=T, do_expand=True)
+    hits = torch.bincount(idx.reshape(-1), minlength=E)
+    start, rows = torch.cumsum(hits, 0) - hits, h.recv_src_metadata[:, 2:].cpu()
+    once = (idx.unsqueeze(2) == torch.arange(E)).any(dim=1).int()   # [T][E]: one row per token and expert
+    want = (start + torch.cumsum(once, 0) - once).gather(1, idx)
+    want[::3, 0] = -1
+    assert torch.equal(rows.long(), want)
+    t, k = (want >= 0).nonzero(as_tuple=True)
+    assert torch.equal(recv.cpu()[want[t, k]], x[t]) and torch.equal(rw.cpu()[want[t, k]], w[t, k])
+    assert torch.equal(h.psum_num_recv_tokens_per_expert.cpu()[:E].long(), start + once.sum(0))
+
+
 def test_counts_of_back_to_back_calls_and_an_empty_batch():
     """Every waiting call gets its own counts, also with nothing to send."""
     T, H, E, K = 700, 128, 8, 2
