@@ -1173,9 +1173,11 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
     const size_t row_bytes = (size_t)p.H * 2;
     const char* x = reinterpret_cast<const char*>(p.x) + (size_t)c * 32;
     char* out = reinterpret_cast<char*>(p.combined_x) + (size_t)c * 32;
-    // a block's groups: every grid-th one, or (p.span) a run of tokens
+    // a block's groups: every grid-th one, or (p.span) a run of tokens, the last run first
+    // where the runs are many (p.backward)
+    const int block = p.backward ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const int step = (p.span ? 1 : gridDim.x) * p.tokens_per_block;
-    const int first = blockIdx.x * (p.span ? p.span : p.tokens_per_block);
+    const int first = block * (p.span ? p.span : p.tokens_per_block);
     const int end = p.span ? min(p.T, first + p.span) : p.T;
 
     // rows that there are (kAbs: a dispatch may have kept some beyond the caller's tensor)
@@ -2205,7 +2207,7 @@ cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx&
 
 // How the kernels that give a warp one tile of a row per token are laid out.
 struct ReduceShape {
-    int tiles_per_block, tokens_per_block, span, threads;
+    int tiles_per_block, tokens_per_block, span, backward, threads;
     dim3 grid;
 };
 static ReduceShape reduce_shape(int T, int K, int H, int num_sms) {
@@ -2231,11 +2233,16 @@ static ReduceShape reduce_shape(int T, int K, int H, int num_sms) {
     // every block an equal run of consecutive groups (1024 tokens to 8: 20.5 us, strided
     // 22.5). More: runs of two, handed out as blocks finish, so that no SM falls behind
     // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
-    // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181).
+    // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181). Those are rows
+    // beyond L2: the last tokens' are taken first, as what was written last is still there
+    // where the rows were made in token order (a layer whose experts' outputs are the rows
+    // just received: 4096 x 14 KB 172.7 us | 169.0, 3000 128.9 | 124.0, 8000 x 8 KB 189.8 | 183.5;
+    // rows made long before 81.3 either way). With fewer waves it gains and loses 1 %.
     const int resident = std::max(1, num_sms * (2 * kReduceWarps * 32 / s.threads) / parts);
     const int waves = (groups + resident - 1) / resident;
     const int run = K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
     s.span = run * s.tokens_per_block;
+    s.backward = run == 2;
     s.grid = dim3(run ? (groups + run - 1) / run : groups < resident ? groups : resident, parts);
     return s;
 }
@@ -2261,6 +2268,7 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
     }
     const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
     p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
+    p.backward = shape.backward;
     void (*k)(DirectCombineParams) = nullptr;
     if (p.absolute) {
         k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, true, 1> : ep_combine_rows_kernel<4, true, 2>;

@@ -110,6 +110,7 @@ struct DirectCombineParams {
     int absolute;               // rowmap names rows of the whole tensor, which has M of them (-1: none), every
                                 // weight is 1; topk_idx and topk_weights are not read
     int tokens_per_block, tiles_per_block, span;  // set by the launcher (span: tokens a block works through)
+    int backward;               // set by the launcher: the last tokens first
     // search: no rowmap; rows are looked up in the handle by the kernel
     int search;
     const int32_t* src_info;
