@@ -1362,18 +1362,17 @@ __device__ __forceinline__ void load_peer_tables(void* const* peer_base, const i
 //  3. fix the receive layout (source-rank order), write `layout_range` and
 //     `recv_count`, leave the verdicts for the receive duty, and answer every
 //     source with the first row of its segment in each of this rank's experts.
-template <bool kCount>
 __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, int* smem_i32,
                                                  char* const* s_peer, const int* s_active) {
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int L = p.E / p.R, n = L * p.R;
-    int* hist = smem_i32;         // [E]
+    const int* hist = smem_i32;   // [E] counts of this rank's tokens
     int* s_cnt = smem_i32 + p.E;  // [L*R]
     MCEP_TRACE(0, 1);
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
         if (!s_active[dr]) continue;
-        const int c = kCount ? hist[x] : p.bits.words != nullptr ? bits_total(p.bits, x) : ld_ro(p.count + x);
+        const int c = hist[x];
         uint64_t* wd = reinterpret_cast<uint64_t*>(s_peer[dr] + p.w.cnt_off) + (p.rank * L + (x - dr * L));
         st_relaxed_sys(wd, ((uint64_t)p.seq << 32) | (uint32_t)(c + 1));
     }
@@ -1566,16 +1565,21 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     const int nsend = nblocks - 1;
     const int nh = nsend < kRecvHelpers ? nsend : kRecvHelpers;
     MCEP_TRACE(0, 0);
-    if (kCount && bid == 0) {  // the counts do not wait for the peer tables (0.8 us)
-        for (int i = tid; i < p.E; i += nthr) smem_i32[i] = 0;
-        __syncthreads();
-        count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
+    if (bid == 0) {  // the counts do not wait for the peer tables (0.8 us)
+        if (kCount) {
+            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = 0;
+            __syncthreads();
+            count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
+        } else {
+            for (int i = tid; i < p.E; i += nthr)
+                smem_i32[i] = p.bits.words != nullptr ? bits_total(p.bits, i) : ld_ro(p.count + i);
+        }
     }
     load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);
 
     if (bid == 0) {
         __syncthreads();
-        dispatch_control<kCount>(p, smem_i32, s_peer, s_active);
+        dispatch_control(p, smem_i32, s_peer, s_active);
         if (kPhases == 3) {
             __syncthreads();
             dispatch_recv_duty<kFP8>(p, nh, nh + 1, smem_i32);
@@ -1701,13 +1705,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, 4) ep_dispatch_recv_kernel(Gro
 // position; one system fence per block, a ticket, and whoever finishes last
 // tells every peer. With zero copy the caller's kernels wrote the rows there
 // already and only the word is sent.
+// `first_lr`: layout_range[tid], requested by the caller ahead of its peer tables.
 __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p, int j, int np,
                                                      int* smem_i32, char* const* s_peer,
-                                                     const int* s_active) {
+                                                     const int* s_active, long long first_lr) {
     const int L = p.E / p.R, n = L * p.R;
     int* pre = smem_i32;  // [n + 1]
     __shared__ int s_wt[32];
-    __shared__ int s_last;
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int RM = p.R * p.M;
@@ -1719,7 +1723,7 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
         bool mine = false;
         for (int i = tid; i < n; i += nthr) {
             const int src = i % p.R;
-            const long long lr = ld_ro(p.layout_range + i);
+            const long long lr = i == tid ? first_lr : ld_ro(p.layout_range + i);
             int c = (int)(lr & 0xffffffffll);
             if (src == p.rank || !s_active[src]) c = 0;
             pre[i] = c;
@@ -1779,18 +1783,19 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
     // more) is for stores that cross NVLink.
     const int any = __syncthreads_or(stored ? 1 : 0);
     MCEP_TRACE(2, 3);  // this block's rows are copied
-    if (tid == 0) {
+    // One thread, of the last warp: the others go on to the reduce duty, whose first loads
+    // are warp 0's, while the ticket is on its way (128 tokens of 7 KB on one rank, the layer:
+    // 16.5 us with a barrier behind the ticket, 15.8 without).
+    if (tid == nthr - 32) {
         if (any || (p.zero_copy && j == 0)) __threadfence();
-        s_last = (atomicAdd(p.ticket, 1u) == (unsigned)(np - 1));
-        if (s_last) *p.ticket = 0;
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        for (int r = tid; r < p.R; r += nthr) {
-            if (r == p.rank || !s_active[r]) continue;
-            uint64_t* f = reinterpret_cast<uint64_t*>(s_peer[r] + p.w.cflag_off) + p.rank;
-            st_relaxed_sys(f, ((uint64_t)p.seq << 32) | 1u);
+        if (atomicAdd(p.ticket, 1u) == (unsigned)(np - 1)) {
+            *p.ticket = 0;
+            __threadfence();
+            for (int r = 0; r < p.R; ++r) {
+                if (r == p.rank || !s_active[r]) continue;
+                uint64_t* f = reinterpret_cast<uint64_t*>(s_peer[r] + p.w.cflag_off) + p.rank;
+                st_relaxed_sys(f, ((uint64_t)p.seq << 32) | 1u);
+            }
         }
     }
 }
@@ -1848,12 +1853,13 @@ __device__ __forceinline__ void combine_body(const GroupCombineParams& p, int bi
     __shared__ char* s_peer[kMaxRanks];
     __shared__ int s_active[kMaxRanks];
     MCEP_TRACE(2, 0);
+    long long first_lr = 0;
+    if ((kPhases & 1) && !p.zero_copy && (int)threadIdx.x < p.E) first_lr = ld_ro(p.layout_range + threadIdx.x);
     load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);
     __syncthreads();
-    if (kPhases & 1) combine_publish_duty(p, bid, nblocks, smem_i32, s_peer, s_active);
+    if (kPhases & 1) combine_publish_duty(p, bid, nblocks, smem_i32, s_peer, s_active, first_lr);
     MCEP_TRACE(2, 1);
     if (kPhases & 2) {
-        __syncthreads();
         combine_reduce_duty(p, bid, nblocks, s_peer);
     }
     MCEP_TRACE(2, 2);
