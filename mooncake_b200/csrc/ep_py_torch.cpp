@@ -13,6 +13,7 @@
 // addresses `bind` was given, so it always drives the same libmcep.so as the
 // ctypes declarations of ep.py.
 #define PY_SSIZE_T_CLEAN
+#include <array>
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -278,6 +279,42 @@ PyObject* py_register_overlap(PyObject*, PyObject* cls) {
     Py_INCREF(cls);
     overlap_type = reinterpret_cast<PyTypeObject*>(cls);
     Py_RETURN_NONE;
+}
+
+// ---- EPHandle ---------------------------------------------------------------------------
+const char* const kHandleNames[] = {
+    "do_expand", "num_experts", "expert_alignment", "num_max_tokens_per_rank", "num_sms", "topk_idx",
+    "psum_num_recv_tokens_per_scaleup_rank", "psum_num_recv_tokens_per_expert", "num_recv_tokens_per_expert_list",
+    "recv_src_metadata", "dst_buffer_slot_idx", "token_metadata_at_forward", "channel_linked_list", "native_handle",
+    "num_recv_tokens"};
+constexpr size_t kHandleFields = sizeof(kHandleNames) / sizeof(kHandleNames[0]);
+PyObject* handle_names[kHandleFields];
+PyTypeObject* handle_type = nullptr;
+
+PyObject* py_register_handle(PyObject*, PyObject* cls) {
+    if (!PyType_Check(cls)) return PyErr_Format(PyExc_TypeError, "a class is wanted");
+    for (size_t i = 0; i < kHandleFields; ++i)
+        if (handle_names[i] == nullptr && (handle_names[i] = PyUnicode_InternFromString(kHandleNames[i])) == nullptr)
+            return nullptr;
+    Py_INCREF(cls);
+    handle_type = reinterpret_cast<PyTypeObject*>(cls);
+    Py_RETURN_NONE;
+}
+
+// A handle made of all its fields, whose references are taken over (null: an error is set).
+PyObject* wrap_handle(const std::array<PyObject*, kHandleFields>& fields) {
+    PyObject* dict = PyDict_New();
+    bool ok = dict != nullptr;
+    for (size_t i = 0; i < kHandleFields; ++i) {
+        ok = ok && fields[i] != nullptr && PyDict_SetItem(dict, handle_names[i], fields[i]) == 0;
+        Py_XDECREF(fields[i]);
+    }
+    PyObject* none = ok ? PyTuple_New(0) : nullptr;
+    PyObject* self = none ? handle_type->tp_new(handle_type, none, nullptr) : nullptr;
+    Py_XDECREF(none);
+    if (self != nullptr && PyObject_GenericSetDict(self, dict, nullptr) != 0) Py_CLEAR(self);
+    Py_XDECREF(dict);
+    return self;
 }
 
 struct HookObject {
@@ -667,16 +704,16 @@ PyObject* runtime_combine_tensors(PyObject* self, PyObject* const* args, Py_ssiz
 }
 
 // elastic_dispatch_tensors(x, topk_idx, topk_weights or None, active_ranks, kept_idx or None, E, M,
-//                          alignment, do_expand, do_cpu_sync, timeout_us, async, in_place or None)
-//   -> (recv_x, recv_topk_idx, recv_topk_weights or None, recv_src_metadata, psum_rank, psum_expert,
-//       dst_buffer_slot_idx, kept_idx, counts or None, event), or None (as above)
+//                          alignment, do_expand, do_cpu_sync, timeout_us, async, in_place or None, num_sms)
+//   -> what ElasticBuffer.dispatch returns: (recv_x, recv_topk_idx, recv_topk_weights or None, EPHandle,
+//       EventOverlap), or None (as above)
 // `kept_idx`: the cached handle's routing (topk_idx is then that tensor); None: a copy is made.
 // psum_expert is [L + 1] with do_expand and its entries 1.. without, as the wrapper hands it out;
-// `counts` is the list of tokens per local expert (do_cpu_sync), the row tensors are then cut to length.
+// With do_cpu_sync the handle has the list of tokens per local expert, and the row tensors are cut to length.
 PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     RuntimeObject* s = self_of(self);
-    if (nargs != 13) return PyErr_Format(PyExc_TypeError, "elastic_dispatch_tensors() takes 13 arguments");
+    if (nargs != 14) return PyErr_Format(PyExc_TypeError, "elastic_dispatch_tensors() takes 14 arguments");
     if (!alive(s)) return nullptr;
     Reader r{const_cast<PyObject**>(args)};
     const at::Tensor *x = tensor_of(args[0]), *idx = tensor_of(args[1]), *w = tensor_of(args[2]);
@@ -740,7 +777,7 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
     if (rc) return fail();
 
     int64_t n = n_cap, n_out = out_cap;
-    PyObject* counts = sync ? PyList_New(L) : new_ref(Py_None);
+    PyObject* counts = PyList_New(sync ? L : 0);
     if (counts == nullptr) return nullptr;
     if (sync) {
         const int32_t* psum = host.data() + R;
@@ -758,18 +795,35 @@ PyObject* runtime_elastic_dispatch_tensors(PyObject* self, PyObject* const* args
         if (!in_place) recv_x.unsafeGetTensorImpl()->set_sizes_contiguous({n_out, H});
     }
     const int64_t first = expand ? 0 : 1;
-    return pack({wrap(std::move(recv_x)), wrap(small.view(o_idx, at::kLong, {n, K})),
-                 !w ? new_ref(Py_None)
-                    : wrap(expand ? small.view(o_w, at::kFloat, {n_out}) : small.view(o_w, at::kFloat, {n, K})),
-                 wrap(small.view(o_md, at::kInt, {n, K + 2})), wrap(small.view(o_rank, at::kInt, {R})),
-                 wrap(small.view(o_expert + 4 * first, at::kInt, {L + 1 - first})),
-                 wrap(small.view(o_slot, at::kInt, {T, K})),
-                 cached ? new_ref(args[4]) : wrap(small.view(o_kept, at::kLong, idx->sizes())), counts, wrap_event(ev)});
+    PyObject* p_rows = wrap(std::move(recv_x));
+    PyObject* p_idx = wrap(small.view(o_idx, at::kLong, {n, K}));
+    PyObject* p_w = !w       ? new_ref(Py_None)
+                    : expand ? wrap(small.view(o_w, at::kFloat, {n_out}))
+                             : wrap(small.view(o_w, at::kFloat, {n, K}));
+    PyObject* p_md = wrap(small.view(o_md, at::kInt, {n, K + 2}));
+    PyObject* p_rank = wrap(small.view(o_rank, at::kInt, {R}));
+    PyObject* p_expert = wrap(small.view(o_expert + 4 * first, at::kInt, {L + 1 - first}));
+    PyObject* p_slot = wrap(small.view(o_slot, at::kInt, {T, K}));
+    PyObject* p_kept = cached ? new_ref(args[4]) : wrap(small.view(o_kept, at::kLong, idx->sizes()));
+    PyObject* keep = nullptr;
+    if (!async)
+        keep = new_ref(Py_None);
+    else if (!p_rows || !p_idx || !p_w || !p_md || !p_rank || !p_expert || !p_slot || !p_kept)
+        keep = nullptr;  // (an error is set)
+    else if (w)
+        keep = PyTuple_Pack(12, args[0], args[1], p_kept, args[3], p_rows, p_idx, p_rank, p_expert, p_md, p_slot, args[2], p_w);
+    else
+        keep = PyTuple_Pack(10, args[0], args[1], p_kept, args[3], p_rows, p_idx, p_rank, p_expert, p_md, p_slot);
+    PyObject* handle = wrap_handle({new_ref(args[8]), new_ref(args[5]), new_ref(args[7]), new_ref(args[6]),
+                                    new_ref(args[13]), p_kept, p_rank, p_expert, counts, p_md, p_slot, new_ref(Py_None),
+                                    new_ref(Py_None), new_ref(Py_True), PyLong_FromLongLong(n)});
+    return pack({p_rows, p_idx, p_w, handle, wrap_overlap(wrap_event(ev), keep)});
     END_HANDLE_TH_ERRORS
 }
 
 // elastic_combine_tensors(x, topk_idx, topk_weights or None, psum_rank, recv_src_metadata, active_ranks,
-//                         E, M, do_expand, timeout_us, async) -> (combined_x, event), or None (as above)
+//                         E, M, do_expand, timeout_us, async)
+//   -> what ElasticBuffer.combine returns: (combined_x, None, EventOverlap), or None (as above)
 PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     RuntimeObject* s = self_of(self);
@@ -803,7 +857,17 @@ PyObject* runtime_elastic_combine_tensors(PyObject* self, PyObject* const* args,
     int rc;
     Py_BEGIN_ALLOW_THREADS rc = lib.elastic_combine(s->buf, &a, &ev);
     Py_END_ALLOW_THREADS if (rc) return fail();
-    return pack({wrap(std::move(out)), wrap_event(ev)});
+    PyObject* p_out = wrap(std::move(out));
+    PyObject* keep = nullptr;
+    if (!async)
+        keep = new_ref(Py_None);
+    else if (!p_out)
+        keep = nullptr;  // (an error is set)
+    else if (w)
+        keep = PyTuple_Pack(6, args[0], args[5], p_out, args[1], args[4], args[2]);
+    else
+        keep = PyTuple_Pack(5, args[0], args[5], p_out, args[1], args[4]);
+    return pack({p_out, new_ref(Py_None), wrap_overlap(wrap_event(ev), keep)});
     END_HANDLE_TH_ERRORS
 }
 
@@ -848,6 +912,7 @@ PyMethodDef module_methods[] = {
     {"adopt_event", py_adopt_event, METH_O, "An EventHandle that owns the mcep_event at this address (None: None)."},
     {"bind", py_bind, METH_O, "bind({name: address}): the entry points of the loaded libmcep.so."},
     {"register_overlap", py_register_overlap, METH_O, "The class (derived from EventOverlapBase) that calls return."},
+    {"register_handle", py_register_handle, METH_O, "The class of the handles that elastic calls return."},
     {"current_stream", py_current_stream, METH_NOARGS, "torch's current CUDA stream as an integer."},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_mcep_torch", "Native binding of libmcep.so for torch tensors.",

@@ -197,6 +197,7 @@ def get_ep_buffer_size_hint(num_max_dispatch_tokens_per_rank: int, hidden: int,
 
 EventHandle = _native.EventHandle  # mooncake-ep/include/mooncake_ep_event.h:9-44
 EventOverlapBase, register_overlap = _native.EventOverlapBase, _native.register_overlap
+register_handle = _native.register_handle
 
 
 class Buffer(_native.Runtime):

@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from . import ep
-from .mooncake_ep_buffer import EventOverlap, _DeviceBytes, _stream_ptr
+from .mooncake_ep_buffer import EventOverlap, _DeviceBytes, _stream_ptr  # noqa: F401  (calls return EventOverlap)
 
 
 class EPHandle:
@@ -64,12 +64,8 @@ class EPHandle:
         # without a CPU sync an upper bound, after one the number of rows received (:79-81)
         self.num_recv_tokens = int(recv_src_metadata.shape[0])
 
-    @classmethod
-    def _of(cls, **fields) -> "EPHandle":
-        """A handle made of all its fields at once (half the time of the constructor)."""
-        handle = cls.__new__(cls)
-        handle.__dict__ = fields
-        return handle
+
+ep.register_handle(EPHandle)
 
 
 class ElasticBuffer:
@@ -243,33 +239,18 @@ class ElasticBuffer:
             num_max_tokens_per_rank = self.num_max_tokens_per_rank or x.shape[0]
         if num_sms is None:
             num_sms = self._num_sms or self.get_theoretical_num_sms(num_experts, topk_idx.shape[1])
-        active_ranks = self._active_ranks(x.device)
         # the handle keeps its own copy of the routing, as the reference's does (:679), written by
         # the call's kernels; a cached handle's is used again
         out = self.runtime.elastic_dispatch_tensors(
-            x, topk_idx, topk_weights, active_ranks, None if handle is None else handle.topk_idx, num_experts,
-            num_max_tokens_per_rank, expert_alignment, do_expand, do_cpu_sync, self._timeout_us(),
-            async_with_compute_stream, self._rows_in_place if self.recv_in_place else None)
+            x, topk_idx, topk_weights, self._active_ranks(x.device), None if handle is None else handle.topk_idx,
+            num_experts, num_max_tokens_per_rank, expert_alignment, do_expand, do_cpu_sync, self._timeout_us(),
+            async_with_compute_stream, self._rows_in_place if self.recv_in_place else None, num_sms)
         if out is None:
             assert x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16
             assert topk_idx.dtype == torch.int64 and topk_idx.is_contiguous()
             assert topk_weights is None or (topk_weights.dtype == torch.float32 and topk_weights.is_contiguous())
             raise AssertionError("dispatch takes CUDA tensors: x [T, H], T * K entries of topk_idx and topk_weights")
-        (recv_x, recv_topk_idx, recv_topk_weights, recv_src_metadata, psum_rank, psum_expert, dst_buffer_slot_idx,
-         kept_idx, counts, event) = out
-        out_handle = EPHandle._of(
-            do_expand=do_expand, num_experts=num_experts, expert_alignment=expert_alignment,
-            num_max_tokens_per_rank=num_max_tokens_per_rank, num_sms=num_sms, topk_idx=kept_idx,
-            psum_num_recv_tokens_per_scaleup_rank=psum_rank, psum_num_recv_tokens_per_expert=psum_expert,
-            num_recv_tokens_per_expert_list=counts or [], recv_src_metadata=recv_src_metadata,
-            dst_buffer_slot_idx=dst_buffer_slot_idx, token_metadata_at_forward=None, channel_linked_list=None,
-            native_handle=True, num_recv_tokens=recv_src_metadata.size(0))
-        keep = None
-        if async_with_compute_stream:
-            keep = (x, topk_idx, kept_idx, active_ranks, recv_x, recv_topk_idx, psum_rank, psum_expert,
-                    recv_src_metadata, dst_buffer_slot_idx) + \
-                (() if topk_weights is None else (topk_weights, recv_topk_weights))
-        return recv_x, recv_topk_idx, recv_topk_weights, out_handle, EventOverlap(event, keep)
+        return out
 
     # ------------------------------------------------------------------ combine
     def combine(self, x: torch.Tensor, handle: EPHandle, topk_weights: Optional[torch.Tensor] = None,
@@ -282,15 +263,9 @@ class ElasticBuffer:
         if handle.do_expand and topk_weights is not None:
             # the reference asserts the same on the device (combine_official.cuh:70)
             raise AssertionError("topk_weights must be None with an expanded layout")
-        active_ranks = self._active_ranks(x.device)
         res = self.runtime.elastic_combine_tensors(
             x, handle.topk_idx, topk_weights, handle.psum_num_recv_tokens_per_scaleup_rank, handle.recv_src_metadata,
-            active_ranks, handle.num_experts, handle.num_max_tokens_per_rank, handle.do_expand, self._timeout_us(),
-            async_with_compute_stream)
+            self._active_ranks(x.device), handle.num_experts, handle.num_max_tokens_per_rank, handle.do_expand,
+            self._timeout_us(), async_with_compute_stream)
         assert res is not None, "combine takes a contiguous [n, H] bf16 CUDA tensor (and topk_weights as a tensor)"
-        combined_x, event = res
-        keep = None
-        if async_with_compute_stream:
-            keep = (x, active_ranks, combined_x, handle.topk_idx, handle.recv_src_metadata) + \
-                (() if topk_weights is None else (topk_weights,))
-        return combined_x, None, EventOverlap(event, keep)
+        return res
