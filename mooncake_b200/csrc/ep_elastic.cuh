@@ -99,11 +99,6 @@ struct ElasticSingleParams {
     int T, K, E, H, alignment;
     int C;                       // tokens per block of the copy kernel, and behind a layout kernel
     int warps_per_row, parts;    // the warps and the blocks that share a row (set by the launcher)
-    RouteBits bits;              // behind a layout kernel: row 0 all tokens that name an expert, 1 + e (expanded)
-                                 // those that name e
-    uint16_t* hits;              // [E][bits.stride] listings per chunk
-    int32_t* starts;             // [E + 1] expanded: where the experts' segments start
-    unsigned* ticket;            // expanded: chunks that are done
     int max_rows;                // expanded: rows recv_x has room for
     int32_t* status;
     int32_t* rows;               // kept for combine: [T] received row of the token, or (expanded) [T][K] row
@@ -121,6 +116,11 @@ struct ElasticSingleParams {
     // [0] flag (host_seq once the rest is there), [1] received rows, [2..] psum_expert
     int32_t* host_counts;
     int32_t host_seq;
+    RouteBits bits;              // behind a layout kernel: row 0 all tokens that name an expert, 1 + e (expanded)
+                                 // those that name e
+    uint16_t* hits;              // [E][bits.stride] listings per chunk
+    int32_t* starts;             // [E + 1] expanded: where the experts' segments start
+    unsigned* ticket;            // expanded: chunks that are done
 };
 // The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
 struct SingleTables {

@@ -549,13 +549,12 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
     __shared__ int s_pos[kEntries];  // received row of token c
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int K = p.K, nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    for (int i = tid; i < (kExpand ? 2 * p.E + 1 : p.E + 1); i += nthr) smem_i32[i] = 0;
+    __syncthreads();
     pdl_wait();
     pdl_launch_dependents();
     if (blockIdx.x == 0) {  // the counts
-        for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
         int* rows = smem_i32 + p.E + 1;
-        if (kExpand)
-            for (int i = tid; i < p.E; i += nthr) rows[i] = 0;
         const int n = sent_before(p, p.T);
         __syncthreads();
         count_hits(p, smem_i32);
@@ -604,9 +603,6 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
     }
     if (kExpand) {
         int* before = smem_i32 + p.E + 1;
-        for (int i = tid; i <= p.E; i += nthr) smem_i32[i] = 0;
-        for (int i = tid; i < p.E; i += nthr) before[i] = 0;
-        __syncthreads();
         count_hits(p, smem_i32);
         count_tokens<1, true>(p.topk_idx, 0, t0, K, p.E, choices_in_pairs(p.topk_idx, K), before);
         __syncthreads();

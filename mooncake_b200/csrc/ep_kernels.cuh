@@ -65,13 +65,9 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx);
 struct DirectDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
-    RouteBits bits;             // from the layout kernel (words null: none), or
-    const int32_t* slot;        // [T*K] from another layout kernel, or null: counted in the send kernel
     int T, K, E, M, H;
     int use_fp8;
     int C;                      // counting: tokens per batch (set by the launcher)
-    int warps_per_row, tokens_per_block, parts;  // else: how a block's warps are dealt out, blocks that share a row
-                                                 // (set by the launcher)
     int32_t* status;
     void* recv_x;
     float* recv_scales;
@@ -79,6 +75,12 @@ struct DirectDispatchParams {
     int32_t* recv_count;        // [E], written without `slot`
     int64_t* layout_range;      // [E], written without `slot`
     int32_t* rowmap;            // [T*K] row of (token, k) inside its expert, kept for combine
+    // Positions from the layout kernel (words null: none), or from another one; neither: they
+    // are counted in the send kernel. (Last, so that what a counting kernel reads lies together.)
+    RouteBits bits;
+    const int32_t* slot;        // [T*K]
+    int warps_per_row, tokens_per_block, parts;  // with positions: how a block's warps are dealt out, blocks that
+                                                 // share a row (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 // whether the send kernels count the slots themselves for this many tokens
@@ -109,8 +111,8 @@ struct DirectCombineParams {
     const int32_t* rowmap;
     int absolute;               // rowmap names rows of the whole tensor, which has M of them (-1: none), every
                                 // weight is 1; topk_idx and topk_weights are not read
-    int tokens_per_block, tiles_per_block, span;  // set by the launcher (span: tokens a block works through)
-    int backward;               // set by the launcher: the last tokens first
+    int tokens_per_block, tiles_per_block, span;  // set by the launcher (span: tokens a block works through, < 0:
+                                                  // the last ones of the batch first)
     // search: no rowmap; rows are looked up in the handle by the kernel
     int search;
     const int32_t* src_info;
@@ -145,9 +147,8 @@ struct WaitCfg {
 struct GroupDispatchParams {
     const void* x;              // [T][H] bf16
     const int64_t* topk_idx;    // [T][K]
-    RouteBits bits;             // from the layout kernel (words null: none), or
     const int32_t* slot;        // [T*K] and
-    const int32_t* count;       // [E] from another layout kernel, or null: counted in the send kernel
+    const int32_t* count;       // [E] from a layout kernel, or null: `bits`, or counted in the send kernel
     void* const* peer_base;     // [R] base of every rank's symmetric buffer
     char* local_base;           // this rank's
     int T, K, E, R, M, H, rank;
@@ -172,6 +173,7 @@ struct GroupDispatchParams {
     int32_t* recv_count;        // [L]
     int64_t* layout_range;      // [L][R]
     int copy_rows;              // recv_x is a tensor of the caller's: copy the rows out
+    RouteBits bits;             // from the layout kernel (words null: none)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms);
