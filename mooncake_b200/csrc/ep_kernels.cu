@@ -2139,22 +2139,25 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
                   ctx, p, epc, words);
 }
 
-bool counts_in_send_kernel(int T, int K, int row_bytes, int num_sms, bool group) {
+bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group) {
     // A group's sender blocks are one resident wave, a token each (one rank on this path,
     // us per layer, counting | layout kernel: rows of 8 KB in bf16 to 8, 200 tokens 17.6 |
     // 17.2, 290 19.0 | 18.4, 400 30.8 | 26.4; of 7 KB in FP8, 290 23.9 | 26.9).
     if (group) return T <= 2 * num_sms;
     // A single rank counts in one resident wave of blocks with as many tokens each as that
-    // takes. Up to two choices per token that is as good as a layout kernel (us per layer,
-    // counting | layout kernel, rows of 8 KB to 2: 1000 tokens 14.6 | 14.4, 4000 39.2 | 38.3;
-    // in FP8 35.7 | 36.2; of 14 KB to 1, 4000 44.3 | 48.0) and saves a launch.
-    if (K <= 2) return T <= 8192 / K;
-    // From three on the layout kernel is the faster one on the device at every size (rows
-    // of 14 KB to 8: 160 tokens 15.2 | 13.8, 300 24.8 | 21.1, 590 32.6 | 31.7; of 4 KB in FP8
-    // to 8: 200 10.0 | 9.6, 400 16.3 | 14.9, 590 20.8 | 20.0; of 4 KB to 4, 590 9.1 | 8.5), but
-    // a layer of three launches takes the host 12.5 us and one of two 10: it is used where
-    // the rows are more than the device moves in that time.
-    return T <= num_sms || (T <= 4 * num_sms && (long long)T * K * row_bytes < 12 << 20);
+    // takes. The layout kernel is the faster one on the device at nearly every size, but a
+    // layer of three launches takes the host 12.4 us and one of two 10: it is used where the
+    // rows, in either type, are more than the device moves in that time. Up to two choices per
+    // token (us per layer, counting | layout kernel): rows of 8 KB to 2, 600 tokens (10 MB) 10.6 |
+    // 12.4, 1000 (16 MB) 14.3 | 14.2, in FP8 13.9 | 12.7, 4000 38.9 | 37.1; of 2 KB 2000 (8 MB) 10.3 |
+    // 12.3, 4000 16.3 | 14.3; of 14 KB to 1, 600 (9 MB) 11.3 | 12.4, 1000 16.1 | 15.5, 4000 44.2 |
+    // 41.7 (8000 in FP8 alone lose, 76.9 | 78.0).
+    const long long bytes = (long long)T * K * H * 2;
+    if (K <= 2) return bytes < 12 << 20 && T <= 8192 / K;
+    // From three on counting is slower by block: rows of 8 KB to 8 in FP8, 200 tokens (13 MB)
+    // 10.0 | 12.4, 300 (20 MB) 13.5 | 12.4, 400 16.3 | 14.9; of 14 KB in bf16, 160 (18 MB) 15.2 |
+    // 13.8, 300 24.8 | 21.1, 590 32.6 | 31.7; of 4 KB to 4, 590 (10 MB) 10.0 | 12.4.
+    return T <= num_sms || (T <= 4 * num_sms && bytes < 17 << 20);
 }
 
 // Tokens per batch and threads per block of the kernels that work through batches.
@@ -2189,6 +2192,10 @@ cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx)
             // two tiles | one: 4096 rows of 14 KB to 3 68.5 | 73.0, to 4 82.4 | 85.5, to 8 145.9 |
             // 145.8; 4000 of 4 KB to 4 29.2 | 29.8; 1500 of 8 KB to 8 37.6 | 36.5
             if (p.K <= 4 && ntiles >= 4) k = ep_dispatch_rows_kernel<true, 2, 4, 10>, tiles = 2, most = 4;
+        } else if (p.K == 1 ? ntiles >= 4 : p.K == 2 && ntiles > 8) {
+            // two tiles | one: 8000 rows of 14 KB to 1 76.3 | 86.1, 1000 of 8 KB 10.1 | 11.0; 4000 of
+            // 14 KB to 2 59.0 | 60.0, 2000 of 8 KB 22.5 | 22.1; to 3 1500 of 8 KB 22.2 | 21.8
+            k = ep_dispatch_rows_kernel<false, 2, 4, 10>, tiles = 2, most = 4;
         } else if ((long long)p.T * p.K * p.H * 2 < 256 << 20) {
             // 42 warps per SM | 32: to 3, 4096 rows of 14 KB (168 MB) 78.4 | 79.8; to 4 (224 MB) 97.4 |
             // 97.2, to 6 135.8 | 135.5, to 8 174.7 | 173.7
@@ -2381,13 +2388,14 @@ cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const Laun
 }
 
 cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx) {
-    // Rows of 8 tiles and more (one rank on this path, us per layer with it | without; 2000
-    // tokens of 4 tiles to 4, the kernel alone 10.1 | 9.0): 8 tiles to 8, 2000 tokens 63.9 |
-    // 69.7, 1024 38.9 | 38.9, 600 30.0 | 28.6, 300 25.6 | 24.5, to 2 2000 32.7 | 33.4; 10
-    // tiles 2000 78.1 | 95.3, 1024 46.2 | 50.4, 300 25.5 | 25.5; 14 tiles 2000 103.8 | 115.8,
-    // 600 39.9 | 40.8, 300 28.2 | 28.6; 16 tiles 1024 63.2 | 71.4. At 8 tiles alone the line
-    // lies too low for fewer than about 1000 tokens.
-    if (p.T > ctx.num_sms && p.H >= 8 * kTileChannels) {
+    // Rows of 8 tiles and more, once a block would have several tokens (one rank on this path,
+    // us per layer with it | without). 4 tiles: 300 tokens to 8 21.1 | 18.5, 1500 32.8 | 29.9. 8
+    // tiles: to 2 300 17.2 | 16.5, 600 18.8 | 18.9, 2000 32.5 | 33.2; to 4 600 22.3 | 22.0, 1000 26.7 |
+    // 27.0; to 8 300 24.1 | 22.0, 1000 36.5 | 35.6, 1500 49.2 | 51.6. 14 tiles: to 2 300 18.6 | 18.9,
+    // 400 20.0 | 19.9, 600 24.8 | 25.9; to 8 300 27.5 | 27.3, 400 30.7 | 29.8, 600 38.5 | 39.5, 2000
+    // 100 | 111.
+    const int tiles = (p.H + kTileChannels - 1) / kTileChannels;
+    if (p.T > (tiles > 8 ? 3 : 2 + p.K) * ctx.num_sms && p.H >= 8 * kTileChannels) {
         const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
         p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
         return launch("ep_combine_reduce", ep_combine_gather_kernel<4>, shape.grid, dim3(shape.threads), 0, ctx, p);

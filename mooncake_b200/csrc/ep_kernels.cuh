@@ -84,7 +84,7 @@ struct DirectDispatchParams {
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 // whether the send kernels count the slots themselves for this many tokens
-bool counts_in_send_kernel(int T, int K, int row_bytes, int num_sms, bool group);
+bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group);
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
 
 struct SendShape {

@@ -924,8 +924,8 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
     // Larger batches get their layout from a kernel of its own.
-    const bool counting = (b->fuse_layout || T == 0) && 
-                          mcep::counts_in_send_kernel(T, K, g.row_bytes, b->num_sms, group);
+    const bool counting = (b->fuse_layout || T == 0) &&
+                          mcep::counts_in_send_kernel(T, K, H, b->num_sms, group);
     mcep::RouteBits bits = {};
     if (!counting) {
         mcep::LayoutParams lp = {};
