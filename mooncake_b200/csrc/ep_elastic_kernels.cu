@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
         raw = ld_ro(p.topk_idx + (size_t)t0 * K + tid);
         if (p.topk_weights) w = ld_ro(p.topk_weights + (size_t)t0 * K + tid);
     }
-    const int e = all_bits(raw) < p.E ? all_bits(raw) : -1;
+    const int e = (uint64_t)raw < (uint64_t)p.E ? (int)raw : -1;
     if (tid < ne) s_exp[tid] = e;
     __syncthreads();
     int pos = sent_before(p, t0);

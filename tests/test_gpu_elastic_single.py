@@ -160,6 +160,21 @@ def test_all_64_bits_of_an_entry_decide(T, K, expand):
     assert torch.equal(out.cpu().view(torch.int16), ref.view(torch.int16))
 
 
+@pytest.mark.parametrize("T,expand", [(40, False), (40, True), (700, False), (700, True)])
+def test_entries_beyond_31_bits_name_no_expert(T, expand):
+    """An entry whose low half is negative as 32 bits is received as -1, like any other that names no expert."""
+    H, E, K = 128, 8, 3
+    x, idx, w = make_rank_inputs(15, 0, T, H, E, K)
+    idx[::2, 1] = torch.tensor([2147483651, 4294967291, 2147483648, 4294967294, -5]).repeat(T)[:T // 2]
+    want = eo.elastic_dispatch([x], [idx], [w], E, T, 1, expand)[0]
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=T, hidden=H, num_topk=K)
+    recv, ridx, _, h, _ = buf.dispatch(x.cuda(), topk_idx=idx.cuda(), topk_weights=w.cuda(), num_experts=E,
+                                       num_max_tokens_per_rank=T, do_expand=expand)
+    assert torch.equal(ridx.cpu(), want["recv_topk_idx"]) and bool((ridx[:, 1] < 0).any())
+    assert h.num_recv_tokens_per_expert_list == want["hits"]
+    assert torch.equal(recv.cpu().view(torch.int16), want["recv_x"].view(torch.int16))
+
+
 def test_shapes_of_the_routing_are_the_callers():
     """T * K entries of topk_idx and topk_weights are read, whatever their shapes: flat weights,
     matrices made for the largest batch, a trailing dimension of one."""
