@@ -433,8 +433,8 @@ int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const 
     mcep::SingleTables tables;
     const mcep::LayoutScratch scratch = mcep::next_layout_scratch(b);
     if (!v.group && !v.defer &&
-        mcep::elastic_single_tables(T, K, E, a->do_expand != 0, v.num_sms, scratch.memory, scratch.bytes,
-                                    scratch.ticket, &tables))
+        mcep::elastic_single_tables(T, K, E, a->do_expand != 0, counts != nullptr, v.num_sms, scratch.memory,
+                                    scratch.bytes, scratch.ticket, &tables))
         return single_dispatch(b, s, v, a, tables, counts, out_event);
     EL_REQUIRE(counts == nullptr || !v.defer);
     const size_t rec_want = record_bytes(R, M, K);

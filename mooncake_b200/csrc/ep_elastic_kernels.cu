@@ -808,20 +808,25 @@ cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int n
 }
 
 namespace {
-// One launch. Flat rows: up to 4096 choices and seven tokens per SM, in one resident wave
-// (us per layer: 500 tokens of 14 KB to 8 10.3, behind a layout kernel 12.5; 1000 of 8 KB
-// to 2 10.2 against 11.5; 700 to 8 11.2 against 10.6, 2000 to 2 14.3 against 14.2).
-// Expanded rows, where every block counts all choices, up to two tokens per SM.
-bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand) {
-    return expand ? T <= 2 * num_sms : T * K <= 4096 && T <= 7 * num_sms;
+// One launch saves the host 2 us of 16, which most of these calls are bound by, and costs the
+// device up to 2. Flat rows, up to seven tokens per SM in one resident wave (the layer, wall |
+// device, counting and behind a layout kernel: 400 tokens of 8 KB to 8 14.5 | 7.7 and 16.4 | 7.4,
+// 1000 14.7 | 11.1 and 16.6 | 8.8, of 14 KB 14.2 | 13.2 and 16.4 | 11.2); a call whose host waits
+// for the counts (`waits`) gets them later, so up to 4096 choices there (1000 to 8: 30.4 - 32.0 and
+// 28.8 - 29.7). Expanded rows, where every block counts all choices: two tokens per SM, to four
+// while they are 16 choices (a call that waits: 400 to 2 25.1 and 26.9, 390 to 6 26.4 and 28.5, 500
+// to 8 28.5 and 27.7).
+bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand, bool waits) {
+    if (expand) return T <= 2 * num_sms || (T <= 4 * num_sms && T * K <= 16 * num_sms);
+    return T <= 7 * num_sms && T * K <= (waits ? 4096 : 8 * 7 * num_sms);
 }
 }  // namespace
 
-bool elastic_single_tables(int T, int K, int E, bool expand, int num_sms, void* scratch, size_t bytes, unsigned* ticket,
-                           SingleTables* tables) {
+bool elastic_single_tables(int T, int K, int E, bool expand, bool waits, int num_sms, void* scratch, size_t bytes,
+                           unsigned* ticket, SingleTables* tables) {
     *tables = SingleTables();
     if (K > kMaxTopk || E > kMaxExperts) return false;
-    if (counts_in_copy_kernel(T, K, num_sms, expand)) return true;
+    if (counts_in_copy_kernel(T, K, num_sms, expand, waits)) return true;
     const size_t starts = ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
     const size_t hits = (size_t)E * (((T + kChunkTokens - 1) / kChunkTokens + 15) / 16 * 16) * sizeof(uint16_t);
     if (starts + hits > bytes) return false;

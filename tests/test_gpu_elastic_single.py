@@ -76,6 +76,13 @@ def test_layout_in_bits(T, H, E, K, expand, alignment):
     test_dispatch_and_combine(T, H, E, K, expand, alignment)
 
 
+@pytest.mark.parametrize("T,H,E,K,expand,alignment", [  # either side of where the counting in the copy kernel ends
+    (1036, 640, 64, 8, False, 1), (1036, 128, 32, 9, False, 1), (592, 640, 16, 4, True, 2), (593, 128, 16, 4, True, 1),
+    (395, 128, 16, 6, True, 1), (394, 1152, 16, 6, True, 4)])
+def test_either_side_of_the_counting_limit(T, H, E, K, expand, alignment):
+    test_dispatch_and_combine(T, H, E, K, expand, alignment)
+
+
 def test_a_repeat_has_its_expanded_row_at_its_last_listing():
     """An expert listed twice takes two rows of its segment and fills one; the first listing names none."""
     T, H, E, K = 700, 1152, 8, 3
