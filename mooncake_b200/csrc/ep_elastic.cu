@@ -129,6 +129,10 @@ struct ElasticState {
     size_t single_entries = 0, single_tokens = 0;
     int32_t* single_rows[2] = {};
     int32_t* single_pos = nullptr;
+    // per parity [MCEP_MAX_EXPERTS]: filled by the layout kernel of a call and cleared by whoever
+    // reads them; `totals_left`: a call failed between the two
+    unsigned long long* single_totals = nullptr;
+    bool totals_left = false;
     int32_t* host_counts = nullptr;
     uint32_t host_seq = 0;
     uint64_t clock = 0;
@@ -206,6 +210,8 @@ int ensure(ElasticState* s, const mcep::BufferView& v, int M, int K, int L, int 
     return MCEP_OK;
 }
 
+constexpr size_t kTotalsBytes = (size_t)MCEP_MAX_EXPERTS * sizeof(unsigned long long);
+
 // Scratch of the single-rank path.
 int ensure_single(ElasticState* s, int M, int K) {
     const size_t entries = (size_t)M * K, tokens = (size_t)M;
@@ -216,10 +222,16 @@ int ensure_single(ElasticState* s, int M, int K) {
     s->single_entries = entries > s->single_entries ? entries : s->single_entries;
     s->single_tokens = tokens > s->single_tokens ? tokens : s->single_tokens;
     const size_t rows = up(s->single_entries * 4 + 4, 256), pos = up(s->single_tokens * 4 + 4, 256);
-    EL_CUDA(cudaMalloc(&s->single_blob, 2 * rows + pos));
-    s->single_rows[0] = reinterpret_cast<int32_t*>(s->single_blob);
-    s->single_rows[1] = reinterpret_cast<int32_t*>(s->single_blob + rows);
-    s->single_pos = reinterpret_cast<int32_t*>(s->single_blob + 2 * rows);
+    EL_CUDA(cudaMalloc(&s->single_blob, 2 * kTotalsBytes + 2 * rows + pos));
+    char* at = s->single_blob + 2 * kTotalsBytes;
+    s->single_totals = reinterpret_cast<unsigned long long*>(s->single_blob);
+    s->totals_left = true;
+    s->single_rows[0] = reinterpret_cast<int32_t*>(at);
+    s->single_rows[1] = reinterpret_cast<int32_t*>(at + rows);
+    s->single_pos = reinterpret_cast<int32_t*>(at + 2 * rows);
+    EL_CUDA(cudaMemset(s->single_totals, 0, 2 * kTotalsBytes));
+    EL_CUDA(cudaDeviceSynchronize());  // (streams that do not wait for the default one)
+    s->totals_left = false;
     for (auto& r : s->rec)
         if (r.single) r = ElasticState::Record();
     if (!s->ev) EL_CUDA(cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming));
@@ -342,7 +354,16 @@ int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, 
     if (counts) p.host_counts = s->host_counts, p.host_seq = (int32_t)++s->host_seq;
     const bool chain = mcep::may_chain(b, stream);
     mcep::LaunchCtx ctx{stream, v.num_sms, chain && !async, chain};
-    EL_CUDA(mcep::launch_elastic_single_dispatch(p, expand, tables, ctx));
+    if (tables.bits.words != nullptr) {
+        p.totals = s->single_totals + (size_t)par * MCEP_MAX_EXPERTS;
+        if (s->totals_left) EL_CUDA(cudaMemsetAsync(s->single_totals, 0, 2 * kTotalsBytes, stream));
+    }
+    if (cudaError_t e = mcep::launch_elastic_single_dispatch(p, expand, tables, ctx); e != cudaSuccess) {
+        s->totals_left = true;
+        EL_CUDA(e);
+    }
+    // (nothing that is being captured has run)
+    if (s->totals_left && tables.bits.words != nullptr && chain) s->totals_left = false;
     mcep::count_dispatch_call(b);
     auto& rec = s->rec[par];
     rec.key = a->recv_src_metadata, rec.par = par, rec.T = T, rec.K = K, rec.E = E, rec.M = M, rec.H = H;

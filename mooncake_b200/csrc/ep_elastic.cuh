@@ -118,14 +118,13 @@ struct ElasticSingleParams {
     int32_t host_seq;
     RouteBits bits;              // behind a layout kernel: row 0 all tokens that name an expert, 1 + e (expanded)
                                  // those that name e
-    uint16_t* hits;              // [E][bits.stride] listings per chunk
+    unsigned long long* totals;  // [E] listings and rows of the experts, zero between calls
     int32_t* starts;             // [E + 1] expanded: where the experts' segments start
     unsigned* ticket;            // expanded: chunks that are done
 };
 // The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
 struct SingleTables {
     RouteBits bits = {};
-    uint16_t* hits = nullptr;
     int32_t* starts = nullptr;
     unsigned* ticket = nullptr;
 };

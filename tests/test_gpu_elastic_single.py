@@ -71,7 +71,8 @@ def test_dispatch_and_combine(T, H, E, K, expand, alignment):
 
 @pytest.mark.parametrize("T,H,E,K,expand,alignment", [  # words, chunks and loads of counts; rows of odd tiles and parts
     (16384, 128, 8, 2, True, 1), (16384, 128, 300, 1, False, 3), (4225, 640, 24, 5, True, 8), (4224, 1152, 9, 7, False, 1),
-    (1153, 4224, 8, 3, True, 2), (2049, 8320, 8, 2, False, 1), (384, 128, 4096, 4, True, 1)])
+    (1153, 4224, 8, 3, True, 2), (2049, 8320, 8, 2, False, 1), (384, 128, 4096, 4, True, 1),
+    (1500, 128, 2048, 8, True, 1), (4000, 256, 1025, 2, False, 2)])
 def test_layout_in_bits(T, H, E, K, expand, alignment):
     test_dispatch_and_combine(T, H, E, K, expand, alignment)
 
@@ -117,6 +118,47 @@ def test_counts_of_back_to_back_calls_and_an_empty_batch():
         assert out.shape == (T, H) and not bool(out.any())
     recv, _, _, h, _ = buf.dispatch(x[:0], topk_idx=idx[:0].cuda(), num_experts=E, num_max_tokens_per_rank=T)
     assert recv.shape == (0, H) and h.num_recv_tokens_per_expert_list == [0] * E
+
+
+@pytest.mark.parametrize("E", [8, 129, 4096])
+def test_totals_of_one_call_are_not_in_the_next(E):
+    """Counts behind a layout kernel, call after call of one buffer: batches, layouts and waits
+    in turn, and a captured pair of calls replayed in between."""
+    M, H, K = 2600, 128, 3
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K)
+    x = torch.randn((M, H), device="cuda").to(torch.bfloat16)
+    _, idx, _ = make_rank_inputs(43, 0, M, H, E, K, "zipf1.2", n_mask=M // 9)
+    idx[::7, 0] = idx[::7, 2]
+    di = idx.cuda()
+
+    def call(T, expand, sync, shift):
+        h = buf.dispatch(x[:T], topk_idx=di[shift:shift + T], num_experts=E, num_max_tokens_per_rank=M,
+                         do_expand=expand, do_cpu_sync=sync)[3]
+        return h, idx[shift:shift + T], expand
+
+    def check(h, chosen, expand):
+        chosen = torch.where(chosen < 0, E, chosen)
+        hits = torch.bincount(chosen.reshape(-1), minlength=E + 1)[:E]
+        once = (chosen.unsqueeze(2) == torch.arange(E)).any(dim=1).sum(0)
+        want = torch.cumsum(hits, 0) - hits + once if expand else torch.cumsum(hits, 0)
+        assert torch.equal(h.psum_num_recv_tokens_per_expert.cpu()[:E].long(), want)
+        assert h.psum_num_recv_tokens_per_scaleup_rank.tolist() == [int((chosen < E).any(dim=1).sum())]
+
+    def calls():
+        return [call(T, expand, sync, 2600 - T) for T, expand, sync in (
+            (2600, False, True), (1500, True, False), (2100, True, True), (1100, False, False), (2600, True, False),
+            (1037, False, True), (1290, False, False))]
+
+    for got in calls():
+        check(*got)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        captured = [call(2000, False, False, 77), call(1111, True, False, 200)]
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        for got in captured + calls():
+            check(*got)
 
 
 @pytest.mark.parametrize("body", ["_first_call_inside_a_failed_capture", "_launch_that_fails"])
