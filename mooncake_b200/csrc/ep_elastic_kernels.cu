@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSi
     for (int x = tid; x < rows; x += kBitsThreads) {
         const uint4 m = smem_u128[x];
         const int n = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
-        p.bits.words[(size_t)x * p.bits.chunks + blockIdx.x] = m;
+        p.bits.words[(size_t)blockIdx.x * p.bits.experts + x] = m;
         p.bits.counts[(size_t)x * p.bits.stride + blockIdx.x] = (uint8_t)n;
         if (kExpand && x > 0) add_hits(p, x - 1, n + extra[x - 1], n);
     }

@@ -684,11 +684,13 @@ __global__ void __launch_bounds__(1024) ep_layout_cluster_kernel(LayoutParams p)
 // ---- the layout as bits, for kernels that look positions up themselves -------------
 // What dispatch uses between the smallest and the largest batches. Every chunk of 128
 // tokens is a block of its own and nothing is summed here: per expert the chunk's bits
-// (RouteBits) and their number, one load, one store. A sender finds its position from them
-// in one round trip more than it would read a finished one (bits_before), but a finished
-// one costs a cluster barrier, remote totals and a prefix over all experts before it
-// exists: from the kernel's start to its end 5.7 us for 2001 tokens to 8 of 128, 9.3 for
-// 4096 to 8 of 256; here 2.4 and 2.
+// (RouteBits) and their number, one load, one store. A block's words lie together: what a warp
+// stores is four lines, as [expert][chunk] it was 32 (elastic calls, the layer: 4096 rows of
+// 4 KB expanded to 8 of 512 55.9 us, now 54.5, to 2 of 2048 34.8, now 30.5). A sender finds
+// its position from them in one round trip more than it would read a finished one
+// (bits_before), but a finished one costs a cluster barrier, remote totals and a prefix over
+// all experts before it exists: from the kernel's start to its end 5.7 us for 2001 tokens to 8
+// of 128, 9.3 for 4096 to 8 of 256; here 2.4 and 2.
 constexpr int kBitsThreads = 256;
 
 template <int KB>
@@ -721,7 +723,7 @@ __global__ void __launch_bounds__(kBitsThreads) ep_layout_bits_kernel(LayoutPara
     __syncthreads();
     for (int e = tid; e < p.E; e += kBitsThreads) {
         const uint4 m = smem_u128[e];
-        p.bits.words[(size_t)e * p.bits.chunks + blockIdx.x] = m;
+        p.bits.words[(size_t)blockIdx.x * p.bits.experts + e] = m;
         p.bits.counts[(size_t)e * p.bits.stride + blockIdx.x] =
             (uint8_t)(__popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w));
     }
@@ -2079,7 +2081,7 @@ RouteBits route_bits(void* memory, size_t capacity, int T, int E) {
     if (chunks < 1 || chunks > 128 || (size_t)E * (chunks * sizeof(uint4) + stride) > capacity) return b;
     b.words = static_cast<uint4*>(memory);
     b.counts = reinterpret_cast<uint8_t*>(b.words + (size_t)E * chunks);
-    b.chunks = chunks, b.stride = stride;
+    b.experts = E, b.chunks = chunks, b.stride = stride;
     return b;
 }
 

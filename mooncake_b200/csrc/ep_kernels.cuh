@@ -35,9 +35,9 @@ struct LaunchCtx {
 // and of the lower bits of its own (bits_before, ep_routing.cuh).
 constexpr int kChunkTokens = 128;
 struct RouteBits {
-    uint4* words;     // [E][chunks], bit t % 128 of chunk t / 128; null: not there
-    uint8_t* counts;  // [E][stride], padding undefined
-    int chunks, stride;
+    uint4* words;     // [chunks][experts], bit t % 128 of chunk t / 128; null: not there
+    uint8_t* counts;  // [experts][stride], padding undefined
+    int experts, chunks, stride;
 };
 // Such bits in `capacity` bytes at `memory` (256-byte aligned); words null where they do
 // not fit or where the batch has more than 128 chunks.

@@ -134,7 +134,7 @@ __device__ __forceinline__ int sum_counts(const uint8_t* row, int n) {
 // Tokens before t that chose expert e.
 __device__ __forceinline__ int bits_before(const RouteBits& b, int e, int t) {
     const int chunk = t / kChunkTokens, bit = t % kChunkTokens;
-    const uint4 v = ld_ro(b.words + (size_t)e * b.chunks + chunk);
+    const uint4 v = ld_ro(b.words + (size_t)chunk * b.experts + e);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     int n = sum_counts<false>(b.counts + (size_t)e * b.stride, chunk);
 #pragma unroll
