@@ -975,6 +975,19 @@ __global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectD
     send_tokens<kFP8, false, true>(v, blockIdx.x, gridDim.x, smem_i32);
 }
 
+// The counts of a batch whose layout is there as bits; whole block. The first block does it once
+// its own rows are out and the others hide it; the last one, an expert per thread ahead of its
+// rows, was waited for (the layer: 885 rows of 11 KB to 2 of 512 14.6 us, now 13.4; 3539 of 256
+// bytes in FP8 to 8 of 2048 28.8, now 23.7; a block of its own ahead of the rows costs 0.4 at few
+// choices, 1000 rows of 14 KB to 2 15.4 against 14.7). Not inlined: what it keeps in registers is
+// not taken from the rows' warps (inlined, 16 bytes are spilled: 1000 rows to 4 22.4, now 21.6).
+__device__ __noinline__ void write_counts(RouteBits bits, int E, int32_t* recv_count, int64_t* layout_range) {
+    bits_totals<4>(bits, E, [&](int x, int n) {
+        recv_count[x] = n;
+        layout_range[x] = n;  // begin 0 | count
+    });
+}
+
 // Single rank, behind a layout kernel: a warp owns one tile of one token and needs no
 // other: lane k finds the token's k-th row, the tile goes to each. Nothing is shared and
 // nobody waits at a barrier. Blocks are small because it is the turnover of independent
@@ -1013,13 +1026,6 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks)
     }
     if (mine) e = (int)ld_ro(p.topk_idx + (size_t)t * K + lane);
     pdl_wait();
-    if (p.bits.words != nullptr && blockIdx.x == gridDim.x - 1) {
-        for (int x = threadIdx.x; x < p.E; x += blockDim.x) {
-            const int n = bits_total(p.bits, x);
-            p.recv_count[x] = n;
-            p.layout_range[x] = n;  // begin 0 | count
-        }
-    }
     // (a repeated expert has the same row and gets the same bytes twice)
     int s = -1;
     if (p.bits.words != nullptr) {
@@ -1072,6 +1078,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks)
             }
         }
     }
+    if (p.bits.words != nullptr && blockIdx.x == 0) write_counts(p.bits, p.E, p.recv_count, p.layout_range);
 }
 
 // Single rank: rowmap[t][k] = packed row of (token t, expert topk[t][k]) as the
@@ -1573,9 +1580,10 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     if (bid == 0) {  // the counts do not wait for the peer tables (0.8 us)
         if (kCount) {
             count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
+        } else if (p.bits.words != nullptr) {
+            bits_totals<4>(p.bits, p.E, [&](int i, int n) { smem_i32[i] = n; });
         } else {
-            for (int i = tid; i < p.E; i += nthr)
-                smem_i32[i] = p.bits.words != nullptr ? bits_total(p.bits, i) : ld_ro(p.count + i);
+            for (int i = tid; i < p.E; i += nthr) smem_i32[i] = ld_ro(p.count + i);
         }
     }
     load_peer_tables(p.peer_base, p.wait.active_ranks, p.R, p.wait.status, s_peer, s_active);

@@ -149,5 +149,35 @@ template <bool kHere = false>
 __device__ __forceinline__ int bits_total(const RouteBits& b, int e) {
     return sum_counts<kHere>(b.counts + (size_t)e * b.stride, b.chunks);
 }
+// use(expert, tokens that chose it) for every expert; whole block. A lane per sixteen chunks
+// of an expert, kAhead loads of a lane requested together (2048 experts of 28 chunks, a thread
+// per expert and one load after the other: 13 us of 224 threads).
+template <int kAhead, typename Use>
+__device__ __forceinline__ void bits_totals(const RouteBits& b, int E, Use use) {
+    const int loads = b.stride / 16, lanes = loads <= 1 ? 1 : loads <= 2 ? 2 : loads <= 4 ? 4 : 8;  // per expert
+    const int per = blockDim.x / lanes, mine = threadIdx.x / lanes, l = threadIdx.x - mine * lanes;
+    for (int x0 = mine; x0 - mine < E; x0 += kAhead * per) {
+        uint4 v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int x = x0 + u * per;
+            v[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (x < E && l < loads) v[u] = ld_ro(reinterpret_cast<const uint4*>(b.counts + (size_t)x * b.stride) + l);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int x = x0 + u * per;
+            const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            unsigned n = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int there = b.chunks - 16 * l - 4 * j;  // bytes of this word that count
+                n = __dp4a(w[j] & (there >= 4 ? 0xffffffffu : there > 0 ? (1u << (8 * there)) - 1u : 0u), 0x01010101u, n);
+            }
+            for (int d = lanes / 2; d > 0; d /= 2) n += __shfl_xor_sync(0xffffffffu, n, d);
+            if (x < E && l == 0) use(x, (int)n);
+        }
+    }
+}
 
 }  // namespace mcep
