@@ -536,7 +536,7 @@ __device__ __forceinline__ bool names_any(const int64_t* q, int n, int E, bool v
     return any;
 }
 
-// Tokens of [0, upto) that name any expert; whole block, once per kernel.
+// Tokens of [0, upto) that name any expert; whole block, once per kernel, with a barrier.
 __device__ __forceinline__ int sent_before(const ElasticSingleParams& p, int upto) {
     __shared__ int s_sent[32];
     const bool vec = choices_in_pairs(p.topk_idx, p.K);
@@ -574,14 +574,16 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
     __shared__ int s_pos[kEntries];  // received row of token c
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
     const int K = p.K, nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
-    for (int i = tid; i < (kExpand ? 2 * p.E + 1 : p.E + 1); i += nthr) smem_i32[i] = 0;
-    __syncthreads();
+    // (only where something is counted, and sent_before has a barrier ahead of that; cleared in every
+    // block and with a barrier of their own, a dispatch of 3 to 54 tokens in a captured graph, where
+    // nothing hides it, took 3.1 us instead of 2.9)
+    if (kExpand || blockIdx.x == 0)
+        for (int i = tid; i < (kExpand ? 2 * p.E + 1 : p.E + 1); i += nthr) smem_i32[i] = 0;
     pdl_wait();
     pdl_launch_dependents();
     if (blockIdx.x == 0) {  // the counts
         int* rows = smem_i32 + p.E + 1;
         const int n = sent_before(p, p.T);
-        __syncthreads();
         count_hits(p, smem_i32);
         if (kExpand) count_tokens<1, true>(p.topk_idx, 0, p.T, K, p.E, choices_in_pairs(p.topk_idx, K), rows);
         __syncthreads();
