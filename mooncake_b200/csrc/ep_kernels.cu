@@ -2161,7 +2161,7 @@ bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group) {
     // token (us per layer, counting | layout kernel): rows of 8 KB to 2, 600 tokens (10 MB) 10.6 |
     // 12.4, 1000 (16 MB) 14.3 | 14.2, in FP8 13.9 | 12.7, 4000 38.9 | 37.1; of 2 KB 2000 (8 MB) 10.3 |
     // 12.3, 4000 16.3 | 14.3; of 14 KB to 1, 600 (9 MB) 11.3 | 12.4, 1000 16.1 | 15.5, 4000 44.2 |
-    // 41.7 (8000 in FP8 alone lose, 76.9 | 78.0).
+    // 41.7, 8000 in FP8 76.6 | 71.1.
     const long long bytes = (long long)T * K * H * 2;
     if (K <= 2) return bytes < 12 << 20 && T <= 8192 / K;
     // From three on counting is slower by block: rows of 8 KB to 8 in FP8, 200 tokens (13 MB)
@@ -2199,9 +2199,14 @@ cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx)
         void (*k)(DirectDispatchParams) = ep_dispatch_rows_kernel<true, 1, 7, 6>;
         int tiles = 1, most = 7;
         if (p.use_fp8) {
+            // four tiles | two: 8192 rows of 14 KB to 1 72.0 | 78.8, 4000 of 4 KB 11.3 | 12.2, 2000 of
+            // 14 KB 19.2 | 20.4; to 2, 2000 of 14 KB 31.1 | 30.3
             // two tiles | one: 4096 rows of 14 KB to 3 68.5 | 73.0, to 4 82.4 | 85.5, to 8 145.9 |
             // 145.8; 4000 of 4 KB to 4 29.2 | 29.8; 1500 of 8 KB to 8 37.6 | 36.5
-            if (p.K <= 4 && ntiles >= 4) k = ep_dispatch_rows_kernel<true, 2, 4, 10>, tiles = 2, most = 4;
+            if (p.K == 1 && ntiles >= 4)
+                k = ep_dispatch_rows_kernel<true, 4, 4, 8>, tiles = 4, most = 4;
+            else if (p.K <= 4 && ntiles >= 4)
+                k = ep_dispatch_rows_kernel<true, 2, 4, 10>, tiles = 2, most = 4;
         } else if (p.K == 1 ? ntiles >= 4 : p.K == 2 && ntiles > 8) {
             // two tiles | one: 8000 rows of 14 KB to 1 76.3 | 86.1, 1000 of 8 KB 10.1 | 11.0; 4000 of
             // 14 KB to 2 59.0 | 60.0, 2000 of 8 KB 22.5 | 22.1; to 3 1500 of 8 KB 22.2 | 21.8

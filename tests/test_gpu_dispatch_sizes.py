@@ -68,7 +68,8 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
 @pytest.mark.parametrize("T,H,E,K", [  # edges of the layout's words, chunks and loads of counts, and where it ends
     (31, 128, 8, 3), (33, 640, 8, 3), (127, 3584, 8, 5), (128, 4096, 300, 2), (129, 8320, 24, 16), (149, 7168, 8, 8),
     (2047, 128, 8, 4), (2049, 384, 64, 3), (600, 128, 2600, 1), (16384, 128, 8, 3), (16385, 128, 8, 3),
-    (150, 128, 4096, 2), (2200, 128, 900, 3), (4300, 128, 300, 2)])
+    (150, 128, 4096, 2), (2200, 128, 900, 3), (4300, 128, 300, 2),
+    (301, 2048, 8, 1), (150, 2688, 16, 1), (149, 8320, 8, 1)])  # four tiles of a row per warp (FP8), whole and not
 def test_positions_from_the_layout_kernel(T, H, E, K, fp8):
     """Positions looked up in bits and counts (or read, beyond them), repeats and empty tokens among them."""
     M = (T + 3) // 4 * 4
