@@ -328,7 +328,7 @@ namespace {
 
 // A single rank: one or two kernels write every output directly.
 int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, const mcep_elastic_dispatch_args* a,
-                    const mcep::SingleTables& tables, const Counts* counts, mcep_event** out_event) {
+                    const mcep::SingleTables& tables, bool may_chain, const Counts* counts, mcep_event** out_event) {
     const int E = a->num_experts, M = a->num_max_tokens_per_rank, T = a->num_tokens, H = a->hidden, K = a->num_topk;
     EL_REQUIRE(H % 16 == 0 && H % 128 == 0);
     EL_REQUIRE(reinterpret_cast<uintptr_t>(a->x) % 32 == 0 && reinterpret_cast<uintptr_t>(a->recv_x) % 32 == 0);
@@ -352,7 +352,7 @@ int single_dispatch(mcep_buffer* b, ElasticState* s, const mcep::BufferView& v, 
     p.copied_topk_idx = a->copied_topk_idx;
     p.psum_rank = a->psum_num_recv_tokens_per_scaleup_rank, p.psum_expert = a->psum_num_recv_tokens_per_expert;
     if (counts) p.host_counts = s->host_counts, p.host_seq = (int32_t)++s->host_seq;
-    const bool chain = mcep::may_chain(b, stream);
+    const bool chain = async ? mcep::may_chain(b, stream) : may_chain;
     mcep::LaunchCtx ctx{stream, v.num_sms, chain && !async, chain};
     if (tables.bits.words != nullptr) {
         p.totals = s->single_totals + (size_t)par * MCEP_MAX_EXPERTS;
@@ -453,10 +453,12 @@ int elastic_dispatch(mcep_buffer* b, const mcep_elastic_dispatch_args* a, const 
     ElasticState* s = state_of(b);
     mcep::SingleTables tables;
     const mcep::LayoutScratch scratch = mcep::next_layout_scratch(b);
+    const bool chain = mcep::may_chain(b, reinterpret_cast<cudaStream_t>(a->compute_stream));  // (not in a capture)
+    const mcep::HostIs host = counts ? mcep::HostIs::kWaiting : chain ? mcep::HostIs::kFree : mcep::HostIs::kCapturing;
     if (!v.group && !v.defer &&
-        mcep::elastic_single_tables(T, K, E, a->do_expand != 0, counts != nullptr, v.num_sms, scratch.memory,
-                                    scratch.bytes, scratch.ticket, &tables))
-        return single_dispatch(b, s, v, a, tables, counts, out_event);
+        mcep::elastic_single_tables(T, K, E, H, a->do_expand != 0, host, v.num_sms, scratch.memory, scratch.bytes,
+                                    scratch.ticket, &tables))
+        return single_dispatch(b, s, v, a, tables, chain, counts, out_event);
     EL_REQUIRE(counts == nullptr || !v.defer);
     const size_t rec_want = record_bytes(R, M, K);
     const size_t rec_bytes = (v.group && s->record_area_bytes != 0) ? s->record_area_bytes : rec_want;

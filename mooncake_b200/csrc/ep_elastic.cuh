@@ -128,10 +128,12 @@ struct SingleTables {
     int32_t* starts = nullptr;
     unsigned* ticket = nullptr;
 };
+// What the host does meanwhile: goes on, waits for the counts, or captures the call.
+enum class HostIs { kFree, kWaiting, kCapturing };
 // Whether the kernels below take this problem (else the general path does), and its tables,
-// in `bytes` bytes at `scratch` (256-byte aligned). `waits`: the host waits for the counts.
-bool elastic_single_tables(int T, int K, int E, bool expand, bool waits, int num_sms, void* scratch, size_t bytes,
-                           unsigned* ticket, SingleTables* tables);
+// in `bytes` bytes at `scratch` (256-byte aligned).
+bool elastic_single_tables(int T, int K, int E, int H, bool expand, HostIs host, int num_sms, void* scratch,
+                           size_t bytes, unsigned* ticket, SingleTables* tables);
 cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, const SingleTables& tables,
                                            const LaunchCtx& ctx);
 

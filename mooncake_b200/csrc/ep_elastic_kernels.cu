@@ -835,25 +835,33 @@ cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int n
 }
 
 namespace {
-// One launch saves the host 2 us of 16, which most of these calls are bound by, and costs the
-// device up to 2. Flat rows, up to seven tokens per SM in one resident wave (the layer, wall |
-// device, counting and behind a layout kernel: 400 tokens of 8 KB to 8 14.5 | 7.7 and 16.4 | 7.4,
-// 1000 14.7 | 11.1 and 16.6 | 8.8, of 14 KB 14.2 | 13.2 and 16.4 | 11.2); a call whose host waits
-// for the counts (`waits`) gets them later, so up to 4096 choices there (1000 to 8: 30.4 - 32.0 and
-// 28.8 - 29.7). Expanded rows, where every block counts all choices: two tokens per SM, to four
-// while they are 16 choices (a call that waits: 400 to 2 25.1 and 26.9, 390 to 6 26.4 and 28.5, 500
-// to 8 28.5 and 27.7).
-bool counts_in_copy_kernel(int T, int K, int num_sms, bool expand, bool waits) {
-    if (expand) return T <= 2 * num_sms || (T <= 4 * num_sms && T * K <= 16 * num_sms);
-    return T <= 7 * num_sms && T * K <= (waits ? 4096 : 8 * 7 * num_sms);
+// One launch saves the host 2 us of 11 - 16, which most of these calls are bound by, and costs the
+// device up to 2 (the layer, wall | device, counting and behind a layout kernel).
+// Flat rows, up to seven tokens per SM in one resident wave: 520 tokens of 8 KB to 8 11.5 | 8.4 and
+// 13.5 | 7.7, 1036 11.5 | 11.3 and 13.5 | 8.9, of 14 KB 13.2 | 13.2 and 13.7 | 11.3. Above 4096
+// choices only where the host's time counts: a call whose host waits for the counts gets them
+// later (1000 to 8: 30.4 - 32.0 and 28.8 - 29.7), a captured one has paid for its launches (the
+// layers in a graph, 520 of 8 KB 8.2 and 7.9, 1036 10.9 and 9.3, of 1 KB 8.6 and 6.4), and with
+// more than eight choices a block counts longer than the launch takes (518 of 1 KB to 16 12.8 | 12.4
+// and 13.7 | 7.1).
+// Expanded rows, where every block counts all choices: two tokens per SM; four while they are 16
+// choices (444 of 4 KB to 4 11.4 | 10.2 and 13.7 | 11.2, 394 of 8 KB to 6 15.1 | 14.9 and 15.0 | 14.9)
+// and the rows have up to eight tiles, a warp each: above, the blocks are two to an SM and more than
+// one wave (444 of 14 KB to 4 17.9 | 17.8 and 16.4 | 16.2), which a host that waits does not notice
+// (a call that waits, 444 to 4 21.5 and 24.3, 394 to 6 22.7 and 24.7).
+bool counts_in_copy_kernel(int T, int K, int H, int num_sms, bool expand, HostIs host) {
+    if (expand)
+        return T <= 2 * num_sms || (T <= 4 * num_sms && T * K <= 16 * num_sms &&
+                                    (host == HostIs::kWaiting || H <= 8 * kTileChannels));
+    return T <= 7 * num_sms && T * K <= (host == HostIs::kFree && K <= 8 ? 8 * 7 * num_sms : 4096);
 }
 }  // namespace
 
-bool elastic_single_tables(int T, int K, int E, bool expand, bool waits, int num_sms, void* scratch, size_t bytes,
-                           unsigned* ticket, SingleTables* tables) {
+bool elastic_single_tables(int T, int K, int E, int H, bool expand, HostIs host, int num_sms, void* scratch,
+                           size_t bytes, unsigned* ticket, SingleTables* tables) {
     *tables = SingleTables();
     if (K > kMaxTopk || E > kMaxExperts) return false;
-    if (counts_in_copy_kernel(T, K, num_sms, expand, waits)) return true;
+    if (counts_in_copy_kernel(T, K, H, num_sms, expand, host)) return true;
     const size_t starts = ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
     if (starts > bytes) return false;
     tables->starts = static_cast<int32_t*>(scratch);

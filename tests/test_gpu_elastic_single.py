@@ -79,7 +79,8 @@ def test_layout_in_bits(T, H, E, K, expand, alignment):
 
 @pytest.mark.parametrize("T,H,E,K,expand,alignment", [  # either side of where the counting in the copy kernel ends
     (1036, 640, 64, 8, False, 1), (1036, 128, 32, 9, False, 1), (592, 640, 16, 4, True, 2), (593, 128, 16, 4, True, 1),
-    (395, 128, 16, 6, True, 1), (394, 1152, 16, 6, True, 4)])
+    (395, 128, 16, 6, True, 1), (394, 1152, 16, 6, True, 4), (394, 4224, 16, 6, True, 1), (394, 4096, 16, 6, True, 1),
+    (460, 640, 16, 9, False, 1), (455, 640, 16, 9, False, 1)])
 def test_either_side_of_the_counting_limit(T, H, E, K, expand, alignment):
     test_dispatch_and_combine(T, H, E, K, expand, alignment)
 
