@@ -2403,14 +2403,16 @@ cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const Laun
 }
 
 cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx) {
-    // Rows of 8 tiles and more, once a block would have several tokens (one rank on this path,
-    // us per layer with it | without). 4 tiles: 300 tokens to 8 21.1 | 18.5, 1500 32.8 | 29.9. 8
-    // tiles: to 2 300 17.2 | 16.5, 600 18.8 | 18.9, 2000 32.5 | 33.2; to 4 600 22.3 | 22.0, 1000 26.7 |
-    // 27.0; to 8 300 24.1 | 22.0, 1000 36.5 | 35.6, 1500 49.2 | 51.6. 14 tiles: to 2 300 18.6 | 18.9,
-    // 400 20.0 | 19.9, 600 24.8 | 25.9; to 8 300 27.5 | 27.3, 400 30.7 | 29.8, 600 38.5 | 39.5, 2000
-    // 100 | 111.
+    // Rows of 6 tiles and more, once a block would have several tokens; the other kernel's block
+    // has a row of up to 8 tiles in one pass, beyond that it has two and loses earlier (one rank on
+    // this path, us per layer with it | without). 5 tiles: 2000 tokens to 2 26.1 | 25.7, to 8 43.8 |
+    // 42.2. 6 tiles: to 1 800 tokens 18.2 | 18.5, 1200 21.2 | 22.7; to 4 800 21.9 | 21.5, 1200 26.4 | 27.4;
+    // to 8 1200 35.5 | 35.2, 1600 42.5 | 42.4, 2000 49.5 | 54.2. 8 tiles: to 2 800 20.8 | 20.2, 1200 25.0 |
+    // 25.5; to 4 1200 30.4 | 30.2, 1600 33.6 | 34.4; to 8 1200 42.0 | 41.1, 1600 51.1 | 54.6. 9 tiles: to 2
+    // 300 17.4 | 18.0; to 8 300 22.8 | 22.5, 450 25.7 | 25.9, 600 32.3 | 30.7, 800 35.0 | 36.7. 14 tiles: to
+    // 8 300 26.3 | 26.2, 600 37.7 | 39.4, 2000 100 | 111.
     const int tiles = (p.H + kTileChannels - 1) / kTileChannels;
-    if (p.T > (tiles > 8 ? 3 : 2 + p.K) * ctx.num_sms && p.H >= 8 * kTileChannels) {
+    if (tiles >= 6 && 2 * p.T > (tiles > 8 ? 6 : 12 + p.K) * ctx.num_sms) {
         const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
         p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
         return launch("ep_combine_reduce", ep_combine_gather_kernel<4>, shape.grid, dim3(shape.threads), 0, ctx, p);
