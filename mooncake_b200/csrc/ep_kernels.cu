@@ -1041,7 +1041,8 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks)
         atomicOr(p.status, kStatusSlotRange);
         s = -1;
     }
-    // (32 bits: a device has no room for 2^31 rows of 128 bytes, nor for as many scales of theirs)
+    // (31 bits: mcep_dispatch has larger tensors filled by the kernel that counts. 64 bits in the
+    // shuffles: 2756 rows of 256 bytes in FP8 to 8 11.5 us, 11.0 so)
     const int to = s >= 0 ? e * M + s : -1;
     if (tile == 0 && mine) {
         p.rowmap[(size_t)t * K + lane] = s;

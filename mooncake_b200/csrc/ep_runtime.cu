@@ -8,6 +8,7 @@
 #include <cuda.h>  // types of the virtual-memory API only; entry points are looked up at run time
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -366,6 +367,8 @@ bool is_capturing(cudaStream_t stream) {
     return st != cudaStreamCaptureStatusNone;
 }
 bool chain_with_pdl(const mcep_buffer* b, cudaStream_t stream) { return b->pdl && !is_capturing(stream); }
+// Whether the rows of E x M, each of `parts` parts, can be numbered in a positive int.
+bool places_fit_31_bits(int E, int M, int parts) { return (long long)E * M <= INT_MAX / parts; }
 }  // namespace
 
 namespace mcep {
@@ -923,9 +926,11 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     // are in place by then (1 - 2 us of launch latency per call).
     mcep::LaunchCtx first{stream, b->num_sms, pdl && !a->async_finish};
 
-    // Larger batches get their layout from a kernel of its own.
-    const bool counting = (b->fuse_layout || T == 0) &&
-                          mcep::counts_in_send_kernel(T, K, H, b->num_sms, group);
+    // Larger batches get their layout from a kernel of its own. (Not a single rank's in tensors of
+    // 2^31 rows or scales and more, whose places the kernel behind it does not tell apart.)
+    const bool far_rows = !group && !places_fit_31_bits(E, M, fp8 ? H / 128 : 1);
+    const bool counting = far_rows || ((b->fuse_layout || T == 0) &&
+                                       mcep::counts_in_send_kernel(T, K, H, b->num_sms, group));
     mcep::RouteBits bits = {};
     if (!counting) {
         mcep::LayoutParams lp = {};
@@ -1105,7 +1110,8 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
             if (rec && rec->T == T && rec->K == K && rec->E == E && rec->M == M && rec->H == H)
                 rowmap = b->scratch[rec->seq & 1].rowmap;
         }
-        const bool search = rowmap == nullptr && (long long)T * K <= 4096;
+        // (the kernels that read kept rows count a tensor's in 31 bits)
+        const bool search = (rowmap == nullptr && (long long)T * K <= 4096) || !places_fit_31_bits(E, M, 1);
         if (rowmap == nullptr && !search) {
             mcep::CombineInvertParams ip = {};
             ip.src_info = a->src_info, ip.layout_range = a->layout_range, ip.topk_idx = a->topk_idx;

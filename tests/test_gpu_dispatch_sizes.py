@@ -138,3 +138,48 @@ def test_rows_of_more_blocks_than_are_resident(T):
     recv, _, handle, _, _ = buf.dispatch(x, idx, active, T, E, 2_000_000, use_fp8=False)
     out, _, _ = buf.combine(recv, idx, w, active, 2_000_000, handle)
     assert torch.equal(recv[0], x) and torch.equal(recv[1], x) and torch.equal(out, x)
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("T,M", [(5, 1 << 29), (700, 1 << 29), (700, (1 << 31) // 8)])
+def test_tensors_of_2_to_the_31_rows(T, M, fp8):
+    """Rows whose number has more than 31 bits. No device holds such tensors whole: every token names the
+    last expert, whose part alone is there, and the bases that are passed lie that far ahead of it."""
+    H, E, K = 128, 8, 2
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=g, device="cuda").to(torch.bfloat16)
+    idx = torch.tensor([[-1, E - 1], [E - 1, E - 1], [-1, -1], [E - 1, E]], device="cuda").repeat(T, 1)[:T].contiguous()
+    sent = (idx == E - 1).any(dim=1).nonzero().flatten()
+    n, width = len(sent), H if fp8 else 2 * H
+    rows = torch.zeros((T, width), dtype=torch.uint8, device="cuda")
+    scales = torch.zeros((T,), dtype=torch.float32, device="cuda")  # (a scale per row: H is 128)
+    src = torch.full((T,), -1, dtype=torch.int32, device="cuda")
+    count, layout = (torch.full((E,), -1, dtype=d, device="cuda") for d in (torch.int32, torch.int64))
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    ahead, stream = (E - 1) * M, torch.cuda.current_stream().cuda_stream
+    buf = ep.Buffer(0, 1, 0)
+    for fuse in (1, 0):
+        buf.set_option("fuse_layout", fuse)
+        buf.dispatch(x.data_ptr(), idx.data_ptr(), active.data_ptr(), T, H, K, M, E, 2_000_000, fp8,
+                     rows.data_ptr() - ahead * width, scales.data_ptr() - ahead * 4 if fp8 else 0, count.data_ptr(),
+                     src.data_ptr() - ahead * 4, layout.data_ptr(), False, False, stream)
+        torch.cuda.synchronize()
+        assert count.tolist() == [0] * (E - 1) + [n] and layout.tolist() == count.tolist()
+        assert torch.equal(src[:n].long(), sent) and bool((src[n:] == -1).all())
+        want = ora.dispatch([x.cpu()], [idx.cpu()], (T + 3) // 4 * 4, E, fp8)[0]
+        assert torch.equal(rows[:n].cpu(), want["recv_x"][E - 1, :n].contiguous().view(torch.uint8))
+        if fp8:
+            assert torch.equal(scales[:n].cpu(), want["scales"][E - 1, :n].flatten())
+    y = torch.randn((T, H), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.rand((T, K), generator=g, device="cuda")
+    out = torch.full((T, H), 7.0, dtype=torch.bfloat16, device="cuda")
+    buf.combine(y.data_ptr() - ahead * 2 * H, idx.data_ptr(), w.data_ptr(), src.data_ptr() - ahead * 4, layout.data_ptr(),
+                active.data_ptr(), E, T, H, K, M, E, 2_000_000, False, out.data_ptr(), False, False, stream)
+    torch.cuda.synchronize()
+    acc = torch.zeros((T, H), device="cuda", dtype=torch.float64)
+    for k in range(K):
+        at = (idx[sent, k] == E - 1).double() * w[sent, k].double()
+        acc[sent] += at.unsqueeze(1) * y[:n].double()
+    # (an fp32 sum of two products and one rounding to bf16: half a step, and both sums' errors)
+    assert bool(((out.double() - acc).abs() <= acc.abs() * 2 ** -8 + 1e-6).all())
+    assert buf.status() == 0
