@@ -39,7 +39,7 @@ struct RouteBits {
     uint8_t* counts;  // [experts][stride], padding undefined
     int experts, chunks, stride;
 };
-// Such bits in `capacity` bytes at `memory` (256-byte aligned); words null where they do
+// Such bits in `capacity` bytes at `memory` (16-byte aligned); words null where they do
 // not fit or where the batch has more than 128 chunks.
 RouteBits route_bits(void* memory, size_t capacity, int T, int E);
 

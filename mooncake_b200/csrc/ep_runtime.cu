@@ -502,10 +502,11 @@ int mcep_buffer_create(int rank, int num_ranks, int64_t num_ep_buffer_bytes, int
     // workspace: [status 256 B][parity 0 scratch][parity 1 scratch]
     b->status = reinterpret_cast<int32_t*>(b->workspace);
     b->dev_next_seq = reinterpret_cast<uint32_t*>(b->workspace + 256 + 192);  // beside parity 0's tickets
-    const size_t words = (size_t)MCEP_MAX_EXPERTS * sizeof(uint64_t);
-    const size_t small = (size_t)(MCEP_MAX_EXPERTS + 64) * sizeof(int32_t);
-    const size_t half = (kWorkspaceBytes - 256) / 2;
-    const size_t fixed = 256 + small + words + 2 * 64 * sizeof(uint64_t) + kChunkHistBytes;
+    constexpr size_t words = (size_t)MCEP_MAX_EXPERTS * sizeof(uint64_t);
+    constexpr size_t small = (size_t)(MCEP_MAX_EXPERTS + 64) * sizeof(int32_t);
+    constexpr size_t half = (kWorkspaceBytes - 256) / 2 / 256 * 256;
+    constexpr size_t fixed = 256 + small + words + 2 * 64 * sizeof(uint64_t) + kChunkHistBytes;
+    static_assert(half % 256 == 0 && fixed % 256 == 0, "the layout scratch of either parity is 256-byte aligned");
     const size_t big = ((half - fixed - 1024) / 3) / 256 * 256;  // bytes for each of slot / rowmap / rowmap_inv
     b->scratch_entries = big / sizeof(int32_t);
     for (int par = 0; par < 2; ++par) {
