@@ -70,7 +70,8 @@ def test_dispatch_and_combine(T, H, E, K, fp8, staged):
     (31, 128, 8, 3), (33, 640, 8, 3), (127, 3584, 8, 5), (128, 4096, 300, 2), (129, 8320, 24, 16), (149, 7168, 8, 8),
     (2047, 128, 8, 4), (2049, 384, 64, 3), (600, 128, 2600, 1), (16384, 128, 8, 3), (16385, 128, 8, 3),
     (150, 128, 4096, 2), (2200, 128, 900, 3), (4300, 128, 300, 2),
-    (301, 2048, 8, 1), (150, 2688, 16, 1), (149, 8320, 8, 1)])  # four tiles of a row per warp (FP8), whole and not
+    (301, 2048, 8, 1), (150, 2688, 16, 1), (149, 8320, 8, 1),  # four tiles of a row per warp (FP8), whole and not
+    (149, 2560, 8, 4), (33, 3584, 16, 2), (150, 4480, 8, 3)])  # two, odd numbers of them
 def test_positions_from_the_layout_kernel(T, H, E, K, fp8):
     """Positions looked up in bits and counts (or read, beyond them), repeats and empty tokens among them."""
     M = (T + 3) // 4 * 4
@@ -83,6 +84,41 @@ def test_positions_from_the_layout_kernel(T, H, E, K, fp8):
     recv, cnt, handle, _, _ = buf.dispatch(x.cuda(), idx.cuda(), active, M, E, 2_000_000, use_fp8=fp8)
     got = [dict(recv_x=recv[0] if fp8 else recv, scales=recv[1] if fp8 else None, recv_count=cnt, handle=handle)]
     torch.cuda.synchronize()
+    _check_dispatch(dict(R=1, E=E, M=M, fp8=fp8), got, ora.dispatch([x], [idx], M, E, fp8), None)
+    y = torch.randn((E, M, H), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
+    out, _, _ = buf.combine(y, idx.cuda(), w.cuda(), active, 2_000_000, handle)
+    ref = ora.combine([y.cpu()], [idx], [w], [dict(src_info=handle[0].cpu(), layout_range=handle[1].cpu())], M, E)
+    assert torch.equal(out.cpu().view(torch.int16), ref[0].view(torch.int16))
+    assert buf.runtime.status() == 0
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("T,H,E,K,counted", [
+    # several tokens per block and more of their tiles than the block has warps, ragged last batches
+    (1001, 4096, 16, 1, True), (1481, 1152, 8, 2, True), (592, 4224, 8, 3, True), (591, 4480, 16, 3, True),
+    # either side of where the layout kernel begins: 12 MB to one and two, 17 MB and a token per SM to more
+    (1535, 4096, 8, 1, True), (1536, 4096, 8, 1, False), (767, 4096, 8, 2, True), (768, 4096, 8, 2, False),
+    (271, 4096, 8, 8, True), (272, 4096, 8, 8, False), (297, 1664, 16, 16, True), (592, 128, 16, 16, True),
+    (593, 128, 16, 16, False), (148, 8320, 8, 8, True), (149, 8320, 8, 8, False)])
+def test_batches_that_count_for_themselves(T, H, E, K, counted, fp8):
+    """Positions counted in the send kernel of a single rank, repeats and empty tokens among them, up to
+    the sizes that it is used for; which kernel ran is looked up, so that the sizes follow the rule."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are those of 148 SMs")
+    M = (T + 3) // 4 * 4
+    x, idx, w = make_rank_inputs(19, 0, T, H, E, K, "zipf1.2", n_mask=T // 7)
+    if K > 1:
+        idx[::5, K - 1] = idx[::5, 0]
+    buf = Buffer(FakeGroup(0, 1), 0)
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    ep.set_kernel_timing(True)
+    try:
+        recv, cnt, handle, _, _ = buf.dispatch(x.cuda(), idx.cuda(), active, M, E, 2_000_000, use_fp8=fp8)
+    finally:
+        ep.set_kernel_timing(False)
+    torch.cuda.synchronize()
+    assert any("layout" in name for name in ep.drain_kernel_times()) == (not counted)
+    got = [dict(recv_x=recv[0] if fp8 else recv, scales=recv[1] if fp8 else None, recv_count=cnt, handle=handle)]
     _check_dispatch(dict(R=1, E=E, M=M, fp8=fp8), got, ora.dispatch([x], [idx], M, E, fp8), None)
     y = torch.randn((E, M, H), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
     out, _, _ = buf.combine(y, idx.cuda(), w.cuda(), active, 2_000_000, handle)

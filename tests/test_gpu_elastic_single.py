@@ -72,7 +72,8 @@ def test_dispatch_and_combine(T, H, E, K, expand, alignment):
 @pytest.mark.parametrize("T,H,E,K,expand,alignment", [  # words, chunks and loads of counts; rows of odd tiles and parts
     (16384, 128, 8, 2, True, 1), (16384, 128, 300, 1, False, 3), (4225, 640, 24, 5, True, 8), (4224, 1152, 9, 7, False, 1),
     (1153, 4224, 8, 3, True, 2), (2049, 8320, 8, 2, False, 1), (384, 128, 4096, 4, True, 1),
-    (1500, 128, 2048, 8, True, 1), (4000, 256, 1025, 2, False, 2)])
+    (1500, 128, 2048, 8, True, 1), (4000, 256, 1025, 2, False, 2),
+    (1983, 8320, 8, 8, True, 1), (9477, 1664, 8, 8, True, 1)])  # combine: the last tokens first, odd remainders
 def test_layout_in_bits(T, H, E, K, expand, alignment):
     test_dispatch_and_combine(T, H, E, K, expand, alignment)
 
