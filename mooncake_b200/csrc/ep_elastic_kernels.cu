@@ -725,11 +725,12 @@ __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel
     const int first = (part * p.warps_per_row + warp - sub * p.warps_per_row) * kTiles;  // tile
     const int t = group * p.C + sub, K = p.K;
     const bool mine = t < p.T && lane < K;
+    const int nchunks = p.H / 16;  // (asked of the parameters each time, 8 bytes spill)
     V32 v[kTiles];
 #pragma unroll
     for (int u = 0; u < kTiles; ++u) {
         const int c = (first + u) * 32 + lane;
-        if (t < p.T && c < p.H / 16)
+        if (t < p.T && c < nchunks)
             v[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
     }
     int64_t raw = -1;
@@ -779,14 +780,14 @@ __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel
 #pragma unroll
             for (int u = 0; u < kTiles; ++u) {
                 const int c = (first + u) * 32 + lane;
-                if (c < p.H / 16) st32(out + (size_t)r * row_bytes + (size_t)c * 32, v[u]);
+                if (c < nchunks) st32(out + (size_t)r * row_bytes + (size_t)c * 32, v[u]);
             }
         }
     } else if (named) {
 #pragma unroll
         for (int u = 0; u < kTiles; ++u) {
             const int c = (first + u) * 32 + lane;
-            if (c < p.H / 16) st32(out + (size_t)pos * row_bytes + (size_t)c * 32, v[u]);
+            if (c < nchunks) st32(out + (size_t)pos * row_bytes + (size_t)c * 32, v[u]);
         }
     }
 }

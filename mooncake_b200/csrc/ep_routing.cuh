@@ -133,10 +133,10 @@ __device__ __forceinline__ int sum_counts(const uint8_t* row, int n) {
 }
 // Tokens before t that chose expert e.
 __device__ __forceinline__ int bits_before(const RouteBits& b, int e, int t) {
-    const int chunk = t / kChunkTokens, bit = t % kChunkTokens;
-    const uint4 v = ld_ro(b.words + (size_t)chunk * b.experts + e);
+    const int chunk = t / kChunkTokens, bit = t % kChunkTokens;  // (the tables lie in 16 MB: 32-bit places)
+    const uint4 v = ld_ro(b.words + (chunk * b.experts + e));
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    int n = sum_counts<false>(b.counts + (size_t)e * b.stride, chunk);
+    int n = sum_counts<false>(b.counts + e * b.stride, chunk);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int lower = bit - 32 * j;  // bits of this word that are lower
