@@ -112,7 +112,7 @@ def algorithmic_bytes(w, R, sel):
     payload = (H + 4 * S) if w["fp8"] else 2 * H   # per (token, selected expert)
     b = {}
     # single rank: x read once, packed outputs written once; combine gathers and writes once
-    b["ep_dispatch_send_direct"] = T * 2 * H + sel * payload + 8 * T * K + 4 * sel
+    b["ep_dispatch_send_direct"] = b["ep_dispatch_rows"] = T * 2 * H + sel * payload + 8 * T * K + 4 * sel
     b["ep_combine_reduce_direct"] = sel * 2 * H + T * 2 * H + 12 * T * K
     # group: rows go straight to their final place (one write per selection, local
     # or over NVLink); the receive duty only moves the small side messages

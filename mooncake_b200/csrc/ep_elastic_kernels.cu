@@ -890,7 +890,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
     const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
     if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;
-    if (cudaError_t e = launch_kernel("ep_elastic_single_layout", layout, dim3(p.bits.chunks), dim3(kBitsThreads), smem,
+    if (cudaError_t e = launch_kernel("ep_elastic_layout_bits", layout, dim3(p.bits.chunks), dim3(kBitsThreads), smem,
                                       1, ctx, p))
         return e;
     LaunchCtx chained = ctx;
@@ -900,7 +900,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     p.warps_per_row = (warps + p.parts - 1) / p.parts;
     p.C = kElasticWarps / p.warps_per_row;
     auto k = expand ? ep_elastic_rows_kernel<true> : ep_elastic_rows_kernel<false>;
-    return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C * p.parts),
+    return launch_kernel("ep_elastic_rows", k, dim3(1 + (p.T + p.C - 1) / p.C * p.parts),
                          dim3(p.C * p.warps_per_row * 32), expand ? 0 : ((size_t)p.E + 1) * sizeof(int), 1, chained, p);
 }
 

@@ -2224,8 +2224,8 @@ cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx)
         p.warps_per_row = (warps + p.parts - 1) / p.parts;
         p.tokens_per_block = most / p.warps_per_row;
         const int groups = (p.T + p.tokens_per_block - 1) / p.tokens_per_block;
-        return launch("ep_dispatch_send_direct", k, dim3(groups * p.parts), dim3(32 * p.warps_per_row * p.tokens_per_block),
-                      0, ctx, p);
+        return launch("ep_dispatch_rows", k, dim3(groups * p.parts), dim3(32 * p.warps_per_row * p.tokens_per_block), 0,
+                      ctx, p);
     }
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, false);
     p.C = s.tokens;

@@ -30,7 +30,7 @@ import torch
 import torch.distributed as dist
 
 from . import ep
-from .mooncake_ep_buffer import EventOverlap, _DeviceBytes, _stream_ptr  # noqa: F401  (calls return EventOverlap)
+from .mooncake_ep_buffer import EventOverlap, _DeviceBytes, _stream_ptr
 
 
 class EPHandle:
@@ -203,7 +203,8 @@ class ElasticBuffer:
                  num_max_tokens_per_rank: Optional[int] = None,
                  expert_alignment: Optional[int] = None, handle: Optional[EPHandle] = None,
                  do_expand: bool = False, do_cpu_sync: Optional[bool] = None,
-                 num_sms: Optional[int] = None, async_with_compute_stream: bool = False):
+                 num_sms: Optional[int] = None, async_with_compute_stream: bool = False
+                 ) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor], EPHandle, EventOverlap]:
         """Reference :437-714. Returns (recv_x, recv_topk_idx, recv_topk_weights, handle, event).
 
         With `do_cpu_sync` the host waits for the counts; the rows are ordered on the current stream
@@ -254,7 +255,8 @@ class ElasticBuffer:
 
     # ------------------------------------------------------------------ combine
     def combine(self, x: torch.Tensor, handle: EPHandle, topk_weights: Optional[torch.Tensor] = None,
-                num_sms: Optional[int] = None, async_with_compute_stream: bool = False):
+                num_sms: Optional[int] = None, async_with_compute_stream: bool = False
+                ) -> Tuple[torch.Tensor, None, EventOverlap]:
         """Reference :716-774. Returns (combined_x, None, event)."""
         if self.runtime is None:
             raise RuntimeError("ElasticBuffer has been destroyed")
