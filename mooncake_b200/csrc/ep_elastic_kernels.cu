@@ -411,8 +411,8 @@ __device__ void tell_host(const ElasticSingleParams& p) {
 // (mooncake_ep_elastic_dispatch_copy_epilogue.cuh:114-141). Every block adds its own to the
 // totals, so that whoever needs them reads one word per expert, however many chunks there
 // are. (One block that reads every chunk's hits, a load after the other, is what the call waits
-// for: the layer, 4826 rows of 11 KB expanded to 1 of 128 experts 44.7 us, now 43.2; 4364 of 5 KB
-// to 1 of 2048 63.1, now 37.4; flat, 10904 of 9 KB to 2 of 1024 81.2, now 66.9.)
+// for: the layer, 4826 rows of 11 KB expanded to 1 of 128 experts 44.7 us, now 43.0; 4364 of 5 KB
+// to 1 of 2048 63.1, now 33.8; flat, 10904 of 9 KB to 2 of 1024 81.2, now 66.9.)
 // An expanded row's place depends on the hits of all experts below its own: the block that
 // finishes last makes the segments of them (kExpand). For flat rows they are results only, and
 // a block of the copy kernel does it, so that no row waits.
@@ -694,11 +694,12 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
 // writes what there is per entry. Block 0 writes and passes on the counts.
 // Two tiles per warp and 40 warps per SM: a row is stored once (or K times, few in general),
 // so it is the bytes requested at a time that matter. Flat, 4096 rows of 14 KB, dispatch
-// alone: 20.4 us, one tile and 32 warps 29.0, 48 warps 25.6, four tiles and 32 warps 20.8 (a
+// alone: 20.3 us, one tile and 32 warps 29.0, 48 warps 25.6, four tiles and 32 warps 20.8 (a
 // block per eight tokens and a layout kernel of one cluster before: 23.5). Expanded, the
 // layer, 4096 rows of 14 KB to 2 and to 8: 64.8 and 176.9 us, one tile and 40 warps 74.9 and
 // 178.3, 42 warps in blocks of seven 71.7 and 176.4, four tiles and 32 warps 67.5 and 182.1
-// (a block per token before: 65.1 and 179.2).
+// (a block per token before: 65.1 and 179.2; with what the layout kernel has lost since 63.2
+// and 172.2).
 constexpr int kElasticWarps = 4, kElasticTiles = 2;
 
 template <bool kExpand>

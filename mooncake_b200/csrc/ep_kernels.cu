@@ -738,12 +738,8 @@ __global__ void __launch_bounds__(kBitsThreads) ep_layout_bits_kernel(LayoutPara
 // area: this GPU's (single rank, or an expert this rank owns) or a peer's, over
 // NVLink.
 //
-// A single rank launches one block per batch, however many there are: the
-// hardware then hands the batches out as SMs come free. Rows of 14 KB to 8
-// experts each, 4096 tokens: 98 us with one resident wave striding over the
-// tokens (the slowest SM decides), 85 us with a block each. Tokens leave in
-// ascending order over the whole grid, which keeps an expert's rows together in
-// time and in HBM pages.
+// A group's launch is one resident wave that strides over the batches; so is a single
+// rank's, which sends small batches this way (larger ones: ep_dispatch_rows_kernel).
 //
 // What goes where for entry (t, k) with expert e, owner rank o, local expert le,
 // row r = first row of this rank's segment in e + earlier tokens of this rank:
@@ -956,8 +952,8 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
 // =============================================================================
 // single rank: dispatch writes the packed outputs directly
 // =============================================================================
-// Bound by HBM for large batches (4096 tokens, hidden 7168, top-8, bf16: 529 MB)
-// and by latency for decode (index load -> count -> row stores, one batch per block).
+// Small batches (counts_in_send_kernel), in one launch: bound by latency, index load ->
+// count -> row stores, one batch per block.
 template <bool kFP8>
 __global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
     extern __shared__ int smem_i32[];  // [E]
@@ -990,11 +986,14 @@ __device__ __noinline__ void write_counts(RouteBits bits, int E, int32_t* recv_c
 
 // Single rank, behind a layout kernel: a warp owns one tile of one token and needs no
 // other: lane k finds the token's k-th row, the tile goes to each. Nothing is shared and
-// nobody waits at a barrier. Blocks are small because it is the turnover of independent
+// nobody waits at a barrier. The hardware hands the blocks out in ascending order as SMs come
+// free, which keeps an expert's rows together in time and in HBM pages (4096 rows of 14 KB to 8
+// with a block per token: 85 us, with one resident wave striding over the tokens, where the
+// slowest SM decides, 98). Blocks are small because it is the turnover of independent
 // warps that hides the chain index -> bits -> stores: with a block per token that met at
 // three barriers a block lived 6 us, 2001 of them behind one another were bound by that
-// and not by HBM (2001 rows of 8 KB to 8 in FP8, the layer 50.1 us, now 46.7; 2000 of 4 KB
-// in bf16 26.2, now 24.9; 4000 of 1 KB 25.0, now 20.2).
+// and not by HBM (2001 rows of 8 KB to 8 in FP8, the layer 49.5 us, now 45.5; 2000 of 4 KB
+// in bf16 25.6, now 22.6; 4000 of 1 KB 19.8, now 14.9).
 // How many warps and tiles of each (us per layer; launch_direct_dispatch chooses): many warps per SM where the
 // time is that of the loads and of quantising (FP8 to 4, 2048 rows of 14 KB: 46.1 with 42
 // warps, 48.1 with 32; bf16 to 8, 1500 rows of 8 KB: 42.0 | 42.9); with few copies per row
@@ -2151,9 +2150,11 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
 }
 
 bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group) {
-    // A group's sender blocks are one resident wave, a token each (one rank on this path,
-    // us per layer, counting | layout kernel: rows of 8 KB in bf16 to 8, 200 tokens 17.6 |
-    // 17.2, 290 19.0 | 18.4, 400 30.8 | 26.4; of 7 KB in FP8, 290 23.9 | 26.9).
+    // A group's sender blocks are one resident wave, a token each (one rank on this path, us per
+    // layer to 8, counting | layout kernel: rows of 4 KB in bf16 150 tokens 11.9 | 14.6, 290 14.4 |
+    // 15.0, in FP8 14.2 | 15.2; of 14 KB in bf16 150 18.6 | 20.1, 290 20.1 | 22.5, in FP8 18.5 | 21.0. Rows
+    // of 8 KB fill a block's warps once, bf16 ones alone lose from 200 on: 200 16.5 | 16.5, 290 17.5 |
+    // 17.1, with hooks 21.3 | 19.5; in FP8 290 15.9 | 16.6; 400 of 8 KB 30.8 | 26.4).
     if (group) return T <= 2 * num_sms;
     // A single rank counts in one resident wave of blocks with as many tokens each as that
     // takes. The layout kernel is the faster one on the device at nearly every size, but a
@@ -2162,12 +2163,18 @@ bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group) {
     // token (us per layer, counting | layout kernel): rows of 8 KB to 2, 600 tokens (10 MB) 10.6 |
     // 12.4, 1000 (16 MB) 14.3 | 14.2, in FP8 13.9 | 12.7, 4000 38.9 | 37.1; of 2 KB 2000 (8 MB) 10.3 |
     // 12.3, 4000 16.3 | 14.3; of 14 KB to 1, 600 (9 MB) 11.3 | 12.4, 1000 16.1 | 15.5, 4000 44.2 |
-    // 41.7, 8000 in FP8 76.6 | 71.1.
+    // 41.7, 8000 in FP8 76.6 | 71.1. Just below the line some lose: of 8 KB to 1, 1500 (12 MB) 11.0 | 11.7,
+    // in FP8 12.2 | 11.8, and a stream that is ahead of the device has 12.4 | 10.7; of 2 KB to 2, 3000
+    // 12.4 | 11.8.
     const long long bytes = (long long)T * K * H * 2;
     if (K <= 2) return bytes < 12 << 20 && T <= 8192 / K;
     // From three on counting is slower by block: rows of 8 KB to 8 in FP8, 200 tokens (13 MB)
     // 10.0 | 12.4, 300 (20 MB) 13.5 | 12.4, 400 16.3 | 14.9; of 14 KB in bf16, 160 (18 MB) 15.2 |
-    // 13.8, 300 24.8 | 21.1, 590 32.6 | 31.7; of 4 KB to 4, 590 (10 MB) 10.0 | 12.4.
+    // 13.8, 300 24.8 | 21.1, 590 32.6 | 31.7; of 4 KB to 4, 590 (10 MB) 10.0 | 12.4. Around the line, wall
+    // and a stream that is ahead: of 8 KB to 8 in FP8, 240 (15 MB) 9.9 | 11.4 and 9.4 | 9.5, 270 (17 MB)
+    // 10.5 | 11.7 and 9.5 | 9.6; in bf16 240 11.1 | 11.3 and 10.0 | 10.5, 270 11.7 | 11.5 and 10.3 | 10.4; of 5 KB
+    // 400 (16 MB) in FP8 11.1 | 11.9 and 10.3 | 9.4, in bf16 11.9 | 11.5 and 11.2 | 10.1; of 3 KB 590 (14 MB) in
+    // FP8 11.4 | 11.6 and 10.7 | 9.2.
     return T <= num_sms || (T <= 4 * num_sms && bytes < 17 << 20);
 }
 
@@ -2274,9 +2281,13 @@ static ReduceShape reduce_shape(int T, int K, int H, int num_sms) {
     // (4096 tokens to 8 after a write of 512 MB, whose last lines are still leaving L2:
     // 96 us, equal runs and strided 100; 8192 tokens 168 against 184 and 181). Those are rows
     // beyond L2: the last tokens' are taken first, as what was written last is still there
-    // where the rows were made in token order (a layer whose experts' outputs are the rows
-    // just received: 4096 x 14 KB 172.7 us | 169.0, 3000 128.9 | 124.0, 8000 x 8 KB 189.8 | 183.5;
-    // rows made long before 81.3 either way). With fewer waves it gains and loses 1 %.
+    // where the rows were made in token order (combine of the rows just received, first | last
+    // tokens first: 4096 x 14 KB 94.2 us | 90.1, 3000 73 | 67.6, 8000 x 8 KB 102.4 | 97.5). Rows that are
+    // written expert by expert just before, as a grouped GEMM does, gain less or nothing (90.1 |
+    // 88.2, 69.6 | 69.6, 98.3 | 96.3), rows made long before nothing (96.3 | 96.3, 74.4 | 75.8, 102.4 |
+    // 104.4). The group's kernel has the order too (one rank on that path, 4096 x 14 KB 101.4 | 97.2,
+    // written by expert 99.4 | 97.3, long before 101.4 | 101.4; rows of peers have not been measured).
+    // With fewer waves it gains and loses 1 %.
     const int resident = std::max(1, num_sms * (2 * kReduceWarps * 32 / s.threads) / parts);
     const int waves = (groups + resident - 1) / resident;
     const int run = K < 8 || waves < 4 ? 0 : waves <= 8 ? waves : 2;
