@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel
     for (int u = 0; u < kTiles; ++u) {
         const int c = (first + u) * 32 + lane;
         if (t < p.T && c < nchunks)
-            v[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+            v[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2, p.x_last);
     }
     int64_t raw = -1;
     float w = 0.f;
@@ -888,6 +888,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
     p.bits = tables.bits, p.starts = tables.starts, p.ticket = tables.ticket;
+    p.x_last = layer_beyond_l2(p.T, expand ? p.K : 1, p.H);
     auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
     const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
     if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;

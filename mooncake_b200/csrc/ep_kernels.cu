@@ -755,6 +755,7 @@ struct SendView {
     int T, K, E, R, M, H, rank;
     int L, RM;
     int C;                    // tokens per batch
+    bool x_last;              // see layer_beyond_l2
     RouteBits bits;           // the layout kernel's bits (words null: none), or
     const int32_t* slot;      // [T*K] position among this rank's tokens for the expert (layout kernel),
                               // or null: counted here (small batches, one per block)
@@ -804,7 +805,7 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
         V32 r = {};
         const int tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
         if (tok < v.C && t + tok < v.T && c < nchunks)
-            r = ld32_readonly(v.x + ((size_t)(t + tok) * v.H + (size_t)c * 16) * 2);
+            r = ld32_readonly(v.x + ((size_t)(t + tok) * v.H + (size_t)c * 16) * 2, !kCount && v.x_last);
         return r;
     };
     int t0 = sid * v.C;
@@ -1021,7 +1022,7 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks)
         const int c = (tile + u) * 32 + lane;
         row[u] = V32{};
         if (t < p.T && c < nchunks)
-            row[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+            row[u] = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2, p.x_last);
     }
     if (mine) e = (int)ld_ro(p.topk_idx + (size_t)t * K + lane);
     pdl_wait();
@@ -1118,7 +1119,7 @@ __global__ void __launch_bounds__(256) ep_combine_invert_kernel(CombineInvertPar
 // one bf16 rounding, one 32-byte store (mooncake_ep_kernel.cu:715-752).
 // kDepth rows are requested before the first of them is used. s_ptr has kMaxTopk
 // entries, null where nothing is to be added.
-template <int kDepth, bool kReadOnly>
+template <int kDepth, bool kReadOnly, bool kLast>
 __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const float* s_w, int K,
                                             int H, void* out_row) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -1137,7 +1138,7 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
                 const char* rp = s_ptr[k0 + b];
                 if (rp != nullptr)
                     v[b] = kReadOnly ? ld32_readonly(rp + (size_t)c * 32)
-                                     : ld32_coherent(rp + (size_t)c * 32);
+                                     : ld32_coherent(rp + (size_t)c * 32, kLast);
             }
 #pragma unroll
             for (int b = 0; b < kDepth; ++b) {
@@ -1168,7 +1169,7 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
 // kAbs: rowmap holds rows of the whole tensor and every weight is 1 (elastic calls).
 constexpr int kReduceWarps = 16;  // 64 registers a thread with two blocks per SM: nothing spills in the kernel below
 
-template <int kDepth, bool kAbs, int kBlocks>
+template <int kDepth, bool kAbs, int kBlocks, bool kLast>
 __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_kernel(DirectCombineParams p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp / p.tiles_per_block;  // which token of the group
@@ -1216,7 +1217,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
 #pragma unroll
             for (int b = 0; b < kDepth; ++b) {
                 const int r = __shfl_sync(kFull, row, k0 + b);
-                if ((unsigned)r < rows && act) v[b] = ld32_readonly(x + (size_t)r * row_bytes);
+                if ((unsigned)r < rows && act) v[b] = ld32_readonly(x + (size_t)r * row_bytes, kLast);
             }
             if (k0 == 0) request(t0 + step + sub);
 #pragma unroll
@@ -1232,14 +1233,14 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
                 }
             }
         }
-        if (act && t0 + sub < end) st32(out + (size_t)(t0 + sub) * row_bytes, pack_bf16x16(acc));
+        if (act && t0 + sub < end) st32(out + (size_t)(t0 + sub) * row_bytes, pack_bf16x16(acc), kLast);
     }
 }
 
 // One row per token (top-1, and every flat elastic combine of a single rank): a gather.
 // The kernel above would have a single load per lane in flight; here a warp requests
 // up to four tiles of its block's `tokens_per_block` rows before it uses the first.
-template <bool kAbs>
+template <bool kAbs, bool kLast>
 __global__ void __launch_bounds__(512, 2) ep_combine_one_row_kernel(DirectCombineParams p) {
     constexpr int kAhead = 4, kMost = 16;
     __shared__ int s_row[kMost];
@@ -1271,7 +1272,8 @@ __global__ void __launch_bounds__(512, 2) ep_combine_one_row_kernel(DirectCombin
         for (int u = 0; u < kAhead; ++u) {
             const int item = i0 + u * nwarps, tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
             const int r = item < items && c < nchunks ? s_row[tok] : -1;
-            if (r >= 0) v[u] = ld32_readonly(reinterpret_cast<const char*>(p.x) + (size_t)r * row_bytes + (size_t)c * 32);
+            if (r >= 0)
+                v[u] = ld32_readonly(reinterpret_cast<const char*>(p.x) + (size_t)r * row_bytes + (size_t)c * 32, kLast);
         }
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
@@ -1341,7 +1343,7 @@ __global__ void __launch_bounds__(512) ep_combine_search_kernel(DirectCombinePar
             s_w[tid] = w;
         }
         __syncthreads();
-        reduce_rows<8, true>(s_ptr, s_w, p.K, p.H,
+        reduce_rows<8, true, false>(s_ptr, s_w, p.K, p.H,
                              reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
     }
 }
@@ -1609,6 +1611,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     v.beg = reinterpret_cast<const uint64_t*>(p.local_base + p.w.beg_off);
     v.seq = p.seq, v.wait = scaled(p.wait, 2), v.rx_off = p.rx_off, v.meta_off = p.meta_off;
     v.meta_stride = p.meta_stride, v.rowmap = p.rowmap, v.s_peer = s_peer, v.s_active = s_active;
+    v.x_last = p.x_last;
     const bool remote = send_tokens<kFP8, true, kCount>(v, sid, nsend, smem_i32);
     MCEP_TRACE(0, 5);  // all rows of this block are issued
 
@@ -1825,6 +1828,7 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
 // or this rank's own expert output) and the K rows are reduced in registers.
 // An owner that is inactive, or whose word does not arrive in time (it is then
 // marked inactive), contributes nothing (mooncake_ep_kernel.cu:685-699, 728-732).
+template <bool kLast>
 __device__ __forceinline__ void combine_reduce_duty(const GroupCombineParams& p, int first_token, int token_stride,
                                                     char* const* s_peer, const int* s_active) {
     __shared__ const char* s_ptr[kMaxTopk];
@@ -1859,14 +1863,14 @@ __device__ __forceinline__ void combine_reduce_duty(const GroupCombineParams& p,
         }
         __syncthreads();
         if (t == first_token) MCEP_TRACE(2, 4);  // the owners' words are in, rows can be read
-        reduce_rows<8, false>(s_ptr, s_w, p.K, p.H,
-                              reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
+        reduce_rows<8, false, kLast>(s_ptr, s_w, p.K, p.H,
+                                     reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
         __syncthreads();  // the rows are done with s_ptr
     }
 }
 
 // kPhases: 1 = publish, 2 = reduce, 3 = both in one launch.
-template <int kPhases>
+template <int kPhases, bool kLast>
 __device__ __forceinline__ void combine_body(const GroupCombineParams& p, int bid, int nblocks,
                                              int* smem_i32) {
     __shared__ char* s_peer[kMaxRanks];
@@ -1879,18 +1883,18 @@ __device__ __forceinline__ void combine_body(const GroupCombineParams& p, int bi
     if (kPhases & 1) combine_publish_duty(p, bid, nblocks, smem_i32, s_peer, s_active, first_lr);
     MCEP_TRACE(2, 1);
     if (kPhases & 2) {
-        combine_reduce_duty(p, bid, nblocks, s_peer, s_active);
+        combine_reduce_duty<kLast>(p, bid, nblocks, s_peer, s_active);
     }
     MCEP_TRACE(2, 2);
 }
 
-template <int kPhases>
+template <int kPhases, bool kLast = false>
 __global__ void __launch_bounds__(512) ep_combine_kernel(GroupCombineParams p) {
     extern __shared__ int smem_i32[];
     pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
-    combine_body<kPhases>(p, blockIdx.x, gridDim.x, smem_i32);
+    combine_body<kPhases, kLast>(p, blockIdx.x, gridDim.x, smem_i32);
 }
 
 // The reduce duty of batches with more tokens than SMs, in a launch of its own: as
@@ -1900,7 +1904,7 @@ __global__ void __launch_bounds__(512) ep_combine_kernel(GroupCombineParams p) {
 // first needs that owner - and keeps the verdict. One rank on this path, 2048 tokens of
 // 14 KB to 8: 47 us, with a barrier per token and the words looked at for every one 59
 // (512 tokens 16.7 and 18.9).
-template <int kDepth>
+template <int kDepth, bool kLast>
 __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel(GroupCombineParams p) {
     __shared__ char* s_peer[kMaxRanks];
     __shared__ int s_active[kMaxRanks];
@@ -1976,7 +1980,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
                     __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(row), k0 + b));
                 if (r != nullptr) {
                     there |= 1u << b;
-                    if (act) v[b] = ld32_coherent(r + (size_t)c * 32);
+                    if (act) v[b] = ld32_coherent(r + (size_t)c * 32, kLast);
                 }
             }
             if (k0 == 0) request(t0 + step + sub);
@@ -1994,7 +1998,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
         }
         if (act && t0 + sub < end)
             st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + sub) * row_bytes + (size_t)c * 32,
-                 pack_bf16x16(acc));
+                 pack_bf16x16(acc), kLast && p.K > 1);
     }
 }
 
@@ -2007,7 +2011,7 @@ __global__ void __launch_bounds__(512)
     const int which = blockIdx.x / per_rank;
     if (threadIdx.x == 0) s_p = ps[which];
     __syncthreads();
-    combine_body<3>(s_p, blockIdx.x - which * per_rank, per_rank, smem_i32);
+    combine_body<3, false>(s_p, blockIdx.x - which * per_rank, per_rank, smem_i32);
 }
 
 // threads per block: one warp per tile, at most 16 warps
@@ -2201,8 +2205,11 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool group) {
     return s;
 }
 
+bool layer_beyond_l2(long long T, int copies, int H) { return T * (copies + 2) * H * 2 > 40ll << 20; }
+
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
     if (!p.counting()) {
+        p.x_last = layer_beyond_l2(p.T, p.K, p.H);
         const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
         void (*k)(DirectDispatchParams) = ep_dispatch_rows_kernel<true, 1, 7, 6>;
         int tiles = 1, most = 7;
@@ -2302,6 +2309,7 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         const int grid = persistent_grid(p.T, ep_combine_search_kernel, threads, 0, ctx);
         return launch("ep_combine_search", ep_combine_search_kernel, dim3(grid), dim3(threads), 0, ctx, p);
     }
+    const bool last = layer_beyond_l2(p.T, p.K, p.H);
     const int row_tiles = (p.H + kTileChannels - 1) / kTileChannels;
     if (p.K == 1) {
         // two rounds of four tiles per warp (4096 rows of 14 KB: 21.0 us, 29 - 32 with the
@@ -2311,18 +2319,23 @@ cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx) {
         const int most = (p.T + 2 * ctx.num_sms - 1) / (2 * ctx.num_sms);
         p.tokens_per_block = c < 1 ? 1 : c < most ? c : most < 1 ? 1 : most;
         const int warps = p.tokens_per_block * row_tiles;
-        auto k = p.absolute ? ep_combine_one_row_kernel<true> : ep_combine_one_row_kernel<false>;
+        void (*k)(DirectCombineParams) = nullptr;
+        if (p.absolute)
+            k = last ? ep_combine_one_row_kernel<true, true> : ep_combine_one_row_kernel<true, false>;
+        else
+            k = last ? ep_combine_one_row_kernel<false, true> : ep_combine_one_row_kernel<false, false>;
         const int grid = p.T > 0 ? (p.T + p.tokens_per_block - 1) / p.tokens_per_block : 1;
         return launch("ep_combine_reduce_direct", k, dim3(grid), dim3(32 * (warps < 16 ? warps : 16)), 0, ctx, p);
     }
     const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
     p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
     void (*k)(DirectCombineParams) = nullptr;
-    if (p.absolute) {
-        k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, true, 1> : ep_combine_rows_kernel<4, true, 2>;
-    } else {
-        k = p.T <= ctx.num_sms ? ep_combine_rows_kernel<8, false, 1> : ep_combine_rows_kernel<4, false, 2>;
-    }
+    if (p.T <= ctx.num_sms)
+        k = p.absolute ? ep_combine_rows_kernel<8, true, 1, false> : ep_combine_rows_kernel<8, false, 1, false>;
+    else if (p.absolute)
+        k = last ? ep_combine_rows_kernel<4, true, 2, true> : ep_combine_rows_kernel<4, true, 2, false>;
+    else
+        k = last ? ep_combine_rows_kernel<4, false, 2, true> : ep_combine_rows_kernel<4, false, 2, false>;
     return launch("ep_combine_reduce_direct", k, shape.grid, dim3(shape.threads), 0, ctx, p);
 }
 
@@ -2362,6 +2375,7 @@ cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& c
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
+    p.x_last = layer_beyond_l2(p.T, p.K, p.H);
     auto k = pick_dispatch<1>(p.use_fp8 != 0, p.counting());
     // the control block, then one block per token (small batches) or a resident wave
     // (a wave, not a block per batch: a block that stored rows in a peer's memory, nearly
@@ -2424,13 +2438,15 @@ cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& c
     // 300 17.4 | 18.0; to 8 300 22.8 | 22.5, 450 25.7 | 25.9, 600 32.3 | 30.7, 800 35.0 | 36.7. 14 tiles: to
     // 8 300 26.3 | 26.2, 600 37.7 | 39.4, 2000 100 | 111.
     const int tiles = (p.H + kTileChannels - 1) / kTileChannels;
+    const bool last = layer_beyond_l2(p.T, p.K, p.H);
     if (tiles >= 6 && 2 * p.T > (tiles > 8 ? 6 : 12 + p.K) * ctx.num_sms) {
         const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
         p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
-        return launch("ep_combine_reduce", ep_combine_gather_kernel<4>, shape.grid, dim3(shape.threads), 0, ctx, p);
+        return launch("ep_combine_reduce", last ? ep_combine_gather_kernel<4, true> : ep_combine_gather_kernel<4, false>,
+                      shape.grid, dim3(shape.threads), 0, ctx, p);
     }
     const int threads = block_threads(p.H);
-    auto k = ep_combine_kernel<2>;
+    auto k = last ? ep_combine_kernel<2, true> : ep_combine_kernel<2>;
     const int grid = persistent_grid(p.T, k, threads, 0, ctx);
     return launch("ep_combine_reduce", k, dim3(grid), dim3(threads), 0, ctx, p);
 }

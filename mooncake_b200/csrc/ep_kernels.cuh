@@ -79,12 +79,19 @@ struct DirectDispatchParams {
     // are counted in the send kernel. (Last, so that what a counting kernel reads lies together.)
     RouteBits bits;
     const int32_t* slot;        // [T*K]
+    bool x_last;                // see layer_beyond_l2 (set by the launcher)
     int warps_per_row, tokens_per_block, parts;  // with positions: how a block's warps are dealt out, blocks that
                                                  // share a row (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 // whether the send kernels count the slots themselves for this many tokens
 bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group);
+// Whether the input of a layer, `copies` rows of each token and the result are so many bytes that the
+// last use of what is used up is worth telling L2 (ld32_readonly with `last`). Of less, all of it stays there anyway, and
+// what a caller uses again is not to be the first that goes (us per layer on three sets of inputs in turn, no
+// mark | all marked: to 1, 1500 rows of 8 KB, 37 MB, 11.3 | 11.7, 2000, 49 MB, 12.7 | 12.2; to 2, 1200, 39 MB, 11.9 | 12.1,
+// 1600, 52 MB, 14.6 | 14.2; flat elastic rows of 4 KB, 2500, 31 MB, 9.7 | 9.9, 4000, 49 MB, 14.5 | 13.5).
+bool layer_beyond_l2(long long T, int copies, int H);
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
 
 struct SendShape {
@@ -174,6 +181,7 @@ struct GroupDispatchParams {
     int64_t* layout_range;      // [L][R]
     int copy_rows;              // recv_x is a tensor of the caller's: copy the rows out
     RouteBits bits;             // from the layout kernel (words null: none)
+    bool x_last;                // see layer_beyond_l2 (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms);

@@ -20,6 +20,7 @@ SIZES = [  # T, H, E, K, fp8
     (2341, 7168, 8, 8, False), (592, 4096, 16, 3, True), (593, 4096, 16, 3, False), (4096, 1024, 8, 2, True), (4097, 640, 8, 2, False), (8192, 128, 8, 1, True),
     (8192, 128, 256, 8, True), (8193, 128, 256, 8, True), (9001, 256, 16, 1, False),
     (400, 12416, 8, 8, False), (4800, 4096, 8, 8, False),
+    (512, 4096, 8, 8, False), (513, 4096, 8, 8, True), (853, 8192, 4, 1, False), (854, 8192, 4, 1, False),  # marks for L2
     (1036, 3584, 8, 2, False), (1037, 3584, 8, 2, False), (1481, 2688, 8, 8, False), (445, 4224, 8, 4, False),  # the two reduce kernels of a group
 ]
 
