@@ -122,11 +122,14 @@ struct ElasticSingleParams {
     unsigned long long* totals;  // [E] listings and rows of the experts, zero between calls
     int32_t* starts;             // [E + 1] expanded: where the experts' segments start
     unsigned* ticket;            // expanded: chunks that are done
+    uint16_t* listings;          // expanded, no starts: [E][listings_stride] of every chunk, segments made of them in
+    int listings_stride;         // the copy kernel
 };
 // The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
 struct SingleTables {
     RouteBits bits = {};
     int32_t* starts = nullptr;
+    uint16_t* listings = nullptr;
     unsigned* ticket = nullptr;
 };
 // What the host does meanwhile: goes on, waits for the counts, or captures the call.

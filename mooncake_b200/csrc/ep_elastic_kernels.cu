@@ -2,6 +2,8 @@
 // another GPU; the exchange between the ranks is the group dispatch / combine.
 #include "ep_elastic.cuh"
 
+#include <type_traits>
+
 #include "ep_device.cuh"
 #include "ep_kernels.cuh"
 #include "ep_launch.cuh"
@@ -466,6 +468,87 @@ __device__ __forceinline__ void take_totals(const ElasticSingleParams& p, Use us
     }
 }
 
+// ---- segments made by every block of the copy kernel -----------------------------------
+// Up to 16 chunks and 256 experts the layout kernel leaves its listings as they are, a word per
+// expert and chunk, and every block of the copy kernel sums up those of all experts. What the block
+// that finishes last does else - a fence, the ticket, the totals, the sums and the segments, five
+// round trips to L2 one after the other - stands ahead of every row; here one load and a scan do, with
+// 4 KB more for a block to read, which on larger tables costs what it saves. Device time
+// per layer, that block's segments | their own: 1024 rows of 8 KB to 8 of 128 27.0 us | 25.0, to 2 of 64 14.7 | 12.6,
+// of 4 KB to 8 of 256 20.2 | 17.3, of 14 KB to 8 of 8 43.6 | 40.4, to 4 of 128 26.3 | 23.9; 2048 of 14 KB to 8 of 256 83.8 |
+// 82.1, to 2 of 64 30.7 | 28.8, to 1 of 8 24.2 | 22.6.
+// It must not spill: with the first listings asked for ahead of the bits in registers, 50 bytes
+// a thread, 1024 of 8 KB to 8 25.7, 2048 of 14 KB 84.3; by cp.async 25.1 and 91.0.
+constexpr int kOwnChunks = 16, kOwnExperts = 256;
+constexpr int kElasticWarps = 4, kElasticTiles = 2;  // of the copy kernel: see there
+
+// [E][listings_stride] words, the ones of chunks that there are not are zero.
+__host__ __device__ constexpr int listings_stride_of(int chunks) { return (chunks + 7) / 8 * 8; }
+__device__ __forceinline__ void leave_listings(const ElasticSingleParams& p, int e, int listings) {
+    uint16_t* row = p.listings + (size_t)e * p.listings_stride;
+    row[blockIdx.x] = (uint16_t)listings;
+    if (blockIdx.x == gridDim.x - 1)
+        for (int c = gridDim.x; c < p.listings_stride; ++c) row[c] = 0;
+}
+__device__ __forceinline__ int sum_words(const uint4& v) {
+    const uint32_t s = (v.x & 0xffffu) + (v.y & 0xffffu) + (v.z & 0xffffu) + (v.w & 0xffffu);
+    return (int)(s + (v.x >> 16) + (v.y >> 16) + (v.z >> 16) + (v.w >> 16));
+}
+// Where the segments start: a thread has `per` experts, whose sums lie in three parts (inside a
+// thread's experts, a warp's threads, the block's warps). The block
+// meets once, in `make`.
+struct OwnSegments {
+    struct Shared {
+        int expert[kOwnExperts], thread[kElasticWarps * 32], warp[kElasticWarps];
+    };
+    Shared& s;
+    const int per, first;
+
+    __device__ __forceinline__ static const uint4* row(const ElasticSingleParams& p, int e) {
+        return reinterpret_cast<const uint4*>(p.listings + e * p.listings_stride);
+    }
+    __device__ __forceinline__ OwnSegments(const ElasticSingleParams& p, Shared& shared)
+        : s(shared), per((p.E + blockDim.x - 1) / blockDim.x), first(threadIdx.x * per) {}
+    __device__ __forceinline__ void make(const ElasticSingleParams& p) {
+        const int lane = threadIdx.x & 31;
+        int sum = 0;
+        for (int x = first; x < min(first + per, p.E); ++x) {
+            int n = sum_words(ld_ro(row(p, x)));
+            if (p.listings_stride > 8) n += sum_words(ld_ro(row(p, x) + 1));
+            s.expert[x] = sum;
+            sum += p.alignment == 1 ? n : aligned_count(n, p.alignment);
+        }
+        int incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(kAll, incl, d);
+            if (lane >= d) incl += u;
+        }
+        s.thread[threadIdx.x] = incl - sum;
+        if (lane == 31) s.warp[threadIdx.x >> 5] = incl;
+        __syncthreads();
+    }
+    __device__ __forceinline__ static int start(const Shared& s, int per, int e) {
+        const int thread = per == 1 ? e : e / per;
+        int n = s.expert[e] + s.thread[thread];
+        for (int w = 0; w < thread >> 5; ++w) n += s.warp[w];
+        return n;
+    }
+};
+
+// The segments' ends; whole block. Not inlined: its registers are not taken from the rows' warps.
+__device__ __noinline__ void write_segments(const OwnSegments::Shared& s, int per, RouteBits bits, int E,
+                                            int32_t* psum_expert, int32_t* psum_rank) {
+    for (int x = threadIdx.x; x < E; x += blockDim.x)
+        psum_expert[x] = OwnSegments::start(s, per, x) + bits_total(bits, 1 + x);
+    if (threadIdx.x != 0) return;
+    int n = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) n += s.warp[w];
+    psum_expert[E] = n;
+    psum_rank[0] = bits_total(bits, 0);
+}
+
+
 template <bool kExpand>
 __global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSingleParams p) {
     extern __shared__ uint4 smem_u128[];  // [1 or 1 + E] bits of this chunk, then [E + 1] listings beyond them
@@ -490,12 +573,17 @@ __global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSi
         const int n = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
         p.bits.words[(size_t)blockIdx.x * p.bits.experts + x] = m;
         p.bits.counts[(size_t)x * p.bits.stride + blockIdx.x] = (uint8_t)n;
-        if (kExpand && x > 0) add_hits(p, x - 1, n + extra[x - 1], n);
+        if (!kExpand || x == 0) continue;
+        if (p.listings != nullptr)
+            leave_listings(p, x - 1, n + extra[x - 1]);
+        else
+            add_hits(p, x - 1, n + extra[x - 1], n);
     }
     if (!kExpand) {
         for (int x = tid; x < p.E; x += kBitsThreads) add_hits(p, x, extra[x], 0);
         return;
     }
+    if (p.listings != nullptr) return;  // the copy kernel makes the segments
     __threadfence();
     __syncthreads();
     if (tid == 0) s_last = atomicInc(p.ticket, gridDim.x - 1) == gridDim.x - 1;
@@ -700,11 +788,11 @@ __global__ void __launch_bounds__(512, 2) ep_elastic_single_copy_kernel(ElasticS
 // 178.3, 42 warps in blocks of seven 71.7 and 176.4, four tiles and 32 warps 67.5 and 182.1
 // (a block per token before: 65.1 and 179.2; with what the layout kernel has lost since 63.2
 // and 172.2).
-constexpr int kElasticWarps = 4, kElasticTiles = 2;
 
-template <bool kExpand>
+template <bool kExpand, bool kOwn>
 __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel(ElasticSingleParams p) {
     extern __shared__ int smem_i32[];  // flat: [E + 1] hits / sums (block 0)
+    __shared__ typename std::conditional<kOwn, OwnSegments::Shared, char>::type s_own;
     constexpr int kTiles = kElasticTiles;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
@@ -716,6 +804,12 @@ __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel
             exclusive_sums(smem_i32, p.E);
             for (int x = tid; x <= p.E; x += blockDim.x) p.psum_expert[x] = smem_i32[x];
             if (tid == 0) p.psum_rank[0] = bits_total<false>(p.bits, 0);
+            __syncthreads();
+        }
+        if constexpr (kOwn) {
+            OwnSegments segments(p, s_own);
+            segments.make(p);
+            write_segments(s_own, segments.per, p.bits, p.E, p.psum_expert, p.psum_rank);
             __syncthreads();
         }
         tell_host(p);
@@ -743,10 +837,19 @@ __global__ void __launch_bounds__(kElasticWarps * 32, 10) ep_elastic_rows_kernel
     const int e = (uint64_t)raw < (uint64_t)p.E ? (int)raw : -1;
     const unsigned named = __ballot_sync(kAll, e >= 0);
     pdl_wait();
-    const int pos = named ? bits_before(p.bits, 0, t) : -1;
-    int row = -1;
+    int row = -1, pos = -1;
     // (a repeat's earlier listings find the last one's row and store the same bytes)
-    if (kExpand && e >= 0) row = row_with_room(p, ld_ro(p.starts + e) + bits_before(p.bits, 1 + e, t));
+    if constexpr (kOwn) {
+        OwnSegments segments(p, s_own);
+        if (named) pos = bits_before(p.bits, 0, t);
+        int before = 0;
+        if (e >= 0) before = bits_before(p.bits, 1 + e, t);
+        segments.make(p);
+        if (e >= 0) row = row_with_room(p, OwnSegments::start(s_own, segments.per, e) + before);
+    } else {
+        if (named) pos = bits_before(p.bits, 0, t);
+        if (kExpand && e >= 0) row = row_with_room(p, ld_ro(p.starts + e) + bits_before(p.bits, 1 + e, t));
+    }
     if (first == 0 && t < p.T) {
         const int master = 31 - __clz(named);
         const unsigned same = __match_any_sync(kAll, e);
@@ -857,6 +960,14 @@ bool counts_in_copy_kernel(int T, int K, int H, int num_sms, bool expand, HostIs
                                     (host == HostIs::kWaiting || H <= 8 * kTileChannels));
     return T <= 7 * num_sms && T * K <= (host == HostIs::kFree && K <= 8 ? 8 * 7 * num_sms : 4096);
 }
+
+// Expanded rows whose segments every block of the copy kernel makes (the figures: OwnSegments). With
+// 256 experts and two loads for each, long rows, whose blocks move least for what they read, lose
+// (1100 tokens of 14 KB to 2 20.8 | 21.2, 2048 to 1 25.2 | 25.7; of 5 KB 13.4 | 12.8 and 14.9 | 14.4; to 2 of 160 20.2 | 20.0).
+bool makes_own_segments(int T, int E, int H) {
+    if (T > kOwnChunks * kChunkTokens || E > kOwnExperts) return false;
+    return E * listings_stride_of((T + kChunkTokens - 1) / kChunkTokens) <= 160 * kOwnChunks || H <= 8 * kTileChannels;
+}
 }  // namespace
 
 bool elastic_single_tables(int T, int K, int E, int H, bool expand, HostIs host, int num_sms, void* scratch,
@@ -864,9 +975,13 @@ bool elastic_single_tables(int T, int K, int E, int H, bool expand, HostIs host,
     *tables = SingleTables();
     if (K > kMaxTopk || E > kMaxExperts) return false;
     if (counts_in_copy_kernel(T, K, H, num_sms, expand, host)) return true;
-    const size_t starts = ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
+    const bool own = expand && makes_own_segments(T, E, H);
+    const size_t starts = own ? (size_t)E * kOwnChunks * sizeof(uint16_t) : ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
     if (starts > bytes) return false;
-    tables->starts = static_cast<int32_t*>(scratch);
+    if (own)
+        tables->listings = static_cast<uint16_t*>(scratch);
+    else
+        tables->starts = static_cast<int32_t*>(scratch);
     tables->bits = route_bits(static_cast<char*>(scratch) + starts, bytes - starts, T, expand ? 1 + E : 1);
     tables->ticket = ticket;
     return tables->bits.words != nullptr;
@@ -889,6 +1004,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     }
     p.bits = tables.bits, p.starts = tables.starts, p.ticket = tables.ticket;
     p.x_last = layer_beyond_l2(p.T, expand ? p.K : 1, p.H);
+    p.listings = tables.listings, p.listings_stride = listings_stride_of(p.bits.chunks);
     auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
     const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
     if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;
@@ -901,7 +1017,9 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     p.parts = (warps + kElasticWarps - 1) / kElasticWarps;
     p.warps_per_row = (warps + p.parts - 1) / p.parts;
     p.C = kElasticWarps / p.warps_per_row;
-    auto k = expand ? ep_elastic_rows_kernel<true> : ep_elastic_rows_kernel<false>;
+    auto k = p.listings ? ep_elastic_rows_kernel<true, true>
+             : expand   ? ep_elastic_rows_kernel<true, false>
+                        : ep_elastic_rows_kernel<false, false>;
     return launch_kernel("ep_elastic_rows", k, dim3(1 + (p.T + p.C - 1) / p.C * p.parts),
                          dim3(p.C * p.warps_per_row * 32), expand ? 0 : ((size_t)p.E + 1) * sizeof(int), 1, chained, p);
 }

@@ -87,6 +87,43 @@ def test_either_side_of_the_counting_limit(T, H, E, K, expand, alignment):
     test_dispatch_and_combine(T, H, E, K, expand, alignment)
 
 
+@pytest.mark.parametrize("T,H,E,K,alignment", [  # loads of listings, experts of a thread, 64 to 128 threads; where it ends
+    (600, 128, 16, 3, 1), (1024, 2560, 256, 2, 4), (1025, 640, 160, 4, 1), (1153, 4096, 256, 1, 8), (2048, 3072, 97, 8, 3),
+    (1025, 4224, 256, 2, 1), (2049, 640, 24, 2, 4), (700, 128, 257, 2, 1), (901, 1664, 129, 16, 128)])
+def test_expanded_segments(T, H, E, K, alignment):
+    """Segments of listings, repeats among them (every one counted, one row, at the last), tokens that go nowhere."""
+    M = T + E * (alignment - 1) // K + 1
+    x, idx, w = make_rank_inputs(41, 0, T, H, E, K, "zipf1.2", n_mask=T // 9)
+    if K > 1:
+        idx[::3, 0] = idx[::3, K - 1]
+    there = torch.zeros((T, E), dtype=torch.int64)
+    for k in range(K):
+        named = (idx[:, k] >= 0).nonzero().flatten()
+        there[named, idx[named, k]] += 1
+    sizes = (there.sum(dim=0) + alignment - 1) // alignment * alignment
+    starts = torch.cat([torch.zeros(1, dtype=torch.int64), sizes.cumsum(0)])
+    once = (there > 0).long()
+    before = once.cumsum(0) - once
+    rows = torch.full((T, K), -1, dtype=torch.int64)
+    for k in range(K):
+        last = (idx[:, k] >= 0) & ~(idx[:, k + 1:] == idx[:, k:k + 1]).any(dim=1)
+        t = last.nonzero().flatten()
+        rows[t, k] = starts[idx[t, k]] + before[t, idx[t, k]]
+    sent = once.any(dim=1)
+    buf = ElasticBuffer(FakeGroup(0, 1), num_max_tokens_per_rank=M, hidden=H, num_topk=K, num_gpu_timeout_secs=2)
+    for wait in (True, False):
+        recv, _, rw, h, _ = buf.dispatch(x.cuda(), topk_idx=idx.cuda(), topk_weights=w.cuda(), num_experts=E,
+                                         num_max_tokens_per_rank=M, expert_alignment=alignment, do_expand=True,
+                                         do_cpu_sync=wait)
+        ends = torch.cat([starts[:E] + once.sum(dim=0), starts[E:]])
+        assert h.psum_num_recv_tokens_per_expert.tolist() == ends.tolist()
+        assert h.psum_num_recv_tokens_per_scaleup_rank.tolist() == [int(sent.sum())]
+        assert torch.equal(h.recv_src_metadata[:int(sent.sum()), 2:].cpu().long(), rows[sent])
+        t, k = (rows >= 0).nonzero(as_tuple=True)
+        assert torch.equal(recv.cpu()[rows[t, k]], x[t]) and torch.equal(rw.cpu()[rows[t, k]], w[t, k])
+    assert buf.runtime.status() == 0
+
+
 def test_a_repeat_has_its_expanded_row_at_its_last_listing():
     """An expert listed twice takes two rows of its segment and fills one; the first listing names none."""
     T, H, E, K = 700, 1152, 8, 3
