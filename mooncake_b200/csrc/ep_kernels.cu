@@ -810,6 +810,7 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
     };
     int t0 = sid * v.C;
     V32 ahead = load_item(t0, warp);
+    if (kGroup && !kCount) pdl_wait();  // (the layout kernel has waited for the rows; it is its tables that come now)
     if (kCount && !kGroup && v.T == 0 && sid == 0)
         for (int e = tid; e < v.E; e += nthr) v.recv_count[e] = 0, v.layout_range[e] = 0;
     int counted = 0;  // tokens that are in hist
@@ -1384,7 +1385,7 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
     MCEP_TRACE(0, 1);
     for (int x = tid; x < p.E; x += nthr) {
         const int dr = x / L;
-        if (!s_active[dr]) continue;
+        if (!s_active[dr] || dr == p.rank) continue;
         const int c = hist[x];
         uint64_t* wd = reinterpret_cast<uint64_t*>(s_peer[dr] + p.w.cnt_off) + (p.rank * L + (x - dr * L));
         st_relaxed_sys(wd, ((uint64_t)p.seq << 32) | (uint32_t)(c + 1));
@@ -1395,8 +1396,12 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
         const int le = i / p.R, src = i - le * p.R;
         int c = -1;  // -1: nothing will come from this source (inactive, or given up on)
         if (s_active[src]) {
-            const uint32_t v = wait_word(my_cnt + src * L + le, p.seq, p.wait, src);
-            c = v ? (int)v - 1 : -1;
+            if (src == p.rank) {
+                c = hist[src * L + le];
+            } else {
+                const uint32_t v = wait_word(my_cnt + src * L + le, p.seq, p.wait, src);
+                c = v ? (int)v - 1 : -1;
+            }
             if (c > p.M) {
                 atomicOr(p.wait.status, kStatusSlotRange);
                 c = 0;
@@ -1580,6 +1585,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     const int nh = nsend < kRecvHelpers ? nsend : kRecvHelpers;
     MCEP_TRACE(0, 0);
     if (bid == 0) {  // the counts do not wait for the peer tables (0.8 us)
+        if (!kCount) pdl_wait();
         if (kCount) {
             count_tokens<2>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
         } else if (p.bits.words != nullptr) {
@@ -1682,8 +1688,8 @@ __global__ void __launch_bounds__(512, 2) ep_dispatch_kernel(GroupDispatchParams
     if (kCount) {
         for (int i = threadIdx.x; i < p.E; i += blockDim.x) smem_i32[i] = 0;
         __syncthreads();
+        pdl_wait();  // (behind a layout kernel: in the body)
     }
-    pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     dispatch_body<kFP8, kCount, kPhases>(p, blockIdx.x, gridDim.x, smem_i32);
@@ -1708,14 +1714,20 @@ __global__ void __launch_bounds__(512)
     dispatch_body<kFP8, kCount, kPhases>(s_p, blockIdx.x - which * per_rank, per_rank, smem_i32);
 }
 
+// Everything that the receive duty reads arrives with words of this call (the control block's verdicts,
+// the peers' payload words), so it starts beside the send kernel and only ends behind it: what the
+// stream sees as done is done. One rank on this path, us per layer with this, the reduce phase's like
+// (ep_combine_kernel), the own counts taken directly and the first tiles ahead of the layout's end:
+// 400 tokens of 14 KB to 8 29.3 -> 26.5, 1024 of 4 KB 24.7 -> 22.1, 2048 of 14 KB 95.3 -> 92.1; in hook mode
+// 27.9, 23.3 and 93.3, 1024 of 8 KB 36.9 -> 35.0.
 template <bool kFP8>
 __global__ void __launch_bounds__(kRowWarps * 32, 4) ep_dispatch_recv_kernel(GroupDispatchParams p) {
     extern __shared__ int smem_i32[];
-    pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     MCEP_TRACE(1, 0);
     dispatch_recv_duty<kFP8>(p, blockIdx.x, gridDim.x, smem_i32);
+    pdl_wait();
 }
 
 // =============================================================================
@@ -1888,13 +1900,19 @@ __device__ __forceinline__ void combine_body(const GroupCombineParams& p, int bi
     MCEP_TRACE(2, 2);
 }
 
+// behind_publish: what the reduce phase reads was complete when the publish phase, the kernel ahead of
+// it, began - that kernel lets the next one start only once it has waited for all before it - and a
+// peer's rows come with the peer's word. So it starts beside the publish phase, and only ends behind
+// it. A hook's reduce phase waits at its top: the caller may have put work between, which may still
+// read the result's memory.
 template <int kPhases, bool kLast = false>
 __global__ void __launch_bounds__(512) ep_combine_kernel(GroupCombineParams p) {
     extern __shared__ int smem_i32[];
-    pdl_wait();
+    if (kPhases != 2 || !p.behind_publish) pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     combine_body<kPhases, kLast>(p, blockIdx.x, gridDim.x, smem_i32);
+    if (kPhases == 2 && p.behind_publish) pdl_wait();
 }
 
 // The reduce duty of batches with more tokens than SMs, in a launch of its own: as
@@ -1912,7 +1930,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
     const int sub = warp / p.tiles_per_block;
     const int c = ((warp - sub * p.tiles_per_block + blockIdx.y * p.tiles_per_block) * 32) + lane;
     const bool act = c < p.H / 16;
-    pdl_wait();
+    if (!p.behind_publish) pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     const int L = p.E / p.R, RM = p.R * p.M;
@@ -2000,6 +2018,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
             st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + sub) * row_bytes + (size_t)c * 32,
                  pack_bf16x16(acc), kLast && p.K > 1);
     }
+    if (p.behind_publish) pdl_wait();
 }
 
 // All logical ranks of an in-process group in one cooperative launch (see

@@ -213,6 +213,7 @@ struct GroupCombineParams {
     uint64_t* res_cflag;        // [R]
     unsigned* ticket;
     void* combined_x;           // [T][H] bf16
+    int behind_publish;         // the reduce phase directly follows the publish phase of its call
     int tokens_per_block, tiles_per_block, span;  // set by the launcher (reduce phase of large batches)
 };
 cudaError_t launch_group_combine(const GroupCombineParams& p, const LaunchCtx& ctx);

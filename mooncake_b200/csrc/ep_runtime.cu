@@ -1185,6 +1185,7 @@ int mcep_combine(mcep_buffer* b, const mcep_combine_args* a, mcep_event** out_ev
     p.wait.hard_timeout_ns = b->hard_timeout_ns, p.wait.status = b->status;
     p.res_cflag = b->scratch[par].res_cflag, p.ticket = b->scratch[par].publish_ticket;
     p.combined_x = a->combined_x;
+    p.behind_publish = !a->return_recv_hook;
 
     const bool one_kernel = !a->return_recv_hook && b->one_kernel &&
                             mcep::group_call_can_be_one_kernel(T, K, E, num_sms);

@@ -163,6 +163,31 @@ def test_a_layout_kernel_for_small_batches(T, staged):
     assert buf.runtime.status() == 0
 
 
+@pytest.mark.parametrize("T,H", [(320, 4096), (1024, 7168)])  # the two reduce kernels of a group
+def test_a_result_is_the_callers_until_its_hook_runs(T, H):
+    """Work between combine and its hook may still read the result's memory, also work that lets the next kernel
+    start early (a dispatch of these rows); without a hook the phases of a call overlap."""
+    E = K = 8
+    x, idx, w = (t.cuda() for t in make_rank_inputs(23, 0, T, H, E, K))
+    buf = Buffer(FakeGroup(0, 1), Buffer.get_ep_buffer_size_hint(T, H, 1, E))
+    buf.runtime.set_option("force_staged", 1)
+    other = Buffer(FakeGroup(0, 1), 0)
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    recv, _, handle, _, _ = buf.dispatch(x, idx, active, T, E, 2_000_000, use_fp8=False)
+    want, _, _ = buf.combine(recv, idx, w, active, 2_000_000, handle)
+    for _ in range(4):
+        recv, _, handle, _, hook = buf.dispatch(x, idx, active, T, E, 2_000_000, use_fp8=False, return_recv_hook=True)
+        hook()
+        out = torch.full((T, H), 7.0, dtype=torch.bfloat16, device="cuda")
+        _, _, hook = buf.combine(recv, idx, w, active, 2_000_000, handle, return_recv_hook=True, out=out)
+        between, count, _, _, _ = other.dispatch(out, idx, active, T, E, 2_000_000, use_fp8=False)
+        hook()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        assert all(bool((between[e, :n] == 7).all()) for e, n in enumerate(count.tolist()))
+    assert buf.runtime.status() == 0
+
+
 @pytest.mark.parametrize("T", [2, 150])
 def test_rows_of_more_blocks_than_are_resident(T):
     """Rows so long that one alone is shared by more combine blocks than the device holds at a time."""
