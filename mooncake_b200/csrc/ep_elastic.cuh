@@ -100,6 +100,7 @@ struct ElasticSingleParams {
     int C;                       // tokens per block of the copy kernel, and behind a layout kernel
     int warps_per_row, parts;    // the warps and the blocks that share a row (set by the launcher)
     bool x_last;                 // see layer_beyond_l2 (set by the launcher)
+    bool own_segments;
     int max_rows;                // expanded: rows recv_x has room for
     int32_t* status;
     int32_t* rows;               // kept for combine: [T] received row of the token, or (expanded) [T][K] row
@@ -120,10 +121,11 @@ struct ElasticSingleParams {
     RouteBits bits;              // behind a layout kernel: row 0 all tokens that name an expert, 1 + e (expanded)
                                  // those that name e
     unsigned long long* totals;  // [E] listings and rows of the experts, zero between calls
-    int32_t* starts;             // [E + 1] expanded: where the experts' segments start
+    union {                      // expanded
+        int32_t* starts;         // [E + 1] where the experts' segments start, or (own_segments)
+        uint16_t* listings;      // [E][chunks, padded] of every chunk, segments made of them in the copy kernel
+    };
     unsigned* ticket;            // expanded: chunks that are done
-    uint16_t* listings;          // expanded, no starts: [E][listings_stride] of every chunk, segments made of them in
-    int listings_stride;         // the copy kernel
 };
 // The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
 struct SingleTables {

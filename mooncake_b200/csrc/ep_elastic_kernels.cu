@@ -482,13 +482,14 @@ __device__ __forceinline__ void take_totals(const ElasticSingleParams& p, Use us
 constexpr int kOwnChunks = 16, kOwnExperts = 256;
 constexpr int kElasticWarps = 4, kElasticTiles = 2;  // of the copy kernel: see there
 
-// [E][listings_stride] words, the ones of chunks that there are not are zero.
+// [E][chunks, a multiple of 8] words, the ones of chunks that there are not are zero.
 __host__ __device__ constexpr int listings_stride_of(int chunks) { return (chunks + 7) / 8 * 8; }
 __device__ __forceinline__ void leave_listings(const ElasticSingleParams& p, int e, int listings) {
-    uint16_t* row = p.listings + (size_t)e * p.listings_stride;
+    const int stride = listings_stride_of(gridDim.x);
+    uint16_t* row = p.listings + (size_t)e * stride;
     row[blockIdx.x] = (uint16_t)listings;
     if (blockIdx.x == gridDim.x - 1)
-        for (int c = gridDim.x; c < p.listings_stride; ++c) row[c] = 0;
+        for (int c = gridDim.x; c < stride; ++c) row[c] = 0;
 }
 __device__ __forceinline__ int sum_words(const uint4& v) {
     const uint32_t s = (v.x & 0xffffu) + (v.y & 0xffffu) + (v.z & 0xffffu) + (v.w & 0xffffu);
@@ -505,7 +506,7 @@ struct OwnSegments {
     const int per, first;
 
     __device__ __forceinline__ static const uint4* row(const ElasticSingleParams& p, int e) {
-        return reinterpret_cast<const uint4*>(p.listings + e * p.listings_stride);
+        return reinterpret_cast<const uint4*>(p.listings + e * listings_stride_of(p.bits.chunks));
     }
     __device__ __forceinline__ OwnSegments(const ElasticSingleParams& p, Shared& shared)
         : s(shared), per((p.E + blockDim.x - 1) / blockDim.x), first(threadIdx.x * per) {}
@@ -514,7 +515,7 @@ struct OwnSegments {
         int sum = 0;
         for (int x = first; x < min(first + per, p.E); ++x) {
             int n = sum_words(ld_ro(row(p, x)));
-            if (p.listings_stride > 8) n += sum_words(ld_ro(row(p, x) + 1));
+            if (p.bits.chunks > 8) n += sum_words(ld_ro(row(p, x) + 1));
             s.expert[x] = sum;
             sum += p.alignment == 1 ? n : aligned_count(n, p.alignment);
         }
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSi
         p.bits.words[(size_t)blockIdx.x * p.bits.experts + x] = m;
         p.bits.counts[(size_t)x * p.bits.stride + blockIdx.x] = (uint8_t)n;
         if (!kExpand || x == 0) continue;
-        if (p.listings != nullptr)
+        if (p.own_segments)
             leave_listings(p, x - 1, n + extra[x - 1]);
         else
             add_hits(p, x - 1, n + extra[x - 1], n);
@@ -583,7 +584,7 @@ __global__ void __launch_bounds__(kBitsThreads) ep_elastic_bits_kernel(ElasticSi
         for (int x = tid; x < p.E; x += kBitsThreads) add_hits(p, x, extra[x], 0);
         return;
     }
-    if (p.listings != nullptr) return;  // the copy kernel makes the segments
+    if (p.own_segments) return;  // the copy kernel makes the segments
     __threadfence();
     __syncthreads();
     if (tid == 0) s_last = atomicInc(p.ticket, gridDim.x - 1) == gridDim.x - 1;
@@ -1002,9 +1003,12 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         return launch_kernel("ep_elastic_single_copy", k, dim3(1 + (p.T + p.C - 1) / p.C), dim3(warps * 32),
                              (size_t)(2 * p.E + 1) * sizeof(int), 1, ctx, p);
     }
-    p.bits = tables.bits, p.starts = tables.starts, p.ticket = tables.ticket;
+    p.bits = tables.bits, p.ticket = tables.ticket, p.own_segments = tables.listings != nullptr;
+    if (p.own_segments)
+        p.listings = tables.listings;
+    else
+        p.starts = tables.starts;
     p.x_last = layer_beyond_l2(p.T, expand ? p.K : 1, p.H);
-    p.listings = tables.listings, p.listings_stride = listings_stride_of(p.bits.chunks);
     auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
     const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
     if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;
@@ -1017,9 +1021,9 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
     p.parts = (warps + kElasticWarps - 1) / kElasticWarps;
     p.warps_per_row = (warps + p.parts - 1) / p.parts;
     p.C = kElasticWarps / p.warps_per_row;
-    auto k = p.listings ? ep_elastic_rows_kernel<true, true>
-             : expand   ? ep_elastic_rows_kernel<true, false>
-                        : ep_elastic_rows_kernel<false, false>;
+    auto k = p.own_segments ? ep_elastic_rows_kernel<true, true>
+             : expand           ? ep_elastic_rows_kernel<true, false>
+                                : ep_elastic_rows_kernel<false, false>;
     return launch_kernel("ep_elastic_rows", k, dim3(1 + (p.T + p.C - 1) / p.C * p.parts),
                          dim3(p.C * p.warps_per_row * 32), expand ? 0 : ((size_t)p.E + 1) * sizeof(int), 1, chained, p);
 }
