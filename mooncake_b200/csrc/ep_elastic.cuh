@@ -32,7 +32,9 @@ struct ElasticRouteParams {
     int64_t* copied_topk_idx;    // [T][K] copy of topk_idx kept with the handle, or null
     void* const* record_base;    // [R] every rank's record area of this call's parity (null: not mapped)
     int record_stride;
+    char fill[16];
 };
+static_assert(cheap_to_launch<ElasticRouteParams>);
 cudaError_t launch_elastic_route(const ElasticRouteParams& p, cudaStream_t stream);
 
 struct ElasticEpilogueParams {
@@ -51,7 +53,9 @@ struct ElasticEpilogueParams {
     int32_t* hist;                // [L] scratch, zero between calls
     unsigned* ticket;             // scratch word, zero between calls
     int32_t* status;
+    char fill[40];
 };
+static_assert(cheap_to_launch<ElasticEpilogueParams>);
 cudaError_t launch_elastic_epilogue(const ElasticEpilogueParams& p, int num_sms, cudaStream_t stream,
                                     bool pdl);
 
@@ -70,7 +74,9 @@ struct ElasticExpandParams {
     float* recv_topk_weights;     // [max_rows] or null
     int max_rows;                 // rows that aligned segments push beyond are dropped (metadata -1, status)
     int32_t* status;
+    char fill[56];
 };
+static_assert(cheap_to_launch<ElasticExpandParams>);
 cudaError_t launch_elastic_expand_scan(const ElasticExpandParams& p, cudaStream_t stream);
 cudaError_t launch_elastic_expand_copy(const ElasticExpandParams& p, int num_sms, cudaStream_t stream);
 
@@ -83,7 +89,9 @@ struct ElasticLocalReduceParams {
     const void* x;                    // [x_rows][H] bf16
     int R, K, H, x_rows;
     void* y;                          // [n][H] bf16
+    char fill[48];
 };
+static_assert(cheap_to_launch<ElasticLocalReduceParams>);
 cudaError_t launch_elastic_local_reduce(const ElasticLocalReduceParams& p, int num_sms,
                                         cudaStream_t stream);
 
@@ -127,6 +135,7 @@ struct ElasticSingleParams {
     };
     unsigned* ticket;            // expanded: chunks that are done
 };
+static_assert(cheap_to_launch<ElasticSingleParams>);
 // The tables of the layout kernel; bits.words null: no launch of its own, the copy kernel counts.
 struct SingleTables {
     RouteBits bits = {};

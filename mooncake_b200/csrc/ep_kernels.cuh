@@ -22,6 +22,16 @@ constexpr int kStatusHardTimeout = 2;
 constexpr int kStatusBadSource = 4;
 constexpr int kStatusNoPeer = 8;  // a rank marked active has no mapped buffer
 
+// What a launch costs the host depends on the size of the kernel's parameters: 1.67 us where it is
+// 32 bytes beyond a multiple of 64 (32, 96, 160, 224, 288, 352), 2.0 - 2.1 for any other from 16 to
+// 1024 (with programmatic serialisation; without 2.0 and 2.5). So parameter blocks are filled up to
+// such a size (us per layer: one token in FP8 10.1 -> 9.8, 128 of 4 KB in bf16 9.9 -> 9.6, elastic decode
+// call of 128 14.2 -> 13.8, expanded, waiting, 1024 30.1 -> 29.4). Not the layout kernel's: calls that have one
+// are the device's, and asynchronous ones lose by a host that is further ahead, as every event between
+// the streams is then waited for (1000 rows of 8 KB to 2 15.7 -> 18.6).
+template <typename P>
+constexpr bool cheap_to_launch = sizeof(P) % 64 == 32;
+
 struct LaunchCtx {
     cudaStream_t stream;
     int num_sms;
@@ -84,6 +94,7 @@ struct DirectDispatchParams {
                                                  // share a row (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
 };
+static_assert(cheap_to_launch<DirectDispatchParams>);
 // whether the send kernels count the slots themselves for this many tokens
 bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group);
 // Whether the input of a layer, `copies` rows of each token and the result are so many bytes that the
@@ -106,7 +117,9 @@ struct CombineInvertParams {
     int L, R, M, T, K, rank;
     int32_t* rowmap;            // scratch [T*K]
     int32_t* status;
+    char fill[32];
 };
+static_assert(cheap_to_launch<CombineInvertParams>);
 cudaError_t launch_combine_invert(const CombineInvertParams& p, const LaunchCtx& ctx);
 
 struct DirectCombineParams {
@@ -125,7 +138,9 @@ struct DirectCombineParams {
     const int32_t* src_info;
     const int64_t* layout_range;
     void* combined_x;           // [T][H] bf16
+    char fill[48];
 };
+static_assert(cheap_to_launch<DirectCombineParams>);
 cudaError_t launch_direct_combine(DirectCombineParams p, const LaunchCtx& ctx);
 
 // ---- groups: words exchanged through symmetric memory -----------------------------
@@ -183,7 +198,9 @@ struct GroupDispatchParams {
     RouteBits bits;             // from the layout kernel (words null: none)
     bool x_last;                // see layer_beyond_l2 (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
+    char fill[40];
 };
+static_assert(cheap_to_launch<GroupDispatchParams>);
 bool group_call_can_be_one_kernel(int T, int K, int E, int num_sms);
 // one launch: control + send + receive duties
 cudaError_t launch_group_dispatch(GroupDispatchParams p, const LaunchCtx& ctx);
@@ -215,7 +232,9 @@ struct GroupCombineParams {
     void* combined_x;           // [T][H] bf16
     int behind_publish;         // the reduce phase directly follows the publish phase of its call
     int tokens_per_block, tiles_per_block, span;  // set by the launcher (reduce phase of large batches)
+    char fill[8];
 };
+static_assert(cheap_to_launch<GroupCombineParams>);
 cudaError_t launch_group_combine(const GroupCombineParams& p, const LaunchCtx& ctx);
 cudaError_t launch_group_combine_publish(const GroupCombineParams& p, const LaunchCtx& ctx);
 cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& ctx);
@@ -244,7 +263,9 @@ struct BarrierParams {
     uint32_t epoch;
     int64_t hard_timeout_ns;
     int32_t* status;
+    char fill[32];
 };
+static_assert(cheap_to_launch<BarrierParams>);
 cudaError_t launch_barrier(const BarrierParams& p, const LaunchCtx& ctx);
 
 // Graph mode: after the last kernel of a call, the word that holds the next
