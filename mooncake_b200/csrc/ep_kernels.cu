@@ -28,6 +28,7 @@
 #include "ep_kernels.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -954,8 +955,8 @@ __device__ __forceinline__ bool send_tokens(const SendView& v, int sid, int nsen
 // =============================================================================
 // single rank: dispatch writes the packed outputs directly
 // =============================================================================
-// Small batches (counts_in_send_kernel), in one launch: bound by latency, index load ->
-// count -> row stores, one batch per block.
+// Small batches (counts_in_send_kernel) of several tokens per block, in one launch: bound by latency,
+// index load -> count -> row stores, one batch per block.
 template <bool kFP8>
 __global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectDispatchParams p) {
     extern __shared__ int smem_i32[];  // [E]
@@ -971,6 +972,113 @@ __global__ void __launch_bounds__(512, 2) ep_dispatch_send_direct_kernel(DirectD
     v.recv_src_info = p.recv_src_info, v.row_bytes = p.H * (kFP8 ? 1 : 2);
     v.rowmap = p.rowmap, v.recv_count = p.recv_count, v.layout_range = p.layout_range;
     send_tokens<kFP8, false, true>(v, blockIdx.x, gridDim.x, smem_i32);
+}
+
+// The same with a token per block (one_token_per_block): what the kernel above spends between its
+// three barriers - a table of all experts, atomics into it, the entries of the batch compared with
+// one another - is here a comparison of every earlier token's choices with this token's own, a
+// thread per token, and one barrier. The last block counts for the outputs. Device time per layer,
+// table | comparison: 1 token of 14 KB in FP8 to 8 7.3 us | 6.0, 128 10.4 | 9.4, 256 of 8 KB 10.0 | 9.4; 128 of 4 KB in
+// bf16 to 4 6.0 | 4.9.
+template <bool kFP8, int KB>
+__device__ __forceinline__ void send_one_token(const DirectDispatchParams& p, int (*s_part)[KB]) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+    const int t = blockIdx.x, K = p.K, M = p.M, nchunks = p.H / 16, ntiles = (p.H + kTileChannels - 1) / kTileChannels;
+    const bool vec = choices_in_pairs(p.topk_idx, K);
+    auto load_tile = [&](int tile) {
+        V32 r = {};
+        const int c = tile * 32 + lane;
+        if (c < nchunks) r = ld32_readonly(static_cast<const char*>(p.x) + ((size_t)t * p.H + (size_t)c * 16) * 2);
+        return r;
+    };
+    V32 row = load_tile(warp);
+    int e = -1, own[KB];
+    if (lane < K) e = (int)ld_ro(p.topk_idx + (size_t)t * K + lane);
+    load_choices<KB, false>(p.topk_idx, t, K, p.E, vec, own);
+    int n = 0;  // lane k: earlier tokens of this warp's that chose the k-th expert
+    for (int j0 = warp * 32; j0 < t; j0 += nthr) {
+        unsigned same = 0;
+        if (j0 + lane < t) {
+            int other[KB];
+            load_choices<KB, false>(p.topk_idx, j0 + lane, K, p.E, vec, other);
+#pragma unroll
+            for (int k = 0; k < KB; ++k) {
+                bool hit = false;
+#pragma unroll
+                for (int a = 0; a < KB; ++a) hit |= other[a] == own[k];
+                if (hit) same |= 1u << k;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KB; ++k) {
+            const unsigned hits = __ballot_sync(kFull, (same >> k) & 1u);
+            if (lane == k) n += __popc(hits);
+        }
+    }
+    const int counting = min(nwarps, (t + 31) / 32);  // warps that have counted
+    if (t > 0) {
+        if (lane < KB && warp < counting) s_part[warp][lane] = n;
+        __syncthreads();
+    }
+    // (a repeated expert has the same row and gets the same bytes twice)
+    int s = -1;
+    if (lane < K && e >= 0 && e < p.E) {
+        s = 0;
+        for (int w = 0; w < counting; ++w) s += s_part[w][lane];
+        if (s >= M) {
+            atomicOr(p.status, kStatusSlotRange);
+            s = -1;
+        }
+    }
+    const int to = s >= 0 ? e * M + s : -1;  // (31 bits: the launcher)
+    if (warp == 0 && lane < K) {
+        p.rowmap[(size_t)t * K + lane] = s;
+        if (s >= 0) p.recv_src_info[to] = t;
+    }
+    char* out = static_cast<char*>(p.recv_x);
+    const int S = p.H / 128, at = s >= 0 ? e * S * M + s : 0;
+    for (int tile = warp; tile < ntiles; tile += nwarps) {
+        if (tile != warp) row = load_tile(tile);
+        const int c = tile * 32 + lane;
+        if (kFP8) {
+            float sinv;
+            const uint4 q = quantize16(row, sinv);
+#pragma unroll 4
+            for (int k = 0; k < K; ++k) {
+                const int r = __shfl_sync(kFull, to, k), sr = __shfl_sync(kFull, at, k);
+                if (r < 0 || c >= nchunks) continue;
+                st16(out + (size_t)r * p.H + (size_t)c * 16, q);
+                if ((lane & 7) == 0) p.recv_scales[(size_t)sr + (size_t)(c >> 3) * M] = sinv;
+            }
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < K; ++k) {
+                const int r = __shfl_sync(kFull, to, k);
+                if (r >= 0 && c < nchunks) st32(out + (size_t)r * p.H * 2 + (size_t)c * 32, row);
+            }
+        }
+    }
+}
+
+template <bool kFP8, int KB>
+__global__ void __launch_bounds__(512, 2) ep_dispatch_one_token_kernel(DirectDispatchParams p) {
+    extern __shared__ int smem_i32[];  // [E]
+    __shared__ int s_part[16][KB];
+    const bool counts = (int)blockIdx.x == p.T;
+    if (counts) {
+        for (int i = threadIdx.x; i < p.E; i += blockDim.x) smem_i32[i] = 0;
+        __syncthreads();
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!counts) return send_one_token<kFP8, KB>(p, s_part);
+    count_tokens_of<KB, 1, false>(p.topk_idx, 0, p.T, p.K, p.E, choices_in_pairs(p.topk_idx, p.K), smem_i32);
+    __syncthreads();
+    for (int x = threadIdx.x; x < p.E; x += blockDim.x) {
+        const int n = smem_i32[x];
+        p.recv_count[x] = n;
+        p.layout_range[x] = n;  // begin 0 | count
+    }
 }
 
 // The counts of a batch whose layout is there as bits; whole block. The first block does it once
@@ -2224,6 +2332,15 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool group) {
     return s;
 }
 
+// Batches that count for themselves, a token per block instead of several (device time per layer,
+// several | one: 300 tokens of 1 KB in FP8 to 8 8.5 us | 7.6, of 8 KB to 2 7.6 | 6.3, to 1 6.7 | 6.0; 400 9.3 | 8.9, 7.8 | 7.4
+// and 6.8 | 6.6, of 4 KB to 8 10.3 | 10.0; 500 10.0 | 9.8, 8.1 | 7.5, but 7.0 | 7.1 and 10.8 | 11.1; 1100 of 4 KB to 1 8.1 | 11.5):
+// as many as are resident at a time, at two blocks of 16 warps, and three per SM, as each compares
+// itself with all earlier ones.
+static bool one_token_per_block(int T, int warps, int num_sms) {
+    return T > 0 && T <= 3 * num_sms && T < 2 * num_sms * (16 / warps);
+}
+
 bool layer_beyond_l2(long long T, int copies, int H) { return T * (copies + 2) * H * 2 > 40ll << 20; }
 
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
@@ -2259,6 +2376,17 @@ cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx)
         const int groups = (p.T + p.tokens_per_block - 1) / p.tokens_per_block;
         return launch("ep_dispatch_rows", k, dim3(groups * p.parts), dim3(32 * p.warps_per_row * p.tokens_per_block), 0,
                       ctx, p);
+    }
+    const int ntiles = (p.H + kTileChannels - 1) / kTileChannels, warps = ntiles < 4 ? 4 : ntiles < 16 ? ntiles : 16;
+    if (one_token_per_block(p.T, warps, ctx.num_sms) && (long long)p.E * p.M * (p.H / 128) <= INT_MAX) {
+        void (*one)(DirectDispatchParams) = nullptr;
+        if (p.K <= 4)
+            one = p.use_fp8 ? ep_dispatch_one_token_kernel<true, 4> : ep_dispatch_one_token_kernel<false, 4>;
+        else if (p.K <= 8)
+            one = p.use_fp8 ? ep_dispatch_one_token_kernel<true, 8> : ep_dispatch_one_token_kernel<false, 8>;
+        else
+            one = p.use_fp8 ? ep_dispatch_one_token_kernel<true, 16> : ep_dispatch_one_token_kernel<false, 16>;
+        return launch("ep_dispatch_send_direct", one, dim3(p.T + 1), dim3(32 * warps), (size_t)p.E * sizeof(int), ctx, p);
     }
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, false);
     p.C = s.tokens;

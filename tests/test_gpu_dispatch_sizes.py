@@ -100,7 +100,10 @@ def test_positions_from_the_layout_kernel(T, H, E, K, fp8):
     # either side of where the layout kernel begins: 12 MB to one and two, 17 MB and a token per SM to more
     (1535, 4096, 8, 1, True), (1536, 4096, 8, 1, False), (767, 4096, 8, 2, True), (768, 4096, 8, 2, False),
     (271, 4096, 8, 8, True), (272, 4096, 8, 8, False), (297, 1664, 16, 16, True), (592, 128, 16, 16, True),
-    (593, 128, 16, 16, False), (148, 8320, 8, 8, True), (149, 8320, 8, 8, False)])
+    (593, 128, 16, 16, False), (148, 8320, 8, 8, True), (149, 8320, 8, 8, False),
+    # a token per block: one warp's tokens and more, several rounds of them, more tiles than warps, its end
+    (1, 4224, 24, 16, True), (32, 128, 8, 5, True), (33, 640, 4096, 1, True), (129, 2048, 8, 3, True), (444, 128, 9, 8, True),
+    (444, 4096, 16, 1, True), (445, 640, 9, 4, True), (147, 8704, 16, 7, True), (295, 4224, 8, 2, True), (296, 4224, 8, 2, True)])
 def test_batches_that_count_for_themselves(T, H, E, K, counted, fp8):
     """Positions counted in the send kernel of a single rank, repeats and empty tokens among them, up to
     the sizes that it is used for; which kernel ran is looked up, so that the sizes follow the rule."""
