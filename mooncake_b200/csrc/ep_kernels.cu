@@ -1227,10 +1227,10 @@ __global__ void __launch_bounds__(256) ep_combine_invert_kernel(CombineInvertPar
 // channels: up to K 32-byte loads in flight, fp32 FMA accumulation in k order,
 // one bf16 rounding, one 32-byte store (mooncake_ep_kernel.cu:715-752).
 // kDepth rows are requested before the first of them is used. s_ptr has kMaxTopk
-// entries, null where nothing is to be added.
+// entries, null where nothing is to be added. hold: the kernel ahead is waited for before a store.
 template <int kDepth, bool kReadOnly, bool kLast>
 __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const float* s_w, int K,
-                                            int H, void* out_row) {
+                                            int H, void* out_row, bool hold = false) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int nchunks = H / 16;
     const int ntiles = (H + kTileChannels - 1) / kTileChannels;
@@ -1260,6 +1260,7 @@ __device__ __forceinline__ void reduce_rows(const char* const* s_ptr, const floa
                 }
             }
         }
+        if (hold) pdl_wait();
         st32(reinterpret_cast<char*>(out_row) + (size_t)c * 32, pack_bf16x16(acc));
     }
 }
@@ -1827,7 +1828,7 @@ __global__ void __launch_bounds__(512)
 // stream sees as done is done. One rank on this path, us per layer with this, the reduce phase's like
 // (ep_combine_kernel), the own counts taken directly and the first tiles ahead of the layout's end:
 // 400 tokens of 14 KB to 8 29.3 -> 26.5, 1024 of 4 KB 24.7 -> 22.1, 2048 of 14 KB 95.3 -> 92.1; in hook mode
-// 27.9, 23.3 and 93.3, 1024 of 8 KB 36.9 -> 35.0.
+// with the wait where the result is stored 26.5, 22.1 and 92.1, 1024 of 8 KB 36.9 -> 33.4.
 template <bool kFP8>
 __global__ void __launch_bounds__(kRowWarps * 32, 4) ep_dispatch_recv_kernel(GroupDispatchParams p) {
     extern __shared__ int smem_i32[];
@@ -1950,7 +1951,7 @@ __device__ __forceinline__ void combine_publish_duty(const GroupCombineParams& p
 // marked inactive), contributes nothing (mooncake_ep_kernel.cu:685-699, 728-732).
 template <bool kLast>
 __device__ __forceinline__ void combine_reduce_duty(const GroupCombineParams& p, int first_token, int token_stride,
-                                                    char* const* s_peer, const int* s_active) {
+                                                    char* const* s_peer, const int* s_active, bool hold) {
     __shared__ const char* s_ptr[kMaxTopk];
     __shared__ float s_w[kMaxTopk];
     const int tid = threadIdx.x;
@@ -1984,7 +1985,7 @@ __device__ __forceinline__ void combine_reduce_duty(const GroupCombineParams& p,
         __syncthreads();
         if (t == first_token) MCEP_TRACE(2, 4);  // the owners' words are in, rows can be read
         reduce_rows<8, false, kLast>(s_ptr, s_w, p.K, p.H,
-                                     reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2);
+                                     reinterpret_cast<char*>(p.combined_x) + (size_t)t * p.H * 2, hold);
         __syncthreads();  // the rows are done with s_ptr
     }
 }
@@ -2003,24 +2004,25 @@ __device__ __forceinline__ void combine_body(const GroupCombineParams& p, int bi
     if (kPhases & 1) combine_publish_duty(p, bid, nblocks, smem_i32, s_peer, s_active, first_lr);
     MCEP_TRACE(2, 1);
     if (kPhases & 2) {
-        combine_reduce_duty<kLast>(p, bid, nblocks, s_peer, s_active);
+        combine_reduce_duty<kLast>(p, bid, nblocks, s_peer, s_active, kPhases == 2 && !p.behind_publish);
     }
     MCEP_TRACE(2, 2);
 }
 
-// behind_publish: what the reduce phase reads was complete when the publish phase, the kernel ahead of
-// it, began - that kernel lets the next one start only once it has waited for all before it - and a
-// peer's rows come with the peer's word. So it starts beside the publish phase, and only ends behind
-// it. A hook's reduce phase waits at its top: the caller may have put work between, which may still
-// read the result's memory.
+// What the reduce phase reads was complete when the publish phase began - that kernel lets the next
+// one start only once it has waited for all before it - and a peer's rows come with the peer's word.
+// So it starts beside the publish phase (or what the caller has put between), and only ends behind
+// it. With a hook (not behind_publish) that work may still read the result's memory: nothing is
+// stored there before it has finished. Waiting at the top, hook mode, one rank on this path, us per layer:
+// 1024 tokens of 8 KB to 8 34.8, so 33.4; 400 of 4 KB in FP8 17.3 and 15.9; 250 of 14 KB 22.3 and 20.9.
 template <int kPhases, bool kLast = false>
 __global__ void __launch_bounds__(512) ep_combine_kernel(GroupCombineParams p) {
     extern __shared__ int smem_i32[];
-    if (kPhases != 2 || !p.behind_publish) pdl_wait();
+    if (kPhases != 2) pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     combine_body<kPhases, kLast>(p, blockIdx.x, gridDim.x, smem_i32);
-    if (kPhases == 2 && p.behind_publish) pdl_wait();
+    if (kPhases == 2) pdl_wait();
 }
 
 // The reduce duty of batches with more tokens than SMs, in a launch of its own: as
@@ -2038,7 +2040,6 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
     const int sub = warp / p.tiles_per_block;
     const int c = ((warp - sub * p.tiles_per_block + blockIdx.y * p.tiles_per_block) * 32) + lane;
     const bool act = c < p.H / 16;
-    if (!p.behind_publish) pdl_wait();
     pdl_launch_dependents();
     resolve_seq(p);
     const int L = p.E / p.R, RM = p.R * p.M;
@@ -2122,11 +2123,12 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
                 }
             }
         }
+        if (!p.behind_publish && t0 == first) pdl_wait();
         if (act && t0 + sub < end)
             st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + sub) * row_bytes + (size_t)c * 32,
                  pack_bf16x16(acc), kLast && p.K > 1);
     }
-    if (p.behind_publish) pdl_wait();
+    pdl_wait();
 }
 
 // All logical ranks of an in-process group in one cooperative launch (see

@@ -230,7 +230,7 @@ struct GroupCombineParams {
     uint64_t* res_cflag;        // [R]
     unsigned* ticket;
     void* combined_x;           // [T][H] bf16
-    int behind_publish;         // the reduce phase directly follows the publish phase of its call
+    int behind_publish;         // the reduce phase directly follows the publish phase of its call (no hook)
     int tokens_per_block, tiles_per_block, span;  // set by the launcher (reduce phase of large batches)
     char fill[8];
 };
