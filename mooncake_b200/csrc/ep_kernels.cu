@@ -338,6 +338,18 @@ __device__ __forceinline__ uint32_t wait_local_word(const uint64_t* word, uint32
     }
 }
 
+// The same from a kernel that may have started beside the writer's, which is ahead of it in the
+// stream: looked at for a while only, then that kernel's end is waited for, which has the word.
+__device__ __forceinline__ uint32_t local_word_of_kernel_ahead(const uint64_t* word, uint32_t seq, const WaitCfg& w) {
+    const uint64_t start = globaltimer_ns();
+    do {
+        const uint64_t v = ld_acquire_gpu(word);
+        if ((uint32_t)(v >> 32) == seq) return (uint32_t)v;
+    } while (globaltimer_ns() - start < 50000);
+    pdl_wait();
+    return wait_local_word(word, seq, w);
+}
+
 // =============================================================================
 // phase trace (diagnostic builds only: -DMCEP_PHASE_TRACE)
 // =============================================================================
@@ -1550,7 +1562,8 @@ __device__ __forceinline__ void dispatch_control(const GroupDispatchParams& p, i
 // final tensors.)
 constexpr int kRowWarps = 8;
 
-template <bool kFP8>
+// kAlone: in a kernel of its own, behind the control block's.
+template <bool kFP8, bool kAlone>
 __device__ __forceinline__ void dispatch_recv_duty(const GroupDispatchParams& p, int j, int np,
                                                    int* smem_i32) {
     const int L = p.E / p.R, n = L * p.R;
@@ -1570,7 +1583,8 @@ __device__ __forceinline__ void dispatch_recv_duty(const GroupDispatchParams& p,
     // the control block's verdicts: what every source sends to every local expert
     bool from_peers = false;
     for (int i = tid; i < n; i += nthr) {
-        const uint32_t v = wait_local_word(p.res_cnt + i, p.seq, scaled(p.wait, 2));
+        const uint32_t v = kAlone ? local_word_of_kernel_ahead(p.res_cnt + i, p.seq, scaled(p.wait, 2))
+                                  : wait_local_word(p.res_cnt + i, p.seq, scaled(p.wait, 2));
         const int c = v ? (int)v - 1 : 0;
         pre[i] = c;
         if (c) atomicAdd(&s_tot[i % p.R], c);
@@ -1710,7 +1724,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
         dispatch_control(p, smem_i32, s_peer, s_active);
         if (kPhases == 3) {
             __syncthreads();
-            dispatch_recv_duty<kFP8>(p, nh, nh + 1, smem_i32);
+            dispatch_recv_duty<kFP8, false>(p, nh, nh + 1, smem_i32);
         }
         return;
     }
@@ -1755,7 +1769,7 @@ __device__ __forceinline__ void dispatch_body(const GroupDispatchParams& p, int 
     }
     if (kPhases == 3 && ticket >= nsend - nh) {
         __syncthreads();
-        dispatch_recv_duty<kFP8>(p, ticket - (nsend - nh), nh + 1, smem_i32);
+        dispatch_recv_duty<kFP8, false>(p, ticket - (nsend - nh), nh + 1, smem_i32);
     }
 }
 
@@ -1835,7 +1849,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 4) ep_dispatch_recv_kernel(Gro
     pdl_launch_dependents();
     resolve_seq(p);
     MCEP_TRACE(1, 0);
-    dispatch_recv_duty<kFP8>(p, blockIdx.x, gridDim.x, smem_i32);
+    dispatch_recv_duty<kFP8, true>(p, blockIdx.x, gridDim.x, smem_i32);
     pdl_wait();
 }
 
