@@ -2296,21 +2296,14 @@ cudaError_t launch_layout(const LayoutParams& p, const LaunchCtx& ctx) {
                   ctx, p, epc, words);
 }
 
-bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group, bool hook) {
-    // A group's sender blocks are one resident wave, a token each: one launch that counts for itself,
-    // or, with the layout kernel, a wave of smaller blocks and a receive and a reduce kernel that start
-    // beside the ones ahead of them (one rank on this path, us per layer to 8, counting | layout kernel: rows
-    // of 4 KB in bf16 150 tokens 11.4 | 12.6, 292 14.4 | 13.8, in FP8 13.9 | 14.0; of 14 KB in bf16 150 18.3 | 18.4, 292
-    // 20.3 | 21.4, in FP8 23.2 | 24.2; of 11 KB 285 17.7 | 19.6). Rows of up to 8 KB, whose smaller blocks are two
-    // to an SM, are faster behind the layout kernel from 12.5 MB on: of 8 KB in bf16 185 (12 MB) 13.5 | 15.3, 200 (13 MB)
-    // 16.4 | 15.3, 292 18.2 | 16.4, with hooks 19.1 | 17.6, in FP8 200 14.9 | 14.7, 292 17.8 | 16.8; of 6 KB 220 (11 MB) 15.3 | 14.7
-    // and in FP8 14.0 | 14.5, 285 (14 MB) 16.3 | 15.1 and 15.0 | 14.9; to 4, of 8 KB 285 (9 MB) 13.3 | 12.8 and 12.7 | 13.0;
-    // to 16, 240 (31 MB) 29.3 | 20.6 and 29.7 | 22.8. With hooks a layer is five launches in place of four, up to 18 us
-    // of the host: as a program sees it, in FP8 200 15.9 | 18.3, 240 (16 MB) 17.1 | 18.2, 292 (19 MB) 19.0 | 18.2.
-    const long long bytes = (long long)T * K * H * 2;
-    if (group)
-        return T <= 2 * num_sms &&
-               (4 * T <= 5 * num_sms || H > 8 * kTileChannels || bytes < (hook ? 36 << 19 : 25 << 19));
+bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group) {
+    // A group's sender blocks are one resident wave, a token each, and up to here a dispatch without a
+    // hook is one launch for all ranks of a process alike (group_call_can_be_one_kernel), whatever
+    // their tokens. One rank on this path, us per layer to 8, counting | layout kernel: rows of 4 KB
+    // in bf16 150 tokens 11.4 | 12.6, 292 14.4 | 13.8; of 14 KB 150 18.3 | 18.4, 292 20.3 | 21.4. Rows of
+    // 8 KB would take the layout kernel from 200 on (16.4 | 15.3, 292 18.2 | 16.4, in FP8 17.8 | 16.8), but
+    // three launches in place of one are not measured where peers have rows to move.
+    if (group) return T <= 2 * num_sms;
     // A single rank counts in one resident wave of blocks with as many tokens each as that
     // takes. The layout kernel is the faster one on the device at nearly every size, but a
     // layer of three launches takes the host 12.4 us and one of two 10: it is used where the
@@ -2321,6 +2314,7 @@ bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group, bool ho
     // 41.7, 8000 in FP8 76.6 | 71.1. Just below the line some lose: of 8 KB to 1, 1500 (12 MB) 11.0 | 11.7,
     // in FP8 12.2 | 11.8, and a stream that is ahead of the device has 12.4 | 10.7; of 2 KB to 2, 3000
     // 12.4 | 11.8.
+    const long long bytes = (long long)T * K * H * 2;
     if (K <= 2) return bytes < 12 << 20 && T <= 8192 / K;
     // From three on counting is slower by block: rows of 8 KB to 8 in FP8, 200 tokens (13 MB)
     // 10.0 | 12.4, 300 (20 MB) 13.5 | 12.4, 400 16.3 | 14.9; of 14 KB in bf16, 160 (18 MB) 15.2 |

@@ -96,7 +96,7 @@ struct DirectDispatchParams {
 };
 static_assert(cheap_to_launch<DirectDispatchParams>);
 // whether the send kernels count the slots themselves for this many tokens
-bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group, bool hook);
+bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group);
 // Whether the input of a layer, `copies` rows of each token and the result are so many bytes that the
 // last use of what is used up is worth telling L2 (ld32_readonly with `last`). Of less, all of it stays there anyway, and
 // what a caller uses again is not to be the first that goes (us per layer on three sets of inputs in turn, no

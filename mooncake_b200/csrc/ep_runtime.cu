@@ -931,7 +931,7 @@ int mcep_dispatch(mcep_buffer* b, const mcep_dispatch_args* a, mcep_event** out_
     // 2^31 rows or scales and more, whose places the kernel behind it does not tell apart.)
     const bool far_rows = !group && !places_fit_31_bits(E, M, fp8 ? H / 128 : 1);
     const bool counting = far_rows || ((b->fuse_layout || T == 0) &&
-                                       mcep::counts_in_send_kernel(T, K, H, b->num_sms, group, a->return_recv_hook != 0));
+                                       mcep::counts_in_send_kernel(T, K, H, b->num_sms, group));
     mcep::RouteBits bits = {};
     if (!counting) {
         mcep::LayoutParams lp = {};

@@ -139,6 +139,13 @@ def test_ranks_on_either_side_of_the_counting_limit(T, fp8, mode):
     _run_case(dict(R=len(T), tokens=list(T), M=320, H=128, E=8 * len(T), K=16, fp8=fp8, seed=3), mode=mode)
 
 
+@pytest.mark.parametrize("mode", ["hook", "sync"])
+@pytest.mark.parametrize("T,H,fp8", [((150, 250), 4096, False), ((150, 250), 4096, True), ((1, 294, 186), 4096, False)])
+def test_ranks_of_one_launch_differ_in_bytes(T, H, fp8, mode):
+    """In-process groups: ranks of up to two tokens per SM share a launch, however many bytes each of them sends."""
+    _run_case(dict(R=len(T), tokens=list(T), M=296, H=H, E=8 * len(T), K=8, fp8=fp8, seed=5), mode=mode)
+
+
 @pytest.mark.parametrize("staged", [False, True])
 @pytest.mark.parametrize("T", [0, 1, 40, 296])
 def test_a_layout_kernel_for_small_batches(T, staged):
