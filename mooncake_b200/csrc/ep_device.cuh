@@ -125,22 +125,17 @@ __device__ __forceinline__ void st32(void* p, const V32& r) {
 }
 // ---- what L2 should give up first -----------------------------------------------
 // A layer of a large batch moves more than the 126 MB of L2, and what stays there decides how much
-// of it HBM sees. Nobody reads the experts' outputs again once combine has them, nor, in general, a
-// dispatch's input: marked so, they make room instead of the rows that the next kernel wants
-// (bytes at the memory: 470 MB of rows handed straight to combine 437 read, marked 390; a flat
-// elastic combine of 59 MB 25, marked 0). us per layer, no mark | rows of combine | input of
-// dispatch too | combine's result too: 4096 rows of 14 KB to 8 in bf16 168.3 | 162.1 | 161.2 | 160.7, in FP8,
-// the outputs made long before, 147.0 | 147.0 | 147.0 | 139.8; 2000 of 8 KB to 8 47.4 | 44.2 | 43.6 | 43.3, 2001
-// in FP8 45.4 | 46.7 | 46.0 | 44.3; 4096 of 8 KB to 2 33.6 | 33.0 | 32.4 | 30.4; to 1, 4000 of 14 KB 38.5 | 38.1 |
-// 36.8 | 35.6; elastic training step of 4096 of 14 KB 78.4 | 76.6 | 74.3 | 73.9.
-// The result is read next, so the same in a program: a kernel that writes the input, dispatch, one
-// that makes the outputs from the rows, combine, one that adds the result to what there was: 2000
-// rows of 8 KB to 8 107.1 | 102.8 | 102.6 | 102.8, in FP8 239.4 | 236.2 | 234.8 | 235.6; 4096 of 14 KB to 8 354.0 | 348.5 |
-// 348.3 | 350.0; 4096 of 8 KB to 2 82.2 | 81.2 | 80.3 | 82.2; of 14 KB to 1 104.7 | 102.3 | 98.9 | 101.2, 3000 to 1 77.7 | - |
-// 75.6 | 79.3. So it is marked where it is the smaller part, not with one row per token (there FP8
-// rows whose outputs were made long before lose: 3000 of 14 KB to 1 33.7 | - | 34.5).
-// The received rows are what the next kernel wants: marked too, 165 us for the first of these.
-// The loads above, and a store of combine's result, with that mark where `last`.
+// of it HBM sees. Nobody reads the experts' outputs again once combine has them, nor, in many
+// models, a dispatch's input: marked evict-first, they make room for the rows that the next kernel wants.
+// (Bytes that combine read from memory: 437 of 470 MB of rows handed straight to it, marked 390; 25 of
+// the 59 MB of a flat elastic layer, marked 0.)
+// us of a program - a kernel that writes the input, dispatch, the experts' kernel, combine, one that
+// adds the result to what there was - with no mark | the experts' outputs | the input too: 2000 rows of
+// 8 KB to 8 107.3 | 103.4 | 103.0, in FP8 238.5 | 235.1 | 234.3; 4096 of 14 KB to 8 354.4 | 348.2 | 348.1, in FP8
+// 834 | 827.5 | 823.5; 4096 of 8 KB to 2 82.6 | 81.7 | 80.2; of 14 KB to 1 104.6 | 101.4 | 99.2.
+// Combine's result is not marked: the next kernel reads it (2 us more for the last but one, 1.5 for
+// 4096 of 14 KB to 8). The received rows are not either: they are what the next kernel wants.
+// The loads above, with that mark where `last`.
 __device__ __forceinline__ V32 ld32_readonly(const void* p, bool last) {
     if (!last) return ld32_readonly(p);
     V32 r;
@@ -161,14 +156,6 @@ __device__ __forceinline__ V32 ld32_coherent(const void* p, bool last) {
         : "l"(p)
         : "memory");
     return r;
-}
-__device__ __forceinline__ void st32(void* p, const V32& r, bool last) {
-    if (!last) return st32(p, r);
-    asm volatile(
-        "st.global.L1::no_allocate.L2::evict_first.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p),
-        "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]),
-        "r"(r.w[7])
-        : "memory");
 }
 __device__ __forceinline__ uint4 ld16_coherent(const void* p) {
     uint4 r;

@@ -1355,7 +1355,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, kBlocks) ep_combine_rows_ke
                 }
             }
         }
-        if (act && t0 + sub < end) st32(out + (size_t)(t0 + sub) * row_bytes, pack_bf16x16(acc), kLast);
+        if (act && t0 + sub < end) st32(out + (size_t)(t0 + sub) * row_bytes, pack_bf16x16(acc));
     }
 }
 
@@ -2140,7 +2140,7 @@ __global__ void __launch_bounds__(kReduceWarps * 32, 2) ep_combine_gather_kernel
         if (!p.behind_publish && t0 == first) pdl_wait();
         if (act && t0 + sub < end)
             st32(reinterpret_cast<char*>(p.combined_x) + (size_t)(t0 + sub) * row_bytes + (size_t)c * 32,
-                 pack_bf16x16(acc), kLast && p.K > 1);
+                 pack_bf16x16(acc));
     }
     pdl_wait();
 }
