@@ -125,8 +125,9 @@ __device__ __forceinline__ void st32(void* p, const V32& r) {
 }
 // ---- what L2 should give up first -----------------------------------------------
 // A layer of a large batch moves more than the 126 MB of L2, and what stays there decides how much
-// of it HBM sees. Nobody reads the experts' outputs again once combine has them, nor, in many
-// models, a dispatch's input: marked evict-first, they make room for the rows that the next kernel wants.
+// of it HBM sees. Nobody reads the experts' outputs again once combine has them, nor, where
+// input_beyond_l2 says so, finds a dispatch's input there: marked evict-first, they make room for the rows
+// that the next kernel wants.
 // (Bytes that combine read from memory: 437 of 470 MB of rows handed straight to it, marked 390; 25 of
 // the 59 MB of a flat elastic layer, marked 0.)
 // us of a program - a kernel that writes the input, dispatch, the experts' kernel, combine, one that

@@ -107,7 +107,7 @@ struct ElasticSingleParams {
     int T, K, E, H, alignment;
     int C;                       // tokens per block of the copy kernel, and behind a layout kernel
     int warps_per_row, parts;    // the warps and the blocks that share a row (set by the launcher)
-    bool x_last;                 // see layer_beyond_l2 (set by the launcher)
+    bool x_last;                 // see input_beyond_l2 (set by the launcher)
     bool own_segments;
     int max_rows;                // expanded: rows recv_x has room for
     int32_t* status;

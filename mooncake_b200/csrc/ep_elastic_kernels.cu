@@ -1008,7 +1008,7 @@ cudaError_t launch_elastic_single_dispatch(ElasticSingleParams p, bool expand, c
         p.listings = tables.listings;
     else
         p.starts = tables.starts;
-    p.x_last = layer_beyond_l2(p.T, expand ? p.K : 1, p.H);
+    p.x_last = input_beyond_l2(p.T, expand ? p.K : 1, p.H, false);
     auto layout = expand ? ep_elastic_bits_kernel<true> : ep_elastic_bits_kernel<false>;
     const size_t smem = (expand ? 1 + (size_t)p.E : 1) * sizeof(uint4) + ((size_t)p.E + 1) * sizeof(int);
     if (cudaError_t e = allow_shared_memory(reinterpret_cast<const void*>(layout), smem)) return e;

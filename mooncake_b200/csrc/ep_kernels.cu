@@ -768,7 +768,7 @@ struct SendView {
     int T, K, E, R, M, H, rank;
     int L, RM;
     int C;                    // tokens per batch
-    bool x_last;              // see layer_beyond_l2
+    bool x_last;              // see input_beyond_l2
     RouteBits bits;           // the layout kernel's bits (words null: none), or
     const int32_t* slot;      // [T*K] position among this rank's tokens for the expert (layout kernel),
                               // or null: counted here (small batches, one per block)
@@ -2359,10 +2359,13 @@ static bool one_token_per_block(int T, int warps, int num_sms) {
 }
 
 bool layer_beyond_l2(long long T, int copies, int H) { return T * (copies + 2) * H * 2 > 40ll << 20; }
+bool input_beyond_l2(long long T, int copies, int H, bool fp8) {
+    return fp8 ? layer_beyond_l2(T, copies, H) : T * (copies + 1) * H * 2 > 120ll << 20;
+}
 
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx) {
     if (!p.counting()) {
-        p.x_last = layer_beyond_l2(p.T, p.K, p.H);
+        p.x_last = input_beyond_l2(p.T, p.K, p.H, p.use_fp8);
         const int ntiles = (p.H + kTileChannels - 1) / kTileChannels;
         void (*k)(DirectDispatchParams) = ep_dispatch_rows_kernel<true, 1, 7, 6>;
         int tiles = 1, most = 7;
@@ -2539,7 +2542,7 @@ cudaError_t launch_group_dispatch_send(GroupDispatchParams p, const LaunchCtx& c
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, true);
     p.C = s.tokens;
     const size_t smem = dispatch_smem(p);
-    p.x_last = layer_beyond_l2(p.T, p.K, p.H);
+    p.x_last = input_beyond_l2(p.T, p.K, p.H, p.use_fp8);
     auto k = pick_dispatch<1>(p.use_fp8 != 0, p.counting());
     // the control block, then one block per token (small batches) or a resident wave
     // (a wave, not a block per batch: a block that stored rows in a peer's memory, nearly

@@ -89,7 +89,7 @@ struct DirectDispatchParams {
     // are counted in the send kernel. (Last, so that what a counting kernel reads lies together.)
     RouteBits bits;
     const int32_t* slot;        // [T*K]
-    bool x_last;                // see layer_beyond_l2 (set by the launcher)
+    bool x_last;                // see input_beyond_l2 (set by the launcher)
     int warps_per_row, tokens_per_block, parts;  // with positions: how a block's warps are dealt out, blocks that
                                                  // share a row (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
@@ -98,11 +98,19 @@ static_assert(cheap_to_launch<DirectDispatchParams>);
 // whether the send kernels count the slots themselves for this many tokens
 bool counts_in_send_kernel(int T, int K, int H, int num_sms, bool group);
 // Whether the input of a layer, `copies` rows of each token and the result are so many bytes that the
-// last use of what is used up is worth telling L2 (ld32_readonly with `last`). Of less, all of it stays there anyway, and
-// what a caller uses again is not to be the first that goes (us per layer on three sets of inputs in turn, no
-// mark | all marked: to 1, 1500 rows of 8 KB, 37 MB, 11.3 | 11.7, 2000, 49 MB, 12.7 | 12.2; to 2, 1200, 39 MB, 11.9 | 12.1,
-// 1600, 52 MB, 14.6 | 14.2; flat elastic rows of 4 KB, 2500, 31 MB, 9.7 | 9.9, 4000, 49 MB, 14.5 | 13.5).
+// last use of the experts' outputs is worth telling L2 (ld32_readonly with `last`). Of less, all of it
+// stays there anyway, and what a caller uses again is not to be the first that goes (us per layer on
+// three sets of inputs in turn, no mark | marked: to 1, 1500 rows of 8 KB, 37 MB, 11.3 | 11.7, 2000, 49 MB,
+// 12.7 | 12.2; to 2, 1200, 39 MB, 11.9 | 12.1, 1600, 52 MB, 14.6 | 14.2).
 bool layer_beyond_l2(long long T, int copies, int H);
+// The same for the input. A shared expert reads it again behind dispatch: in bf16 it is marked only where
+// input and rows are more than L2's 120 MiB, and it would not be found there anyway. us of a program with
+// such a reader, only the outputs marked | the input too: 2096 rows of 10 KB to 2 74.1 | 75.5, 6368 of 2 KB
+// to 4 67.6 | 69.1, flat elastic 3496 of 12 KB 95.8 | 97.6; beyond the line 3488 of 14 KB to 3 144.0 | 144.1,
+// 4592 of 8 KB to 4 122.8 | 122.2 (without the reader 101.2 | 100.5 and 89.7 | 88.4). FP8 rows are half as
+// long and the reader loses next to nothing: 2684 of 12 KB to 1 125.9 | 125.4, 1032 of 14 KB to 3 110.8 |
+// 109.5, 2320 to 2 177.8 | 178.0 (with outputs made long before 2096 of 10 KB to 8 91.7 | 93.0, no mark 95.4).
+bool input_beyond_l2(long long T, int copies, int H, bool fp8);
 cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx);
 
 struct SendShape {
@@ -196,7 +204,7 @@ struct GroupDispatchParams {
     int64_t* layout_range;      // [L][R]
     int copy_rows;              // recv_x is a tensor of the caller's: copy the rows out
     RouteBits bits;             // from the layout kernel (words null: none)
-    bool x_last;                // see layer_beyond_l2 (set by the launcher)
+    bool x_last;                // see input_beyond_l2 (set by the launcher)
     bool counting() const { return slot == nullptr && bits.words == nullptr; }
     char fill[40];
 };

@@ -21,6 +21,7 @@ SIZES = [  # T, H, E, K, fp8
     (8192, 128, 256, 8, True), (8193, 128, 256, 8, True), (9001, 256, 16, 1, False),
     (400, 12416, 8, 8, False), (4800, 4096, 8, 8, False),
     (512, 4096, 8, 8, False), (513, 4096, 8, 8, True), (853, 8192, 4, 1, False), (854, 8192, 4, 1, False),  # marks for L2
+    (1706, 4096, 8, 8, False), (1707, 4096, 8, 8, False),
     (199, 4096, 16, 8, True), (200, 4096, 16, 8, False), (292, 2816, 16, 8, True), (185, 4096, 16, 9, False),  # a group's counting
     (1036, 3584, 8, 2, False), (1037, 3584, 8, 2, False), (1481, 2688, 8, 8, False), (445, 4224, 8, 4, False),  # the two reduce kernels of a group
 ]

@@ -23,6 +23,7 @@ SIZES = [  # T, H, E, K, expand, alignment
     (1024, 1152, 24, 6, False, 1), (2049, 128, 64, 8, True, 16), (2500, 256, 4096, 1, False, 1),
     (512, 4096, 16, 8, False, 1), (513, 1152, 16, 8, False, 1), (256, 7168, 24, 16, False, 1), (1036, 640, 8, 3, False, 4), (1037, 640, 8, 1, False, 1),
     (1706, 4096, 8, 2, False, 1), (1707, 4096, 8, 2, False, 1), (1280, 4096, 8, 2, True, 1), (1281, 4096, 8, 2, True, 1),
+    (4388, 7168, 8, 1, False, 1), (4389, 7168, 8, 1, False, 1), (2925, 7168, 8, 2, True, 1), (2926, 7168, 8, 2, True, 1),  # its input too
     (4097, 128, 8, 5, False, 1), (16385, 128, 4, 1, False, 1), (600, 128, 5000, 2, False, 1),
 ]
 
