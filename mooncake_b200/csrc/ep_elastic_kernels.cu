@@ -473,10 +473,9 @@ __device__ __forceinline__ void take_totals(const ElasticSingleParams& p, Use us
 // expert and chunk, and every block of the copy kernel sums up those of all experts. What the block
 // that finishes last does else - a fence, the ticket, the totals, the sums and the segments, five
 // round trips to L2 one after the other - stands ahead of every row; here one load and a scan do, with
-// 4 KB more for a block to read, which on larger tables costs what it saves. Device time
-// per layer, that block's segments | their own: 1024 rows of 8 KB to 8 of 128 27.0 us | 25.0, to 2 of 64 14.7 | 12.6,
-// of 4 KB to 8 of 256 20.2 | 17.3, of 14 KB to 8 of 8 43.6 | 40.4, to 4 of 128 26.3 | 23.9; 2048 of 14 KB to 8 of 256 83.8 |
-// 82.1, to 2 of 64 30.7 | 28.8, to 1 of 8 24.2 | 22.6.
+// 4 KB more for a block to read, which on larger tables costs what it saves. Device us per layer, that
+// block's segments | their own: 1024 rows of 8 KB to 8 of 128 27.0 | 25.0, to 2 of 64 14.7 | 12.6; 2048 of 14 KB to 8
+// of 256 83.8 | 82.1, to 1 of 8 24.2 | 22.6.
 // It must not spill: with the first listings asked for ahead of the bits in registers, 50 bytes
 // a thread, 1024 of 8 KB to 8 25.7, 2048 of 14 KB 84.3; by cp.async 25.1 and 91.0.
 constexpr int kOwnChunks = 16, kOwnExperts = 256;
@@ -964,7 +963,7 @@ bool counts_in_copy_kernel(int T, int K, int H, int num_sms, bool expand, HostIs
 
 // Expanded rows whose segments every block of the copy kernel makes (the figures: OwnSegments). With
 // 256 experts and two loads for each, long rows, whose blocks move least for what they read, lose
-// (1100 tokens of 14 KB to 2 20.8 | 21.2, 2048 to 1 25.2 | 25.7; of 5 KB 13.4 | 12.8 and 14.9 | 14.4; to 2 of 160 20.2 | 20.0).
+// (1100 tokens of 14 KB to 2 20.8 | 21.2, of 5 KB 13.4 | 12.8; of 14 KB to 2 of 160 20.2 | 20.0).
 bool makes_own_segments(int T, int E, int H) {
     if (T > kOwnChunks * kChunkTokens || E > kOwnExperts) return false;
     return E * listings_stride_of((T + kChunkTokens - 1) / kChunkTokens) <= 160 * kOwnChunks || H <= 8 * kTileChannels;
@@ -977,7 +976,8 @@ bool elastic_single_tables(int T, int K, int E, int H, bool expand, HostIs host,
     if (K > kMaxTopk || E > kMaxExperts) return false;
     if (counts_in_copy_kernel(T, K, H, num_sms, expand, host)) return true;
     const bool own = expand && makes_own_segments(T, E, H);
-    const size_t starts = own ? (size_t)E * kOwnChunks * sizeof(uint16_t) : ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
+    const size_t starts =
+        own ? (size_t)E * kOwnChunks * sizeof(uint16_t) : ((size_t)(E + 1) * sizeof(int32_t) + 15) / 16 * 16;
     if (starts > bytes) return false;
     if (own)
         tables->listings = static_cast<uint16_t*>(scratch);

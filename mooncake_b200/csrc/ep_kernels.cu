@@ -1394,8 +1394,8 @@ __global__ void __launch_bounds__(512, 2) ep_combine_one_row_kernel(DirectCombin
         for (int u = 0; u < kAhead; ++u) {
             const int item = i0 + u * nwarps, tok = item / ntiles, c = (item - tok * ntiles) * 32 + lane;
             const int r = item < items && c < nchunks ? s_row[tok] : -1;
-            if (r >= 0)
-                v[u] = ld32_readonly(reinterpret_cast<const char*>(p.x) + (size_t)r * row_bytes + (size_t)c * 32, kLast);
+            const char* x = reinterpret_cast<const char*>(p.x) + (size_t)c * 32;
+            if (r >= 0) v[u] = ld32_readonly(x + (size_t)r * row_bytes, kLast);
         }
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
@@ -1841,8 +1841,9 @@ __global__ void __launch_bounds__(512)
 // the peers' payload words), so it starts beside the send kernel and only ends behind it: what the
 // stream sees as done is done. One rank on this path, us per layer with this, the reduce phase's like
 // (ep_combine_kernel), the own counts taken directly and the first tiles ahead of the layout's end:
-// 400 tokens of 14 KB to 8 29.3 -> 26.5, 1024 of 4 KB 24.7 -> 22.1, 2048 of 14 KB 95.3 -> 92.1; in hook mode
-// with the wait where the result is stored 26.5, 22.1 and 92.1, 1024 of 8 KB 36.9 -> 33.4.
+// 400 tokens of 14 KB to 8 29.3 -> 26.5, 1024 of 4 KB 24.7 -> 22.1, 2048 of 14 KB 95.3 -> 92.1; in hook mode 1024
+// of 8 KB 36.9 -> 33.4, where the host has queued the phases ahead. Rows of peers have not been moved by it
+// beside a send kernel: that takes several GPUs.
 template <bool kFP8>
 __global__ void __launch_bounds__(kRowWarps * 32, 4) ep_dispatch_recv_kernel(GroupDispatchParams p) {
     extern __shared__ int smem_i32[];
@@ -2349,11 +2350,10 @@ static SendShape send_shape(int T, int K, int H, int num_sms, bool group) {
     return s;
 }
 
-// Batches that count for themselves, a token per block instead of several (device time per layer,
-// several | one: 300 tokens of 1 KB in FP8 to 8 8.5 us | 7.6, of 8 KB to 2 7.6 | 6.3, to 1 6.7 | 6.0; 400 9.3 | 8.9, 7.8 | 7.4
-// and 6.8 | 6.6, of 4 KB to 8 10.3 | 10.0; 500 10.0 | 9.8, 8.1 | 7.5, but 7.0 | 7.1 and 10.8 | 11.1; 1100 of 4 KB to 1 8.1 | 11.5):
-// as many as are resident at a time, at two blocks of 16 warps, and three per SM, as each compares
-// itself with all earlier ones.
+// Batches that count for themselves, a token per block instead of several: as many as are resident at
+// a time, at two blocks of 16 warps, and three per SM, as each compares itself with all earlier ones.
+// Device us per layer, several | one: 300 tokens of 1 KB in FP8 to 8 8.5 | 7.6, of 8 KB to 2 7.6 | 6.3; 400 9.3 | 8.9
+// and 7.8 | 7.4; 500 of 8 KB to 1 7.0 | 7.1, of 4 KB to 8 10.8 | 11.1; 1100 of 4 KB to 1 8.1 | 11.5.
 static bool one_token_per_block(int T, int warps, int num_sms) {
     return T > 0 && T <= 3 * num_sms && T < 2 * num_sms * (16 / warps);
 }
@@ -2406,7 +2406,8 @@ cudaError_t launch_direct_dispatch(DirectDispatchParams p, const LaunchCtx& ctx)
             one = p.use_fp8 ? ep_dispatch_one_token_kernel<true, 8> : ep_dispatch_one_token_kernel<false, 8>;
         else
             one = p.use_fp8 ? ep_dispatch_one_token_kernel<true, 16> : ep_dispatch_one_token_kernel<false, 16>;
-        return launch("ep_dispatch_send_direct", one, dim3(p.T + 1), dim3(32 * warps), (size_t)p.E * sizeof(int), ctx, p);
+        return launch("ep_dispatch_send_direct", one, dim3(p.T + 1), dim3(32 * warps), (size_t)p.E * sizeof(int), ctx,
+                      p);
     }
     const SendShape s = send_shape(p.T, p.K, p.H, ctx.num_sms, false);
     p.C = s.tokens;
@@ -2609,8 +2610,8 @@ cudaError_t launch_group_combine_reduce(GroupCombineParams p, const LaunchCtx& c
     if (tiles >= 6 && 2 * p.T > (tiles > 8 ? 6 : 12 + p.K) * ctx.num_sms) {
         const ReduceShape shape = reduce_shape(p.T, p.K, p.H, ctx.num_sms);
         p.tiles_per_block = shape.tiles_per_block, p.tokens_per_block = shape.tokens_per_block, p.span = shape.span;
-        return launch("ep_combine_reduce", last ? ep_combine_gather_kernel<4, true> : ep_combine_gather_kernel<4, false>,
-                      shape.grid, dim3(shape.threads), 0, ctx, p);
+        auto k = last ? ep_combine_gather_kernel<4, true> : ep_combine_gather_kernel<4, false>;
+        return launch("ep_combine_reduce", k, shape.grid, dim3(shape.threads), 0, ctx, p);
     }
     const int threads = block_threads(p.H);
     auto k = last ? ep_combine_kernel<2, true> : ep_combine_kernel<2>;

@@ -26,9 +26,10 @@ constexpr int kStatusNoPeer = 8;  // a rank marked active has no mapped buffer
 // 32 bytes beyond a multiple of 64 (32, 96, 160, 224, 288, 352), 2.0 - 2.1 for any other from 16 to
 // 1024 (with programmatic serialisation; without 2.0 and 2.5). So parameter blocks are filled up to
 // such a size (us per layer: one token in FP8 10.1 -> 9.8, 128 of 4 KB in bf16 9.9 -> 9.6, elastic decode
-// call of 128 14.2 -> 13.8, expanded, waiting, 1024 30.1 -> 29.4). Not the layout kernel's: calls that have one
-// are the device's, and asynchronous ones lose by a host that is further ahead, as every event between
-// the streams is then waited for (1000 rows of 8 KB to 2 15.7 -> 18.6).
+// call of 128 14.2 -> 13.8, expanded, waiting, 1024 30.1 -> 29.4). The layout kernel's are not (128 bytes): a
+// synchronous layer with that kernel would have 0.4 us less of the host, but an asynchronous one whose
+// host is just behind the device gets ahead of it, and waits for every event between the streams, as any
+// program does whose host is ahead (1000 rows of 8 KB to 2 15.7 -> 18.6).
 template <typename P>
 constexpr bool cheap_to_launch = sizeof(P) % 64 == 32;
 

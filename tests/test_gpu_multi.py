@@ -41,6 +41,14 @@ def _cases(R):
         "mixtral_t4096": dict(T=4096, M=4096, H=4096, E=8, K=2, fp8=False, check="properties"),
         "prefill_t4096": dict(T=4096, M=4096, H=7168, E=256, K=8, fp8=False, check="properties"),
     }
+    # behind a layout kernel: receive and reduce phases that start beside the phase ahead of them, with
+    # rows of peers to move; and ranks of one launch that differ in bytes
+    c["layout_fp8"] = dict(T=400, M=400, H=4096, E=8 * R, K=8, fp8=True, seed=13)
+    c["layout_bf16_hook"] = dict(T=400, M=400, H=4096, E=8 * R, K=8, fp8=False, seed=14, mode="hook")
+    c["layout_fp8_caller_recv_x"] = dict(T=400, M=400, H=4096, E=8 * R, K=8, fp8=True, seed=15, mode="hook",
+                                         recv_in_place=False)
+    c["uneven_one_launch"] = dict(tokens=[150 + 100 * (r % 2) for r in range(R)], M=256, H=4096, E=8 * R, K=8,
+                                  fp8=False, seed=16)
     # the elastic-style interface (ElasticBuffer): the route plan of the reference's own test, and
     # random routing with masked entries and an expert alignment
     c["elastic_alltoall_plan"] = dict(elastic=True, plan="alltoall", T=32, M=128, H=4096, E=256, K=8)
