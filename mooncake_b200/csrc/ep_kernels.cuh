@@ -27,9 +27,10 @@ constexpr int kStatusNoPeer = 8;  // a rank marked active has no mapped buffer
 // 1024 (with programmatic serialisation; without 2.0 and 2.5). So parameter blocks are filled up to
 // such a size (us per layer: one token in FP8 10.1 -> 9.8, 128 of 4 KB in bf16 9.9 -> 9.6, elastic decode
 // call of 128 14.2 -> 13.8, expanded, waiting, 1024 30.1 -> 29.4). The layout kernel's are not (128 bytes): a
-// synchronous layer with that kernel would have 0.4 us less of the host, but an asynchronous one whose
-// host is just behind the device gets ahead of it, and waits for every event between the streams, as any
-// program does whose host is ahead (1000 rows of 8 KB to 2 15.7 -> 18.6).
+// synchronous layer that the host bounds would gain 0.3 us (not filled | filled: 300 tokens of 8 KB in FP8
+// to 8 11.7 | 11.3, 1000 in bf16 to 2 11.5 | 11.1, from 400 to 8 on none), but the host of an asynchronous one gets
+// ahead of the device and then waits for every event between the streams (300 14.9 | 18.2, 900 to 2 15.7 |
+// 18.3; whoever is ahead anyway has 18.2 and 18.3 with either).
 template <typename P>
 constexpr bool cheap_to_launch = sizeof(P) % 64 == 32;
 
